@@ -42,7 +42,7 @@ struct Plan {
 
 // Cheapest kernel for this shape and number of K ranges according to the cost models (gemm_units.cuh), never below the
 // time HBM needs for the weight.
-Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
+Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   const int sms = 148;
   const int kb_total = static_cast<int>(ceil_div(K, 64));
   Plan best{3, 1e30};
@@ -68,6 +68,12 @@ Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz
   if (best.clocks < hbm) best.clocks = hbm;
   return best;
+}
+
+Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
+  static ModelCache<5, Plan> cache;
+  const int64_t key[5] = {epi, M, N, K, splits};
+  return cache.get(key, [&] { return model_kernel(epi, M, N, K, splits); });
 }
 
 int dispatch(int epi, int variant, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
@@ -145,20 +151,29 @@ extern "C" int ojb_gemm_set_probe(int32_t mma_repeat, int32_t knob) {
 extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_splits, int32_t* variant, int32_t* splits,
                              float* microseconds) {
   OJB_REQUIRE(M > 0 && N > 0 && K > 0 && kind >= 0 && kind <= 2 && max_splits >= 1 && max_splits <= 16 && variant && splits);
-  const int kb_total = static_cast<int>(ceil_div(K, 64));
-  Plan best{0, 1e30};
-  int best_s = 1;
-  for (int s = 1; s <= (kind == kEpiPartialF32 ? max_splits : 1); ++s) {
-    const int per = static_cast<int>(ceil_div(kb_total, s));
-    if (static_cast<int64_t>(s - 1) * per >= kb_total) continue;
-    Plan p = plan_kernel(kind, M, N, K, s);
-    // the kernel that sums the partial planes reads S * M * N floats (mostly from L2)
-    if (kind == kEpiPartialF32) p.clocks += (s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
-    if (p.clocks < best.clocks * 0.97) { best = p; best_s = s; }
-  }
-  *variant = best.variant;
-  *splits = best_s;
-  if (microseconds) *microseconds = static_cast<float>(best.clocks / 1800.0);
+  struct Ranges {
+    Plan plan;
+    int splits;
+  };
+  static ModelCache<5, Ranges> cache;
+  const int64_t key[5] = {M, N, K, kind, max_splits};
+  const Ranges r = cache.get(key, [&] {
+    const int kb_total = static_cast<int>(ceil_div(K, 64));
+    Plan best{0, 1e30};
+    int best_s = 1;
+    for (int s = 1; s <= (kind == kEpiPartialF32 ? max_splits : 1); ++s) {
+      const int per = static_cast<int>(ceil_div(kb_total, s));
+      if (static_cast<int64_t>(s - 1) * per >= kb_total) continue;
+      Plan p = model_kernel(kind, M, N, K, s);
+      // the kernel that sums the partial planes reads S * M * N floats (mostly from L2)
+      if (kind == kEpiPartialF32) p.clocks += (s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
+      if (p.clocks < best.clocks * 0.97) { best = p; best_s = s; }
+    }
+    return Ranges{best, best_s};
+  });
+  *variant = r.plan.variant;
+  *splits = r.splits;
+  if (microseconds) *microseconds = static_cast<float>(r.plan.clocks / 1800.0);
   return OJB_OK;
 }
 

@@ -13,6 +13,8 @@
 #define OJB_PROBE_DBG(g) 0
 #endif
 #include "gemm_common.cuh"
+#include <cstring>
+#include <mutex>
 
 namespace ojb {
 namespace {
@@ -152,39 +154,99 @@ inline double block_kernel_clocks(int64_t N, int bn, int n_xblk, int tail_box, i
   }
   if (grid_out) *grid_out = grid;
   if (grid <= 0) return 0.0;
-  double load[160] = {0.0};
   if (grid > 160) return 1e30;
-  int64_t i = 0;
+  // Runs of equal units: units_run[w] holds the difference array of what starts at worker w, `all` what every worker gets. All
+  // costs are whole numbers of clocks, so the sums are exact in any order.
+  double step[161] = {0.0}, all = 0.0;
+  int at = 0;                        // worker of the next unit
+  auto run = [&](int64_t n, double cost) {
+    all += static_cast<double>(n / grid) * cost;
+    const int r = static_cast<int>(n % grid), end = at + r;
+    step[at] += cost;
+    if (end <= grid) {
+      step[end] -= cost;
+    } else {
+      step[grid] -= cost;
+      step[0] += cost;
+      step[end - grid] -= cost;
+    }
+    at = end < grid ? end : end - grid;
+  };
   auto kbs = [&](int s) { const int k1 = (s + 1) * per < kb_total ? (s + 1) * per : kb_total; return k1 - s * per; };
   auto tails_before = [&](int j) {
     if (!has_tail) return 0;
     const int t = n_xblk > 0 ? (j * bn + 255) / 256 : j;
     return t < n_wtile256 ? t : n_wtile256;
   };
+  const int s_full = kb_total / per < splits ? kb_total / per : splits;      // K ranges of full length; one shorter may follow
+  const double block_full = per * c.block_kb + c.block_epi, tail_full = per * c.tail_kb + c.tail_epi;
   for (int j = 0; j < n_wtile; ++j) {
-    for (int s = 0; s < splits; ++s)
-      for (int xb = 0; xb < n_xblk; ++xb) load[i++ % grid] += kbs(s) * c.block_kb + c.block_epi;
+    run(static_cast<int64_t>(s_full) * n_xblk, block_full);
+    for (int s = s_full; s < splits; ++s) run(n_xblk, kbs(s) * c.block_kb + c.block_epi);
     const int nt = (j + 1 < n_wtile ? tails_before(j + 1) : (has_tail ? n_wtile256 : 0)) - tails_before(j);
-    for (int t = 0; t < nt; ++t)
-      for (int s = 0; s < splits; ++s)
-        for (int xc = 0; xc < n_xchunk; ++xc) load[i++ % grid] += kbs(s) * c.tail_kb + c.tail_epi;
+    for (int t = 0; t < nt; ++t) {
+      run(static_cast<int64_t>(s_full) * n_xchunk, tail_full);
+      for (int s = s_full; s < splits; ++s) run(n_xchunk, kbs(s) * c.tail_kb + c.tail_epi);
+    }
   }
-  double worst = 0.0;
-  for (int k = 0; k < grid; ++k) worst = load[k] > worst ? load[k] : worst;
+  double worst = 0.0, sum = 0.0;
+  for (int k = 0; k < grid; ++k) {
+    sum += step[k];
+    worst = all + sum > worst ? all + sum : worst;
+  }
   return worst + 5000.0;      // launch, TMEM allocation, first stages
 }
+
+// Answers of the cost model, which depend on nothing but their whole-number arguments: a forward asks for the same handful of
+// shapes in every layer. Direct-mapped and of fixed size, shared by all threads under a lock. Measured on the host before /
+// after (with the runs above): the K ranges of a [5120, 17408] projection at 400 rows 572 / 0.2 us (0.12 ms when first
+// asked), at 16 672 rows 16.7 ms / 0.2 us (0.20 ms).
+template <int KEYS, typename Value>
+class ModelCache {
+ public:
+  template <typename Make>
+  Value get(const int64_t (&key)[KEYS], Make make) {
+    uint64_t hash = 1469598103934665603ull;
+    for (int i = 0; i < KEYS; ++i) hash = (hash ^ static_cast<uint64_t>(key[i])) * 1099511628211ull;
+    Slot& slot = slots_[(hash ^ (hash >> 32)) % kSlots];
+    {
+      std::lock_guard<std::mutex> hold(lock_);
+      if (slot.used && memcmp(slot.key, key, sizeof(key)) == 0) return slot.value;
+    }
+    const Value v = make();
+    std::lock_guard<std::mutex> hold(lock_);
+    memcpy(slot.key, key, sizeof(key));
+    slot.value = v;
+    slot.used = true;
+    return v;
+  }
+
+ private:
+  static constexpr int kSlots = 1024;
+  struct Slot {
+    int64_t key[KEYS];
+    Value value;
+    bool used;
+  };
+  std::mutex lock_;
+  Slot slots_[kSlots] = {};
+};
 
 // Width of the w tile of the block units: the multiple of 16 with the smallest modelled time, wider tiles preferred.
 inline int choose_bn(int64_t N, int n_xblk, int tail_box, int n_xchunk, bool has_tail, int splits, int kb_total, int workers,
                      int epi) {
   if (n_xblk == 0) return 256;
-  int best = 256;
-  double best_cost = 1e30;
-  for (int bn = 256; bn >= 64; bn -= 16) {
-    const double cost = block_kernel_clocks(N, bn, n_xblk, tail_box, n_xchunk, has_tail, splits, kb_total, workers, epi);
-    if (cost < best_cost * 0.98) { best_cost = cost; best = bn; }
-  }
-  return best;
+  static ModelCache<9, int> cache;
+  const int64_t key[9] = {N, n_xblk, tail_box, n_xchunk, has_tail, splits, kb_total, workers, epi};
+  return cache.get(key, [&] {
+    int best = 256;
+    double best_cost = 1e30;
+    for (int bn = 256; bn >= 64; bn -= 16) {
+      const double cost = block_kernel_clocks(N, bn, n_xblk, tail_box, n_xchunk, has_tail, splits, kb_total, workers, epi);
+      if (cost < best_cost * 0.98) { best_cost = cost; best = bn; }
+    }
+    return best;
+  });
 }
 
 }  // namespace

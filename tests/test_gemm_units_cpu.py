@@ -76,3 +76,23 @@ def test_rejects_bad_geometry():
               ctypes.c_int32(8), ctypes.c_int32(0), p, ctypes.c_int64(4)) == -1                 # BN not a multiple of 16
     assert fn(ctypes.c_int32(2), ctypes.c_int32(0), ctypes.c_int32(1), ctypes.c_int32(256), ctypes.c_int64(1024), ctypes.c_int32(1),
               ctypes.c_int32(8), ctypes.c_int32(0), p, ctypes.c_int64(4)) == -4                 # more units than the buffer holds
+
+
+def test_plan_is_the_same_from_every_thread():
+    """The cost model's answers are kept in a table shared by all threads: more shapes than it has slots, asked for by several
+    threads in different orders, get the answer they get alone."""
+    import random
+    from concurrent.futures import ThreadPoolExecutor
+
+    from ojb200 import lt_ext
+
+    shapes = [(M, N, K, kind) for M in range(16, 2400, 48) for N, K, kind in ((12352, 5120, 0), (1024, 512, 1), (5120, 4096, 2),
+                                                                             (136, 200, 0), (5120, 17408, 2), (264, 72, 2), (512, 640, 1))]
+    alone = {s: lt_ext.gemm_plan(*s, max_splits=4) for s in shapes}
+
+    def ask(seed):
+        order = random.Random(seed).sample(shapes * 4, len(shapes) * 4)
+        return all(lt_ext.gemm_plan(*s, max_splits=4) == alone[s] for s in order)
+
+    with ThreadPoolExecutor(8) as pool:
+        assert all(pool.map(ask, range(8)))
