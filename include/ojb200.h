@@ -314,6 +314,24 @@ int ojb_tree_attn(const void* qt, const void* kt, const void* vt, const void* ga
 int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const void* gate, const int32_t* krange, void* y,
                      int64_t N, int64_t HQ, int64_t HKV, int64_t D, float scale, int32_t* status, ojb_stream_t stream);
 
+/* The same for any rows of the tree as queries: query row n (of NQ) goes by row q_rows[n] of krange (q_rows null: by row n), and
+ * its gate is read at gate + n * gate_ld + head * gate_hs (elements, multiples of 8), e.g. inside the in-projection output.
+ * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0, any NQ. */
+int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
+                       const void* gate, int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ,
+                       int64_t HKV, float scale, int32_t* status, ojb_stream_t stream);
+
+/* Its operands (ojb_fullattn_prep without the copies of the gate and of V in row order): q_src = NQ rows, q_ld elements apart,
+ * of [q(256) | gate(256)] per query head; kv_src = N rows, kv_ld apart, of HKV k heads then HKV v heads. Query row n takes its
+ * rotary angles from row q_rows[n] of cosb / sinb (null: row n). RD a power of two in [16, 256]; N % 8 == 0. */
+int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t* q_rows, int64_t NQ, const void* kv_src, int64_t kv_ld,
+                      const float* qw1, const float* kw1, const void* cosb, const void* sinb, void* qt, void* kt, void* vt_t,
+                      int64_t N, int64_t HQ, int64_t HKV, int64_t RD, float eps, ojb_stream_t stream);
+
+/* out[i, :] = in[rows[i], :] for one or two matrices (b may be null) of a_bytes / b_bytes per row (multiples of 16). */
+int ojb_gather_rows(const int64_t* rows, int64_t n_rows, const void* a, void* a_out, int64_t a_bytes, const void* b, void* b_out,
+                    int64_t b_bytes, ojb_stream_t stream);
+
 /* Measurement hook of ojb_tree_attn_tc (no counterpart in the reference): `records` = null switches it off; otherwise a device
  * buffer of 16 uint64 words. The CTA of kv head 0 and the last-but-one block of 16 query rows stores %globaltimer at kernel
  * entry [0], after its set-up [1], at the first scores of pass 1 [2] and of pass 2 [3], when the last P tile is handed over
@@ -323,7 +341,7 @@ int ojb_tree_attn_set_trace(uint64_t* records);
 
 /* Scoring head — replaces src/server.py:37 `mdl.head(forward_gtree(...).float())` together with the gather
  * src/fastmodel.py:482 `hn[lay.lastidx]`: out[s, a] = bias[a] + sum_h float(hn[rows[s], h]) * W[a, h], all fp32.
- * hn bf16 [N, H] (final-norm output), rows int64 [S] (last row of each candidate), W fp32 [A, H], bias fp32 [A] or null. */
+ * hn bf16 [N, H] (final-norm output), rows int64 [S] (last row of each candidate; null: row s), W fp32 [A, H], bias fp32 [A] or null. */
 int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S, int64_t A,
                    int64_t H, ojb_stream_t stream);
 

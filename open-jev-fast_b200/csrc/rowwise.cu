@@ -3,6 +3,7 @@
 // All of them are HBM-bound streaming kernels: 16-byte accesses, one pass over the data, rows held in registers.
 #include "common.cuh"
 #include <cuda_fp8.h>
+#include <initializer_list>
 
 namespace ojb {
 namespace {
@@ -317,6 +318,108 @@ fullattn_prep_kernel(const bf16_t* __restrict__ proj, const float* __restrict__ 
   store(dst + (static_cast<int64_t>(hh) * N + n) * D + d0, ov);
 }
 
+// Operands of the tcgen05 tree attention (head dim 256) from the in-projection: q and k normalised and rotated, head-major; V with
+// keys contiguous. The first blocks (8 warps) do q and k: a warp takes kPrepRows rows of one head, so the norm weights are read
+// once and the rows' loads are in flight together. The other blocks transpose tiles of 64 keys x 64 dims of V through shared
+// memory, so that both sides move in 128-byte pieces.
+// Bound by memory: 2 x 2 bytes per q / k / v element, N * (HQ + 2 HKV) * 256 of them. fullattn_prep_kernel, which the attention
+// path used before, also copies the gate (the attention now reads it in place), writes V a second time in row order and stores
+// the transposed V element by element (2-byte stores N apart).
+constexpr int kPrepRows = 4;
+constexpr int kPrepTile = 64;
+
+__global__ void __launch_bounds__(256)
+attn_operands_kernel(const bf16_t* __restrict__ q_src, int64_t q_ld, const int64_t* __restrict__ q_rows, int NQ,
+                     const bf16_t* __restrict__ kv_src, int64_t kv_ld, const float* __restrict__ qw1, const float* __restrict__ kw1,
+                     const bf16_t* __restrict__ cosb, const bf16_t* __restrict__ sinb, bf16_t* __restrict__ qt,
+                     bf16_t* __restrict__ kt, bf16_t* __restrict__ vt_t, int N, int HQ, int HKV, int RD, float eps, int q_blocks,
+                     int k_blocks) {
+  pdl_begin();
+  constexpr int D = 256;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ bf16_t tile[kPrepTile][kPrepTile + 2];
+  const int blk = blockIdx.x;
+  if (blk < q_blocks + k_blocks) {
+    // block = 8 groups of kPrepRows rows of one head: consecutive blocks take consecutive heads of the same rows
+    const bool isq = blk < q_blocks;
+    const int heads = isq ? HQ : HKV, rows = isq ? NQ : N;
+    const int b = isq ? blk : blk - q_blocks;
+    const int hh = b % heads, n0 = (b / heads * 8 + warp) * kPrepRows;
+    const bf16_t* src = isq ? q_src + static_cast<int64_t>(hh) * 2 * D : kv_src + static_cast<int64_t>(hh) * D;
+    const int64_t ld = isq ? q_ld : kv_ld;
+    bf16_t* dst = (isq ? qt : kt) + static_cast<int64_t>(hh) * rows * D;
+    const float* w1 = isq ? qw1 : kw1;
+    const int d0 = lane * 8;
+    uint4 raw[kPrepRows];
+#pragma unroll
+    for (int r = 0; r < kPrepRows; ++r)
+      raw[r] = n0 + r < rows ? ldg_stream(src + (n0 + r) * ld + d0) : make_uint4(0u, 0u, 0u, 0u);
+    const float4 wa = __ldg(reinterpret_cast<const float4*>(w1 + d0)), wb = __ldg(reinterpret_cast<const float4*>(w1 + d0 + 4));
+    const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+    const bool rope = d0 < RD, first = d0 < RD / 2;
+    const int partner = RD / 16;      // lane distance of the rotate-half partner
+#pragma unroll
+    for (int r = 0; r < kPrepRows; ++r) {
+      const int n = n0 + r;
+      if (n >= rows) break;
+      float x[8], nv[8], pv[8];
+      unpack8(raw[r], x);
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ss += x[e] * x[e];
+      ss = warp_sum(ss);
+      const float rstd = rsqrtf(ss / static_cast<float>(D) + eps);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) nv[e] = round_bf((x[e] * rstd) * w[e]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) pv[e] = __shfl_xor_sync(0xffffffffu, nv[e], partner);
+      if (rope) {
+        const int64_t tn = (isq && q_rows != nullptr) ? q_rows[n] : n;
+        float c[8], s[8];
+        unpack8(*reinterpret_cast<const uint4*>(cosb + tn * RD + d0), c);
+        unpack8(*reinterpret_cast<const uint4*>(sinb + tn * RD + d0), s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) nv[e] = round_bf(nv[e] * c[e]) + round_bf((first ? -pv[e] : pv[e]) * s[e]);
+      }
+      *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(n) * D + d0) = pack8(nv);
+    }
+    return;
+  }
+  const int b = blk - q_blocks - k_blocks, cols = HKV * D / kPrepTile;
+  const int c0 = b % cols * kPrepTile, n0 = b / cols * kPrepTile;
+  const bf16_t* v = kv_src + static_cast<int64_t>(HKV) * D + c0;
+#pragma unroll
+  for (int u = 0; u < kPrepTile * kPrepTile / 8 / 256; ++u) {
+    const int i = threadIdx.x + u * 256, r = i >> 3, c = (i & 7) * 8;
+    if (n0 + r < N) {
+      const uint4 x = ldg_stream(v + (n0 + r) * kv_ld + c);
+      uint32_t* t = reinterpret_cast<uint32_t*>(&tile[r][c]);
+      t[0] = x.x; t[1] = x.y; t[2] = x.z; t[3] = x.w;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < kPrepTile * kPrepTile / 8 / 256; ++u) {
+    const int i = threadIdx.x + u * 256, c = i >> 3, r = (i & 7) * 8;
+    if (n0 + r < N) {      // N is a multiple of 8: all eight keys or none
+      alignas(16) bf16_t o[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[e] = tile[r + e][c];
+      *reinterpret_cast<uint4*>(vt_t + static_cast<int64_t>(c0 + c) * N + n0 + r) = *reinterpret_cast<const uint4*>(o);
+    }
+  }
+}
+
+// Rows rows[i] of one or two matrices, one block per output row.
+__global__ void __launch_bounds__(256)
+gather_rows_kernel(const int64_t* __restrict__ rows, const uint4* __restrict__ a, uint4* __restrict__ a_out, int a_vecs,
+                   const uint4* __restrict__ b, uint4* __restrict__ b_out, int b_vecs) {
+  pdl_begin();
+  const int64_t i = blockIdx.x, n = rows[i];
+  for (int c = threadIdx.x; c < a_vecs; c += blockDim.x) a_out[i * a_vecs + c] = a[n * a_vecs + c];
+  for (int c = threadIdx.x; c < b_vecs; c += blockDim.x) b_out[i * b_vecs + c] = b[n * b_vecs + c];
+}
+
 // Per-row e4m3 quantisation for the 8-bit GEMM: scale[m] = max|x[m,:]| / 448 (1 for an all-zero row), q = x / scale rounded
 // to e4m3 (saturating). One CTA per row, two passes over the row (the second one hits L1 / L2).
 __global__ void __launch_bounds__(kRowThreads)
@@ -385,7 +488,7 @@ extern "C" int ojb_l2_prefetch(const void* data, int64_t nbytes, int64_t chunk, 
   return launch_status(cudaGetLastError());
 }
 
-extern "C" int ojb_abi_version(void) { return 6; }
+extern "C" int ojb_abi_version(void) { return 7; }
 
 extern "C" int ojb_add_rmsnorm(const void* x, const void* delta, const float* w1, const int32_t* rowmask, void* h_out,
                                void* hn_out, int64_t rows, int64_t H, float eps, ojb_stream_t stream) {
@@ -538,6 +641,42 @@ extern "C" int ojb_fullattn_prep(const void* proj, const float* qw1, const float
   return launch_status(cudaGetLastError());
 }
 
+extern "C" int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t* q_rows, int64_t NQ, const void* kv_src, int64_t kv_ld,
+                                 const float* qw1, const float* kw1, const void* cosb, const void* sinb, void* qt, void* kt,
+                                 void* vt_t, int64_t N, int64_t HQ, int64_t HKV, int64_t RD, float eps, ojb_stream_t stream) {
+  constexpr int D = 256;
+  OJB_REQUIRE(q_src && kv_src && qw1 && kw1 && cosb && sinb && qt && kt && vt_t && N > 0 && NQ > 0 && HQ > 0 && HKV > 0);
+  OJB_REQUIRE(N % 8 == 0 && N < (1 << 24) && NQ < (1 << 24) && HQ <= 1024 && HKV <= 1024);
+  OJB_REQUIRE(RD > 0 && RD <= D && RD % 16 == 0 && (RD & (RD - 1)) == 0);
+  OJB_REQUIRE(q_ld >= HQ * 2 * D && q_ld % 8 == 0 && kv_ld >= HKV * 2 * D && kv_ld % 8 == 0);
+  for (const void* p : {q_src, kv_src, static_cast<const void*>(qw1), static_cast<const void*>(kw1), cosb, sinb,
+                        static_cast<const void*>(qt), static_cast<const void*>(kt), static_cast<const void*>(vt_t)})
+    OJB_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15u) == 0);
+  const int64_t q_blocks = ceil_div(NQ, 8 * kPrepRows) * HQ, k_blocks = ceil_div(N, 8 * kPrepRows) * HKV;
+  const int64_t v_blocks = ceil_div(N, kPrepTile) * (HKV * D / kPrepTile);
+  OJB_REQUIRE(q_blocks + k_blocks + v_blocks < (int64_t{1} << 31));
+  launch_kernel(attn_operands_kernel, dim3(static_cast<unsigned>(q_blocks + k_blocks + v_blocks)), dim3(256), 0,
+                static_cast<cudaStream_t>(stream), static_cast<const bf16_t*>(q_src), q_ld, q_rows, static_cast<int>(NQ),
+                static_cast<const bf16_t*>(kv_src), kv_ld, qw1, kw1, static_cast<const bf16_t*>(cosb),
+                static_cast<const bf16_t*>(sinb), static_cast<bf16_t*>(qt), static_cast<bf16_t*>(kt), static_cast<bf16_t*>(vt_t),
+                static_cast<int>(N), static_cast<int>(HQ), static_cast<int>(HKV), static_cast<int>(RD), eps,
+                static_cast<int>(q_blocks), static_cast<int>(k_blocks));
+  return launch_status(cudaGetLastError());
+}
+
+extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, const void* a, void* a_out, int64_t a_bytes, const void* b,
+                               void* b_out, int64_t b_bytes, ojb_stream_t stream) {
+  if (n_rows == 0) return OJB_OK;
+  OJB_REQUIRE(rows && n_rows > 0 && n_rows < (int64_t{1} << 31) && a && a_out && a_bytes > 0 && a_bytes % 16 == 0 && a_bytes < (1 << 30));
+  OJB_REQUIRE(b ? (b_out && b_bytes > 0 && b_bytes % 16 == 0 && b_bytes < (1 << 30)) : (b_bytes == 0));
+  for (const void* p : {a, static_cast<const void*>(a_out), b, static_cast<const void*>(b_out)})
+    OJB_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15u) == 0);
+  launch_kernel(gather_rows_kernel, dim3(static_cast<unsigned>(n_rows)), dim3(256), 0, static_cast<cudaStream_t>(stream), rows,
+                static_cast<const uint4*>(a), static_cast<uint4*>(a_out), static_cast<int>(a_bytes / 16),
+                static_cast<const uint4*>(b), static_cast<uint4*>(b_out), static_cast<int>(b_bytes / 16));
+  return launch_status(cudaGetLastError());
+}
+
 // ------------------------------------------------------------------------------------------------------- scoring head
 namespace ojb {
 namespace {
@@ -550,7 +689,7 @@ score_head_kernel(const bf16_t* __restrict__ hn, const int64_t* __restrict__ row
   if (wid >= S * A) return;
   const int lane = threadIdx.x & 31;
   const int s = wid / A, a = wid - s * A;
-  const bf16_t* x = hn + rows[s] * static_cast<int64_t>(H);
+  const bf16_t* x = hn + (rows ? rows[s] : s) * static_cast<int64_t>(H);
   const float* w = W + static_cast<int64_t>(a) * H;
   float acc = 0.f;
   for (int c = lane * 8; c < H; c += 256) {
@@ -568,7 +707,7 @@ score_head_kernel(const bf16_t* __restrict__ hn, const int64_t* __restrict__ row
 extern "C" int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
                               int64_t A, int64_t H, ojb_stream_t stream) {
   if (S == 0 || A == 0) return OJB_OK;
-  OJB_REQUIRE(hn && rows && W && out && S > 0 && A > 0 && H > 0 && H % 8 == 0);
+  OJB_REQUIRE(hn && W && out && S > 0 && A > 0 && H > 0 && H % 8 == 0);
   const int64_t warps = S * A;
   launch_kernel(ojb::score_head_kernel, dim3(static_cast<unsigned>(ojb::ceil_div(warps, 8))), dim3(256), 0, static_cast<cudaStream_t>(stream), 
       static_cast<const ojb::bf16_t*>(hn), rows, W, bias, out, static_cast<int>(S), static_cast<int>(A), static_cast<int>(H));

@@ -61,6 +61,10 @@ struct AttnArgs {
   int N, HQ, HKV, G;
   float scale_log2e;
   int wait_ms;
+  int NQ;                    // query rows
+  const int64_t* q_rows;     // null, or the row of krange that query row n goes by
+  int64_t gate_ld;           // gate: elements between rows, and between heads of a row
+  int gate_hs;
 };
 
 // bits of keys [32 * w, 32 * w + 32) that fall in [lo, hi)
@@ -118,7 +122,10 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
   pdl_wait();      // from here on the previous kernel of the stream has completed
   // key ranges of the 16 rows
-  if (tid < kQRows * 8) kr[tid] = g.krange[static_cast<int64_t>(r0) * 8 + tid];
+  if (tid < kQRows * 8) {      // rows past the last query row see nothing
+    const int r = r0 + (tid >> 3);
+    kr[tid] = r < g.NQ ? g.krange[(g.q_rows ? g.q_rows[r] : r) * 8 + (tid & 7)] : 0;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -127,7 +134,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     mbar_expect_tx(bar(kBarQ), static_cast<uint32_t>(G) * 4u * (kQRows * 128u));
     for (int w = 0; w < G; ++w)
       for (int kb4 = 0; kb4 < 4; ++kb4)
-        tma_load_2d(smem_u32(Qs) + kb4 * qstride + w * (kQRows * 128), &map_q, bar(kBarQ), kb4 * 64, (hq0 + w) * N + r0);
+        tma_load_2d(smem_u32(Qs) + kb4 * qstride + w * (kQRows * 128), &map_q, bar(kBarQ), kb4 * 64, (hq0 + w) * g.NQ + r0);
   }
   // ordered list of the key blocks that at least one of the 16 rows sees
   const int NB = (N + kSub - 1) / kSub;
@@ -168,10 +175,9 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (int u = 0; u < kBatch; ++u) {
       const int i = base + u * kTcThreads;
       gq[u] = make_uint4(0u, 0u, 0u, 0u);
-      if (i < pieces) {
-        const int row = i >> 5, piece = i & 31;             // tile row = 16 * head + query row
-        gq[u] = *reinterpret_cast<const uint4*>(g.gate + (static_cast<int64_t>(r0 + (row & 15)) * g.HQ + (hq0 + (row >> 4))) * kD + piece * 8);
-      }
+      const int row = i >> 5, piece = i & 31;               // tile row = 16 * head + query row
+      if (i < pieces && r0 + (row & 15) < g.NQ)
+        gq[u] = *reinterpret_cast<const uint4*>(g.gate + (r0 + (row & 15)) * g.gate_ld + (hq0 + (row >> 4)) * g.gate_hs + piece * 8);
     }
   };
   if (trace && tid == 0) { trace[0] = t_entry; trace[1] = global_timer_ns(); trace[15] = static_cast<unsigned long long>(nblk); }
@@ -401,8 +407,8 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
       for (int u = 0; u < kBatch; ++u) {
         const int i = base + u * kTcThreads;
-        if (i < pieces) {
-          const int row = i >> 5, piece = i & 31;
+        const int row = i >> 5, piece = i & 31;
+        if (i < pieces && r0 + (row & 15) < g.NQ) {
           float gv[8], a[8], out[8];
           unpack8(gq[u], gv);
           unpack8(*reinterpret_cast<const uint4*>(smem + row * kStagePitch + piece * 16), a);
@@ -442,24 +448,34 @@ extern "C" int ojb_tree_attn_set_trace(uint64_t* records) {
   return launch_status(cudaMemcpyToSymbol(ojb::g_attn_trace, &p, sizeof(p)));
 }
 
-extern "C" int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const void* gate, const int32_t* krange, void* y,
-                                int64_t N, int64_t HQ, int64_t HKV, int64_t D, float scale, int32_t* status,
-                                ojb_stream_t stream) {
-  if (N == 0) return OJB_OK;
-  OJB_REQUIRE(qt && kt && vt_t && gate && krange && y && N > 0 && N % 32 == 0 && D == kD);
+extern "C" int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
+                                  const void* gate, int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ,
+                                  int64_t HKV, float scale, int32_t* status, ojb_stream_t stream) {
+  if (N == 0 || NQ == 0) return OJB_OK;
+  OJB_REQUIRE(qt && kt && vt_t && gate && krange && y && N > 0 && N % 8 == 0 && NQ > 0);
   OJB_REQUIRE(HQ > 0 && HKV > 0 && HQ % HKV == 0 && HQ / HKV <= kMaxG);
+  OJB_REQUIRE(gate_ld >= 0 && gate_hs >= 0 && gate_ld % 8 == 0 && gate_hs % 8 == 0 && gate_hs < (1 << 30));
   OJB_REQUIRE(aligned16(qt) && aligned16(kt) && aligned16(vt_t) && aligned16(gate) && aligned16(y));
-  if ((N + kSub - 1) / kSub > kMaxBlocks) return OJB_ERR_LIMIT;
+  if ((N + kSub - 1) / kSub > kMaxBlocks || NQ > static_cast<int64_t>(kMaxBlocks) * kSub) return OJB_ERR_LIMIT;
   CUtensorMap map_q, map_k, map_vt;
-  int rc = make_map(&map_q, qt, HQ * N, kD, kQRows);
+  int rc = make_map(&map_q, qt, HQ * NQ, kD, kQRows);
   if (rc == OJB_OK) rc = make_map(&map_k, kt, HKV * N, kD, kSub);
   if (rc == OJB_OK) rc = make_map(&map_vt, vt_t, HKV * kD, N, kD);
   if (rc != OJB_OK) return rc;
   static int smem_set[kMaxDevices] = {};
   if (!raise_smem_limit(tree_attn_tc_kernel, static_cast<int>(kSmemBytes), smem_set)) return OJB_ERR_LAUNCH;
   AttnArgs a{static_cast<const bf16_t*>(gate), krange, static_cast<bf16_t*>(y), status, static_cast<int>(N), static_cast<int>(HQ),
-             static_cast<int>(HKV), static_cast<int>(HQ / HKV), scale * 1.4426950408889634f, gemm_wait_limit_ms()};
-  launch_kernel(tree_attn_tc_kernel, dim3(static_cast<unsigned>(HKV), static_cast<unsigned>(N / kQRows)), dim3(kTcThreads),
+             static_cast<int>(HKV), static_cast<int>(HQ / HKV), scale * 1.4426950408889634f, gemm_wait_limit_ms(),
+             static_cast<int>(NQ), q_rows, gate_ld, static_cast<int>(gate_hs)};
+  launch_kernel(tree_attn_tc_kernel, dim3(static_cast<unsigned>(HKV), static_cast<unsigned>(ceil_div(NQ, kQRows))), dim3(kTcThreads),
                 kSmemBytes, static_cast<cudaStream_t>(stream), map_q, map_k, map_vt, a);
   return launch_status(cudaGetLastError());
+}
+
+extern "C" int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const void* gate, const int32_t* krange, void* y,
+                                int64_t N, int64_t HQ, int64_t HKV, int64_t D, float scale, int32_t* status,
+                                ojb_stream_t stream) {
+  if (N == 0) return OJB_OK;
+  OJB_REQUIRE(N > 0 && N % 32 == 0 && D == kD);
+  return ojb_tree_attn_rows(qt, N, nullptr, kt, vt_t, N, gate, HQ * kD, kD, krange, y, HQ, HKV, scale, status, stream);
 }

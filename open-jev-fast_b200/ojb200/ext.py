@@ -168,6 +168,33 @@ def fullattn_prep2(proj, qw1, kw1, cosb, sinb, B, T, HQ, HKV, D, eps, with_vt_t=
 fullattn_prep = fullattn_prep2   # src/ext.py:10 — same contract
 
 
+def attn_operands_ok(HQ, HKV, D, RD, N):
+    """Whether attn_operands / tree_attn_rows serve these sizes; the operators above and fattn_tree* serve the rest."""
+    return D == 256 and HQ // HKV <= 6 and N % 8 == 0 and 16 <= RD <= D and RD & (RD - 1) == 0
+
+
+def attn_operands(q_src, kv_src, qw1, kw1, cosb, sinb, HQ, HKV, eps, q_rows=None):
+    """Operands of tree_attn_rows. q_src: rows of per-head [q(256) | gate(256)], kv_src [N, ...]: rows of k heads, then v heads;
+    both may be column slices of one in-projection output (rows apart by their stride). q_rows int64 or None: query row n is
+    row q_rows[n] of the packed rows (of the rotary tables). -> qt [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N]."""
+    _chk(qw1, kw1, cosb, sinb, q_rows)
+    D, RD = 256, cosb.shape[-1]
+    NQ, N = q_src.shape[0], kv_src.shape[0]
+    for t, cols in ((q_src, HQ * 2 * D), (kv_src, 2 * HKV * D)):
+        if not t.is_cuda or t.dtype != bf16 or t.dim() != 2 or t.shape[1] != cols or t.stride(1) != 1:
+            raise RuntimeError("attn_operands: CUDA bf16 rows of HQ * 512 and of HKV * 512 columns expected")
+    if cosb.shape != (N, RD) or sinb.shape != (N, RD) or (q_rows is None and NQ != N) or \
+            (q_rows is not None and (q_rows.dtype != torch.int64 or q_rows.numel() != NQ)):
+        raise RuntimeError("attn_operands: shapes do not match")
+    dev = q_src.device
+    qt = torch.empty(HQ, NQ, D, dtype=bf16, device=dev)
+    kt = torch.empty(HKV, N, D, dtype=bf16, device=dev)
+    vt_t = torch.empty(HKV, D, N, dtype=bf16, device=dev)
+    call("ojb_attn_operands", ptr(q_src), i64(q_src.stride(0)), ptr(q_rows), i64(NQ), ptr(kv_src), i64(kv_src.stride(0)), ptr(qw1),
+         ptr(kw1), ptr(cosb), ptr(sinb), ptr(qt), ptr(kt), ptr(vt_t), i64(N), i64(HQ), i64(HKV), i64(RD), f32(eps), stream_ptr())
+    return qt, kt, vt_t
+
+
 # ------------------------------------------------------------------------------------------------ Gated DeltaNet
 def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV, HK, HD, l2norm=True):
     _chk(proj, hist, rep_ptr, rep_pos, convw, A_log, dt_bias)
@@ -576,6 +603,35 @@ def fattn_tree_tc(qt, kt, vt_t, gate, krange, scale):
     return y
 
 
+def tree_attn_rows(qt, kt, vt_t, q_src, krange, scale, q_rows=None):
+    """fattn_tree_tc on the operands of attn_operands: the gate is read where the in-projection left it (the second 256 columns
+    of every head of q_src), and the query rows may be any rows of the tree (q_rows int64). -> y [NQ, HQ*256]."""
+    _chk(qt, kt, vt_t, krange, q_rows)
+    HQ, NQ, D = qt.shape
+    HKV, N, _ = kt.shape
+    if D != 256 or HQ % HKV or HQ // HKV > 6 or tuple(vt_t.shape) != (HKV, D, N) or tuple(krange.shape) != (N, 8):
+        raise RuntimeError("tree_attn_rows: operands of attn_operands and krange [N, 8] expected")
+    if tuple(q_src.shape) != (NQ, HQ * 2 * D) or q_src.stride(1) != 1 or q_src.dtype != bf16 or (q_rows is None and NQ != N):
+        raise RuntimeError("tree_attn_rows: q_src does not belong to qt")
+    y = torch.empty(NQ, HQ * D, dtype=bf16, device=qt.device)
+    call("ojb_tree_attn_rows", ptr(qt), i64(NQ), ptr(q_rows), ptr(kt), ptr(vt_t), i64(N), ptr(q_src[:, D:]), i64(q_src.stride(0)),
+         i64(2 * D), ptr(krange), ptr(y), i64(HQ), i64(HKV), f32(scale), ptr(_lib.status_word(qt.device)), stream_ptr())
+    return y
+
+
+def gather_rows(rows, a, b=None):
+    """a[rows] (and b[rows]) of contiguous matrices, one launch. rows int64."""
+    _chk(rows, a, b)
+    S = rows.numel()
+    outs = [torch.empty((S,) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in (a, b) if t is not None]
+    size = [t[0].numel() * t.element_size() for t in (a, b) if t is not None] + [0]
+    if rows.dtype != torch.int64:
+        raise RuntimeError("gather_rows: int64 rows expected")
+    call("ojb_gather_rows", ptr(rows), i64(S), ptr(a), ptr(outs[0]), i64(size[0]), ptr(b), ptr(outs[1] if b is not None else None),
+         i64(size[1] if b is not None else 0), stream_ptr())
+    return outs if b is not None else outs[0]
+
+
 def fattn_tree2(proj, qw1, kw1, cosb, sinb, sig, vbits, HQ, HKV, scale, eps):
     """src/ext.py:38 — q/k preparation + attention + gate from the in-projection output (two launches here)."""
     N = proj.shape[0]
@@ -617,10 +673,10 @@ def embed_rope(ids, table, pos, inv_freq, scaling=1.0):
 
 # ------------------------------------------------------------------------------------------------ scoring head
 def score_head(hn, rows, W, bias):
-    """hn bf16 [N, H], rows int64 [S], W f32 [A, H], bias f32 [A] or None -> f32 [S, A] (gather + fp32 linear in one
+    """hn bf16 [N, H], rows int64 [S] or None (every row of hn), W f32 [A, H], bias f32 [A] or None -> f32 [S, A] (gather + fp32 linear in one
     launch; the reference does `head(hn[lastidx].float())` with torch, src/server.py:37)."""
     _chk(hn, rows, W, bias)
-    S, (A, H) = rows.numel(), W.shape
+    S, (A, H) = hn.shape[0] if rows is None else rows.numel(), W.shape
     out = torch.empty(S, A, dtype=torch.float32, device=hn.device)
     call("ojb_score_head", ptr(hn), ptr(rows), ptr(W), ptr(bias), ptr(out), i64(S), i64(A), i64(H), stream_ptr())
     return out

@@ -132,12 +132,13 @@ class FastQwen35(torch.nn.Module):
     # kernel, tile width and K split for any shape (lt_ext.gemm_plan); `tune(M)` refines that choice for one row count by
     # timing the candidates on this model's own weights, back to back over all layers (so under the power cap and with the
     # weights coming from HBM, as in the real forward).
-    def _mm(self, x, w):
-        """out = x @ w^T, bf16 (src/fastmodel.py:168 _mm)."""
+    def _mm(self, x, w, lo=0, hi=None):
+        """out = x @ w[lo:hi]^T, bf16 (src/fastmodel.py:168 _mm)."""
         q8 = self._q8.get(w.data_ptr()) if self.fp8 else None
         if q8 is not None:
             xq, sx = LT.quantize_rows_e4m3(x)
-            return LT.gemm_e4m3(xq, sx, q8[0], q8[1], 0)
+            return LT.gemm_e4m3(xq, sx, q8[0][lo:hi], q8[1][lo:hi], 0)
+        w = w[lo:hi]
         return LT.lt_matmul(x, w, self._force.get("mm", self._plan.get(("mm", x.shape[0], w.shape[0], w.shape[1]), 0)))
 
     @staticmethod
@@ -309,10 +310,20 @@ class FastQwen35(torch.nn.Module):
                            g.view(S, L2, d.HV), beta.view(S, L2, d.HV), d.HD ** -0.5)
         return K.gated_rmsnorm_inv2(o_r, lay.inv, proj, d.normw, None, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
 
+    def _attn_tc(self, d, lay, cos, N):
+        """Whether the tcgen05 attention serves this layer, and whether its operands come straight from the in-projection."""
+        tc = FATTN_TC and hasattr(lay, "krange") and d.D == 256 and d.HQ // d.HKV <= 6 and N % 32 == 0
+        return tc, tc and K.attn_operands_ok(d.HQ, d.HKV, d.D, cos.shape[-1], N)
+
     def _attn_tree(self, d, proj, lay, cos, sin):
         N = proj.shape[0]
         G = d.HQ // d.HKV
-        if FATTN_TC and hasattr(lay, "krange") and d.D == 256 and G <= 6 and N % 32 == 0:
+        tc, in_place = self._attn_tc(d, lay, cos, N)
+        if in_place:
+            q_src, kv_src = proj[:, :d.HQ * 2 * d.D], proj[:, d.HQ * 2 * d.D:]
+            qt, kt, vt_t = K.attn_operands(q_src, kv_src, d.qw1, d.kw1, cos, sin, d.HQ, d.HKV, self.eps)
+            return K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale)
+        if tc:
             qt, kt, vt, gate, vt_t = K.fullattn_prep2(proj, d.qw1, d.kw1, cos, sin, 1, N, d.HQ, d.HKV, d.D, self.eps, with_vt_t=True)
             return K.fattn_tree_tc(qt, kt, vt_t, gate, lay.krange, d.scale)
         qt, kt, vt, gate = K.fullattn_prep2(proj, d.qw1, d.kw1, cos, sin, 1, N, d.HQ, d.HKV, d.D, self.eps)
@@ -324,10 +335,37 @@ class FastQwen35(torch.nn.Module):
             return K.fattn_tree_ranges(qt, kt, vt, gate, lay.krange, d.scale, gq)
         return K.fattn_tree(qt, kt, vt, gate, None, lay.vbits, d.scale, gq)
 
+    # Behind its token mixer the last layer is a function of single rows, and only the candidates' last rows are asked for: its
+    # queries, output projection and MLP run on those alone. Below ASKED_MIN_ROWS rows every projection takes the time its weight
+    # takes to arrive whatever the row count, and the extra launches (a gather, two projections in the place of one) would only
+    # add to it.
+    ASKED_MIN_ROWS = 192
+
+    def _asked_rows_only(self, lay, N):
+        i = lay.lastidx
+        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and i.dtype == torch.int64 and i.is_contiguous()
+
+    def _mix_asked(self, d, h, hn, rows, lay, cos, sin, linear):
+        """Token mixer of the last layer for the asked rows: (their residual stream, their mixer output)."""
+        if not linear and self._attn_tc(d, lay, cos, hn.shape[0])[1]:
+            nq = d.HQ * 2 * d.D
+            hq, h = K.gather_rows(rows, hn, h)
+            q_src, kv_src = self._mm(hq, d.w_in, 0, nq), self._mm(hn, d.w_in, nq)
+            qt, kt, vt_t = K.attn_operands(q_src, kv_src, d.qw1, d.kw1, cos, sin, d.HQ, d.HKV, self.eps, rows)
+            return h, K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale, rows)
+        proj = self._mm(hn, d.w_in)
+        y = self._linear_tree(d, proj, lay) if linear else self._attn_tree(d, proj, lay, cos, sin)
+        return K.gather_rows(rows, h, y.view(y.shape[0], -1))
+
     @torch.no_grad()
     def forward_gtree(self, ids, lay, return_all=False):
         """src/fastmodel.py:400-482: ids int64 [N] packed rows, lay from gtree_build -> bf16 [S, H] (final norm applied) of
-        every candidate's last row; return_all=True gives all N rows (the scoring head gathers by itself)."""
+        every candidate's last row; return_all=True gives all N rows."""
+        hn, rows = self._forward(ids, lay, return_all)
+        return hn if return_all or rows is None else hn[rows]
+
+    def _forward(self, ids, lay, return_all=False):
+        """(final-norm hidden states, the rows of them that are asked for — None when those are all)."""
         if self._own_rope and ids.dtype == torch.int64 and lay.pos.dtype == torch.int64:
             x, cos, sin = K.embed_rope(ids, self.embed.weight, lay.pos, self._inv_freq, self._rope_scale)
         else:                                   # other rope types: the backbone's own module (torch)
@@ -338,21 +376,25 @@ class FastQwen35(torch.nn.Module):
         h = torch.empty(x.shape, dtype=torch.float32, device=x.device)        # the residual stream, fp32 throughout
         hn = K.resnorm_f32(h, x, None, None, self.in_w1[0], rowmask if lin[0] else None, self.eps)
         nl = len(self.L)
+        rows = None if return_all or not self._asked_rows_only(lay, x.shape[0]) else lay.lastidx
         for i, d in enumerate(self.L):
-            proj = self._mm(hn, d.w_in)
-            y = self._linear_tree(d, proj, lay) if lin[i] else self._attn_tree(d, proj, lay, cos, sin)
+            if rows is not None and i == nl - 1:
+                h, y = self._mix_asked(d, h, hn, rows, lay, cos, sin, lin[i])
+            else:
+                proj = self._mm(hn, d.w_in)
+                y = self._linear_tree(d, proj, lay) if lin[i] else self._attn_tree(d, proj, lay, cos, sin)
             h, hn = self._res(h, y, d.w_out, d.sk_out, self.post_w1[i], None)
             m = self._mlp_in(hn, d)
             last = i == nl - 1
             h, hn = self._res(h, m, d.w_down, d.sk_down, self.final_w1 if last else self.in_w1[i + 1],
                               None if last or not lin[i + 1] else rowmask)
-        return hn if return_all else hn[lay.lastidx]
+        return hn, (lay.lastidx if rows is None else None)
 
     @torch.no_grad()
     def score_gtree(self, ids, lay, head_w, head_b=None):
         """Forward + scoring head: fp32 [S, A] (src/server.py:37 `head(forward_gtree(ids, lay).float())`)."""
-        hn = self.forward_gtree(ids, lay, return_all=True)
-        return K.score_head(hn, lay.lastidx, head_w, head_b)
+        hn, rows = self._forward(ids, lay)
+        return K.score_head(hn, rows, head_w, head_b)
 
     # ------------------------------------------------------------------------------------------------ single-level tree
     def tree_layout(self, pre_ids, suf_ids, suf_mask, pad=0, dense=True, cap=None):
@@ -364,11 +406,20 @@ class FastQwen35(torch.nn.Module):
         """src/fastmodel.py:266-314: long shared prefix, S suffixes -> [S, H]. Both modes of the reference ("replicate" and
         "state") give the same result; here the prefix is always computed once and its Gated DeltaNet state handed to every
         suffix inside the state kernel."""
+        return self.forward_gtree(*self._single_level(pre_ids, suf_ids, lay), return_all)
+
+    @torch.no_grad()
+    def score_tree(self, pre_ids, suf_ids, lay, head_w, head_b=None):
+        """forward_tree + scoring head: fp32 [S, A]."""
+        return self.score_gtree(*self._single_level(pre_ids, suf_ids, lay), head_w, head_b)
+
+    @staticmethod
+    def _single_level(pre_ids, suf_ids, lay):
         ids = torch.zeros(lay.N32, dtype=pre_ids.dtype, device=pre_ids.device)
         ids[:lay.N] = torch.cat([pre_ids, suf_ids.reshape(-1)])
         inner = SimpleNamespace(N=lay.N32, S=lay.S, pos=lay.pos32, rowmask=lay.rowmask32, hist=lay.hist, krange=lay.krange,
                                 chunks=lay.chunks, steps=lay.steps, walk_ptr=lay.walk_ptr, n_walks=1, lastidx=lay.lastidx)
-        return self.forward_gtree(ids, inner, return_all)
+        return ids, inner
 
     # ------------------------------------------------------------------------------------------------ batch forward
     @torch.no_grad()

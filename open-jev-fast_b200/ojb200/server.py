@@ -136,7 +136,6 @@ class EntryState:
     FIELDS = ("pos32", "rowmask32", "hist", "krange", "chunks", "steps", "walk_ptr", "lastidx")
 
     def __init__(self, scorer, Lpb, S, Lsb):
-        from . import ext as K
         fast, dev = scorer.fast, scorer.device
         self.pre = torch.zeros(Lpb, dtype=torch.long, device=dev)
         self.suf = torch.zeros(S, Lsb, dtype=torch.long, device=dev)
@@ -144,8 +143,7 @@ class EntryState:
         self.cap = -(-Lpb // 64) + S * -(-Lsb // 64)
         self.lay = fast.tree_layout(self.pre, self.suf, self.msk, pad=0, dense=False, cap=self.cap)
         fast.tune(self.lay.N32)
-        body = lambda: K.score_head(fast.forward_tree(self.pre, self.suf, self.lay, "state", return_all=True), self.lay.lastidx,
-                                    scorer.head_w, scorer.head_b)
+        body = lambda: fast.score_tree(self.pre, self.suf, self.lay, scorer.head_w, scorer.head_b)
         st = torch.cuda.Stream(device=dev)
         st.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(st):

@@ -83,6 +83,61 @@ def test_tree_attention_tcgen05(N_case, HQ, HKV):
     assert ((got[real] - old[real]).norm() / old[real].norm()).item() < 4e-3
 
 
+@pytest.mark.parametrize("N_case,HQ,HKV", [("baseline", 24, 4), ("ragged", 4, 2), ("long", 12, 2), ("nostem", 5, 1)])
+def test_tree_attention_of_any_rows(N_case, HQ, HKV):
+    """tree_attn_rows (gate read inside the in-projection output; all rows, or some as queries) against fattn_tree_tc. All rows:
+    the same kernel on the same tiles, the same bits. Some rows: other tiles see other lists of key blocks, so sums of the same
+    terms in another order (P in bf16): a bf16 ulp of the result, 2^-8, on single values."""
+    from ojb200 import ext as K, _lib
+    from ojb200 import layout as PL
+    D, RD = 256, 64
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()[N_case]
+    ids, lay = PL.gtree_build(seqs, groups, pad_id, NB, PB, dev="cuda", dense=False)
+    N = lay.N
+    g = torch.Generator(device="cuda").manual_seed(29)
+    proj = torch.randn(N, 2 * HQ * D + 2 * HKV * D, generator=g, device="cuda").to(bf16)
+    w1 = 1.0 + torch.randn(D, generator=g, device="cuda") * 0.02
+    cosb, sinb = (torch.randn(N, RD, generator=g, device="cuda").to(bf16) for _ in range(2))
+    qt, kt, vt, gate, vt_t = K.fullattn_prep2(proj, w1, w1, cosb, sinb, 1, N, HQ, HKV, D, 1e-6, with_vt_t=True)
+    want = K.fattn_tree_tc(qt, kt, vt_t, gate, lay.krange, D ** -0.5)
+    q_src = proj[:, :HQ * 2 * D]
+    assert torch.equal(K.tree_attn_rows(qt[0], kt[0], vt_t[0], q_src, lay.krange, D ** -0.5), want)
+    real = lay.rowmask.nonzero().flatten()
+    for n in (1, 16, 17, 45):
+        rows = real[torch.randint(0, real.numel(), (n,), generator=g, device="cuda")]
+        y = K.tree_attn_rows(qt[0][:, rows].contiguous(), kt[0], vt_t[0], q_src[rows], lay.krange, D ** -0.5, rows)
+        assert (y.float() - want[rows].float()).norm() <= 4e-3 * want[rows].float().norm()
+        assert torch.allclose(y.float(), want[rows].float(), rtol=2 ** -6, atol=2 ** -7)
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("case", ["doc", "baseline", "nostem"])
+@pytest.mark.parametrize("last", ["full_attention", "linear_attention"])
+@pytest.mark.parametrize("head_dim,fp8", [(256, False), (256, True), (64, False)])
+def test_last_layer_on_the_asked_rows(case, last, head_dim, fp8, monkeypatch):
+    """The last layer's queries, output projection and MLP on the asked rows alone against the same layer on every row: the
+    same terms, projections of another row count (another K split): bf16 roundings of one layer."""
+    from ojb200 import fastmodel as FM
+    from ojb200 import modelgen as MG
+    over = dict(MG.SMALL, head_dim=head_dim)
+    layers = 3
+    cfg = MG.make_config(**dict(over, num_hidden_layers=layers, layer_types=["linear_attention", "full_attention", last]))
+    core = MG.build_core(cfg, device="cpu", seed=3, std=0.05, draw_on="cpu").to("cuda")
+    fast = FM.FastQwen35(core, fp8=fp8)
+    W, b = MG.make_head(cfg.hidden_size, A=2, seed=1, device="cuda")
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()[case]
+    ids, lay = fast.gtree_build([[t % cfg.vocab_size for t in s] for s in seqs], groups, pad_id, NB, PB, dev="cuda")
+    monkeypatch.setattr(FM.FastQwen35, "ASKED_MIN_ROWS", 1 << 30)
+    want = fast.forward_gtree(ids, lay).float()
+    want_s = fast.score_gtree(ids, lay, W, b)
+    monkeypatch.setattr(FM.FastQwen35, "ASKED_MIN_ROWS", 1)
+    assert fast._asked_rows_only(lay, lay.N)
+    got = fast.forward_gtree(ids, lay).float()
+    assert (got - want).norm() <= (2e-2 if fp8 else 6e-3) * want.norm()
+    got_s = fast.score_gtree(ids, lay, W, b)
+    assert (got_s - want_s).norm() <= (2e-2 if fp8 else 6e-3) * want_s.norm().clamp_min(1.0)
+
+
 def _small_model(seed=0):
     from ojb200 import modelgen as MG
     cfg = MG.make_config(**MG.SMALL)

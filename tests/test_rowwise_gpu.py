@@ -130,3 +130,34 @@ def test_embed_rope_matches_torch_embedding_and_the_backbone_rotary_module():
     bad[5] = V + 7                                   # an id outside the table: a zero row, not a fault
     x2, _, _ = K.embed_rope(bad, table, pos, rot.inv_freq.float().contiguous(), 1.0)
     assert x2[5].abs().max().item() == 0 and torch.equal(x2[6:], want_x[6:])
+
+
+@pytest.mark.parametrize("N,HQ,HKV,RD", [(8, 6, 1, 64), (40, 4, 4, 16), (72, 24, 4, 256), (544, 24, 4, 64)])
+@pytest.mark.parametrize("asked", [False, True])
+def test_attn_operands_equal_fullattn_prep(N, HQ, HKV, RD, asked):
+    """The operands of the attention straight from the in-projection are those of fullattn_prep bit for bit: all rows, and any
+    rows as queries (repeated and out of order) with the rotary angles of the rows they stand for."""
+    from ojb200 import ext as K
+    D = 256
+    g = torch.Generator().manual_seed(N)
+    proj = _randn(N, 2 * HQ * D + 2 * HKV * D, seed=13).cuda()
+    qw1, kw1 = ((1.0 + torch.randn(D, generator=g) * 0.02).cuda() for _ in range(2))
+    ang = torch.rand(N, RD // 2, generator=g) * 6.28
+    cosb, sinb = (torch.cat([f(ang)] * 2, -1).to(bf16).cuda() for f in (torch.cos, torch.sin))
+    want_q, want_k, _, _, want_v = K.fullattn_prep2(proj, qw1, kw1, cosb, sinb, 1, N, HQ, HKV, D, 1e-6, with_vt_t=True)
+    rows = torch.randint(0, N, (min(N, 19),), generator=g).cuda() if asked else None
+    q_src = proj[:, :HQ * 2 * D]
+    if asked:
+        q_src = K.gather_rows(rows, proj)[:, :HQ * 2 * D]
+        want_q = want_q[:, :, rows]
+    qt, kt, vt_t = K.attn_operands(q_src, proj[:, HQ * 2 * D:], qw1, kw1, cosb, sinb, HQ, HKV, 1e-6, rows)
+    assert torch.equal(qt, want_q[0]) and torch.equal(kt, want_k[0]) and torch.equal(vt_t, want_v[0])
+
+
+@pytest.mark.parametrize("rows", [1, 3, 700])
+def test_gather_rows(rows):
+    from ojb200 import ext as K
+    a, b = _randn(50, 24, seed=14).cuda(), torch.randn(50, 4, generator=torch.Generator().manual_seed(1)).cuda()
+    idx = torch.randint(0, 50, (rows,), generator=torch.Generator().manual_seed(2)).cuda()
+    ga, gb = K.gather_rows(idx, a, b)
+    assert torch.equal(ga, a[idx]) and torch.equal(gb, b[idx]) and torch.equal(K.gather_rows(idx, b), b[idx])
