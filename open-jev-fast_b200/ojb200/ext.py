@@ -14,6 +14,7 @@ from . import _lib
 from ._lib import call, f32, i32, i64, ptr, stream_ptr
 
 bf16 = torch.bfloat16
+SM_COUNT = 148
 
 
 def load(verbose=False):
@@ -420,8 +421,13 @@ def gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walk_ptr, n_walks, init_
     scratch = torch.empty(nbytes(i64(nch), i64(HV)), dtype=torch.uint8, device=v.device)
     if out is None:
         out = torch.empty(v.shape, dtype=bf16, device=v.device)
-    call("ojb_gdn_chunked", ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(chunks), i64(nch), ptr(steps), ptr(walk_ptr),
-         i64(n_walks), ptr(init_state), ptr(final_state), ptr(scratch), ptr(out), i64(HK), i64(HV), f32(scale),
+    park = None
+    if 4 * HV * n_walks > SM_COUNT:      # more CTAs than SMs in the state pass: room for the form that puts two on an SM
+        pbytes = _lib.lib().ojb_gdn_park_bytes
+        pbytes.restype = _lib.ctypes.c_int64
+        park = torch.empty(pbytes(i64(n_walks), i64(HV)), dtype=torch.uint8, device=v.device)
+    call("ojb_gdn_chunked_park", ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(chunks), i64(nch), ptr(steps), ptr(walk_ptr),
+         i64(n_walks), ptr(init_state), ptr(final_state), ptr(scratch), ptr(out), i64(HK), i64(HV), f32(scale), ptr(park),
          ptr(_lib.status_word(v.device)), stream_ptr())
     return out
 

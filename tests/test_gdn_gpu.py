@@ -241,3 +241,35 @@ def test_prep_refuses_projection_rows_that_are_not_16_byte_aligned():
     one = torch.ones(HV, dtype=bf16, device="cuda")
     with pytest.raises(RuntimeError):
         K.linattn_prep_rows(proj, hist, convw, one, one, 128, 128, HV, HK, 128)
+
+
+@pytest.mark.parametrize("name,HV,copies", [("baseline", 48, 1), ("example", 40, 1), ("single", 48, 1), ("wide", 16, 4), ("ragged", 32, 3)])
+def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
+    """More CTAs than SMs: the dense form of the state pass (operands refilled in two parts, states parked in global memory)
+    against the full form, outputs and exported states, for one wide tree and for several trees as walks of one call."""
+    from ojb200 import ext as K, _lib
+    from ojb200 import layout as PL
+    HK = 8
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()[name]
+    ids, lay, _ = PL.pack_requests([(seqs, groups)] * copies, pad_id, NB, PB, dev="cuda")
+    assert 4 * HV * copies > K.SM_COUNT
+    q, k, v, g, beta = (t.cuda() for t in _inputs(lay.N, HK, HV, 5))
+    steps = lay.steps.clone()
+    for i in range(copies):
+        steps[int(lay.walk_ptr[i + 1]) - 1, 3] = i + 1                 # export the last state of every walk
+    outs = []
+    for dense in (True, False):
+        out = torch.zeros(lay.N, HV, 128, dtype=bf16, device="cuda")
+        fin = torch.zeros(copies, HV, 128, 128, device="cuda")
+        if dense:
+            K.gdn_chunked(q, k, v, g, beta, 128 ** -0.5, lay.chunks, steps, lay.walk_ptr, copies, None, fin, out)
+        else:
+            scratch = torch.empty(lay.chunks.shape[0] * HV * 81936, dtype=torch.uint8, device="cuda")
+            K.call("ojb_gdn_chunked", *(K.ptr(t) for t in (q, k, v, g, beta, lay.chunks)), K.i64(lay.chunks.shape[0]), K.ptr(steps),
+                   K.ptr(lay.walk_ptr), K.i64(copies), K.ptr(None), K.ptr(fin), K.ptr(scratch), K.ptr(out), K.i64(HK), K.i64(HV),
+                   K.f32(128 ** -0.5), K.ptr(_lib.status_word(v.device)), K.stream_ptr())
+        outs.append((out, fin))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert float(outs[0][0].float().abs().max()) > 0
