@@ -243,6 +243,62 @@ def test_prep_refuses_projection_rows_that_are_not_16_byte_aligned():
         K.linattn_prep_rows(proj, hist, convw, one, one, 128, 128, HV, HK, 128)
 
 
+def _branching_hist(N, gen):
+    """A history table of random paths: runs of consecutive rows, some starting a path, some branching off an earlier row, some
+    rows on no path at all."""
+    hist = np.full((N + 1, 4), -1, np.int32)
+    for n in range(N):
+        u = float(torch.rand((), generator=gen))
+        if u < 0.08:
+            continue
+        prev = n - 1 if u < 0.7 or n == 0 else int(torch.randint(0, n, (), generator=gen))
+        if n > 0 and u < 0.95 and hist[prev, 3] >= 0:
+            hist[n, :3] = hist[prev, 1:]
+        hist[n, 3] = n
+    return torch.as_tensor(hist).cuda()
+
+
+@pytest.mark.parametrize("N", [1, 3, 127, 128, 261, 2047, 2048, 2061])       # one, four and eight rows to a thread, with remainders
+@pytest.mark.parametrize("l2", [True, False])
+def test_prep_of_packed_rows_equals_the_scatter_form(N, l2):
+    """Rows on random paths: the form that reuses rows in registers against the one that reads every tap (each row scattered to
+    its own slot), bit for bit."""
+    from ojb200 import ext as K
+    HK, HV = 2, 4 if N < 300 else 8
+    KD, VD = HK * 128, HV * 128
+    gen = torch.Generator().manual_seed(N)
+    proj = torch.randn(N, 2 * KD + 2 * VD + 2 * HV, generator=gen).to(bf16).cuda()
+    convw = (torch.randn(2 * KD + VD, 4, generator=gen) * 0.3).to(bf16).cuda()
+    A_log, dt_bias = (torch.randn(HV, generator=gen).to(bf16).cuda() for _ in range(2))
+    hist = _branching_hist(N, gen)
+    ptr_ = torch.cat([torch.arange(N + 1), torch.tensor([N])]).to(torch.int32).cuda()
+    pos = torch.arange(N, dtype=torch.int32).cuda()
+    got = K._prep(proj, hist, None, None, N, convw, A_log, dt_bias, KD, VD, HV, HK, 128, l2)
+    want = K._prep(proj, hist, ptr_, pos, N, convw, A_log, dt_bias, KD, VD, HV, HK, 128, l2)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,HV", [(1, 1), (37, 4), (1023, 17), (2048, 16), (2501, 48)])
+@pytest.mark.parametrize("gather", [False, True])
+def test_gated_rmsnorm_wide_accesses_equal_the_narrow_ones(N, HV, gather):
+    """16-byte form (aligned columns) against the 8-byte form (the same gate four columns further right): sums of the same 128
+    squares in another order, so at most an ulp of the bf16 result, on few values."""
+    from ojb200 import ext as K
+    gen = torch.Generator().manual_seed(N + HV)
+    x = torch.randn(N + 5, HV, 128, generator=gen).to(bf16).cuda()
+    proj = torch.randn(N, HV * 128 + 24, generator=gen).to(bf16).cuda()
+    w = (1 + 0.02 * torch.randn(128, generator=gen)).to(bf16).cuda()
+    inv = torch.randint(0, N + 5, (N,), generator=gen).to(torch.int32).cuda() if gather else None
+    moved = torch.zeros(N, HV * 128 + 24, dtype=bf16, device="cuda")
+    moved[:, 12:12 + HV * 128] = proj[:, 8:8 + HV * 128]
+    src = x if gather else x[:N].contiguous()
+    a = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6).float()
+    b = K._gated_norm(src, inv, moved, w, HV, 128, 12, 1e-6).float()
+    assert bool(((a - b).abs() <= b.abs() * 2 ** -7 + 1e-30).all())
+    assert (a == b).float().mean().item() > 0.99
+
+
 @pytest.mark.parametrize("name,HV,copies", [("baseline", 48, 1), ("example", 40, 1), ("single", 48, 1), ("wide", 16, 4), ("ragged", 32, 3)])
 def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
     """More CTAs than SMs: the dense form of the state pass (operands refilled in two parts, states parked in global memory)
@@ -273,3 +329,32 @@ def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
     _lib.check_status()
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     assert float(outs[0][0].float().abs().max()) > 0
+
+
+def test_silu_and_sigmoid_of_every_bf16_value():
+    """The element-wise functions of the preparation on all 65 536 bf16 inputs (a convolution whose last tap is 1), against
+    64 bits: the bf16 result is the correctly rounded one wherever the fp32 value before rounding, a few units of 2^-24 off, does
+    not cross a rounding boundary — all but a handful. Infinities and not-a-numbers as x / (1 + e^-x) gives them."""
+    from ojb200 import ext as K
+    HK, HV, N = 1, 4, 128                       # 128 rows x 512 value channels: every bf16 value once
+    KD, VD = 128, 512
+    bits = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(torch.int16)
+    x = bits.view(bf16).view(N, VD)
+    proj = torch.zeros(N, 2 * KD + 2 * VD + 2 * HV, dtype=bf16)
+    proj[:, 2 * KD:2 * KD + VD] = x
+    convw = torch.zeros(2 * KD + VD, 4, dtype=bf16)
+    convw[:, 3] = 1
+    hist = torch.full((N + 1, 4), -1, dtype=torch.int32)
+    hist[:N, 3] = torch.arange(N)
+    one = torch.zeros(HV, dtype=bf16)
+    _, _, v, _, _ = K._prep(proj.cuda(), hist.cuda(), None, None, N, convw.cuda(), one.cuda(), one.cuda(), KD, VD, HV, HK, 128, False)
+    got, x64 = v.cpu().flatten(), x.double().flatten()
+    want = (x64 / (1.0 + torch.exp(-x64)))
+    nan = torch.isnan(want)
+    assert torch.equal(torch.isnan(got), nan)
+    normal = ~nan & (want.abs() > 2.0 ** -120)
+    wrong = got[normal] != want[normal].to(bf16)
+    assert wrong.float().mean().item() < 2e-3
+    a, b = got[normal].double(), want[normal]
+    assert bool((((a - b).abs() <= b.abs() * 2.0 ** -8) | (a == b)).all())
+    assert bool((got[~nan & ~normal].double().abs() <= 2.0 ** -119).all())
