@@ -5,6 +5,8 @@
 //   block256  (gemm_block256.cu)  256 rows of x share each w tile between two MMAs (one third less shared-memory fill per
 //             flop), w-tile width chosen per shape, the last M mod 256 <= 128 rows (or all rows when M <= 2048, on request) run with
 //             swapped operands at their true cost.
+//   skinny    (gemm_skinny.cu)    up to 128 rows of x against w tiles of any width, every CTA's shared memory full of weight in
+//             flight; the choice for at most 32 rows.
 //   pair256   (gemm_pair256.cu)   the same units on CTA pairs with tcgen05.mma.cta_group::2; measured on par with block256
 //             (both are bound by shared-memory bandwidth), kept as variants 5 / 6.
 // With variant 0 the kernel is the one with the smallest modelled time (plan_kernel): the models replay the round-robin
@@ -20,19 +22,34 @@ namespace {
 // units (M <= 2048).
 // 5 = pair256 (CTA pairs, cta_group::2) with automatic width; 6 = pair256 with every row of x in swapped-operand units
 // (any M); 512 + a multiple of 16 in [16, 256] = pair256 with that w-tile width; 7 = block256 with the last 257..511 rows of x in
-// two swapped-operand chunks and the rows before them in block units.
+// two swapped-operand chunks and the rows before them in block units; 1024 = skinny (M <= 128, K % 64 == 0, not for SwiGLU; else as 0) with automatic
+// width;
+// 1024 + a multiple of 16 in [16, 128] = skinny with that w-tile width.
 bool variant_ok(int v) {
-  return (v >= 0 && v <= 7) || (v >= 16 && v <= 256 && v % 16 == 0) || (v >= 528 && v <= 768 && v % 16 == 0);
+  return (v >= 0 && v <= 7) || (v >= 16 && v <= 256 && v % 16 == 0) || (v >= 528 && v <= 768 && v % 16 == 0) ||
+         (v >= 1024 && v <= 1152 && v % 16 == 0);
 }
 
 // Modelled SM clocks of the 128-row tile kernel: per k-block a CTA fills (128 + BN) rows and its MMAs read them once,
 // 128 bytes per clock; the epilogue overlaps the next tile.
-double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, int sms) {
+double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, int sms, int epi) {
   const int64_t units = ceil_div(M, 128) * ceil_div(N, bn) * splits;
   const int64_t grid = units < sms ? units : sms;
   const int per = static_cast<int>(ceil_div(kb_total, splits));
   const double kb = bn == 256 ? 900.0 : 600.0;   // fitted to back-to-back runs against the power cap (133 us at 288 rows, 206 us at 544 for gate/up)
-  return static_cast<double>(ceil_div(units, grid)) * (per * kb + 1500.0) + 9000.0;
+  return static_cast<double>(ceil_div(units, grid)) * (per * kb + (epi == kEpiPartialF32 ? 33.0 * bn : 1500.0)) + 9000.0;
+}
+
+// The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (wait, four MMAs, its share of a commit) in less than 280
+// clocks. Measured on [12352, 5120] at 12 / 32 / 64 rows: 26.0 / 26.0 / 33 us against 41 / 28.6 / 29.1 of the 128-row tile kernel
+// (the rows of x that every CTA fetches again cost more from there on, hence kSkinnyRows); [2048, 5120] 18 against 26 us, [5120, 4096]
+// 11.7 against 12.3 us and [5120, 17408] 33.2 against 34.4 us of the best other kernel and K ranges.
+constexpr int kSkinnyRows = 32;
+double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
+  const int bn = skinny_bn(N, splits);
+  const double waves = static_cast<double>(ceil_div(ceil_div(N, bn) * splits, sms));
+  const double fill = (bn + ceil_div(M, 8) * 8) * 128.0 / 30.0, per = static_cast<double>(ceil_div(kb_total, splits));
+  return waves * per * (fill > 280.0 ? fill : 280.0) + 6000.0;
 }
 
 struct Plan {
@@ -49,8 +66,8 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   auto consider = [&](int variant, double clocks) {
     if (clocks < best.clocks) best = Plan{variant, clocks};
   };
-  consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms));
-  if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms));
+  if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, epi));
+  if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, epi));
   {  // block256: full blocks + swapped tail
     int n_xblk = static_cast<int>(M / 256), r = static_cast<int>(M % 256);
     if (r > 128) { n_xblk += 1; r = 0; }
@@ -65,6 +82,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
     const int tail_box = static_cast<int>(ceil_div(ceil_div(M, n_xchunk), 16) * 16);
     consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, epi));
   }
+  if (M <= kSkinnyRows && epi != kEpiSwiglu && skinny_serves(M, K)) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz
   if (best.clocks < hbm) best.clocks = hbm;
   return best;
@@ -78,7 +96,9 @@ Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
 
 int dispatch(int epi, int variant, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
              int64_t ldo, int32_t* status, cudaStream_t st) {
+  if (variant == 1024 && (epi == kEpiSwiglu || !skinny_serves(M, K))) variant = 0;
   if (variant == 0) variant = plan_kernel(epi, M, N, K, splits).variant;
+  if (variant >= 1024) return gemm_skinny_launch(epi, variant - 1024, x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 5 || variant == 6 || variant >= 512)
     return gemm_pair256_launch(epi, variant == 5 ? 0 : (variant == 6 ? -1 : variant - 512), x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 1 || variant == 2)
@@ -98,7 +118,7 @@ extern "C" int ojb_gemm_bf16(const void* x, const void* w, void* out, int64_t M,
 extern "C" int ojb_gemm_bf16_swiglu_v(const void* x, const void* w_blk, void* out, int64_t M, int64_t N, int64_t K, int variant,
                                       int32_t* status, ojb_stream_t stream) {
   OJB_REQUIRE(x && w_blk && out && M > 0 && N > 0 && K > 0 && K % 8 == 0 && N % 256 == 0);
-  OJB_REQUIRE(aligned16(x) && aligned16(w_blk) && aligned16(out) && (variant == 0 || variant == 1 || variant == 3 || variant == 4 || variant == 5 || variant == 6 || variant == 7));
+  OJB_REQUIRE(aligned16(x) && aligned16(w_blk) && aligned16(out) && (variant == 0 || variant == 1 || variant == 3 || variant == 4 || variant == 5 || variant == 6 || variant == 7 || variant == 1024));
   return dispatch(kEpiSwiglu, variant, x, w_blk, out, M, N, K, 1, N / 2, status, static_cast<cudaStream_t>(stream));
 }
 
@@ -185,6 +205,8 @@ extern "C" int ojb_gemm_e4m3(const void* xq, const float* sx, const void* wq, co
   OJB_REQUIRE(kind == 2 ? (splits >= 1 && splits <= 16) : splits == 1);
   OJB_REQUIRE(kind != 1 || N % 256 == 0);
   const int epi = kind == 0 ? kEpiBf16 : (kind == 1 ? kEpiSwiglu : kEpiPartialF32);
+  if (M <= kSkinnyRows && K % 128 == 0 && epi != kEpiSwiglu)
+    return gemm_skinny_launch(epi, 0, xq, wq, out, M, N, K, splits, N, status, static_cast<cudaStream_t>(stream), sx, sw);
   return gemm_block256_launch_e4m3(epi, xq, sx, wq, sw, out, M, N, K, splits, kind == 1 ? N / 2 : N, status,
                                    static_cast<cudaStream_t>(stream));
 }

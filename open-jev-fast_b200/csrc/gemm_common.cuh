@@ -239,6 +239,8 @@ void gemm_block256_set_trace(unsigned long long* buf, int cap);
 // e4m3 operands with one fp32 scale per row of x (sx) and per row of w (sw): out = (xq . wq^T) * sx[m] * sw[n]
 int gemm_block256_launch_e4m3(int epi, const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M,
                               int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
+int gemm_skinny_launch(int epi, int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
+                       int64_t ldo, int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr);
 int gemm_pair256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,
                         int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
 void gemm_pair256_set_trace(unsigned long long* buf, int cap);

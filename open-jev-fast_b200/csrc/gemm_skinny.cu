@@ -1,0 +1,267 @@
+// GEMM of few rows (M <= 128), sm_100a: out[M,N] = x[M,K] · w[N,K]^T for a weight that has to come from HBM.
+//
+// With so few rows the time is that of the weight's bytes, if enough of them are under way: at 6.4 TB/s and about 2 us from request
+// to arrival that is 12 MB, 85 KB on every SM. The larger kernels fix the w tile at 128 or 256 rows and carry 128 rows of x (or
+// two accumulators) beside it: 97 tiles for 12 352 outputs, 16 for 2048, each SM's share of the link idle on the rest. Here the w
+// tile has any multiple of 16 rows up to 128, chosen so that the tiles (times the K ranges) fill the SMs once, and a stage holds
+// the rows of x that exist and no more, so that all of the shared memory is weight in flight.
+// A stage is several k-blocks, one three-dimensional copy each for x and w: with one k-block per stage the chain wait, MMAs, commit of
+// the issuing thread (0.31 us; the commit alone about 0.15) and the producer's wait and two copies (0.2 us) set the pace, 26 us
+// for K = 5120 whatever the weight's size.
+//
+// One CTA per (w tile, K range), 192 threads: warp 0 asks for the tiles (plain cp.async.bulk.tensor, 128-byte swizzle, mbarrier), one
+// lane of warp 1 issues tcgen05.mma, warps 2-5 read the accumulator back and store. The MMA has M = 128 whatever the number of
+// rows: its A operand starts at the stage's x rows and runs on into whatever shared memory follows them (the w tile, the next
+// stage); a row of the product depends on its own row of A alone, and the rows past M are never read back.
+#include "gemm_units.cuh"
+
+namespace ojb {
+namespace {
+
+constexpr int kSkinnyThreads = 192;
+constexpr int kSkinnyMaxStages = 40;
+constexpr int kSkinnyMaxRows = 128;
+constexpr size_t kSkinnySmem = 227 * 1024;
+
+struct SkinnyArgs {
+  int M, N;
+  int BN, x_rows;                  // rows of w and of x in a stage
+  int splits, kb_per_split, kb_total;
+  int nk;                          // k-blocks per stage
+  int stages;
+  uint32_t stage_bytes, tmem_cols;
+  void* out;
+  int64_t ldo, split_stride;
+  int32_t* status;
+  int wait_ms, drop_copy;
+  const float* sx;                 // e4m3 operands: scale per row of x and of w
+  const float* sw;
+};
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
+// A row-major matrix of `cols` elements (elt bytes each) to a row as [k-block][row][128 bytes]: box = nk k-blocks of box_rows rows,
+// 128-byte swizzle. cols * elt is a multiple of 128: the last k-block of the last row would otherwise reach past the matrix.
+int make_kblock_map(CUtensorMap* map, const void* base, int elt, int64_t rows, int64_t cols, int box_rows, int nk) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return OJB_ERR_DRIVER;
+  const cuuint64_t inner = 128 / elt;
+  cuuint64_t dims[3] = {inner, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols) / inner};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * elt, 128};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(inner), static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(nk)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, elt == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? OJB_OK : OJB_ERR_ARG;
+}
+
+template <int EPI, bool FP8>
+__global__ void __launch_bounds__(kSkinnyThreads, 1)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, SkinnyArgs g) {
+  pdl_launch_dependents();
+  constexpr int kKE = FP8 ? 128 : kBK;      // elements of K per 128-byte k-block
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  __shared__ __align__(8) uint64_t bars[2 * kSkinnyMaxStages + 1];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag[2];
+  const uint32_t tiles0 = smem_u32(smem), full0 = smem_u32(bars), empty0 = full0 + 8 * kSkinnyMaxStages;
+  const uint32_t accfull = empty0 + 8 * kSkinnyMaxStages;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = blockIdx.x / g.splits, split = blockIdx.x - tile * g.splits;
+  const int kb0 = split * g.kb_per_split, nkb = min(kb0 + g.kb_per_split, g.kb_total) - kb0;
+  const int n0 = tile * g.BN;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < g.stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    mbar_init(accfull, 1);
+    abort_flag[0] = 0;
+    abort_flag[1] = g.wait_ms;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_slot), g.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  pdl_wait();
+
+  const uint32_t x_bytes = static_cast<uint32_t>(g.x_rows) * 128, w_bytes = static_cast<uint32_t>(g.BN) * 128;      // of one k-block
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      for (int kb = 0; kb < nkb; kb += g.nk) {
+        if (!mbar_wait(empty0 + 8 * stage, phase ^ 1u, abort_flag)) break;
+        const uint32_t dst = tiles0 + stage * g.stage_bytes, fb = full0 + 8 * stage;
+        mbar_expect_tx(fb, g.stage_bytes);
+        if (!(g.drop_copy && kb == g.nk)) {      // tests only: the announced bytes never arrive
+          // (k-blocks past the end of this range are not multiplied; past the end of K they arrive as zeros)
+          tma_load_3d(dst + g.nk * x_bytes, &map_w, fb, 0, n0, kb0 + kb);
+          tma_load_3d(dst, &map_x, fb, 0, 0, kb0 + kb);
+        }
+        if (++stage == g.stages) { stage = 0; phase ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      const uint32_t idesc = FP8 ? umma_idesc_e4m3(g.BN) : umma_idesc(g.BN);
+      bool ok = true;
+      for (int kb = 0; kb < nkb; kb += g.nk) {
+        if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t src = tiles0 + stage * g.stage_bytes;
+        for (int j = 0; j < g.nk && kb + j < nkb; ++j) {
+          const uint64_t adesc = smem_desc_sw128(src + j * x_bytes), bdesc = smem_desc_sw128(src + g.nk * x_bytes + j * w_bytes);
+#pragma unroll
+          for (int k = 0; k < kBK / kUmmaK; ++k) {
+            const uint32_t accum = (kb + j > 0 || k > 0) ? 1u : 0u;
+            if constexpr (FP8) umma_f8(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+            else umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+          }
+        }
+        umma_commit(empty0 + 8 * stage);
+        if (++stage == g.stages) { stage = 0; phase ^= 1u; }
+      }
+      if (ok) umma_commit(accfull);
+    }
+  } else {
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    if (mbar_wait(accfull, 0, abort_flag)) {
+      tc_fence_after();
+      if (quarter * 32 < g.M) {
+        const bool row_ok = row < g.M;
+        const int ncols = min(g.N - n0, g.BN);
+        float rs = 1.f;
+        if constexpr (FP8) rs = row_ok ? __ldg(g.sx + row) : 1.f;
+        const int64_t off = static_cast<int64_t>(split) * g.split_stride + static_cast<int64_t>(row) * g.ldo + n0;
+        const bool vec_ok = (g.ldo & 7) == 0 && (g.split_stride & 3) == 0;      // n0 and the 16-column steps keep the alignment
+#pragma unroll 1
+        for (int c = 0; c < ncols; c += 16) {
+          uint32_t r[16];
+          tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
+          tmem_ld_wait();
+          if (row_ok) {
+            float v[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+              v[e] = __uint_as_float(r[e]);
+              if constexpr (FP8) v[e] *= rs * __ldg(g.sw + min(n0 + c + e, g.N - 1));
+            }
+            if constexpr (EPI == kEpiPartialF32) {
+              float* o = reinterpret_cast<float*>(g.out) + off + c;
+              if (vec_ok && c + 16 <= ncols) {
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(o + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                  if (c + e < ncols) o[e] = v[e];
+              }
+            } else {
+              bf16_t* o = reinterpret_cast<bf16_t*>(g.out) + off + c;
+              if (vec_ok && c + 16 <= ncols) {
+#pragma unroll
+                for (int e = 0; e < 16; e += 8)
+                  *reinterpret_cast<uint4*>(o + e) = make_uint4(pack2(v[e], v[e + 1]), pack2(v[e + 2], v[e + 3]), pack2(v[e + 4], v[e + 5]),
+                                                                pack2(v[e + 6], v[e + 7]));
+              } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                  if (c + e < ncols) o[e] = f2bf(v[e]);
+              }
+            }
+          }
+          __syncwarp();
+        }
+      }
+      tc_fence_before();
+    }
+  }
+
+  __syncthreads();
+  if (abort_flag[0]) {
+    if (threadIdx.x == 0) report_status(g.status, OJB_DEV_WAIT_TIMEOUT);
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);      // copies that were already issued land before the CTA leaves
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, g.tmem_cols);
+  }
+}
+
+template <int EPI, bool FP8>
+int launch_skinny(int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits, int64_t ldo,
+                  int32_t* status, cudaStream_t stream, const float* sx, const float* sw) {
+  static int smem_set[kMaxDevices] = {};
+  auto kern = gemm_skinny_kernel<EPI, FP8>;
+  if (!raise_smem_limit(kern, static_cast<int>(kSkinnySmem - 2048), smem_set)) return OJB_ERR_LAUNCH;      // 2 KB: the static part
+  SkinnyArgs g{};
+  g.M = static_cast<int>(M);
+  g.N = static_cast<int>(N);
+  g.BN = bn;
+  g.x_rows = static_cast<int>(ceil_div(M, 8) * 8);
+  g.splits = splits;
+  g.kb_total = static_cast<int>(ceil_div(K, FP8 ? 128 : kBK));
+  g.kb_per_split = static_cast<int>(ceil_div(g.kb_total, splits));
+  if (static_cast<int64_t>(splits - 1) * g.kb_per_split >= g.kb_total) return OJB_ERR_ARG;      // empty K range
+  // k-blocks per stage: as many as leave at least six stages, up to four
+  const uint32_t kb_bytes = static_cast<uint32_t>(g.x_rows + bn) * 128;
+  const uint32_t budget = static_cast<uint32_t>(kSkinnySmem - 2048 - 1024);
+  g.nk = 4;
+  while (g.nk > 1 && (g.nk * kb_bytes * 6 > budget || g.nk > g.kb_per_split)) --g.nk;
+  g.stage_bytes = g.nk * kb_bytes;
+  // the A operand of the last k-block may run on behind the last stage
+  const uint32_t reach = (g.nk - 1) * static_cast<uint32_t>(g.x_rows) * 128 + kBM * 128u;
+  const uint32_t over = reach > g.stage_bytes ? reach - g.stage_bytes : 0u;
+  g.stages = static_cast<int>((budget - over) / g.stage_bytes);
+  if (g.stages > kSkinnyMaxStages) g.stages = kSkinnyMaxStages;
+  g.tmem_cols = 32;
+  while (static_cast<int>(g.tmem_cols) < bn) g.tmem_cols *= 2;
+  g.out = out;
+  g.ldo = ldo;
+  g.split_stride = EPI == kEpiPartialF32 ? M * N : 0;
+  g.status = status;
+  g.wait_ms = gemm_wait_limit_ms();
+  g.drop_copy = gemm_drop_copy();
+  g.sx = sx;
+  g.sw = sw;
+  CUtensorMap map_x, map_w;
+  int rc = make_kblock_map(&map_x, x, FP8 ? 1 : 2, M, K, g.x_rows, g.nk);
+  if (rc == OJB_OK) rc = make_kblock_map(&map_w, w, FP8 ? 1 : 2, N, K, bn, g.nk);
+  if (rc != OJB_OK) return rc;
+  const size_t smem = 1024 + static_cast<size_t>(g.stages) * g.stage_bytes + over;
+  launch_kernel(kern, dim3(static_cast<unsigned>(ceil_div(N, bn) * splits)), dim3(kSkinnyThreads), smem, stream, map_x, map_w, g);
+  return launch_status(cudaGetLastError());
+}
+
+}  // namespace
+
+// bn = 0: the narrowest multiple of 16 (at most 128) with which the tiles times the K ranges fill the SMs at most once
+int gemm_skinny_launch(int epi, int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
+                       int64_t ldo, int32_t* status, cudaStream_t stream, const float* sx, const float* sw) {
+  if (M > kSkinnyMaxRows || K % (sx != nullptr ? 128 : kBK) != 0 || (epi != kEpiBf16 && epi != kEpiPartialF32)) return OJB_ERR_LIMIT;
+  if (bn == 0) bn = skinny_bn(N, splits);
+  if (bn < 16 || bn > 128 || bn % 16) return OJB_ERR_ARG;
+  if (sx != nullptr)
+    return epi == kEpiBf16 ? launch_skinny<kEpiBf16, true>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw)
+                           : launch_skinny<kEpiPartialF32, true>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw);
+  return epi == kEpiBf16 ? launch_skinny<kEpiBf16, false>(bn, x, w, out, M, N, K, splits, ldo, status, stream, nullptr, nullptr)
+                         : launch_skinny<kEpiPartialF32, false>(bn, x, w, out, M, N, K, splits, ldo, status, stream, nullptr, nullptr);
+}
+
+}  // namespace ojb

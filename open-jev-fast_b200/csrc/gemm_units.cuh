@@ -232,6 +232,14 @@ class ModelCache {
   Slot slots_[kSlots] = {};
 };
 
+// The few-row kernel (gemm_skinny.cu): what it takes, and the rows of its w tile.
+inline bool skinny_serves(int64_t M, int64_t K) { return M <= 128 && K % 64 == 0; }
+inline int skinny_bn(int64_t N, int splits) {
+  const int64_t per = 148 / splits > 0 ? 148 / splits : 1;
+  const int64_t bn = ceil_div(ceil_div(N, per), 16) * 16;
+  return static_cast<int>(bn < 128 ? bn : 128);
+}
+
 // Width of the w tile of the block units: the multiple of 16 with the smallest modelled time, wider tiles preferred.
 inline int choose_bn(int64_t N, int n_xblk, int tail_box, int n_xchunk, bool has_tail, int splits, int kb_total, int workers,
                      int epi) {

@@ -229,9 +229,10 @@ class FastQwen35(torch.nn.Module):
             return out
 
         kernels = [1, 3] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
+        few = [11] if M <= 32 else []
         for (N, Kd), layers in groups("w_in").items():
             x = rnd(M, Kd)
-            res = race({i: (lambda d, i=i: LT.lt_matmul(x, d.w_in, i)) for i in kernels + [2]}, layers)
+            res = race({i: (lambda d, i=i: LT.lt_matmul(x, d.w_in, i)) for i in kernels + [2] + few}, layers)
             best = min(res, key=res.get)
             self._plan[("mm", M, N, Kd)] = best
             if report is not None:
@@ -251,7 +252,7 @@ class FastQwen35(torch.nn.Module):
                 for S in (1, 2, 3, 4, 6, 8):
                     if (S - 1) * -(-kb // S) >= kb:
                         continue
-                    for i in kernels:
+                    for i in kernels + few:
                         cands[(i, S)] = lambda d, i=i, S=S: K.resnorm_f32(h, None, None, LT.gemm_splitk(y, getattr(d, attr), S, i),
                                                                           w1, None, self.eps)
                 res = race(cands, layers)

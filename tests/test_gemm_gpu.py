@@ -257,3 +257,48 @@ def test_x_larger_than_l2_runs_in_bands(M):
     gg, uu = ref[:, :I], ref[:, I:]
     want = torch.nn.functional.silu(gg) * uu
     assert (out.float() - want).abs().max().item() <= want.abs().max().item() * 2 ** -7 + 2e-3
+
+
+@pytest.mark.parametrize("M", [1, 2, 8, 9, 31, 32, 33, 100, 128])
+@pytest.mark.parametrize("N,K", [(24, 64), (264, 320), (100, 192), (2048, 1280), (4100, 448)])
+def test_few_row_kernel(M, N, K):
+    """The few-row kernel at every edge of its tiles: rows that are no multiple of 8, w tiles past the last output, outputs that are
+    no multiple of 8 (element-wise stores), K ranges that are no multiple of a stage. fp32 sums of K products: K * 2^-24 of
+    sum |x w|; the bf16 output half an ulp, 2^-8, beside it."""
+    from ojb200 import _lib
+    from ojb200._lib import call, i32, i64, ptr, stream_ptr
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * K * 2.0 ** -24
+    st = _lib.status_word(x.device)
+    for v in (1024, 1040, 1088, 1152):
+        out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        call("ojb_gemm_bf16", ptr(x), ptr(w), ptr(out), i64(M), i64(N), i64(K), i32(v), ptr(st), stream_ptr())
+        assert bool(((out.double() - ref).abs() <= bound + ref.abs() * 2.0 ** -8).all())
+        for S in (1, 2, 3):
+            per = -(-(K // 64) // S)
+            if (S - 1) * per >= K // 64:
+                continue
+            parts = torch.full((S, M, N), float("nan"), device="cuda")
+            call("ojb_gemm_bf16_splitk", ptr(x), ptr(w), ptr(parts), i64(M), i64(N), i64(K), i32(S), i32(v), ptr(st), stream_ptr())
+            assert bool(((parts.double().sum(0) - ref).abs() <= bound).all())
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 24, 128), (7, 264, 384), (32, 2048, 1280), (12, 1000, 640)])
+def test_few_row_kernel_e4m3(M, N, K):
+    """Its 8-bit form against the same products in 64 bits (e4m3 products are exact in fp32)."""
+    from ojb200 import lt_ext as LT, _lib
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    wq, sw = LT.quantize_weight_e4m3(torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16))
+    xq, sx = LT.quantize_rows_e4m3(x)
+    xf, wf = (t.view(torch.float8_e4m3fn).double() * s.double()[:, None] for t, s in ((xq, sx), (wq, sw)))
+    ref, bound = xf @ wf.t(), (xf.abs() @ wf.abs().t()) * (K + 4) * 2.0 ** -24
+    assert bool(((LT.gemm_e4m3(xq, sx, wq, sw, 0).double() - ref).abs() <= bound + ref.abs() * 2.0 ** -8).all())
+    for S in (1, 2, 3):
+        if (S - 1) * -(-(K // 128) // S) < K // 128:
+            assert bool(((LT.gemm_e4m3(xq, sx, wq, sw, 2, S).double().sum(0) - ref).abs() <= bound).all())
+    _lib.check_status()
