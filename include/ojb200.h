@@ -89,8 +89,8 @@ int64_t ojb_gemm_unit_order(int32_t n_xblk, int32_t tail_rows, int32_t n_xchunk,
                             int32_t kb_total, int32_t band_xblk, int32_t* out, int64_t cap);
 
 /* Host-side plan (no GPU work): which kernel variant and how many K ranges the library's cost model picks for a shape.
- * kind = 0 bf16 output, 1 SwiGLU-fused, 2 fp32 split-K partials (the only kind that may use more than one range, up to
- * max_splits). *microseconds (optional) receives the modelled time. Takes the place of the algorithm search of
+ * kind = 0 bf16 output, 1 SwiGLU-fused, 2 fp32 split-K partials, 3 those of an 8-bit product with K counted in pairs of
+ * elements (the kinds that may use more than one range, up to max_splits). *microseconds (optional) receives the modelled time. Takes the place of the algorithm search of
  * src/lt.cpp:93 (lt2_search), which times cuBLASLt candidates on the device. */
 int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_splits, int32_t* variant, int32_t* splits,
                   float* microseconds);
@@ -137,6 +137,11 @@ int ojb_add_rmsnorm_sk(const void* x, const float* parts, int splits, const floa
  * hn = bf16(h * rsqrt(mean(h^2) + eps) * w1), zero where rowmask[n] == 0 (rowmask may be null). H % 8 == 0, H <= 8192. */
 int ojb_resnorm_f32(float* h, const void* x_init, const void* delta, const float* parts, int splits, const float* w1,
                     const int32_t* rowmask, void* hn_out, int64_t rows, int64_t H, float eps, ojb_stream_t stream);
+
+/* The same with the normed row handed on as e4m3 operands of the 8-bit GEMM, q [rows, H] bytes and scale fp32 [rows], instead of
+ * bf16: what ojb_quantize_rows_e4m3 makes of that bf16 row, bit for bit. */
+int ojb_resnorm_f32_e4m3(float* h, const void* x_init, const float* parts, int splits, const float* w1, const int32_t* rowmask,
+                         void* q, float* scale, int64_t rows, int64_t H, float eps, ojb_stream_t stream);
 
 /* src/kernels.cu:1288,1296 act_tables. silu_tab[65536] bf16 and sig_tab[65536] fp32, indexed by the bf16 bit pattern:
  * silu_tab[b] = bf16(x / (1 + expf(-x))), sig_tab[b] = 1 / (1 + expf(-x)). */
@@ -209,10 +214,16 @@ int ojb_gtree_fill(const int64_t* tokens, const int64_t* seq_off, const int32_t*
  * l2norm = 0 leaves q and k un-normalised (src/kernels.cu:96 linattn_prep and linattn_prep2 with do_l2 = false, whose callers
  * let the attention kernel normalise); every other prep variant of the reference normalises. The same entry point serves
  * the reference's older layouts (per-sequence [B, T], single-level tree, src-mapped slots): they differ only in `hist` and in
- * the slot tables, which the Python layer derives. */
+ * the slot tables, which the Python layer derives.  */
 int ojb_gdn_prep(const void* proj, const int32_t* hist, const int32_t* rep_ptr, const int32_t* rep_pos, int64_t n_slots,
                  const void* convw, const void* A_log, const void* dt_bias, void* q, void* k, void* v, float* g,
                  void* beta, int64_t N, int64_t KD, int64_t VD, int64_t HV, int64_t HK, int32_t l2norm, ojb_stream_t stream);
+/* The same; ieee != 0 (packed rows only): sigmoids with expf and an IEEE division instead of the special-function unit's exp2 and
+ * reciprocal, a few units of 2^-24 apart before the rounding to bf16. */
+int ojb_gdn_prep_v(const void* proj, const int32_t* hist, const int32_t* rep_ptr, const int32_t* rep_pos, int64_t n_slots,
+                   const void* convw, const void* A_log, const void* dt_bias, void* q, void* k, void* v, float* g,
+                   void* beta, int64_t N, int64_t KD, int64_t VD, int64_t HV, int64_t HK, int32_t l2norm, int32_t ieee,
+                   ojb_stream_t stream);
 
 /* Bytes of scratch that ojb_gdn_chunked needs for n_chunks chunk-table entries and HV value heads. */
 int64_t ojb_gdn_scratch_bytes(int64_t n_chunks, int64_t HV);
@@ -296,6 +307,9 @@ int ojb_gdn_set_trace(uint64_t* records);
  * rstd = 1/sqrt(mean(x^2) + eps) over the 128 dims. x bf16 [*, HV, 128]; proj bf16 [N, P]; w bf16 [128]. */
 int ojb_gated_rmsnorm(const void* x, const int32_t* inv, const void* proj, const void* w, void* out, int64_t N,
                       int64_t HV, int64_t HD, int64_t zoff, int64_t P, float eps, ojb_stream_t stream);
+/* The same; ieee != 0: sigmoids as in ojb_gdn_prep_v (16-byte aligned operands, zoff and P multiples of 8). */
+int ojb_gated_rmsnorm_v(const void* x, const int32_t* inv, const void* proj, const void* w, void* out, int64_t N,
+                        int64_t HV, int64_t HD, int64_t zoff, int64_t P, float eps, int32_t ieee, ojb_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------------------------
  * Tree attention — replaces src/kernels.cu:4287-4458 fattn_tree (and, above 384 rows, the reference's

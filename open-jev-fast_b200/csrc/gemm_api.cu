@@ -32,12 +32,12 @@ bool variant_ok(int v) {
 
 // Modelled SM clocks of the 128-row tile kernel: per k-block a CTA fills (128 + BN) rows and its MMAs read them once,
 // 128 bytes per clock; the epilogue overlaps the next tile.
-double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, int sms, int epi) {
+double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, int sms, bool f32) {
   const int64_t units = ceil_div(M, 128) * ceil_div(N, bn) * splits;
   const int64_t grid = units < sms ? units : sms;
   const int per = static_cast<int>(ceil_div(kb_total, splits));
   const double kb = bn == 256 ? 900.0 : 600.0;   // fitted to back-to-back runs against the power cap (133 us at 288 rows, 206 us at 544 for gate/up)
-  return static_cast<double>(ceil_div(units, grid)) * (per * kb + (epi == kEpiPartialF32 ? 33.0 * bn : 1500.0)) + 9000.0;
+  return static_cast<double>(ceil_div(units, grid)) * (per * kb + (f32 ? 33.0 * bn : 1500.0)) + 9000.0;
 }
 
 // The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (wait, four MMAs, its share of a commit) in less than 280
@@ -59,15 +59,18 @@ struct Plan {
 
 // Cheapest kernel for this shape and number of K ranges according to the cost models (gemm_units.cuh), never below the
 // time HBM needs for the weight.
-Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
+// eight_bit: the ranges of K of an 8-bit product. They regroup its sums, and on e4m3 operands a regrouped sum moves the result of
+// a deep model by percents, so that choice stays on the model it was first made with.
+Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eight_bit = false) {
   const int sms = 148;
   const int kb_total = static_cast<int>(ceil_div(K, 64));
   Plan best{3, 1e30};
+  const bool f32 = epi == kEpiPartialF32 && !eight_bit;
   auto consider = [&](int variant, double clocks) {
     if (clocks < best.clocks) best = Plan{variant, clocks};
   };
-  if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, epi));
-  if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, epi));
+  if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, f32));
+  if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, f32));
   {  // block256: full blocks + swapped tail
     int n_xblk = static_cast<int>(M / 256), r = static_cast<int>(M % 256);
     if (r > 128) { n_xblk += 1; r = 0; }
@@ -82,7 +85,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
     const int tail_box = static_cast<int>(ceil_div(ceil_div(M, n_xchunk), 16) * 16);
     consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, epi));
   }
-  if (M <= kSkinnyRows && epi != kEpiSwiglu && skinny_serves(M, K)) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
+  if (M <= kSkinnyRows && epi != kEpiSwiglu && skinny_serves(M, K) && !eight_bit) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz
   if (best.clocks < hbm) best.clocks = hbm;
   return best;
@@ -170,7 +173,7 @@ extern "C" int ojb_gemm_set_probe(int32_t mma_repeat, int32_t knob) {
 
 extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_splits, int32_t* variant, int32_t* splits,
                              float* microseconds) {
-  OJB_REQUIRE(M > 0 && N > 0 && K > 0 && kind >= 0 && kind <= 2 && max_splits >= 1 && max_splits <= 16 && variant && splits);
+  OJB_REQUIRE(M > 0 && N > 0 && K > 0 && kind >= 0 && kind <= 3 && max_splits >= 1 && max_splits <= 16 && variant && splits);
   struct Ranges {
     Plan plan;
     int splits;
@@ -179,14 +182,15 @@ extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int3
   const int64_t key[5] = {M, N, K, kind, max_splits};
   const Ranges r = cache.get(key, [&] {
     const int kb_total = static_cast<int>(ceil_div(K, 64));
+    const bool eight_bit = kind == 3, parts = kind >= 2;
     Plan best{0, 1e30};
     int best_s = 1;
-    for (int s = 1; s <= (kind == kEpiPartialF32 ? max_splits : 1); ++s) {
+    for (int s = 1; s <= (parts ? max_splits : 1); ++s) {
       const int per = static_cast<int>(ceil_div(kb_total, s));
       if (static_cast<int64_t>(s - 1) * per >= kb_total) continue;
-      Plan p = model_kernel(kind, M, N, K, s);
+      Plan p = model_kernel(eight_bit ? kEpiPartialF32 : kind, M, N, K, s, eight_bit);
       // the kernel that sums the partial planes reads S * M * N floats (mostly from L2)
-      if (kind == kEpiPartialF32) p.clocks += (s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
+      if (parts) p.clocks += (s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
       if (p.clocks < best.clocks * 0.97) { best = p; best_s = s; }
     }
     return Ranges{best, best_s};

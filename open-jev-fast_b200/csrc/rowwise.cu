@@ -32,6 +32,15 @@ __device__ __forceinline__ float block_sum_256(float v, float* red) {
   return t;  // every warp reduces the same 8 partials in the same order -> identical value in all threads
 }
 
+// The same for any number of whole warps (red: 32 floats).
+__device__ __forceinline__ float block_sum(float v, float* red) {
+  v = warp_sum(v);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) red[w] = v;
+  __syncthreads();
+  return warp_sum(lane < static_cast<int>(blockDim.x >> 5) ? red[lane] : 0.f);
+}
+
 // One CTA per row. SPLITS == 0: delta is an optional bf16 row; SPLITS > 0: delta = bf16(sum of SPLITS fp32 partial rows).
 template <int SPLITS>
 __global__ void __launch_bounds__(kRowThreads)
@@ -94,23 +103,52 @@ add_rmsnorm_kernel(const bf16_t* __restrict__ x, const bf16_t* __restrict__ delt
   }
 }
 
+// e4m3 scale of a row from the largest magnitude that each thread of its block of kRowThreads has seen: max|x| / 448, 1 for an
+// all-zero row. red: one float per warp.
+__device__ __forceinline__ float e4m3_scale(float amax, float* red, float& inv) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red[0];
+#pragma unroll
+  for (int w = 1; w < kRowThreads / 32; ++w) amax = fmaxf(amax, red[w]);
+  const float sc = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
+  inv = 1.0f / sc;
+  return sc;
+}
+// Eight values times inv, rounded to e4m3 (saturating).
+__device__ __forceinline__ uint2 e4m3x8(const float (&f)[8], float inv) {
+  uint32_t out[2];
+#pragma unroll
+  for (int e = 0; e < 8; e += 4) {
+    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(f[e] * inv, f[e + 1] * inv), __NV_SATFINITE, __NV_E4M3);
+    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(f[e + 2] * inv, f[e + 3] * inv), __NV_SATFINITE, __NV_E4M3);
+    out[e >> 2] = lo | (hi << 16);
+  }
+  return make_uint2(out[0], out[1]);
+}
+
 // Residual stream kept in fp32. One CTA per row: h = x_init (bf16, first norm of a forward) or h + delta, where delta is the
 // sum of SPLITS fp32 partial rows (SPLITS > 0) or one bf16 row or nothing; the sum is added in fp32 and h is never rounded.
 // hn = bf16(h * rstd * w1): the only rounding is the one the consuming GEMM needs for its operand.
-template <int SPLITS>
-__global__ void __launch_bounds__(kRowThreads)
+// THREADS = 256 with four 16-byte vectors to a thread, or, for few rows, 1024 with one: one round of loads per row instead of three.
+template <int SPLITS, int THREADS, bool E4M3 = false>
+__global__ void __launch_bounds__(THREADS)
 resnorm_f32_kernel(float* __restrict__ h, const bf16_t* __restrict__ x_init, const bf16_t* __restrict__ delta,
                    const float* __restrict__ parts, int64_t part_stride, const float* __restrict__ w1,
-                   const int32_t* __restrict__ rowmask, bf16_t* __restrict__ hn_out, int H, float eps) {
+                   const int32_t* __restrict__ rowmask, bf16_t* __restrict__ hn_out, int H, float eps,
+                   uint8_t* __restrict__ q_out = nullptr, float* __restrict__ q_scale = nullptr) {
   pdl_begin();
-  __shared__ float red[kRowThreads / 32];
+  constexpr int kVecs = kRowThreads * kRowVecs / THREADS;
+  __shared__ float red[32];
   const int64_t row = blockIdx.x;
   const int nvec = H >> 3;
-  float v[kRowVecs][8];
+  float v[kVecs][8];
   float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < kRowVecs; ++i) {
-    const int vi = threadIdx.x + i * kRowThreads;
+  for (int i = 0; i < kVecs; ++i) {
+    const int vi = threadIdx.x + i * THREADS;
     if (vi < nvec) {
       const int64_t off = row * H + static_cast<int64_t>(vi) * 8;
       if (x_init != nullptr) {
@@ -147,12 +185,13 @@ resnorm_f32_kernel(float* __restrict__ h, const bf16_t* __restrict__ x_init, con
       for (int e = 0; e < 8; ++e) ss += v[i][e] * v[i][e];
     }
   }
-  ss = block_sum_256(ss, red);
+  ss = block_sum(ss, red);
   const float rstd = rsqrtf(ss / static_cast<float>(H) + eps);
+  float amax = 0.f;
   const bool keep = rowmask ? (rowmask[row] != 0) : true;
 #pragma unroll
-  for (int i = 0; i < kRowVecs; ++i) {
-    const int vi = threadIdx.x + i * kRowThreads;
+  for (int i = 0; i < kVecs; ++i) {
+    const int vi = threadIdx.x + i * THREADS;
     if (vi < nvec) {
       const int col = vi * 8;
       const float4 wa = __ldg(reinterpret_cast<const float4*>(w1 + col));
@@ -161,7 +200,25 @@ resnorm_f32_kernel(float* __restrict__ h, const bf16_t* __restrict__ x_init, con
       float o[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) o[e] = keep ? (v[i][e] * rstd) * w[e] : 0.f;
-      *reinterpret_cast<uint4*>(hn_out + row * H + col) = pack8(o);
+      const uint4 packed = pack8(o);
+      if constexpr (E4M3) {
+        unpack8(packed, v[i]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(v[i][e]));
+      } else {
+        *reinterpret_cast<uint4*>(hn_out + row * H + col) = packed;
+      }
+    }
+  }
+  if constexpr (E4M3) {      // the bf16 row, quantised as quantize_rows_e4m3_kernel does it, without its way through memory
+    __syncthreads();         // (red is read by every warp of block_sum)
+    float inv;
+    const float sc = e4m3_scale(amax, red, inv);
+    if (threadIdx.x == 0) q_scale[row] = sc;
+#pragma unroll
+    for (int i = 0; i < kVecs; ++i) {
+      const int vi = threadIdx.x + i * THREADS;
+      if (vi < nvec) *reinterpret_cast<uint2*>(q_out + row * H + vi * 8) = e4m3x8(v[i], inv);
     }
   }
 }
@@ -420,8 +477,8 @@ gather_rows_kernel(const int64_t* __restrict__ rows, const uint4* __restrict__ a
   for (int c = threadIdx.x; c < b_vecs; c += blockDim.x) b_out[i * b_vecs + c] = b[n * b_vecs + c];
 }
 
-// Per-row e4m3 quantisation for the 8-bit GEMM: scale[m] = max|x[m,:]| / 448 (1 for an all-zero row), q = x / scale rounded
-// to e4m3 (saturating). One CTA per row, two passes over the row (the second one hits L1 / L2).
+// Per-row e4m3 quantisation for the 8-bit GEMM (e4m3_scale, e4m3x8). One CTA per row, two passes over the row (the second one hits
+// L1 / L2).
 __global__ void __launch_bounds__(kRowThreads)
 quantize_rows_e4m3_kernel(const bf16_t* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int K) {
   pdl_begin();
@@ -430,37 +487,19 @@ quantize_rows_e4m3_kernel(const bf16_t* __restrict__ x, uint8_t* __restrict__ q,
   const bf16_t* xr = x + row * K;
   float amax = 0.f;
   for (int i = threadIdx.x * 8; i < K; i += kRowThreads * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(xr + i), f);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __bfloat1622float2(h[e]);
-      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
+    for (int e = 0; e < 8; ++e) amax = fmaxf(amax, fabsf(f[e]));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  amax = red[0];
-#pragma unroll
-  for (int w = 1; w < kRowThreads / 32; ++w) amax = fmaxf(amax, red[w]);
-  const float sc = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
-  const float inv = 1.0f / sc;
+  float inv;
+  const float sc = e4m3_scale(amax, red, inv);
   if (threadIdx.x == 0) scale[row] = sc;
   uint8_t* qr = q + row * K;
   for (int i = threadIdx.x * 8; i < K; i += kRowThreads * 8) {
-    const uint4 v = *reinterpret_cast<const uint4*>(xr + i);
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-    uint32_t out[2];
-#pragma unroll
-    for (int e = 0; e < 4; e += 2) {
-      const float2 a = __bfloat1622float2(h[e]), b = __bfloat1622float2(h[e + 1]);
-      const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a.x * inv, a.y * inv), __NV_SATFINITE, __NV_E4M3);
-      const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(b.x * inv, b.y * inv), __NV_SATFINITE, __NV_E4M3);
-      out[e >> 1] = lo | (hi << 16);
-    }
-    *reinterpret_cast<uint2*>(qr + i) = make_uint2(out[0], out[1]);
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(xr + i), f);
+    *reinterpret_cast<uint2*>(qr + i) = e4m3x8(f, inv);
   }
 }
 
@@ -533,17 +572,47 @@ extern "C" int ojb_resnorm_f32(float* h, const void* x_init, const void* delta, 
   if (H > kRowThreads * kRowVecs * 8) return OJB_ERR_LIMIT;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t ps = rows * H;
-#define OJB_RN(S)                                                                                                      \
-  case S:                                                                                                              \
-    launch_kernel(resnorm_f32_kernel<S>, dim3(static_cast<unsigned>(rows)), dim3(kRowThreads), 0, st, h,               \
-                  static_cast<const bf16_t*>(x_init), static_cast<const bf16_t*>(delta), parts, ps, w1, rowmask,        \
-                  static_cast<bf16_t*>(hn_out), static_cast<int>(H), eps);                                             \
+  // measured (us, one / six K ranges): 32 rows 3.7 / 5.1 -> 3.1 / 3.9, 288 rows 4.6 / 7.4 -> 4.2 / 7.1, 544 rows 6.9 / 11.5 against
+  // 7.8 / 13.0: with two wide rows to an SM a second wave begins
+  const bool wide = rows <= 296;
+#define OJB_RN_T(S, T, THREADS)                                                                                          \
+  launch_kernel(resnorm_f32_kernel<S, T>, dim3(static_cast<unsigned>(rows)), dim3(THREADS), 0, st, h,                    \
+                static_cast<const bf16_t*>(x_init), static_cast<const bf16_t*>(delta), parts, ps, w1, rowmask,           \
+                static_cast<bf16_t*>(hn_out), static_cast<int>(H), eps, static_cast<uint8_t*>(nullptr),                  \
+                static_cast<float*>(nullptr))
+#define OJB_RN(S)                                                                                                       \
+  case S:                                                                                                               \
+    if (wide) OJB_RN_T(S, 1024, static_cast<unsigned>(ceil_div(H / 8, 32) * 32));                                       \
+    else OJB_RN_T(S, kRowThreads, kRowThreads);                                                                         \
     break;
   switch (splits) {
     OJB_RN(0) OJB_RN(1) OJB_RN(2) OJB_RN(3) OJB_RN(4) OJB_RN(5) OJB_RN(6) OJB_RN(7) OJB_RN(8)
     OJB_RN(9) OJB_RN(10) OJB_RN(11) OJB_RN(12) OJB_RN(13) OJB_RN(14) OJB_RN(15) OJB_RN(16)
   }
 #undef OJB_RN
+#undef OJB_RN_T
+  return launch_status(cudaGetLastError());
+}
+
+extern "C" int ojb_resnorm_f32_e4m3(float* h, const void* x_init, const float* parts, int splits, const float* w1,
+                                    const int32_t* rowmask, void* q, float* scale, int64_t rows, int64_t H, float eps,
+                                    ojb_stream_t stream) {
+  if (rows == 0) return OJB_OK;
+  OJB_REQUIRE(h && w1 && q && scale && rows > 0 && H > 0 && H % 8 == 0 && splits >= 0 && splits <= 16);
+  OJB_REQUIRE((splits == 0) == (parts == nullptr) && !(x_init && parts));
+  if (H > kRowThreads * kRowVecs * 8) return OJB_ERR_LIMIT;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+#define OJB_RQ(S)                                                                                                       \
+  case S:                                                                                                               \
+    launch_kernel(resnorm_f32_kernel<S, kRowThreads, true>, dim3(static_cast<unsigned>(rows)), dim3(kRowThreads), 0, st, h, \
+                  static_cast<const bf16_t*>(x_init), static_cast<const bf16_t*>(nullptr), parts, rows * H, w1, rowmask, \
+                  static_cast<bf16_t*>(nullptr), static_cast<int>(H), eps, static_cast<uint8_t*>(q), scale);             \
+    break;
+  switch (splits) {
+    OJB_RQ(0) OJB_RQ(1) OJB_RQ(2) OJB_RQ(3) OJB_RQ(4) OJB_RQ(5) OJB_RQ(6) OJB_RQ(7) OJB_RQ(8)
+    OJB_RQ(9) OJB_RQ(10) OJB_RQ(11) OJB_RQ(12) OJB_RQ(13) OJB_RQ(14) OJB_RQ(15) OJB_RQ(16)
+  }
+#undef OJB_RQ
   return launch_status(cudaGetLastError());
 }
 
@@ -680,26 +749,27 @@ extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, const void* 
 // ------------------------------------------------------------------------------------------------------- scoring head
 namespace ojb {
 namespace {
-// one warp per (candidate, output): out[s, a] = bias[a] + sum_h float(hn[rows[s], h]) * W[a, h]
-__global__ void __launch_bounds__(256)
+// one block per (candidate, output): out[s, a] = bias[a] + sum_h float(hn[rows[s], h]) * W[a, h]. A handful of outputs of 30 KB of
+// reads each: what counts is one round of loads instead of twenty (one warp per output: 10-12 us).
+constexpr int kHeadThreads = 320;
+__global__ void __launch_bounds__(kHeadThreads)
 score_head_kernel(const bf16_t* __restrict__ hn, const int64_t* __restrict__ rows, const float* __restrict__ W,
-                  const float* __restrict__ bias, float* __restrict__ out, int S, int A, int H) {
+                  const float* __restrict__ bias, float* __restrict__ out, int A, int H) {
   pdl_begin();
-  const int wid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (wid >= S * A) return;
-  const int lane = threadIdx.x & 31;
-  const int s = wid / A, a = wid - s * A;
+  __shared__ float red[32];
+  const int s = blockIdx.x / A, a = blockIdx.x - s * A;
   const bf16_t* x = hn + (rows ? rows[s] : s) * static_cast<int64_t>(H);
   const float* w = W + static_cast<int64_t>(a) * H;
   float acc = 0.f;
-  for (int c = lane * 8; c < H; c += 256) {
+#pragma unroll 2
+  for (int c = threadIdx.x * 8; c < H; c += kHeadThreads * 8) {
     float f[8];
     unpack8(*reinterpret_cast<const uint4*>(x + c), f);
     const float4 w0 = *reinterpret_cast<const float4*>(w + c), w1 = *reinterpret_cast<const float4*>(w + c + 4);
     acc += f[0] * w0.x + f[1] * w0.y + f[2] * w0.z + f[3] * w0.w + f[4] * w1.x + f[5] * w1.y + f[6] * w1.z + f[7] * w1.w;
   }
-  acc = warp_sum(acc);
-  if (lane == 0) out[wid] = acc + (bias ? bias[a] : 0.f);
+  acc = block_sum(acc, red);
+  if (threadIdx.x == 0) out[blockIdx.x] = acc + (bias ? bias[a] : 0.f);
 }
 }  // namespace
 }  // namespace ojb
@@ -708,9 +778,9 @@ extern "C" int ojb_score_head(const void* hn, const int64_t* rows, const float* 
                               int64_t A, int64_t H, ojb_stream_t stream) {
   if (S == 0 || A == 0) return OJB_OK;
   OJB_REQUIRE(hn && W && out && S > 0 && A > 0 && H > 0 && H % 8 == 0);
-  const int64_t warps = S * A;
-  launch_kernel(ojb::score_head_kernel, dim3(static_cast<unsigned>(ojb::ceil_div(warps, 8))), dim3(256), 0, static_cast<cudaStream_t>(stream), 
-      static_cast<const ojb::bf16_t*>(hn), rows, W, bias, out, static_cast<int>(S), static_cast<int>(A), static_cast<int>(H));
+  OJB_REQUIRE(S * A < (int64_t{1} << 31));
+  launch_kernel(ojb::score_head_kernel, dim3(static_cast<unsigned>(S * A)), dim3(ojb::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
+      static_cast<const ojb::bf16_t*>(hn), rows, W, bias, out, static_cast<int>(A), static_cast<int>(H));
   return ojb::launch_status(cudaGetLastError());
 }
 

@@ -72,6 +72,20 @@ def resnorm_f32(h, x_init, delta, parts, w1, rowmask, eps):
     return hn
 
 
+def resnorm_f32_e4m3(h, x_init, parts, w1, rowmask, eps):
+    """resnorm_f32 with the normed rows as e4m3 operands: (bytes [N, H] uint8, scale fp32 [N]), bit for bit those that
+    quantize_rows_e4m3 makes of its bf16 result."""
+    _chk(h, x_init, parts, w1, rowmask)
+    N, H = h.shape
+    if h.dtype != torch.float32 or (parts is not None and (parts.dtype != torch.float32 or tuple(parts.shape[1:]) != (N, H))):
+        raise RuntimeError("resnorm_f32_e4m3: h must be fp32 [N, H] and parts fp32 [S, N, H]")
+    q = torch.empty(N, H, dtype=torch.uint8, device=h.device)
+    scale = torch.empty(N, dtype=torch.float32, device=h.device)
+    call("ojb_resnorm_f32_e4m3", ptr(h), ptr(x_init), ptr(parts), i32(0 if parts is None else parts.shape[0]), ptr(w1), ptr(rowmask),
+         ptr(q), ptr(scale), i64(N), i64(H), f32(eps), stream_ptr())
+    return q, scale
+
+
 def act_tables(like):
     """src/ext.py:23 — [silu_tab bf16[65536], sig_tab f32[65536]] on like's device."""
     silu_tab = torch.empty(65536, dtype=bf16, device=like.device)
@@ -197,7 +211,7 @@ def attn_operands(q_src, kv_src, qw1, kw1, cosb, sinb, HQ, HKV, eps, q_rows=None
 
 
 # ------------------------------------------------------------------------------------------------ Gated DeltaNet
-def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV, HK, HD, l2norm=True):
+def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV, HK, HD, l2norm=True, ieee=False):
     _chk(proj, hist, rep_ptr, rep_pos, convw, A_log, dt_bias)
     if HD != 128 or HK * HD != KD or HV * HD != VD or convw.shape[1] != 4:
         raise RuntimeError("linattn_prep: head dim must be 128 and the conv width 4")
@@ -214,9 +228,9 @@ def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV
     v = torch.empty(n_out, VD, dtype=bf16, device=dev)
     g = torch.empty(n_out, HV, dtype=torch.float32, device=dev)
     beta = torch.empty(n_out, HV, dtype=bf16, device=dev)
-    call("ojb_gdn_prep", ptr(proj), ptr(hist), ptr(rep_ptr), ptr(rep_pos), i64(0 if rep_pos is None else rep_pos.numel()),
+    call("ojb_gdn_prep_v", ptr(proj), ptr(hist), ptr(rep_ptr), ptr(rep_pos), i64(0 if rep_pos is None else rep_pos.numel()),
          ptr(convw), ptr(A_log), ptr(dt_bias), ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), i64(N), i64(KD), i64(VD),
-         i64(HV), i64(HK), i32(1 if l2norm else 0), stream_ptr())
+         i64(HV), i64(HK), i32(1 if l2norm else 0), i32(1 if ieee else 0), stream_ptr())
     return q, k, v, g, beta
 
 
@@ -224,10 +238,11 @@ def _expand(x, HK, HV, HD):
     return x.view(-1, HK, 1, HD).expand(-1, HK, HV // HK, HD).reshape(-1, HV * HD).contiguous()
 
 
-def linattn_prep_rows(proj, hist, convw, A_log, dt_bias, KD, VD, HV, HK, HD):
+def linattn_prep_rows(proj, hist, convw, A_log, dt_bias, KD, VD, HV, HK, HD, ieee=False):
     """One output row per packed row (no replication): [q [N,KD], k [N,KD], v [N,VD], g f32 [N,HV], beta [N,HV]].
-    Not in the reference; the tree-native Gated DeltaNet pass consumes this layout."""
-    return list(_prep(proj, hist, None, None, proj.shape[0], convw, A_log, dt_bias, KD, VD, HV, HK, HD))
+    Not in the reference; the tree-native Gated DeltaNet pass consumes this layout. ieee: sigmoids with expf and an IEEE
+    division (ojb_gdn_prep_v)."""
+    return list(_prep(proj, hist, None, None, proj.shape[0], convw, A_log, dt_bias, KD, VD, HV, HK, HD, ieee=ieee))
 
 
 def linattn_prep_dedup2(proj, hist, rep_ptr, rep_pos, L2, convw, A_log, dt_bias, KD, VD, HV, HK, HD, rep_qk):
@@ -539,18 +554,18 @@ def gated_rmsnorm_map(x, proj, w, HV, HD, zoff, eps, Lp, Ls):
     return _gated_norm(x, _hist_cache[key], proj, w, HV, HD, zoff, eps)
 
 
-def _gated_norm(x, inv, proj, w, HV, HD, zoff, eps):
+def _gated_norm(x, inv, proj, w, HV, HD, zoff, eps, ieee=False):
     _chk(x, inv, proj, w)
     N, P = proj.shape
     out = torch.empty(N, HV * HD, dtype=bf16, device=proj.device)
-    call("ojb_gated_rmsnorm", ptr(x), ptr(inv), ptr(proj), ptr(w), ptr(out), i64(N), i64(HV), i64(HD), i64(zoff), i64(P),
-         f32(eps), stream_ptr())
+    call("ojb_gated_rmsnorm_v", ptr(x), ptr(inv), ptr(proj), ptr(w), ptr(out), i64(N), i64(HV), i64(HD), i64(zoff), i64(P),
+         f32(eps), i32(1 if ieee else 0), stream_ptr())
     return out
 
 
-def gated_rmsnorm(x, proj, w, HV, HD, zoff, eps):
-    """src/ext.py:9 — x [N, HV, HD] in packed-row order."""
-    return _gated_norm(x, None, proj, w, HV, HD, zoff, eps)
+def gated_rmsnorm(x, proj, w, HV, HD, zoff, eps, ieee=False):
+    """src/ext.py:9 — x [N, HV, HD] in packed-row order. ieee as in linattn_prep_rows."""
+    return _gated_norm(x, None, proj, w, HV, HD, zoff, eps, ieee)
 
 
 def gated_rmsnorm_inv(x, inv, proj, w, HV, HD, zoff, eps):

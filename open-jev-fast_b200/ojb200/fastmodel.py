@@ -133,10 +133,10 @@ class FastQwen35(torch.nn.Module):
     # timing the candidates on this model's own weights, back to back over all layers (so under the power cap and with the
     # weights coming from HBM, as in the real forward).
     def _mm(self, x, w, lo=0, hi=None):
-        """out = x @ w[lo:hi]^T, bf16 (src/fastmodel.py:168 _mm)."""
+        """out = x @ w[lo:hi]^T, bf16 (src/fastmodel.py:168 _mm). With 8-bit projections x may come as (e4m3 bytes, row scales)."""
         q8 = self._q8.get(w.data_ptr()) if self.fp8 else None
         if q8 is not None:
-            xq, sx = LT.quantize_rows_e4m3(x)
+            xq, sx = x if isinstance(x, tuple) else LT.quantize_rows_e4m3(x)
             return LT.gemm_e4m3(xq, sx, q8[0][lo:hi], q8[1][lo:hi], 0)
         w = w[lo:hi]
         return LT.lt_matmul(x, w, self._force.get("mm", self._plan.get(("mm", x.shape[0], w.shape[0], w.shape[1]), 0)))
@@ -147,7 +147,14 @@ class FastQwen35(torch.nn.Module):
         N, Kd = W.shape
         return W.view(N, S, Kd // S).permute(1, 2, 0).contiguous()
 
-    def _res(self, h, y, w, S, w1, mask):
+    def _norm(self, h, x_init, parts, w1, mask, last=False):
+        """Residual add + RMSNorm; the operand of the next projection: bf16 rows, or e4m3 rows and their scales where the
+        projections are 8-bit (`last`: the final norm, bf16)."""
+        if self.fp8 and not last:
+            return K.resnorm_f32_e4m3(h, x_init, parts, w1, mask, self.eps)
+        return K.resnorm_f32(h, x_init, None, parts, w1, mask, self.eps)
+
+    def _res(self, h, y, w, S, w1, mask, last=False):
         """Output projection + residual + RMSNorm (src/fastmodel.py:196 _res): fp32 partial products over S ranges of K, then
         one kernel for partial sum + residual + norm. S = 0 lets the plan choose. The residual stream `h` is fp32 [N, H] and is
         updated in place: the partial sums are added in fp32 and the stream is never rounded (the reference rounds the sum
@@ -158,18 +165,18 @@ class FastQwen35(torch.nn.Module):
         q8 = self._q8.get(w.data_ptr()) if self.fp8 else None
         if q8 is not None:
             yq, sy = LT.quantize_rows_e4m3(y)
-            S8 = S if S > 0 else LT.plan_splitk(M, w.shape[0], Kd // 2)      # a 128-byte k-block holds twice the elements
-            return [h, K.resnorm_f32(h, None, None, LT.gemm_e4m3(yq, sy, q8[0], q8[1], 2, S8), w1, mask, self.eps)]
+            S8 = S if S > 0 else LT.plan_splitk(M, w.shape[0], Kd // 2, eight_bit=True)      # a 128-byte k-block holds twice the elements
+            return [h, self._norm(h, None, LT.gemm_e4m3(yq, sy, q8[0], q8[1], 2, S8), w1, mask, last)]
         if S == 0:
             idx, S = self._force.get("res", self._plan.get(("res", M, w.shape[0], Kd), (0, 0)))
             if S == 0:
                 S = LT.plan_splitk(M, w.shape[0], Kd)
-        return [h, K.resnorm_f32(h, None, None, LT.gemm_splitk(y, w, S, idx), w1, mask, self.eps)]
+        return [h, self._norm(h, None, LT.gemm_splitk(y, w, S, idx), w1, mask, last)]
 
     def _mlp_in(self, hn, d):
         if d.fused_mlp and self.fp8:
             q8 = self._q8[d.w_gu_blk.data_ptr()]
-            xq, sx = LT.quantize_rows_e4m3(hn)
+            xq, sx = hn if isinstance(hn, tuple) else LT.quantize_rows_e4m3(hn)
             return LT.gemm_e4m3(xq, sx, q8[0], q8[1], 1)
         if d.fused_mlp:
             return LT.gemm_swiglu(hn, d.w_gu_blk, self._force.get("gu", self._plan.get(("gu", hn.shape[0]) + tuple(d.w_gu_blk.shape), 0)))
@@ -291,7 +298,7 @@ class FastQwen35(torch.nn.Module):
                 K.gdn_chunked_proj(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD ** -0.5, lay.chunks,
                                    lay.steps, lay.walk_ptr, lay.n_walks, None, None, o)
                 return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
-            q, k, v, g, beta = K.linattn_prep_rows(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD)
+            q, k, v, g, beta = K.linattn_prep_rows(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD, self.fp8)
             if hasattr(lay, "lsteps") and TREE_LEVELS:
                 st = self._bufs.get(("gdn_states", lay.S, d.HV))
                 if st is None:
@@ -302,7 +309,7 @@ class FastQwen35(torch.nn.Module):
             else:
                 K.gdn_chunked(q.view(N, d.HK, d.HD), k.view(N, d.HK, d.HD), v.view(N, d.HV, d.HD), g, beta, d.HD ** -0.5,
                               lay.chunks, lay.steps, lay.walk_ptr, lay.n_walks, None, None, o)
-            return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
+            return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps, self.fp8)
         # the reference's route: every candidate path replicated, one sequence per candidate (src/fastmodel.py:420-454)
         S, L2 = lay.S, lay.L2
         q, k, v, g, beta = K.linattn_prep_dedup2(proj, lay.hist, lay.rep_ptr, lay.rep_pos, L2, d.convw, d.A_log, d.dt_bias,
@@ -346,11 +353,16 @@ class FastQwen35(torch.nn.Module):
         i = lay.lastidx
         return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and i.dtype == torch.int64 and i.is_contiguous()
 
-    def _mix_asked(self, d, h, hn, rows, lay, cos, sin, linear):
-        """Token mixer of the last layer for the asked rows: (their residual stream, their mixer output)."""
-        if not linear and self._attn_tc(d, lay, cos, hn.shape[0])[1]:
+    def _mix_asked(self, i, h, hn, rows, lay, cos, sin, linear):
+        """Token mixer of the last layer (i) for the asked rows: (their residual stream, their mixer output)."""
+        d = self.L[i]
+        if not linear and self._attn_tc(d, lay, cos, h.shape[0])[1]:
             nq = d.HQ * 2 * d.D
-            hq, h = K.gather_rows(rows, hn, h)
+            if self.fp8:
+                h = K.gather_rows(rows, h)
+                hq = self._norm(h, None, None, self.in_w1[i], None)
+            else:
+                hq, h = K.gather_rows(rows, hn, h)
             q_src, kv_src = self._mm(hq, d.w_in, 0, nq), self._mm(hn, d.w_in, nq)
             qt, kt, vt_t = K.attn_operands(q_src, kv_src, d.qw1, d.kw1, cos, sin, d.HQ, d.HKV, self.eps, rows)
             return h, K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale, rows)
@@ -375,12 +387,12 @@ class FastQwen35(torch.nn.Module):
         lin = [t == "linear_attention" for t in self.layer_types]
         rowmask = lay.rowmask
         h = torch.empty(x.shape, dtype=torch.float32, device=x.device)        # the residual stream, fp32 throughout
-        hn = K.resnorm_f32(h, x, None, None, self.in_w1[0], rowmask if lin[0] else None, self.eps)
+        hn = self._norm(h, x, None, self.in_w1[0], rowmask if lin[0] else None)
         nl = len(self.L)
         rows = None if return_all or not self._asked_rows_only(lay, x.shape[0]) else lay.lastidx
         for i, d in enumerate(self.L):
             if rows is not None and i == nl - 1:
-                h, y = self._mix_asked(d, h, hn, rows, lay, cos, sin, lin[i])
+                h, y = self._mix_asked(i, h, hn, rows, lay, cos, sin, lin[i])
             else:
                 proj = self._mm(hn, d.w_in)
                 y = self._linear_tree(d, proj, lay) if lin[i] else self._attn_tree(d, proj, lay, cos, sin)
@@ -388,7 +400,7 @@ class FastQwen35(torch.nn.Module):
             m = self._mlp_in(hn, d)
             last = i == nl - 1
             h, hn = self._res(h, m, d.w_down, d.sk_down, self.final_w1 if last else self.in_w1[i + 1],
-                              None if last or not lin[i + 1] else rowmask)
+                              None if last or not lin[i + 1] else rowmask, last)
         return hn, (lay.lastidx if rows is None else None)
 
     @torch.no_grad()

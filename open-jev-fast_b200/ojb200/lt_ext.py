@@ -78,15 +78,16 @@ def interleave_gate_up(w_gate, w_up, block=128):
 
 def gemm_plan(M, N, K, kind, max_splits=16):
     """(variant code, K ranges, modelled microseconds) that the library's cost model picks for a shape; kind = 0 bf16
-    output, 1 SwiGLU-fused, 2 fp32 split-K partials. Host arithmetic only."""
+    output, 1 SwiGLU-fused, 2 fp32 split-K partials, 3 those of an 8-bit product. Host arithmetic only."""
     v, s, us = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_float()
     call("ojb_gemm_plan", i64(M), i64(N), i64(K), i32(kind), i32(max_splits), ctypes.byref(v), ctypes.byref(s), ctypes.byref(us))
     return v.value, s.value, us.value
 
 
-def plan_splitk(M, N, K, sms=SM_COUNT):
-    """Number of K ranges for a projection whose output goes through the partial-sum reduction (residual + RMSNorm kernel)."""
-    return gemm_plan(M, N, K, 2)[1]
+def plan_splitk(M, N, K, sms=SM_COUNT, eight_bit=False):
+    """Number of K ranges for a projection whose output goes through the partial-sum reduction (residual + RMSNorm kernel);
+    eight_bit: of an e4m3 product, K counted in pairs of elements."""
+    return gemm_plan(M, N, K, 3 if eight_bit else 2)[1]
 
 
 def gemm_splitk(x, w, S, idx=0):

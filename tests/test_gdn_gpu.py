@@ -282,8 +282,8 @@ def test_prep_of_packed_rows_equals_the_scatter_form(N, l2):
 @pytest.mark.parametrize("N,HV", [(1, 1), (37, 4), (1023, 17), (2048, 16), (2501, 48)])
 @pytest.mark.parametrize("gather", [False, True])
 def test_gated_rmsnorm_wide_accesses_equal_the_narrow_ones(N, HV, gather):
-    """16-byte form (aligned columns) against the 8-byte form (the same gate four columns further right): sums of the same 128
-    squares in another order, so at most an ulp of the bf16 result, on few values."""
+    """16-byte form (aligned columns) against the 8-byte form (the same gate four columns further right): sums in the same order, the
+    same bits; with the IEEE sigmoid an ulp of bf16 on few values."""
     from ojb200 import ext as K
     gen = torch.Generator().manual_seed(N + HV)
     x = torch.randn(N + 5, HV, 128, generator=gen).to(bf16).cuda()
@@ -293,8 +293,10 @@ def test_gated_rmsnorm_wide_accesses_equal_the_narrow_ones(N, HV, gather):
     moved = torch.zeros(N, HV * 128 + 24, dtype=bf16, device="cuda")
     moved[:, 12:12 + HV * 128] = proj[:, 8:8 + HV * 128]
     src = x if gather else x[:N].contiguous()
-    a = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6).float()
-    b = K._gated_norm(src, inv, moved, w, HV, 128, 12, 1e-6).float()
+    a = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6)
+    assert torch.equal(a, K._gated_norm(src, inv, moved, w, HV, 128, 12, 1e-6))
+    b = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6, ieee=True)
+    a, b = a.float(), b.float()
     assert bool(((a - b).abs() <= b.abs() * 2 ** -7 + 1e-30).all())
     assert (a == b).float().mean().item() > 0.99
 
@@ -331,7 +333,8 @@ def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
     assert float(outs[0][0].float().abs().max()) > 0
 
 
-def test_silu_and_sigmoid_of_every_bf16_value():
+@pytest.mark.parametrize("ieee", [False, True])
+def test_silu_and_sigmoid_of_every_bf16_value(ieee):
     """The element-wise functions of the preparation on all 65 536 bf16 inputs (a convolution whose last tap is 1), against
     64 bits: the bf16 result is the correctly rounded one wherever the fp32 value before rounding, a few units of 2^-24 off, does
     not cross a rounding boundary — all but a handful. Infinities and not-a-numbers as x / (1 + e^-x) gives them."""
@@ -347,7 +350,7 @@ def test_silu_and_sigmoid_of_every_bf16_value():
     hist = torch.full((N + 1, 4), -1, dtype=torch.int32)
     hist[:N, 3] = torch.arange(N)
     one = torch.zeros(HV, dtype=bf16)
-    _, _, v, _, _ = K._prep(proj.cuda(), hist.cuda(), None, None, N, convw.cuda(), one.cuda(), one.cuda(), KD, VD, HV, HK, 128, False)
+    _, _, v, _, _ = K._prep(proj.cuda(), hist.cuda(), None, None, N, convw.cuda(), one.cuda(), one.cuda(), KD, VD, HV, HK, 128, False, ieee)
     got, x64 = v.cpu().flatten(), x.double().flatten()
     want = (x64 / (1.0 + torch.exp(-x64)))
     nan = torch.isnan(want)

@@ -161,3 +161,28 @@ def test_gather_rows(rows):
     idx = torch.randint(0, 50, (rows,), generator=torch.Generator().manual_seed(2)).cuda()
     ga, gb = K.gather_rows(idx, a, b)
     assert torch.equal(ga, a[idx]) and torch.equal(gb, b[idx]) and torch.equal(K.gather_rows(idx, b), b[idx])
+
+
+@pytest.mark.parametrize("rows", [1, 295, 296, 297, 400])          # one wide CTA per row up to 296 rows, a narrow one above
+@pytest.mark.parametrize("H,S", [(8, 0), (256, 1), (5120, 3), (8192, 6)])
+def test_resnorm_f32_and_its_e4m3_form(rows, H, S):
+    """Both row shapes against 64 bits (a bf16 ulp), and the e4m3 form against quantising the bf16 rows of the narrow shape: the same
+    bytes and scales."""
+    from ojb200 import ext as K, lt_ext as LT
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    h = torch.randn(rows, H, generator=g, device="cuda")
+    parts = torch.randn(S, rows, H, generator=g, device="cuda") if S else None
+    w1 = 1.0 + torch.randn(H, generator=g, device="cuda") * 0.1
+    mask = (torch.rand(rows, generator=g, device="cuda") > 0.2).int()
+    total = h.double() + (parts.double().sum(0) if S else 0.0)
+    want = total / torch.sqrt((total * total).mean(1, keepdim=True) + 1e-6) * w1.double() * mask[:, None]
+    h1, h2 = h.clone(), h.clone()
+    hn = K.resnorm_f32(h1, None, None, parts, w1, mask, 1e-6)
+    assert bool(((hn.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all())
+    q, scale = K.resnorm_f32_e4m3(h2, None, parts, w1, mask, 1e-6)
+    assert torch.equal(h1, h2)
+    n = max(1, -(-400 // rows))                                      # the same rows often enough for the narrow shape
+    tall = lambda t: None if t is None else t.repeat(*([1] * (t.dim() - 2)), n, 1)
+    hn = K.resnorm_f32(tall(h), None, None, tall(parts), w1, mask.repeat(n), 1e-6)[:rows].contiguous()
+    qw, sw = LT.quantize_rows_e4m3(hn)
+    assert torch.equal(q, qw) and torch.equal(scale, sw)
