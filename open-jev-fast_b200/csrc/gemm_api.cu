@@ -66,6 +66,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
   const int kb_total = static_cast<int>(ceil_div(K, 64));
   Plan best{3, 1e30};
   const bool f32 = epi == kEpiPartialF32 && !eight_bit;
+  const int model_epi = eight_bit ? kEpi8BitRanges : epi;
   auto consider = [&](int variant, double clocks) {
     if (clocks < best.clocks) best = Plan{variant, clocks};
   };
@@ -76,14 +77,14 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
     if (r > 128) { n_xblk += 1; r = 0; }
     if (n_xblk > 0) {
       const int tail_box = (r + 15) / 16 * 16;
-      const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, epi);
-      consider(3, block_kernel_clocks(N, bn, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, epi));
+      const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, model_epi);
+      consider(3, block_kernel_clocks(N, bn, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, model_epi));
     }
   }
   if (M <= 2048) {  // block256 with every row in swapped-operand units
     const int n_xchunk = static_cast<int>(ceil_div(M, 256));
     const int tail_box = static_cast<int>(ceil_div(ceil_div(M, n_xchunk), 16) * 16);
-    consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, epi));
+    consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, model_epi));
   }
   if (M <= kSkinnyRows && epi != kEpiSwiglu && skinny_serves(M, K) && !eight_bit) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz

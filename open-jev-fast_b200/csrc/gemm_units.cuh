@@ -123,6 +123,9 @@ __host__ __device__ __forceinline__ Unit decode_unit(const GemmArgs& g, int unit
 // and the operand reads of its MMAs), an MMA with M = 128 never takes less than 64 clocks, a swapped-operand unit keeps
 // too few bytes in flight to run faster than about 1200 clocks per k-block, and the epilogue of a block unit costs about 19
 // (bf16), 33 (fp32) or 40 (SwiGLU) clocks per accumulator column.
+// The model as the K ranges of 8-bit products are chosen by (see model_kernel): fp32 partials, every tile width alike.
+constexpr int kEpi8BitRanges = 3;
+
 struct UnitCost {
   double block_kb, block_epi, tail_kb, tail_epi;
 };
@@ -130,7 +133,11 @@ inline UnitCost unit_cost(int bn, int tail_box, int epi) {
   UnitCost c;
   const double smem = 512.0 + 3.0 * bn, mma = 4.0 * bn;
   c.block_kb = smem > mma ? smem : mma;
-  c.block_epi = 900.0 + bn * (epi == kEpiPartialF32 ? 33.0 : (epi == kEpiSwiglu ? 40.0 : 19.0));
+  // tiles of whole 128-byte pieces leave by bulk stores, others by the threads' own, three times as long (before the model knew,
+  // it took 208-wide tiles for fp32 results: [5120, 4096] at 4160 rows 184 us, with 224 149 us)
+  const bool bulk = epi == kEpi8BitRanges || bn % (epi == kEpiPartialF32 ? 32 : 64) == 0;
+  const bool f32 = epi == kEpiPartialF32 || epi == kEpi8BitRanges;
+  c.block_epi = 900.0 + bn * (f32 ? (bulk ? 33.0 : 115.0) : (epi == kEpiSwiglu ? 40.0 : (bulk ? 19.0 : 55.0)));
   const double tsm = 512.0 + 3.0 * tail_box;
   c.tail_kb = tsm > 1200.0 ? tsm : 1200.0;
   c.tail_epi = 3200.0 + 24.0 * tail_box;
