@@ -338,10 +338,12 @@ int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const voi
 
 /* The same for any rows of the tree as queries: query row n (of NQ) goes by row q_rows[n] of krange (q_rows null: by row n), and
  * its gate is read at gate + n * gate_ld + head * gate_hs (elements, multiples of 8), e.g. inside the in-projection output.
- * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0, any NQ. */
+ * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0, any NQ.
+ * one_pass = 1: 256 keys and more (scale > 0) go to a kernel that takes 128 operand rows and goes over the keys once, with a running
+ * maximum; 2: any number does; 0: always the two-pass kernel. */
 int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
                        const void* gate, int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ,
-                       int64_t HKV, float scale, int32_t* status, ojb_stream_t stream);
+                       int64_t HKV, float scale, int32_t one_pass, int32_t* status, ojb_stream_t stream);
 
 /* Its operands (ojb_fullattn_prep without the copies of the gate and of V in row order): q_src = NQ rows, q_ld elements apart,
  * of [q(256) | gate(256)] per query head; kv_src = N rows, kv_ld apart, of HKV k heads then HKV v heads. Query row n takes its

@@ -18,6 +18,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 // Bulk tensor store of one shared-memory tile (box of the map) to global memory; x = column, y = row, z = plane.
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(src), "r"(x),
@@ -176,6 +181,22 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int
   return r == CUDA_SUCCESS ? OJB_OK : OJB_ERR_ARG;
 }
 
+// A row-major matrix of `cols` elements (elt bytes each) to a row as [k-block][row][128 bytes]: box = nk k-blocks of box_rows rows,
+// 128-byte swizzle. cols * elt is a multiple of 128: the last k-block of the last row would otherwise reach past the matrix.
+int make_kblock_map(CUtensorMap* map, const void* base, int elt, int64_t rows, int64_t cols, int box_rows, int nk) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return OJB_ERR_DRIVER;
+  const cuuint64_t inner = 128 / elt;
+  cuuint64_t dims[3] = {inner, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols) / inner};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * elt, 128};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(inner), static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(nk)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, elt == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? OJB_OK : OJB_ERR_ARG;
+}
+
 // The same for a row-major matrix of bytes (e4m3 operands): a box is box_rows rows of 128 bytes = 128 elements of K.
 int make_map_u8(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int box_rows) {
   EncodeTiledFn fn = encode_fn();
@@ -239,6 +260,9 @@ void gemm_block256_set_trace(unsigned long long* buf, int cap);
 // e4m3 operands with one fp32 scale per row of x (sx) and per row of w (sw): out = (xq . wq^T) * sx[m] * sw[n]
 int gemm_block256_launch_e4m3(int epi, const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M,
                               int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
+int tree_attn_long_launch(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N, const void* gate,
+                          int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ, int64_t HKV, float scale,
+                          int32_t* status, cudaStream_t st);
 int gemm_skinny_launch(int epi, int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
                        int64_t ldo, int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr);
 int gemm_pair256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,

@@ -38,27 +38,6 @@ struct SkinnyArgs {
   const float* sw;
 };
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-               ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
-}
-
-// A row-major matrix of `cols` elements (elt bytes each) to a row as [k-block][row][128 bytes]: box = nk k-blocks of box_rows rows,
-// 128-byte swizzle. cols * elt is a multiple of 128: the last k-block of the last row would otherwise reach past the matrix.
-int make_kblock_map(CUtensorMap* map, const void* base, int elt, int64_t rows, int64_t cols, int box_rows, int nk) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return OJB_ERR_DRIVER;
-  const cuuint64_t inner = 128 / elt;
-  cuuint64_t dims[3] = {inner, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols) / inner};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * elt, 128};
-  cuuint32_t box[3] = {static_cast<cuuint32_t>(inner), static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(nk)};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = fn(map, elt == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
-                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? OJB_OK : OJB_ERR_ARG;
-}
-
 template <int EPI, bool FP8>
 __global__ void __launch_bounds__(kSkinnyThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, SkinnyArgs g) {

@@ -38,6 +38,10 @@ constexpr uint32_t kQBytes = kMaxG * kQRows * kD * 2;    // 4 k-blocks of [16 G 
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 0, kColS = 256;               // O: 256 columns; S: two buffers of 128 columns
 constexpr int kStagePitch = kD * 2 + 16;                 // bytes per row of the output staging tile
+// Keys from which tree_attn_long.cu is the faster one. Two-pass / one-pass, all rows as queries (us): 128 rows 11.3 / 12.9, 320 rows
+// 17.1 / 16.2, 544 rows 22.6 / 17.9, 1120 rows 53 / 34, 2592 rows 192 / 115, 16 512 rows 5283 / 2804; seven rows as queries: 128 keys
+// 9.8 / 9.5, 320 keys 15.7 / 12.7, 2592 keys 59 / 42.
+constexpr int64_t kOnePassKeys = 256;
 constexpr int kMaxBlocks = 2048;                         // 64-key blocks a CTA can list (131 072 keys)
 constexpr int kSub = 64;               // keys per visibility block
 constexpr int kKB = 128;               // keys per product (two blocks)
@@ -450,13 +454,16 @@ extern "C" int ojb_tree_attn_set_trace(uint64_t* records) {
 
 extern "C" int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
                                   const void* gate, int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ,
-                                  int64_t HKV, float scale, int32_t* status, ojb_stream_t stream) {
+                                  int64_t HKV, float scale, int32_t one_pass, int32_t* status, ojb_stream_t stream) {
   if (N == 0 || NQ == 0) return OJB_OK;
   OJB_REQUIRE(qt && kt && vt_t && gate && krange && y && N > 0 && N % 8 == 0 && NQ > 0);
   OJB_REQUIRE(HQ > 0 && HKV > 0 && HQ % HKV == 0 && HQ / HKV <= kMaxG);
   OJB_REQUIRE(gate_ld >= 0 && gate_hs >= 0 && gate_ld % 8 == 0 && gate_hs % 8 == 0 && gate_hs < (1 << 30));
   OJB_REQUIRE(aligned16(qt) && aligned16(kt) && aligned16(vt_t) && aligned16(gate) && aligned16(y));
   if ((N + kSub - 1) / kSub > kMaxBlocks || NQ > static_cast<int64_t>(kMaxBlocks) * kSub) return OJB_ERR_LIMIT;
+  if (scale > 0.f && (one_pass == 2 || (one_pass == 1 && N >= kOnePassKeys)))
+    return tree_attn_long_launch(qt, NQ, q_rows, kt, vt_t, N, gate, gate_ld, gate_hs, krange, y, HQ, HKV, scale, status,
+                                 static_cast<cudaStream_t>(stream));
   CUtensorMap map_q, map_k, map_vt;
   int rc = make_map(&map_q, qt, HQ * NQ, kD, kQRows);
   if (rc == OJB_OK) rc = make_map(&map_k, kt, HKV * N, kD, kSub);
@@ -477,5 +484,5 @@ extern "C" int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t
                                 ojb_stream_t stream) {
   if (N == 0) return OJB_OK;
   OJB_REQUIRE(N > 0 && N % 32 == 0 && D == kD);
-  return ojb_tree_attn_rows(qt, N, nullptr, kt, vt_t, N, gate, HQ * kD, kD, krange, y, HQ, HKV, scale, status, stream);
+  return ojb_tree_attn_rows(qt, N, nullptr, kt, vt_t, N, gate, HQ * kD, kD, krange, y, HQ, HKV, scale, 0, status, stream);
 }

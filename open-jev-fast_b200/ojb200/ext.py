@@ -624,9 +624,11 @@ def fattn_tree_tc(qt, kt, vt_t, gate, krange, scale):
     return y
 
 
-def tree_attn_rows(qt, kt, vt_t, q_src, krange, scale, q_rows=None):
+def tree_attn_rows(qt, kt, vt_t, q_src, krange, scale, q_rows=None, one_pass=True):
     """fattn_tree_tc on the operands of attn_operands: the gate is read where the in-projection left it (the second 256 columns
-    of every head of q_src), and the query rows may be any rows of the tree (q_rows int64). -> y [NQ, HQ*256]."""
+    of every head of q_src), and the query rows may be any rows of the tree (q_rows int64). one_pass: False keeps long trees on
+    the two-pass kernel, 2 takes the one-pass kernel for any number of keys.
+    -> y [NQ, HQ*256]."""
     _chk(qt, kt, vt_t, krange, q_rows)
     HQ, NQ, D = qt.shape
     HKV, N, _ = kt.shape
@@ -636,7 +638,8 @@ def tree_attn_rows(qt, kt, vt_t, q_src, krange, scale, q_rows=None):
         raise RuntimeError("tree_attn_rows: q_src does not belong to qt")
     y = torch.empty(NQ, HQ * D, dtype=bf16, device=qt.device)
     call("ojb_tree_attn_rows", ptr(qt), i64(NQ), ptr(q_rows), ptr(kt), ptr(vt_t), i64(N), ptr(q_src[:, D:]), i64(q_src.stride(0)),
-         i64(2 * D), ptr(krange), ptr(y), i64(HQ), i64(HKV), f32(scale), ptr(_lib.status_word(qt.device)), stream_ptr())
+         i64(2 * D), ptr(krange), ptr(y), i64(HQ), i64(HKV), f32(scale), i32(int(one_pass)), ptr(_lib.status_word(qt.device)),
+         stream_ptr())
     return y
 
 

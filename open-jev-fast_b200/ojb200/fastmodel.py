@@ -323,6 +323,8 @@ class FastQwen35(torch.nn.Module):
         tc = FATTN_TC and hasattr(lay, "krange") and d.D == 256 and d.HQ // d.HKV <= 6 and N % 32 == 0
         return tc, tc and K.attn_operands_ok(d.HQ, d.HKV, d.D, cos.shape[-1], N)
 
+    # (8-bit projections stay on the two-pass attention: the one-pass kernel sums in another order, and on e4m3 operands a rounding
+    # that falls the other way grows to percents of the result)
     def _attn_tree(self, d, proj, lay, cos, sin):
         N = proj.shape[0]
         G = d.HQ // d.HKV
@@ -330,7 +332,7 @@ class FastQwen35(torch.nn.Module):
         if in_place:
             q_src, kv_src = proj[:, :d.HQ * 2 * d.D], proj[:, d.HQ * 2 * d.D:]
             qt, kt, vt_t = K.attn_operands(q_src, kv_src, d.qw1, d.kw1, cos, sin, d.HQ, d.HKV, self.eps)
-            return K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale)
+            return K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale, one_pass=not self.fp8)
         if tc:
             qt, kt, vt, gate, vt_t = K.fullattn_prep2(proj, d.qw1, d.kw1, cos, sin, 1, N, d.HQ, d.HKV, d.D, self.eps, with_vt_t=True)
             return K.fattn_tree_tc(qt, kt, vt_t, gate, lay.krange, d.scale)
@@ -365,7 +367,7 @@ class FastQwen35(torch.nn.Module):
                 hq, h = K.gather_rows(rows, hn, h)
             q_src, kv_src = self._mm(hq, d.w_in, 0, nq), self._mm(hn, d.w_in, nq)
             qt, kt, vt_t = K.attn_operands(q_src, kv_src, d.qw1, d.kw1, cos, sin, d.HQ, d.HKV, self.eps, rows)
-            return h, K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale, rows)
+            return h, K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, d.scale, rows, one_pass=not self.fp8)
         proj = self._mm(hn, d.w_in)
         y = self._linear_tree(d, proj, lay) if linear else self._attn_tree(d, proj, lay, cos, sin)
         return K.gather_rows(rows, h, y.view(y.shape[0], -1))

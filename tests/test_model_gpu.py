@@ -101,7 +101,7 @@ def test_tree_attention_of_any_rows(N_case, HQ, HKV):
     qt, kt, vt, gate, vt_t = K.fullattn_prep2(proj, w1, w1, cosb, sinb, 1, N, HQ, HKV, D, 1e-6, with_vt_t=True)
     want = K.fattn_tree_tc(qt, kt, vt_t, gate, lay.krange, D ** -0.5)
     q_src = proj[:, :HQ * 2 * D]
-    assert torch.equal(K.tree_attn_rows(qt[0], kt[0], vt_t[0], q_src, lay.krange, D ** -0.5), want)
+    assert torch.equal(K.tree_attn_rows(qt[0], kt[0], vt_t[0], q_src, lay.krange, D ** -0.5, one_pass=False), want)
     real = lay.rowmask.nonzero().flatten()
     for n in (1, 16, 17, 45):
         rows = real[torch.randint(0, real.numel(), (n,), generator=g, device="cuda")]
@@ -109,6 +109,44 @@ def test_tree_attention_of_any_rows(N_case, HQ, HKV):
         assert (y.float() - want[rows].float()).norm() <= 4e-3 * want[rows].float().norm()
         assert torch.allclose(y.float(), want[rows].float(), rtol=2 ** -6, atol=2 ** -7)
     _lib.check_status()
+
+
+@pytest.mark.parametrize("N_case,HQ,HKV", [("baseline", 24, 4), ("example", 24, 4), ("ragged", 4, 2), ("doc", 6, 1), ("wide", 6, 2),
+                                           ("long", 12, 2), ("nostem", 5, 1), ("single", 3, 3)])
+@pytest.mark.parametrize("spread", [1.0, 30.0])
+def test_one_pass_attention(N_case, HQ, HKV, spread):
+    """The one-pass kernel against the masked-softmax oracle: query rows and keys that fill no tile, one and two heads to a tile, rows
+    that see a single key, and (spread 30) scores whose running maximum moves again and again, so that O is rescaled. Bound
+    as for the two-pass kernel: P in bf16 on both sides."""
+    from ojb200 import ext as K, _lib
+    from ojb200 import layout as PL
+    D, RD = 256, 64
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()[N_case]
+    ids, lay = PL.gtree_build(seqs, groups, pad_id, NB, PB, dev="cuda", dense=False)
+    N = lay.N
+    g = torch.Generator(device="cuda").manual_seed(31)
+    proj = torch.randn(N, 2 * HQ * D + 2 * HKV * D, generator=g, device="cuda").to(bf16)
+    w1 = 1.0 + torch.randn(D, generator=g, device="cuda") * 0.02
+    cosb, sinb = (torch.randn(N, RD, generator=g, device="cuda").to(bf16) for _ in range(2))
+    q_src, kv_src = proj[:, :HQ * 2 * D], proj[:, HQ * 2 * D:]
+    qt, kt, vt_t = K.attn_operands(q_src, kv_src, w1, w1, cosb, sinb, HQ, HKV, 1e-6)
+    scale = D ** -0.5 * spread
+    y = K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, scale, one_pass=2)
+    rows = torch.randint(0, N, (37,), generator=g, device="cuda")
+    some = K.tree_attn_rows(qt[:, rows].contiguous(), kt, vt_t, q_src[rows].contiguous(), lay.krange, scale, rows, one_pass=2)
+    nothing = torch.zeros_like(lay.krange)
+    none = K.tree_attn_rows(qt, kt, vt_t, q_src, nothing, scale, one_pass=2)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert float(none.float().abs().max()) == 0.0                       # a row that sees no key gives zeros
+    vis = torch.as_tensor(OL.gtree_layout(seqs, groups, pad_id, NB, PB)["vis"])
+    gate = q_src.reshape(N, HQ, 2, D)[:, :, 1].reshape(N, HQ * D)
+    ref = O.tree_attention(qt.cpu(), kt.cpu(), vt_t.transpose(1, 2).contiguous().cpu(), gate.cpu(), vis, scale).float()
+    real = lay.rowmask.cpu().bool()
+    assert torch.isfinite(y).all()
+    for got, want, keep in ((y.float().cpu(), ref, real), (some.float().cpu(), ref[rows.cpu()], real[rows.cpu()])):
+        assert ((got[keep] - want[keep]).norm() / want[keep].norm()).item() < 4e-3
+        assert (got[keep] - want[keep]).abs().max().item() < 6e-2
 
 
 @pytest.mark.parametrize("case", ["doc", "baseline", "nostem"])
