@@ -6,7 +6,7 @@
 //             flop), w-tile width chosen per shape, the last M mod 256 <= 128 rows (or all rows when M <= 2048, on request) run with
 //             swapped operands at their true cost.
 //   skinny    (gemm_skinny.cu)    up to 128 rows of x against w tiles of any width, every CTA's shared memory full of weight in
-//             flight; the choice for at most 32 rows.
+//             flight; the choice for all shapes it serves.
 //   pair256   (gemm_pair256.cu)   the same units on CTA pairs with tcgen05.mma.cta_group::2; measured on par with block256
 //             (both are bound by shared-memory bandwidth), kept as variants 5 / 6.
 // With variant 0 the kernel is the one with the smallest modelled time (plan_kernel): the models replay the round-robin
@@ -40,16 +40,16 @@ double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, in
   return static_cast<double>(ceil_div(units, grid)) * (per * kb + (f32 ? 33.0 * bn : 1500.0)) + 9000.0;
 }
 
-// The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (wait, four MMAs, its share of a commit) in less than 280
-// clocks. Measured on [12352, 5120] at 12 / 32 / 64 rows: 26.0 / 26.0 / 33 us against 41 / 28.6 / 29.1 of the 128-row tile kernel
-// (the rows of x that every CTA fetches again cost more from there on, hence kSkinnyRows); [2048, 5120] 18 against 26 us, [5120, 4096]
-// 11.7 against 12.3 us and [5120, 17408] 33.2 against 34.4 us of the best other kernel and K ranges.
-constexpr int kSkinnyRows = 32;
+// The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (its share of a wait, a commit and the MMAs) in less
+// than 220 clocks. Measured against the best of the other kernels (us): [12352, 5120] at 12 / 32 / 64 / 128 rows 24.2 / 24.5 / 27.7 /
+// 27.9 against 36 / 27.2 / 27.3 / 28.7; [2048, 5120] at 32 / 128 rows 15.4 / 18.4 against 21.3 / 21.8; [5120, 4096] at 12 / 128 rows 11.2 /
+// 14.4 against 11.4 / 14.5; [5120, 17408] 32.0 / 38.2 against 32.9 / 39.2.
+constexpr int kSkinnyRows = 128;
 double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
   const int bn = skinny_bn(N, splits);
   const double waves = static_cast<double>(ceil_div(ceil_div(N, bn) * splits, sms));
   const double fill = (bn + ceil_div(M, 8) * 8) * 128.0 / 30.0, per = static_cast<double>(ceil_div(kb_total, splits));
-  return waves * per * (fill > 280.0 ? fill : 280.0) + 6000.0;
+  return waves * per * (fill > 220.0 ? fill : 220.0) + 6000.0;
 }
 
 struct Plan {

@@ -113,7 +113,8 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -127,30 +128,30 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
           const int nh = 2 * (u.kb1 - u.kb0);
           for (int h0 = 0; h0 < nh; h0 += 3) {
             const int cnt = nh - h0 < 3 ? nh - h0 : 3;
-            if (!mbar_wait(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
             const uint32_t a_dst = tiles0 + stage * g.stage_bytes;
             const uint32_t fb = full0 + 8 * stage;
-            mbar_expect_tx(fb, static_cast<uint32_t>(cnt * g.tail_sub));
+            if (one) mbar_expect_tx(fb, static_cast<uint32_t>(cnt * g.tail_sub));
             for (int j = 0; j < cnt; ++j) {
               const int h = h0 + j, kb = u.kb0 + (h >> 1);
-              tma_load_2d(a_dst + j * g.tail_sub, &map_w128, fb, kb * kKE, u.wt * 256 + (h & 1) * kBM);
-              tma_load_2d(a_dst + j * g.tail_sub + kSubBytes, &map_xt, fb, kb * kKE, g.n_xblk * kBlockM + u.xc * g.tail_box);
+              if (one) tma_load_2d(a_dst + j * g.tail_sub, &map_w128, fb, kb * kKE, u.wt * 256 + (h & 1) * kBM);
+              if (one) tma_load_2d(a_dst + j * g.tail_sub + kSubBytes, &map_xt, fb, kb * kKE, g.n_xblk * kBlockM + u.xc * g.tail_box);
             }
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
           continue;
         }
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
-          if (!mbar_wait(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t a_dst = tiles0 + stage * g.stage_bytes;
           const uint32_t fb = full0 + 8 * stage;
-          mbar_expect_tx(fb, tx);
+          if (one) mbar_expect_tx(fb, tx);
           if (!u.tail) {
-            tma_load_2d(a_dst, &map_x, fb, kb * kKE, u.xb * kBlockM);
-            tma_load_2d(a_dst + kABytes, &map_w, fb, kb * kKE, u.wt * g.BN);
+            if (one) tma_load_2d(a_dst, &map_x, fb, kb * kKE, u.xb * kBlockM);
+            if (one) tma_load_2d(a_dst + kABytes, &map_w, fb, kb * kKE, u.wt * g.BN);
           } else {
-            tma_load_2d(a_dst, &map_w256, fb, kb * kKE, u.wt * 256);
-            tma_load_2d(a_dst + kABytes, &map_xt, fb, kb * kKE, g.n_xblk * kBlockM + u.xc * g.tail_box);
+            if (one) tma_load_2d(a_dst, &map_w256, fb, kb * kKE, u.wt * 256);
+            if (one) tma_load_2d(a_dst + kABytes, &map_xt, fb, kb * kKE, g.n_xblk * kBlockM + u.xc * g.tail_box);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -158,20 +159,21 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int stage = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
         const Unit u = decode_unit(g, unit, total_block);
         const uint32_t idesc = FP8 ? umma_idesc_e4m3(u.tail ? g.tail_box : g.BN) : umma_idesc(u.tail ? g.tail_box : g.BN);
-        if (!mbar_wait(accempty, acc_phase ^ 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(accempty, acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         if (u.tail && g.tail_sub) {
           const int nh = 2 * (u.kb1 - u.kb0);
           for (int h0 = 0; h0 < nh; h0 += 3) {
             const int cnt = nh - h0 < 3 ? nh - h0 : 3;
-            if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t a_addr = tiles0 + stage * g.stage_bytes;
             for (int j = 0; j < cnt; ++j) {
@@ -180,18 +182,18 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
               const uint64_t adesc = smem_desc_sw128(a_addr + j * g.tail_sub);
               const uint64_t bdesc = smem_desc_sw128(a_addr + j * g.tail_sub + kSubBytes);
 #pragma unroll
-              for (int k = 0; k < kBK / kUmmaK; ++k) mma(acc, adesc + 2 * k, bdesc + 2 * k, idesc, (h >= 2 || k > 0) ? 1u : 0u);
+              for (int k = 0; k < kBK / kUmmaK; ++k) if (one) mma(acc, adesc + 2 * k, bdesc + 2 * k, idesc, (h >= 2 || k > 0) ? 1u : 0u);
             }
-            umma_commit(empty0 + 8 * stage);
+            if (one) umma_commit(empty0 + 8 * stage);
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
           }
           if (!ok) break;
-          umma_commit(accfull);
+          if (one) umma_commit(accfull);
           acc_phase ^= 1u;
           continue;
         }
         for (int kb = u.kb0; kb < u.kb1; ++kb) {
-          if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = tiles0 + stage * g.stage_bytes;
           const uint64_t adesc0 = smem_desc_sw128(a_addr);
@@ -202,8 +204,8 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             for (int k = 0; k < kBK / kUmmaK; ++k) {
               // advancing K by 16 bf16 = 32 bytes inside the swizzle row: +2 in the (address >> 4) field
               const uint32_t accum = (kb > u.kb0 || k > 0) ? 1u : 0u;
-              mma(tmem_base, adesc0 + 2 * k, bdesc + 2 * k, idesc, accum);
-              mma(tmem_base + kAcc1Col, adesc1 + 2 * k, bdesc + 2 * k, idesc, accum);
+              if (one) mma(tmem_base, adesc0 + 2 * k, bdesc + 2 * k, idesc, accum);
+              if (one) mma(tmem_base + kAcc1Col, adesc1 + 2 * k, bdesc + 2 * k, idesc, accum);
             }
           } else {                                   // probe builds only
             // knob 102: the same MMAs with M = 64 in the instruction descriptor (what does a half-height MMA cost?)
@@ -211,15 +213,15 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             for (int rep = 0; rep < OJB_PROBE_REPEAT(g); ++rep)
               for (int k = 0; k < kBK / kUmmaK; ++k) {
                 const uint32_t accum = (kb > u.kb0 || k > 0 || rep > 0) ? 1u : 0u;
-                mma(tmem_base, adesc0 + 2 * k, bdesc + 2 * k, idesc_m, accum);
-                mma(tmem_base + kAcc1Col, adesc1 + 2 * k, bdesc + 2 * k, idesc_m, accum);
+                if (one) mma(tmem_base, adesc0 + 2 * k, bdesc + 2 * k, idesc_m, accum);
+                if (one) mma(tmem_base + kAcc1Col, adesc1 + 2 * k, bdesc + 2 * k, idesc_m, accum);
               }
           }
-          umma_commit(empty0 + 8 * stage);
+          if (one) umma_commit(empty0 + 8 * stage);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit(accfull);
+        if (one) umma_commit(accfull);
         acc_phase ^= 1u;
       }
     }

@@ -72,6 +72,19 @@ __device__ __forceinline__ void umma_f8(uint32_t tmem_d, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
       : "memory");
 }
+// One lane of a converged warp, the same one every time. A warp that walks its loop as a whole and issues from the elected lane
+// keeps addresses and descriptors in uniform registers, where tcgen05.mma and the copies want them; behind `lane == 0` every
+// operand is moved there anew. Measured on 32 x 2048 x 5120 (80 k-blocks of wait, four MMAs, commit): 30.3 -> 21.0 us with one k-block
+// per commit, 17.9 -> 12.9 us with four.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
+// mbar_wait of a whole warp: one result for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 // Arrive on an mbarrier once every tcgen05.mma issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");

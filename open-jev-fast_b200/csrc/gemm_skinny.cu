@@ -5,9 +5,8 @@
 // two accumulators) beside it: 97 tiles for 12 352 outputs, 16 for 2048, each SM's share of the link idle on the rest. Here the w
 // tile has any multiple of 16 rows up to 128, chosen so that the tiles (times the K ranges) fill the SMs once, and a stage holds
 // the rows of x that exist and no more, so that all of the shared memory is weight in flight.
-// A stage is several k-blocks, one three-dimensional copy each for x and w: with one k-block per stage the chain wait, MMAs, commit of
-// the issuing thread (0.31 us; the commit alone about 0.15) and the producer's wait and two copies (0.2 us) set the pace, 26 us
-// for K = 5120 whatever the weight's size.
+// A stage is several k-blocks, one three-dimensional copy each for x and w: with one k-block per stage the issuing warp's chain of wait,
+// MMAs and commit (0.2 us) sets the pace, 21 us for K = 5120 whatever the weight's size, against 12.9 us with four.
 //
 // One CTA per (w tile, K range), 192 threads: warp 0 asks for the tiles (plain cp.async.bulk.tensor, 128-byte swizzle, mbarrier), one
 // lane of warp 1 issues tcgen05.mma, warps 2-5 read the accumulator back and store. The MMA has M = 128 whatever the number of
@@ -78,29 +77,31 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 
   const uint32_t x_bytes = static_cast<uint32_t>(g.x_rows) * 128, w_bytes = static_cast<uint32_t>(g.BN) * 128;      // of one k-block
   if (warp == 0) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       for (int kb = 0; kb < nkb; kb += g.nk) {
-        if (!mbar_wait(empty0 + 8 * stage, phase ^ 1u, abort_flag)) break;
+        if (!mbar_wait_warp(empty0 + 8 * stage, phase ^ 1u, abort_flag)) break;
         const uint32_t dst = tiles0 + stage * g.stage_bytes, fb = full0 + 8 * stage;
-        mbar_expect_tx(fb, g.stage_bytes);
+        if (one) mbar_expect_tx(fb, g.stage_bytes);
         if (!(g.drop_copy && kb == g.nk)) {      // tests only: the announced bytes never arrive
           // (k-blocks past the end of this range are not multiplied; past the end of K they arrive as zeros)
-          tma_load_3d(dst + g.nk * x_bytes, &map_w, fb, 0, n0, kb0 + kb);
-          tma_load_3d(dst, &map_x, fb, 0, 0, kb0 + kb);
+          if (one) tma_load_3d(dst + g.nk * x_bytes, &map_w, fb, 0, n0, kb0 + kb);
+          if (one) tma_load_3d(dst, &map_x, fb, 0, 0, kb0 + kb);
         }
         if (++stage == g.stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       const uint32_t idesc = FP8 ? umma_idesc_e4m3(g.BN) : umma_idesc(g.BN);
       bool ok = true;
       for (int kb = 0; kb < nkb; kb += g.nk) {
-        if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t src = tiles0 + stage * g.stage_bytes;
         for (int j = 0; j < g.nk && kb + j < nkb; ++j) {
@@ -108,14 +109,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             const uint32_t accum = (kb + j > 0 || k > 0) ? 1u : 0u;
-            if constexpr (FP8) umma_f8(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
-            else umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+            if (one) {
+              if constexpr (FP8) umma_f8(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+              else umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, accum);
+            }
           }
         }
-        umma_commit(empty0 + 8 * stage);
+        if (one) umma_commit(empty0 + 8 * stage);
         if (++stage == g.stages) { stage = 0; phase ^= 1u; }
       }
-      if (ok) umma_commit(accfull);
+      if (ok && one) umma_commit(accfull);
     }
   } else {
     const int quarter = warp & 3, row = quarter * 32 + lane;

@@ -90,7 +90,8 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int stage = 0, issued = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -101,16 +102,16 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const int kb0 = split * g.kb_per_split;
         const int kb1 = min(kb0 + g.kb_per_split, g.kb_total);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(empty0 + 8 * stage, phase ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t a_dst = tiles0 + stage * Plan::kStageBytes;
           const uint32_t fb = full0 + 8 * stage;
-          mbar_expect_tx(fb, Plan::kStageBytes);
+          if (one) mbar_expect_tx(fb, Plan::kStageBytes);
           if (g.drop_copy && issued++ == 1) {
             // tests only (ojb_gemm_test_drop_copy): the bytes announced for this stage never arrive, the consumer's bounded
             // wait on its barrier runs out, the CTA reports OJB_DEV_WAIT_TIMEOUT and leaves in order
           } else {
-            tma_load_2d(a_dst, &map_x, fb, kb * kBK, m_blk * kBM);
-            tma_load_2d(a_dst + Plan::kABytes, &map_w, fb, kb * kBK, n_blk * BN);
+            if (one) tma_load_2d(a_dst, &map_x, fb, kb * kBK, m_blk * kBM);
+            if (one) tma_load_2d(a_dst + Plan::kABytes, &map_w, fb, kb * kBK, n_blk * BN);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
@@ -118,7 +119,8 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       constexpr uint32_t idesc = umma_idesc(BN);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
@@ -128,11 +130,11 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const int split = rest % g.splits;
         const int kb0 = split * g.kb_per_split;
         const int kb1 = min(kb0 + g.kb_per_split, g.kb_total);
-        if (!mbar_wait(accempty0 + 8 * acc, acc_phase ^ 1u, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(accempty0 + 8 * acc, acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = tiles0 + stage * Plan::kStageBytes;
           const uint64_t adesc = smem_desc_sw128(a_addr);
@@ -140,13 +142,13 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // advancing K by 16 bf16 = 32 bytes inside the swizzle row: +2 in the (address >> 4) field
-            umma_bf16(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            if (one) umma_bf16(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(empty0 + 8 * stage);
+          if (one) umma_commit(empty0 + 8 * stage);
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit(accfull0 + 8 * acc);
+        if (one) umma_commit(accfull0 + 8 * acc);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
       }

@@ -169,30 +169,31 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && T > 0) {
+    if (T > 0) {
+      const bool one = elect_one();
       int use = 0;
       bool ok = true;
       auto slot = [&](uint32_t& dst, uint32_t& fb) {
         const int s = use % kLSlots;
-        if (!mbar_wait(bar(kLBarEmpty + s), ((use / kLSlots) & 1) ^ 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kLBarEmpty + s), ((use / kLSlots) & 1) ^ 1, abort_flag)) return false;
         ++use;
         dst = smem_u32(Rg) + s * kLSlot;
         fb = bar(kLBarFull + s);
-        mbar_expect_tx(fb, kLSlot);
+        if (one) mbar_expect_tx(fb, kLSlot);
         return true;
       };
       auto keys = [&](int kb) {
         for (int c = 0; c < 2 && ok; ++c) {      // 128 dims
           uint32_t dst, fb;
           if (!(ok = slot(dst, fb))) break;
-          tma_load_3d(dst, &map_k, fb, 0, kvh * N + kb * kLKeys, 2 * c);
+          if (one) tma_load_3d(dst, &map_k, fb, 0, kvh * N + kb * kLKeys, 2 * c);
         }
       };
       auto values = [&](int kb) {
         for (int c = 0; c < 2 && ok; ++c) {      // 64 keys
           uint32_t dst, fb;
           if (!(ok = slot(dst, fb))) break;
-          tma_load_2d(dst, &map_vt, fb, kb * kLKeys + c * 64, kvh * kLD);
+          if (one) tma_load_2d(dst, &map_vt, fb, kb * kLKeys + c * 64, kvh * kLD);
         }
       };
       int kb = next_block(0);
@@ -209,42 +210,43 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && T > 0) {
+    if (T > 0) {
+      const bool one = elect_one();
       constexpr uint32_t idesc_s = umma_idesc(kLKeys), idesc_o = umma_idesc(kLD);
       int use = 0;
-      bool ok = mbar_wait(bar(kLBarQ), 0, abort_flag);
+      bool ok = mbar_wait_warp(bar(kLBarQ), 0, abort_flag);
       // (S of block j goes where S and P of block j - 2 were: its scores have been read, or P V (j - 2) would not have been issued,
       // and the tensor pipe runs the products in the order of their issue)
       auto qk = [&](int j) {
         const uint32_t acc = tmem_base + kLColS + static_cast<uint32_t>(j & 1) * kLKeys;
         for (int c = 0; c < 2; ++c, ++use) {
           const int s = use % kLSlots;
-          if (!mbar_wait(bar(kLBarFull + s), (use / kLSlots) & 1, abort_flag)) return false;
+          if (!mbar_wait_warp(bar(kLBarFull + s), (use / kLSlots) & 1, abort_flag)) return false;
           tc_fence_after();
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             const uint64_t qd = smem_desc_sw128(smem_u32(Qs) + (2 * c + t) * kLTile), kd = smem_desc_sw128(smem_u32(Rg) + s * kLSlot + t * kLTile);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_bf16(acc, qd + 2 * k, kd + 2 * k, idesc_s, (c > 0 || t > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < 4; ++k) if (one) umma_bf16(acc, qd + 2 * k, kd + 2 * k, idesc_s, (c > 0 || t > 0 || k > 0) ? 1u : 0u);
           }
-          umma_commit(bar(kLBarEmpty + s));
+          if (one) umma_commit(bar(kLBarEmpty + s));
         }
-        umma_commit(bar(kLBarSFull + (j & 1)));
+        if (one) umma_commit(bar(kLBarSFull + (j & 1)));
         return true;
       };
       auto pv = [&](int j) {
-        if (!mbar_wait(bar(kLBarPFull), j & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kLBarPFull), j & 1, abort_flag)) return false;
         for (int c = 0; c < 2; ++c, ++use) {
           const int s = use % kLSlots;
-          if (!mbar_wait(bar(kLBarFull + s), (use / kLSlots) & 1, abort_flag)) return false;
+          if (!mbar_wait_warp(bar(kLBarFull + s), (use / kLSlots) & 1, abort_flag)) return false;
           tc_fence_after();
           const uint32_t p = tmem_base + kLColS + static_cast<uint32_t>((j & 1) * kLKeys + c * 32);      // two keys per column
           const uint64_t vd = smem_desc_sw128(smem_u32(Rg) + s * kLSlot);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16_ts(tmem_base + kLColO, p + 8 * k, vd + 2 * k, idesc_o, (j > 0 || c > 0 || k > 0) ? 1u : 0u);
-          umma_commit(bar(kLBarEmpty + s));
+          for (int k = 0; k < 4; ++k) if (one) umma_bf16_ts(tmem_base + kLColO, p + 8 * k, vd + 2 * k, idesc_o, (j > 0 || c > 0 || k > 0) ? 1u : 0u);
+          if (one) umma_commit(bar(kLBarEmpty + s));
         }
-        umma_commit(bar(kLBarRest));
+        if (one) umma_commit(bar(kLBarRest));
         return true;
       };
       if (ok) ok = qk(0);
@@ -252,7 +254,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         if (j + 1 < T) ok = qk(j + 1);
         if (ok) ok = pv(j);
       }
-      if (ok) umma_commit(bar(kLBarO));
+      if (ok && one) umma_commit(bar(kLBarO));
     }
   } else {
     // ------------------------------------------------------------------ softmax: warps w and w + 4 share 32 rows, 64 keys each

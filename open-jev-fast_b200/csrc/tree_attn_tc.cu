@@ -188,22 +188,23 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == kSoftWarps) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       int use[2] = {0, 0};
       bool ok = true;
       auto load = [&](int R, bool is_v, int p) {      // the K blocks or the V blocks of pair p into region R
-        if (!mbar_wait(bar(kBarFree + R), (use[R] & 1) ^ 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kBarFree + R), (use[R] & 1) ^ 1, abort_flag)) return false;
         ++use[R];
-        mbar_expect_tx(bar(kBarFull + R), kRegion);
+        if (one) mbar_expect_tx(bar(kBarFull + R), kRegion);
         const uint32_t dst = smem_u32(Rg) + R * kRegion;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int kb = vis_list[min(2 * p + h, nblk - 1)];      // an odd count repeats the last block (masked out later)
           if (!is_v) {
             for (int kb4 = 0; kb4 < 4; ++kb4)
-              tma_load_2d(dst + kb4 * (kKB * 128) + h * (kSub * 128), &map_k, bar(kBarFull + R), kb4 * 64, kvh * N + kb * kSub);
+              if (one) tma_load_2d(dst + kb4 * (kKB * 128) + h * (kSub * 128), &map_k, bar(kBarFull + R), kb4 * 64, kvh * N + kb * kSub);
           } else {
-            tma_load_2d(dst + h * (kD * 128), &map_vt, bar(kBarFull + R), kb * kSub, kvh * kD);
+            if (one) tma_load_2d(dst + h * (kD * 128), &map_vt, bar(kBarFull + R), kb * kSub, kvh * kD);
           }
         }
         return true;
@@ -226,15 +227,16 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
   } else if (warp == kSoftWarps + 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       constexpr uint32_t idesc_s = umma_idesc(kKB), idesc_o = umma_idesc(kD);
       int use[2] = {0, 0}, use_s[2] = {0, 0};
-      bool ok = mbar_wait(bar(kBarQ), 0, abort_flag);
-      if (trace) trace[8] = global_timer_ns();          // Q has landed
+      bool ok = mbar_wait_warp(bar(kBarQ), 0, abort_flag);
+      if (trace && one) trace[8] = global_timer_ns();          // Q has landed
       auto qk = [&](int R, int sb) {                    // S[sb] = Q K^T with the K block in region R
-        if (!mbar_wait(bar(kBarFull + R), use[R] & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kBarFull + R), use[R] & 1, abort_flag)) return false;
         ++use[R];
-        if (!one_pass && !mbar_wait(bar(kBarSFree + sb), (use_s[sb] & 1) ^ 1, abort_flag)) return false;
+        if (!one_pass && !mbar_wait_warp(bar(kBarSFree + sb), (use_s[sb] & 1) ^ 1, abort_flag)) return false;
         ++use_s[sb];
         tc_fence_after();
         const uint32_t tmem_s = tmem_base + kColS + static_cast<uint32_t>(sb) * kKB;
@@ -243,15 +245,15 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const uint64_t qdesc = smem_desc_sw128(smem_u32(Qs) + kb4 * qstride);
           const uint64_t kdesc = smem_desc_sw128(smem_u32(Rg) + R * kRegion + kb4 * (kKB * 128));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_bf16(tmem_s, qdesc + 2 * k, kdesc + 2 * k, idesc_s, (kb4 > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) if (one) umma_bf16(tmem_s, qdesc + 2 * k, kdesc + 2 * k, idesc_s, (kb4 > 0 || k > 0) ? 1u : 0u);
         }
-        umma_commit(bar(kBarFree + R));
-        umma_commit(bar(kBarSFull + sb));
+        if (one) umma_commit(bar(kBarFree + R));
+        if (one) umma_commit(bar(kBarSFull + sb));
         return true;
       };
       auto pv = [&](int j, int R) {                     // O += P V of pass-2 block j, V block in region R
-        if (!mbar_wait(bar(kBarPFull), j & 1, abort_flag)) return false;
-        if (!mbar_wait(bar(kBarFull + R), use[R] & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kBarPFull), j & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(kBarFull + R), use[R] & 1, abort_flag)) return false;
         ++use[R];
         tc_fence_after();
 #pragma unroll
@@ -260,10 +262,10 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const uint64_t vdesc = smem_desc_sw128(smem_u32(Rg) + R * kRegion + kb2 * (kD * 128));
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + kColO, pdesc + 2 * k, vdesc + 2 * k, idesc_o, (j > 0 || kb2 > 0 || k > 0) ? 1u : 0u);
+            if (one) umma_bf16(tmem_base + kColO, pdesc + 2 * k, vdesc + 2 * k, idesc_o, (j > 0 || kb2 > 0 || k > 0) ? 1u : 0u);
         }
-        umma_commit(bar(kBarFree + R));
-        umma_commit(bar(kBarPFree));
+        if (one) umma_commit(bar(kBarFree + R));
+        if (one) umma_commit(bar(kBarPFree));
         return true;
       };
       if (one_pass) {
@@ -277,8 +279,8 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         if (ok && nvis > 0) ok = pv(nvis - 1, kHalf + (nvis - 1) % kHalf);
       }
-      if (ok) umma_commit(bar(kBarO));
-      if (trace) trace[9] = global_timer_ns();          // every MMA issued
+      if (ok && one) umma_commit(bar(kBarO));
+      if (trace && one) trace[9] = global_timer_ns();          // every MMA issued
     }
   } else if (warp < kSoftWarps && (warp & 3) < nw) {
     // ------------------------------------------------------------------ softmax + epilogue: two threads per (head, row).

@@ -236,7 +236,7 @@ class FastQwen35(torch.nn.Module):
             return out
 
         kernels = [1, 3] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
-        few = [11] if M <= 32 else []
+        few = [11] if M <= 128 else []
         for (N, Kd), layers in groups("w_in").items():
             x = rnd(M, Kd)
             res = race({i: (lambda d, i=i: LT.lt_matmul(x, d.w_in, i)) for i in kernels + [2] + few}, layers)
