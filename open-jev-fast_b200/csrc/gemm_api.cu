@@ -36,7 +36,9 @@ double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, in
   const int64_t units = ceil_div(M, 128) * ceil_div(N, bn) * splits;
   const int64_t grid = units < sms ? units : sms;
   const int per = static_cast<int>(ceil_div(kb_total, splits));
-  const double kb = bn == 256 ? 900.0 : 600.0;   // fitted to back-to-back runs against the power cap (133 us at 288 rows, 206 us at 544 for gate/up)
+  // against the power cap; in short runs a k-block takes 740 and 440 clocks, but the second reading of x costs energy: gate/up at 1600
+  // rows, chosen by those, ran 405 us in place of the 370 of 256-row blocks, and everything after it slower
+  const double kb = bn == 256 ? 900.0 : 600.0;
   return static_cast<double>(ceil_div(units, grid)) * (per * kb + (f32 ? 33.0 * bn : 1500.0)) + 9000.0;
 }
 

@@ -120,8 +120,8 @@ __host__ __device__ __forceinline__ Unit decode_unit(const GemmArgs& g, int unit
 
 // ---- Cost model (host). Times are SM clocks; the constants come from unit timelines measured on B200 (ojb_gemm_set_trace):
 // the main loops are bound by shared-memory bandwidth (128 bytes per clock per SM shared between the TMA fill of a stage
-// and the operand reads of its MMAs), an MMA with M = 128 never takes less than 64 clocks, a swapped-operand unit keeps
-// too few bytes in flight to run faster than about 1200 clocks per k-block, and the epilogue of a block unit costs about 19
+// and the operand reads of its MMAs), an MMA with M = 128 never takes less than 64 clocks, a k-block of a
+// swapped-operand unit takes its wait, commit and eight MMAs at least 600 clocks, and the epilogue of a block unit costs about 19
 // (bf16), 33 (fp32) or 40 (SwiGLU) clocks per accumulator column.
 // The model as the K ranges of 8-bit products are chosen by (see model_kernel): fp32 partials, every tile width alike.
 constexpr int kEpi8BitRanges = 3;
@@ -139,7 +139,8 @@ inline UnitCost unit_cost(int bn, int tail_box, int epi) {
   const bool f32 = epi == kEpiPartialF32 || epi == kEpi8BitRanges;
   c.block_epi = 900.0 + bn * (f32 ? (bulk ? 33.0 : 115.0) : (epi == kEpiSwiglu ? 40.0 : (bulk ? 19.0 : 55.0)));
   const double tsm = 512.0 + 3.0 * tail_box;
-  c.tail_kb = tsm > 1200.0 ? tsm : 1200.0;
+  const double floor = epi == kEpi8BitRanges ? 1200.0 : 600.0;
+  c.tail_kb = tsm > floor ? tsm : floor;
   c.tail_epi = 3200.0 + 24.0 * tail_box;
   return c;
 }
