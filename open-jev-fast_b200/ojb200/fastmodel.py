@@ -347,9 +347,10 @@ class FastQwen35(torch.nn.Module):
 
     # Behind its token mixer the last layer is a function of single rows, and only the candidates' last rows are asked for: its
     # queries, output projection and MLP run on those alone. Below ASKED_MIN_ROWS rows every projection takes the time its weight
-    # takes to arrive whatever the row count, and the extra launches (a gather, two projections in the place of one) would only
-    # add to it.
-    ASKED_MIN_ROWS = 192
+    # takes to arrive whatever the row count, and the extra launches (a gather, two projections in the place of one) eat up the
+    # rest. Eight layers, all rows / the asked rows (us): 128 rows 1624 / 1620, 160 rows 1783 / 1766, 192 rows 1848 / 1823, 384 rows
+    # 2540 / 2418.
+    ASKED_MIN_ROWS = 160
 
     def _asked_rows_only(self, lay, N):
         i = lay.lastidx
