@@ -354,8 +354,9 @@ int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t* q_rows, in
                       const float* qw1, const float* kw1, const void* cosb, const void* sinb, void* qt, void* kt, void* vt_t,
                       int64_t N, int64_t HQ, int64_t HKV, int64_t RD, float eps, ojb_stream_t stream);
 
-/* out[i, :] = in[rows[i], :] for one or two matrices (b may be null) of a_bytes / b_bytes per row (multiples of 16). */
-int ojb_gather_rows(const int64_t* rows, int64_t n_rows, const void* a, void* a_out, int64_t a_bytes, const void* b, void* b_out,
+/* out[i, :] = in[rows[i], :] for one or two matrices (b may be null) of n_src rows of a_bytes / b_bytes (multiples of 16); an index
+ * outside is moved to the nearest row. */
+int ojb_gather_rows(const int64_t* rows, int64_t n_rows, int64_t n_src, const void* a, void* a_out, int64_t a_bytes, const void* b, void* b_out,
                     int64_t b_bytes, ojb_stream_t stream);
 
 /* Measurement hook of ojb_tree_attn_tc (no counterpart in the reference): `records` = null switches it off; otherwise a device

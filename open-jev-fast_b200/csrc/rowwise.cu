@@ -431,7 +431,7 @@ attn_operands_kernel(const bf16_t* __restrict__ q_src, int64_t q_ld, const int64
 #pragma unroll
       for (int e = 0; e < 8; ++e) pv[e] = __shfl_xor_sync(0xffffffffu, nv[e], partner);
       if (rope) {
-        const int64_t tn = (isq && q_rows != nullptr) ? q_rows[n] : n;
+        const int64_t tn = (isq && q_rows != nullptr) ? min(max(q_rows[n], int64_t{0}), static_cast<int64_t>(N - 1)) : n;
         float c[8], s[8];
         unpack8(*reinterpret_cast<const uint4*>(cosb + tn * RD + d0), c);
         unpack8(*reinterpret_cast<const uint4*>(sinb + tn * RD + d0), s);
@@ -467,12 +467,12 @@ attn_operands_kernel(const bf16_t* __restrict__ q_src, int64_t q_ld, const int64
   }
 }
 
-// Rows rows[i] of one or two matrices, one block per output row.
+// Rows rows[i] (kept inside the matrix) of one or two matrices, one block per output row.
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const int64_t* __restrict__ rows, const uint4* __restrict__ a, uint4* __restrict__ a_out, int a_vecs,
+gather_rows_kernel(const int64_t* __restrict__ rows, int64_t n_src, const uint4* __restrict__ a, uint4* __restrict__ a_out, int a_vecs,
                    const uint4* __restrict__ b, uint4* __restrict__ b_out, int b_vecs) {
   pdl_begin();
-  const int64_t i = blockIdx.x, n = rows[i];
+  const int64_t i = blockIdx.x, n = min(max(rows[i], int64_t{0}), n_src - 1);
   for (int c = threadIdx.x; c < a_vecs; c += blockDim.x) a_out[i * a_vecs + c] = a[n * a_vecs + c];
   for (int c = threadIdx.x; c < b_vecs; c += blockDim.x) b_out[i * b_vecs + c] = b[n * b_vecs + c];
 }
@@ -733,14 +733,14 @@ extern "C" int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t*
   return launch_status(cudaGetLastError());
 }
 
-extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, const void* a, void* a_out, int64_t a_bytes, const void* b,
+extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, int64_t n_src, const void* a, void* a_out, int64_t a_bytes, const void* b,
                                void* b_out, int64_t b_bytes, ojb_stream_t stream) {
   if (n_rows == 0) return OJB_OK;
-  OJB_REQUIRE(rows && n_rows > 0 && n_rows < (int64_t{1} << 31) && a && a_out && a_bytes > 0 && a_bytes % 16 == 0 && a_bytes < (1 << 30));
+  OJB_REQUIRE(rows && n_rows > 0 && n_rows < (int64_t{1} << 31) && n_src > 0 && a && a_out && a_bytes > 0 && a_bytes % 16 == 0 && a_bytes < (1 << 30));
   OJB_REQUIRE(b ? (b_out && b_bytes > 0 && b_bytes % 16 == 0 && b_bytes < (1 << 30)) : (b_bytes == 0));
   for (const void* p : {a, static_cast<const void*>(a_out), b, static_cast<const void*>(b_out)})
     OJB_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15u) == 0);
-  launch_kernel(gather_rows_kernel, dim3(static_cast<unsigned>(n_rows)), dim3(256), 0, static_cast<cudaStream_t>(stream), rows,
+  launch_kernel(gather_rows_kernel, dim3(static_cast<unsigned>(n_rows)), dim3(256), 0, static_cast<cudaStream_t>(stream), rows, n_src,
                 static_cast<const uint4*>(a), static_cast<uint4*>(a_out), static_cast<int>(a_bytes / 16),
                 static_cast<const uint4*>(b), static_cast<uint4*>(b_out), static_cast<int>(b_bytes / 16));
   return launch_status(cudaGetLastError());

@@ -651,7 +651,9 @@ def gather_rows(rows, a, b=None):
     size = [t[0].numel() * t.element_size() for t in (a, b) if t is not None] + [0]
     if rows.dtype != torch.int64:
         raise RuntimeError("gather_rows: int64 rows expected")
-    call("ojb_gather_rows", ptr(rows), i64(S), ptr(a), ptr(outs[0]), i64(size[0]), ptr(b), ptr(outs[1] if b is not None else None),
+    if b is not None and b.shape[0] != a.shape[0]:
+        raise RuntimeError("gather_rows: both matrices need the same number of rows")
+    call("ojb_gather_rows", ptr(rows), i64(S), i64(a.shape[0]), ptr(a), ptr(outs[0]), i64(size[0]), ptr(b), ptr(outs[1] if b is not None else None),
          i64(size[1] if b is not None else 0), stream_ptr())
     return outs if b is not None else outs[0]
 

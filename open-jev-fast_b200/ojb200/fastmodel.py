@@ -354,7 +354,7 @@ class FastQwen35(torch.nn.Module):
 
     def _asked_rows_only(self, lay, N):
         i = lay.lastidx
-        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and i.dtype == torch.int64 and i.is_contiguous()
+        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and i.dtype == torch.int64 and i.is_cuda and i.is_contiguous()
 
     def _mix_asked(self, i, h, hn, rows, lay, cos, sin, linear):
         """Token mixer of the last layer (i) for the asked rows: (their residual stream, their mixer output)."""
