@@ -340,7 +340,8 @@ int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const voi
 
 /* The same for any rows of the tree as queries: query row n (of NQ) goes by row q_rows[n] of krange (q_rows null: by row n), and
  * its gate is read at gate + n * gate_ld + head * gate_hs (elements, multiples of 8), e.g. inside the in-projection output.
- * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0, any NQ.
+ * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0; any NQ with q_rows, at most
+ * N without.
  * one_pass = 1: 256 keys and more (scale > 0) go to a kernel that takes 128 operand rows and goes over the keys once, with a running
  * maximum; 2: any number does; 0: always the two-pass kernel. */
 int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
@@ -349,7 +350,8 @@ int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const 
 
 /* Its operands (ojb_fullattn_prep without the copies of the gate and of V in row order): q_src = NQ rows, q_ld elements apart,
  * of [q(256) | gate(256)] per query head; kv_src = N rows, kv_ld apart, of HKV k heads then HKV v heads. Query row n takes its
- * rotary angles from row q_rows[n] of cosb / sinb (null: row n). RD a power of two in [16, 256]; N % 8 == 0. */
+ * rotary angles from row q_rows[n] of cosb / sinb [N, RD] (null: row n; NQ is then at most N). RD a power of two in [16, 256];
+ * N % 8 == 0. */
 int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t* q_rows, int64_t NQ, const void* kv_src, int64_t kv_ld,
                       const float* qw1, const float* kw1, const void* cosb, const void* sinb, void* qt, void* kt, void* vt_t,
                       int64_t N, int64_t HQ, int64_t HKV, int64_t RD, float eps, ojb_stream_t stream);

@@ -716,6 +716,7 @@ extern "C" int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t*
   constexpr int D = 256;
   OJB_REQUIRE(q_src && kv_src && qw1 && kw1 && cosb && sinb && qt && kt && vt_t && N > 0 && NQ > 0 && HQ > 0 && HKV > 0);
   OJB_REQUIRE(N % 8 == 0 && N < (1 << 24) && NQ < (1 << 24) && HQ <= 1024 && HKV <= 1024);
+  OJB_REQUIRE(q_rows != nullptr || NQ <= N);      // without q_rows query row n takes row n of the rotary tables, which have N
   OJB_REQUIRE(RD > 0 && RD <= D && RD % 16 == 0 && (RD & (RD - 1)) == 0);
   OJB_REQUIRE(q_ld >= HQ * 2 * D && q_ld % 8 == 0 && kv_ld >= HKV * 2 * D && kv_ld % 8 == 0);
   for (const void* p : {q_src, kv_src, static_cast<const void*>(qw1), static_cast<const void*>(kw1), cosb, sinb,

@@ -459,6 +459,7 @@ extern "C" int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_r
                                   int64_t HKV, float scale, int32_t one_pass, int32_t* status, ojb_stream_t stream) {
   if (N == 0 || NQ == 0) return OJB_OK;
   OJB_REQUIRE(qt && kt && vt_t && gate && krange && y && N > 0 && N % 8 == 0 && NQ > 0);
+  OJB_REQUIRE(q_rows != nullptr || NQ <= N);      // without q_rows query row n goes by row n of krange, which has N
   OJB_REQUIRE(HQ > 0 && HKV > 0 && HQ % HKV == 0 && HQ / HKV <= kMaxG);
   OJB_REQUIRE(gate_ld >= 0 && gate_hs >= 0 && gate_ld % 8 == 0 && gate_hs % 8 == 0 && gate_hs < (1 << 30));
   OJB_REQUIRE(aligned16(qt) && aligned16(kt) && aligned16(vt_t) && aligned16(gate) && aligned16(y));

@@ -44,6 +44,20 @@ def test_argument_checks_need_no_gpu():
     assert rc == -1      # N must be a multiple of 32
 
 
+def test_more_query_rows_than_rows_need_their_row_indices():
+    """Without q_rows, query row n goes by row n of the key ranges and of the rotary tables, which have N rows: more query rows
+    than that are refused before anything is launched."""
+    from ojb200 import _lib
+    from ojb200._lib import f32, i32, i64
+    lib, p, none = _lib.lib(), ctypes.c_void_p(1 << 20), ctypes.c_void_p(0)
+    for NQ in (9, 16, 1000):
+        for one_pass in (0, 1, 2):
+            assert lib.ojb_tree_attn_rows(p, i64(NQ), none, p, p, i64(8), p, i64(512), i64(512), p, p, i64(2), i64(1), f32(1.0),
+                                          i32(one_pass), none, none) == -1
+        assert lib.ojb_attn_operands(p, i64(1024), none, i64(NQ), p, i64(512), p, p, p, p, p, p, p, i64(8), i64(2), i64(1), i64(64),
+                                     f32(1e-6), none) == -1
+
+
 def test_gemm_plan_is_host_arithmetic():
     """ojb_gemm_plan needs no GPU: it returns a valid variant, a split count within bounds, and a finite time."""
     from ojb200 import lt_ext
