@@ -6,7 +6,8 @@
  * (ojb_gemm_set_trace, ojb_gdn_set_trace) change process-wide state and the second synchronises; the first call of
  * ojb_gdn_chunked_static on a device does a one-time look-up. Kernel attributes and the SM count are cached per device, so
  * one process may drive several GPUs (make each call with its device current). Return value: OJB_OK or a negative OJB_ERR_* code. Kernels with device-side
- * waits additionally take `status`, a device int32 that stays 0 unless a bounded wait ran out.
+ * waits, and those that follow row indices, additionally take `status`, a device int32 that stays 0 unless a bounded wait ran out
+ * or an index lay outside.
  *
  * Each declaration names the interface of lyuyiqi/open-jev-fast that it stands in for (path inside that project).
  * Tensors are row-major and contiguous; "bf16" is __nv_bfloat16; shapes are written [rows, cols].
@@ -28,6 +29,7 @@ extern "C" {
 
 /* device-side status codes written into `status` */
 #define OJB_DEV_WAIT_TIMEOUT 1
+#define OJB_DEV_ROW_INDEX 2      /* a row index outside [-n, n) of n rows; what it asked for is not-a-number */
 
 typedef void* ojb_stream_t;
 
@@ -341,7 +343,8 @@ int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const voi
 /* The same for any rows of the tree as queries: query row n (of NQ) goes by row q_rows[n] of krange (q_rows null: by row n), and
  * its gate is read at gate + n * gate_ld + head * gate_hs (elements, multiples of 8), e.g. inside the in-projection output.
  * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0; any NQ with q_rows, at most
- * N without.
+ * N without. An index -n counts from the end (here and in ojb_attn_operands); one outside [-N, N) is moved to the nearest row, so that
+ * nothing outside is read: ojb_gather_rows, which takes the same indices, reports it.
  * one_pass = 1: 256 keys and more (scale > 0) go to a kernel that takes 128 operand rows and goes over the keys once, with a running
  * maximum; 2: any number does; 0: always the two-pass kernel. */
 int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
@@ -356,10 +359,10 @@ int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t* q_rows, in
                       const float* qw1, const float* kw1, const void* cosb, const void* sinb, void* qt, void* kt, void* vt_t,
                       int64_t N, int64_t HQ, int64_t HKV, int64_t RD, float eps, ojb_stream_t stream);
 
-/* out[i, :] = in[rows[i], :] for one or two matrices (b may be null) of n_src rows of a_bytes / b_bytes (multiples of 16); an index
- * outside is moved to the nearest row. */
+/* out[i, :] = in[rows[i], :] for one or two matrices (b may be null) of n_src rows of a_bytes / b_bytes (multiples of 16). Index -n counts
+ * from the end; one outside [-n_src, n_src) gives a row of 0xff bytes (not-a-number in bf16 and fp32) and OJB_DEV_ROW_INDEX in `status`. */
 int ojb_gather_rows(const int64_t* rows, int64_t n_rows, int64_t n_src, const void* a, void* a_out, int64_t a_bytes, const void* b, void* b_out,
-                    int64_t b_bytes, ojb_stream_t stream);
+                    int64_t b_bytes, int32_t* status, ojb_stream_t stream);
 
 /* Measurement hook of ojb_tree_attn_tc (no counterpart in the reference): `records` = null switches it off; otherwise a device
  * buffer of 16 uint64 words. The CTA of kv head 0 and the last-but-one block of 16 query rows stores %globaltimer at kernel
@@ -374,6 +377,9 @@ int ojb_tree_attn_set_trace(uint64_t* records);
 int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S, int64_t A,
                    int64_t H, ojb_stream_t stream);
 
+/* The same with the row count of hn: indices as in ojb_gather_rows, the scores of one outside are not-a-number. */
+int ojb_score_head_rows(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
+                        int64_t A, int64_t H, int32_t* status, ojb_stream_t stream);
 #ifdef __cplusplus
 }
 #endif

@@ -69,6 +69,17 @@ __device__ __forceinline__ void report_status(int32_t* status, int32_t code) {
   if (status) atomicCAS(status, 0, code);
 }
 
+// Row that an index of a caller means: -n counts from the end; -1 for an index outside [-rows, rows).
+__device__ __forceinline__ int64_t row_of_index(int64_t i, int64_t rows) {
+  if (i < 0) i += rows;
+  return i >= 0 && i < rows ? i : -1;
+}
+// The same where an index outside has been reported before: moved to the nearest row.
+__device__ __forceinline__ int64_t nearest_row(int64_t i, int64_t rows) {
+  const int64_t n = i < 0 ? i + rows : i;
+  return n < 0 ? 0 : (n < rows ? n : rows - 1);
+}
+
 // ---- mbarrier primitives shared by every kernel that waits for asynchronous copies or tensor-core work
 constexpr int kDefaultWaitMs = 2000;   // limit of every device-side wait unless ojb_gemm_set_wait_limit_ms changed it
 

@@ -431,7 +431,7 @@ attn_operands_kernel(const bf16_t* __restrict__ q_src, int64_t q_ld, const int64
 #pragma unroll
       for (int e = 0; e < 8; ++e) pv[e] = __shfl_xor_sync(0xffffffffu, nv[e], partner);
       if (rope) {
-        const int64_t tn = (isq && q_rows != nullptr) ? min(max(q_rows[n], int64_t{0}), static_cast<int64_t>(N - 1)) : n;
+        const int64_t tn = (isq && q_rows != nullptr) ? nearest_row(q_rows[n], N) : n;
         float c[8], s[8];
         unpack8(*reinterpret_cast<const uint4*>(cosb + tn * RD + d0), c);
         unpack8(*reinterpret_cast<const uint4*>(sinb + tn * RD + d0), s);
@@ -467,12 +467,19 @@ attn_operands_kernel(const bf16_t* __restrict__ q_src, int64_t q_ld, const int64
   }
 }
 
-// Rows rows[i] (kept inside the matrix) of one or two matrices, one block per output row.
+// Rows rows[i] of one or two matrices, one block per output row; an index outside gives a row of ones (not-a-number) and is reported.
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const int64_t* __restrict__ rows, int64_t n_src, const uint4* __restrict__ a, uint4* __restrict__ a_out, int a_vecs,
-                   const uint4* __restrict__ b, uint4* __restrict__ b_out, int b_vecs) {
+                   const uint4* __restrict__ b, uint4* __restrict__ b_out, int b_vecs, int32_t* status) {
   pdl_begin();
-  const int64_t i = blockIdx.x, n = min(max(rows[i], int64_t{0}), n_src - 1);
+  const int64_t i = blockIdx.x, n = row_of_index(rows[i], n_src);
+  if (n < 0) {
+    const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int c = threadIdx.x; c < a_vecs; c += blockDim.x) a_out[i * a_vecs + c] = ones;
+    for (int c = threadIdx.x; c < b_vecs; c += blockDim.x) b_out[i * b_vecs + c] = ones;
+    if (threadIdx.x == 0) report_status(status, OJB_DEV_ROW_INDEX);
+    return;
+  }
   for (int c = threadIdx.x; c < a_vecs; c += blockDim.x) a_out[i * a_vecs + c] = a[n * a_vecs + c];
   for (int c = threadIdx.x; c < b_vecs; c += blockDim.x) b_out[i * b_vecs + c] = b[n * b_vecs + c];
 }
@@ -527,7 +534,7 @@ extern "C" int ojb_l2_prefetch(const void* data, int64_t nbytes, int64_t chunk, 
   return launch_status(cudaGetLastError());
 }
 
-extern "C" int ojb_abi_version(void) { return 7; }
+extern "C" int ojb_abi_version(void) { return 8; }
 
 extern "C" int ojb_add_rmsnorm(const void* x, const void* delta, const float* w1, const int32_t* rowmask, void* h_out,
                                void* hn_out, int64_t rows, int64_t H, float eps, ojb_stream_t stream) {
@@ -735,7 +742,7 @@ extern "C" int ojb_attn_operands(const void* q_src, int64_t q_ld, const int64_t*
 }
 
 extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, int64_t n_src, const void* a, void* a_out, int64_t a_bytes, const void* b,
-                               void* b_out, int64_t b_bytes, ojb_stream_t stream) {
+                               void* b_out, int64_t b_bytes, int32_t* status, ojb_stream_t stream) {
   if (n_rows == 0) return OJB_OK;
   OJB_REQUIRE(rows && n_rows > 0 && n_rows < (int64_t{1} << 31) && n_src > 0 && a && a_out && a_bytes > 0 && a_bytes % 16 == 0 && a_bytes < (1 << 30));
   OJB_REQUIRE(b ? (b_out && b_bytes > 0 && b_bytes % 16 == 0 && b_bytes < (1 << 30)) : (b_bytes == 0));
@@ -743,7 +750,7 @@ extern "C" int ojb_gather_rows(const int64_t* rows, int64_t n_rows, int64_t n_sr
     OJB_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15u) == 0);
   launch_kernel(gather_rows_kernel, dim3(static_cast<unsigned>(n_rows)), dim3(256), 0, static_cast<cudaStream_t>(stream), rows, n_src,
                 static_cast<const uint4*>(a), static_cast<uint4*>(a_out), static_cast<int>(a_bytes / 16),
-                static_cast<const uint4*>(b), static_cast<uint4*>(b_out), static_cast<int>(b_bytes / 16));
+                static_cast<const uint4*>(b), static_cast<uint4*>(b_out), static_cast<int>(b_bytes / 16), status);
   return launch_status(cudaGetLastError());
 }
 
@@ -754,12 +761,20 @@ namespace {
 // reads each: what counts is one round of loads instead of twenty (one warp per output: 10-12 us).
 constexpr int kHeadThreads = 320;
 __global__ void __launch_bounds__(kHeadThreads)
-score_head_kernel(const bf16_t* __restrict__ hn, const int64_t* __restrict__ rows, const float* __restrict__ W,
-                  const float* __restrict__ bias, float* __restrict__ out, int A, int H) {
+score_head_kernel(const bf16_t* __restrict__ hn, int64_t n_src, const int64_t* __restrict__ rows, const float* __restrict__ W,
+                  const float* __restrict__ bias, float* __restrict__ out, int A, int H, int32_t* status) {
   pdl_begin();
   __shared__ float red[32];
   const int s = blockIdx.x / A, a = blockIdx.x - s * A;
-  const bf16_t* x = hn + (rows ? rows[s] : s) * static_cast<int64_t>(H);
+  const int64_t n = rows ? row_of_index(rows[s], n_src) : s;
+  if (n < 0) {      // the whole block
+    if (threadIdx.x == 0) {
+      out[blockIdx.x] = __int_as_float(0x7fffffff);
+      report_status(status, OJB_DEV_ROW_INDEX);
+    }
+    return;
+  }
+  const bf16_t* x = hn + n * static_cast<int64_t>(H);
   const float* w = W + static_cast<int64_t>(a) * H;
   float acc = 0.f;
 #pragma unroll 2
@@ -775,14 +790,20 @@ score_head_kernel(const bf16_t* __restrict__ hn, const int64_t* __restrict__ row
 }  // namespace
 }  // namespace ojb
 
-extern "C" int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
-                              int64_t A, int64_t H, ojb_stream_t stream) {
+extern "C" int ojb_score_head_rows(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out,
+                                   int64_t S, int64_t A, int64_t H, int32_t* status, ojb_stream_t stream) {
   if (S == 0 || A == 0) return OJB_OK;
   OJB_REQUIRE(hn && W && out && S > 0 && A > 0 && H > 0 && H % 8 == 0);
-  OJB_REQUIRE(S * A < (int64_t{1} << 31));
+  OJB_REQUIRE(S * A < (int64_t{1} << 31) && n_src > 0 && (rows || S <= n_src));
   launch_kernel(ojb::score_head_kernel, dim3(static_cast<unsigned>(S * A)), dim3(ojb::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
-      static_cast<const ojb::bf16_t*>(hn), rows, W, bias, out, static_cast<int>(A), static_cast<int>(H));
+      static_cast<const ojb::bf16_t*>(hn), n_src, rows, W, bias, out, static_cast<int>(A), static_cast<int>(H), status);
   return ojb::launch_status(cudaGetLastError());
+}
+
+// without the row count of hn nothing is known to lie outside (and an index cannot count from the end)
+extern "C" int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
+                              int64_t A, int64_t H, ojb_stream_t stream) {
+  return ojb_score_head_rows(hn, INT64_MAX, rows, W, bias, out, S, A, H, nullptr, stream);
 }
 
 extern "C" int ojb_quantize_rows_e4m3(const void* x, void* q, float* scale, int64_t rows, int64_t K, ojb_stream_t stream) {

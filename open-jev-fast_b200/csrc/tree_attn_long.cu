@@ -145,7 +145,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   for (int i = tid; i < g.R * 3; i += kLThreads) {
     const int r = r0 + i / 3, which = i % 3;
     if (r < g.NQ) {
-      const int32_t* q = g.krange + (g.q_rows ? min(max(g.q_rows[r], int64_t{0}), static_cast<int64_t>(N - 1)) : r) * 8;      // (e0, a1, e1, a2, e2, a0)
+      const int32_t* q = g.krange + (g.q_rows ? nearest_row(g.q_rows[r], N) : r) * 8;      // (e0, a1, e1, a2, e2, a0)
       const int lo = max(which == 0 ? q[5] : which == 1 ? q[1] : q[3], 0), hi = min(which == 0 ? q[0] : which == 1 ? q[2] : q[4], N);
       if (lo < hi) {
         const int b0 = lo / kLKeys, b1 = (hi - 1) / kLKeys;
@@ -262,7 +262,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const int qr = r0 + my % g.R;
     int lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0, lo2 = 0, hi2 = 0;
     if (qr < g.NQ) {
-      const int32_t* q = g.krange + (g.q_rows ? min(max(g.q_rows[qr], int64_t{0}), static_cast<int64_t>(N - 1)) : qr) * 8;
+      const int32_t* q = g.krange + (g.q_rows ? nearest_row(g.q_rows[qr], N) : qr) * 8;
       hi0 = q[0]; lo1 = q[1]; hi1 = q[2]; lo2 = q[3]; hi2 = q[4]; lo0 = q[5];
     }
     const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;

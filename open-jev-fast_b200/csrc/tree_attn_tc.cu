@@ -128,7 +128,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // key ranges of the 16 rows
   if (tid < kQRows * 8) {      // rows past the last query row see nothing
     const int r = r0 + (tid >> 3);
-    kr[tid] = r < g.NQ ? g.krange[(g.q_rows ? min(max(g.q_rows[r], int64_t{0}), static_cast<int64_t>(N - 1)) : r) * 8 + (tid & 7)] : 0;
+    kr[tid] = r < g.NQ ? g.krange[(g.q_rows ? nearest_row(g.q_rows[r], N) : r) * 8 + (tid & 7)] : 0;
   }
   tc_fence_before();
   __syncthreads();

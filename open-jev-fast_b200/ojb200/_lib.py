@@ -9,7 +9,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libojb200.so")
-ABI_VERSION = 7
+ABI_VERSION = 8
 
 _ERR = {-1: "invalid argument (shape / alignment / null pointer)", -2: "CUDA launch or API failure",
         -3: "CUDA driver tensor-map encoder unavailable", -4: "size beyond the documented maximum"}
@@ -56,7 +56,7 @@ def f32(v):
 
 
 def status_word(device):
-    """Per-device int32 word that kernels with bounded waits write on a timeout."""
+    """Per-device int32 word that kernels write when a bounded wait runs out or a row index lies outside."""
     key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
     t = _status.get(key)
     if t is None:
@@ -65,13 +65,15 @@ def status_word(device):
 
 
 def check_status(device=None):
-    """Read the status word back (synchronises). Raises if a device-side wait ran out."""
+    """Read the status word back (synchronises). Raises if a device-side wait ran out or a row index lay outside its matrix."""
     key = torch.cuda.current_device() if device is None else torch.device(device).index
     t = _status.get(key)
     if t is not None:
         v = int(t.item())
         if v != 0:
             t.zero_()
+            if v == 2:
+                raise RuntimeError("ojb200: a row index lies outside the rows it points into; its results are not-a-number")
             raise RuntimeError(f"ojb200: device-side wait ran out (status {v}); results of the last calls are invalid")
 
 

@@ -644,7 +644,8 @@ def tree_attn_rows(qt, kt, vt_t, q_src, krange, scale, q_rows=None, one_pass=Tru
 
 
 def gather_rows(rows, a, b=None):
-    """a[rows] (and b[rows]) of contiguous matrices, one launch. rows int64."""
+    """a[rows] (and b[rows]) of contiguous matrices, one launch. rows int64; -n counts from the end, an index outside gives a row of
+    not-a-numbers and is reported through the status word (_lib.check_status raises)."""
     _chk(rows, a, b)
     S = rows.numel()
     outs = [torch.empty((S,) + tuple(t.shape[1:]), dtype=t.dtype, device=t.device) for t in (a, b) if t is not None]
@@ -654,7 +655,7 @@ def gather_rows(rows, a, b=None):
     if b is not None and b.shape[0] != a.shape[0]:
         raise RuntimeError("gather_rows: both matrices need the same number of rows")
     call("ojb_gather_rows", ptr(rows), i64(S), i64(a.shape[0]), ptr(a), ptr(outs[0]), i64(size[0]), ptr(b), ptr(outs[1] if b is not None else None),
-         i64(size[1] if b is not None else 0), stream_ptr())
+         i64(size[1] if b is not None else 0), ptr(_lib.status_word(a.device)), stream_ptr())
     return outs if b is not None else outs[0]
 
 
@@ -700,9 +701,12 @@ def embed_rope(ids, table, pos, inv_freq, scaling=1.0):
 # ------------------------------------------------------------------------------------------------ scoring head
 def score_head(hn, rows, W, bias):
     """hn bf16 [N, H], rows int64 [S] or None (every row of hn), W f32 [A, H], bias f32 [A] or None -> f32 [S, A] (gather + fp32 linear in one
-    launch; the reference does `head(hn[lastidx].float())` with torch, src/server.py:37)."""
+    launch; the reference does `head(hn[lastidx].float())` with torch, src/server.py:37). Indices as in gather_rows."""
     _chk(hn, rows, W, bias)
+    if rows is not None and rows.dtype != torch.int64:
+        raise RuntimeError("score_head: int64 rows expected")
     S, (A, H) = hn.shape[0] if rows is None else rows.numel(), W.shape
     out = torch.empty(S, A, dtype=torch.float32, device=hn.device)
-    call("ojb_score_head", ptr(hn), ptr(rows), ptr(W), ptr(bias), ptr(out), i64(S), i64(A), i64(H), stream_ptr())
+    call("ojb_score_head_rows", ptr(hn), i64(hn.shape[0]), ptr(rows), ptr(W), ptr(bias), ptr(out), i64(S), i64(A), i64(H),
+         ptr(_lib.status_word(hn.device)), stream_ptr())
     return out

@@ -352,9 +352,14 @@ class FastQwen35(torch.nn.Module):
     # 2540 / 2418.
     ASKED_MIN_ROWS = 160
 
+    @staticmethod
+    def _plain_index(i):
+        """Whether the library's kernels take this index; torch takes the others."""
+        return i.dtype == torch.int64 and i.is_cuda and i.is_contiguous()
+
     def _asked_rows_only(self, lay, N):
         i = lay.lastidx
-        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and i.dtype == torch.int64 and i.is_cuda and i.is_contiguous()
+        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and self._plain_index(i)
 
     def _mix_asked(self, i, h, hn, rows, lay, cos, sin, linear):
         """Token mixer of the last layer (i) for the asked rows: (their residual stream, their mixer output)."""
@@ -376,9 +381,12 @@ class FastQwen35(torch.nn.Module):
     @torch.no_grad()
     def forward_gtree(self, ids, lay, return_all=False):
         """src/fastmodel.py:400-482: ids int64 [N] packed rows, lay from gtree_build -> bf16 [S, H] (final norm applied) of
-        every candidate's last row; return_all=True gives all N rows."""
+        every candidate's last row; return_all=True gives all N rows. lay.lastidx: -n counts from the end; an index outside gives
+        not-a-numbers and is reported through the status word (_lib.check_status)."""
         hn, rows = self._forward(ids, lay, return_all)
-        return hn if return_all or rows is None else hn[rows]
+        if return_all or rows is None:
+            return hn
+        return K.gather_rows(rows, hn) if self._plain_index(rows) else hn[rows]
 
     def _forward(self, ids, lay, return_all=False):
         """(final-norm hidden states, the rows of them that are asked for — None when those are all)."""
@@ -410,6 +418,8 @@ class FastQwen35(torch.nn.Module):
     def score_gtree(self, ids, lay, head_w, head_b=None):
         """Forward + scoring head: fp32 [S, A] (src/server.py:37 `head(forward_gtree(ids, lay).float())`)."""
         hn, rows = self._forward(ids, lay)
+        if rows is not None and not self._plain_index(rows):
+            hn, rows = hn[rows], None
         return K.score_head(hn, rows, head_w, head_b)
 
     # ------------------------------------------------------------------------------------------------ single-level tree

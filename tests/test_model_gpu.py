@@ -176,6 +176,37 @@ def test_last_layer_on_the_asked_rows(case, last, head_dim, fp8, monkeypatch):
     assert (got_s - want_s).norm() <= (2e-2 if fp8 else 6e-3) * want_s.norm().clamp_min(1.0)
 
 
+@pytest.mark.parametrize("last", ["full_attention", "linear_attention"])
+@pytest.mark.parametrize("asked", [False, True])
+@pytest.mark.parametrize("fp8", [False, True])
+def test_last_rows_by_index_from_the_end_and_outside(last, asked, fp8, monkeypatch):
+    """lay.lastidx follows one rule whether the last layer runs on every row or on the asked ones: -n counts from the end (the same
+    bits as the row it stands for), an index outside gives not-a-numbers for its candidate alone and an error from check_status."""
+    from ojb200 import fastmodel as FM
+    from ojb200 import modelgen as MG, _lib
+    cfg = MG.make_config(**dict(MG.SMALL, head_dim=256, num_hidden_layers=2, layer_types=["linear_attention", last]))
+    fast = FM.FastQwen35(MG.build_core(cfg, device="cpu", seed=3, std=0.05, draw_on="cpu").to("cuda"), fp8=fp8)
+    W, b = MG.make_head(cfg.hidden_size, A=2, seed=1, device="cuda")
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()["baseline"]
+    ids, lay = fast.gtree_build([[t % cfg.vocab_size for t in s] for s in seqs], groups, pad_id, NB, PB, dev="cuda")
+    monkeypatch.setattr(FM.FastQwen35, "ASKED_MIN_ROWS", 1 if asked else 1 << 30)
+    last_rows = lay.lastidx.clone()
+    assert fast._asked_rows_only(lay, lay.N) == asked and last_rows.numel() >= 3
+    want, want_s = fast.forward_gtree(ids, lay), fast.score_gtree(ids, lay, W, b)
+    lay.lastidx = last_rows - lay.N
+    assert torch.equal(fast.forward_gtree(ids, lay), want) and torch.equal(fast.score_gtree(ids, lay, W, b), want_s)
+    _lib.check_status()
+    keep = torch.arange(last_rows.numel(), device="cuda") != 1
+    for bad in (lay.N, -lay.N - 1):
+        lay.lastidx = last_rows.clone()
+        lay.lastidx[1] = bad
+        for call, ref in ((lambda: fast.forward_gtree(ids, lay), want), (lambda: fast.score_gtree(ids, lay, W, b), want_s)):
+            got = call()
+            with pytest.raises(RuntimeError, match="row index"):
+                _lib.check_status()
+            assert bool(torch.isnan(got[1]).all()) and torch.equal(got[keep], ref[keep])
+
+
 def _small_model(seed=0):
     from ojb200 import modelgen as MG
     cfg = MG.make_config(**MG.SMALL)

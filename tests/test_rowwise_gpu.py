@@ -163,6 +163,32 @@ def test_gather_rows(rows):
     assert torch.equal(ga, a[idx]) and torch.equal(gb, b[idx]) and torch.equal(K.gather_rows(idx, b), b[idx])
 
 
+def test_row_indices_count_from_the_end_and_an_index_outside_is_reported():
+    """One rule for the row indices of gather_rows and score_head: [-n, n) as torch has it; outside, not-a-numbers in that row alone
+    and an error from check_status, once."""
+    from ojb200 import ext as K, _lib
+    n = 50
+    a, b = _randn(n, 24, seed=15).cuda(), torch.randn(n, 8, generator=torch.Generator().manual_seed(3)).cuda()
+    W, bias = torch.randn(3, 24, device="cuda"), torch.randn(3, device="cuda")
+    ok = torch.tensor([-1, 0, -n, n - 1, -7], device="cuda")
+    ga, gb = K.gather_rows(ok, a, b)
+    assert torch.equal(ga, a[ok]) and torch.equal(gb, b[ok])
+    same = K.score_head(a, ok % n, W, bias)
+    assert torch.equal(K.score_head(a, ok, W, bias), same)
+    _lib.check_status()
+    for bad in (n, -n - 1, 1 << 40, -(1 << 62)):
+        idx = ok.clone()
+        idx[2] = bad
+        keep = torch.tensor([0, 1, 3, 4], device="cuda")
+        for call, wants in ((lambda: K.gather_rows(idx, a, b), (a[ok], b[ok])), (lambda: [K.gather_rows(idx, a)], (a[ok],)),
+                            (lambda: [K.score_head(a, idx, W, bias)], (same,))):
+            for got, want in zip(call(), wants):
+                assert torch.equal(got[keep], want[keep]) and bool(torch.isnan(got[2]).all())
+            with pytest.raises(RuntimeError, match="row index"):
+                _lib.check_status()
+            _lib.check_status()
+
+
 @pytest.mark.parametrize("rows", [1, 295, 296, 297, 400])          # one wide CTA per row up to 296 rows, a narrow one above
 @pytest.mark.parametrize("H,S", [(8, 0), (256, 1), (5120, 3), (8192, 6)])
 def test_resnorm_f32_and_its_e4m3_form(rows, H, S):
