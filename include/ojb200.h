@@ -107,8 +107,9 @@ int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_spl
 int ojb_gemm_set_wait_limit_ms(int32_t ms);
 
 /* Failure injection for the tests of that path (host-side switch, off by default): while on, the producer warp of the 128-row
- * tile kernel (variants 1 / 2) announces the bytes of the second k-block it handles but does not issue the copies, so the
- * consumer's bounded wait runs out as described above. Nothing faults, traps or spins without a limit. */
+ * tile kernel (variants 1 / 2), of the few-row kernel (variant 1024: second stage), of the one-pass attention (second half of the first
+ * keys) and of the Gated DeltaNet state pass (second step) announces the bytes of the second piece it handles but does not issue
+ * the copies, so the consumer's bounded wait runs out as described above. Nothing faults, traps or spins without a limit. */
 int ojb_gemm_test_drop_copy(int32_t on);
 
 /* Measurement hook of the 256-row block GEMM kernel and the CTA-pair kernel (no counterpart in the reference). `records` =
@@ -376,10 +377,10 @@ int ojb_tree_attn_set_trace(uint64_t* records);
  * hn bf16 [N, H] (final-norm output), rows int64 [S] (last row of each candidate; null: row s), W fp32 [A, H], bias fp32 [A] or null. */
 int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S, int64_t A,
                    int64_t H, ojb_stream_t stream);
-
 /* The same with the row count of hn: indices as in ojb_gather_rows, the scores of one outside are not-a-number. */
 int ojb_score_head_rows(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
                         int64_t A, int64_t H, int32_t* status, ojb_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -238,7 +238,7 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       const Unit u = decode_unit(g, unit, total_block);
       const bool tracing = g.trace != nullptr && warp == 2 && lane == 0;
       const unsigned long long t_begin = tracing ? global_timer_ns() : 0ull;
-      if (!mbar_wait(accfull, acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(accfull, acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const unsigned long long t_full = tracing ? global_timer_ns() : 0ull;
       const uint32_t tlane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);

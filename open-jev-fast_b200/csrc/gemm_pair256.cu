@@ -296,7 +296,7 @@ gemm_pair256_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_con
       const uint32_t use = static_cast<uint32_t>(nbuf == 2 ? (it >> 1) : it);
       const bool tracing = g.trace != nullptr && warp == 2 && lane == 0 && leader;
       const unsigned long long t_begin = tracing ? global_timer_ns() : 0ull;
-      if (!mbar_wait(accfull0 + 8 * buf, use & 1u, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(accfull0 + 8 * buf, use & 1u, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const unsigned long long t_full = tracing ? global_timer_ns() : 0ull;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf) * kAccCols;

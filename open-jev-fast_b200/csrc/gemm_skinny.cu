@@ -122,7 +122,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     }
   } else {
     const int quarter = warp & 3, row = quarter * 32 + lane;
-    if (mbar_wait(accfull, 0, abort_flag)) {
+    if (mbar_wait_warp(accfull, 0, abort_flag)) {
       tc_fence_after();
       if (quarter * 32 < g.M) {
         const bool row_ok = row < g.M;

@@ -163,7 +163,7 @@ gemm_tile128_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const int m_blk = unit % g.num_m;
       const int rest = unit / g.num_m;
       const int split = rest % g.splits, n_blk = rest / g.splits;
-      if (!mbar_wait(accfull0 + 8 * acc, acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(accfull0 + 8 * acc, acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const int row = m_blk * kBM + quarter * 32 + lane;
       const bool row_ok = row < g.M;

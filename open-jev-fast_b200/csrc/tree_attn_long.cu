@@ -47,7 +47,7 @@ struct LongArgs {
   int32_t* status;
   int N, NQ, HQ, HKV, G, hp, R;      // hp heads x R query rows = 128
   float scale_log2e;
-  int wait_ms;
+  int wait_ms, drop_copy;
   const int64_t* q_rows;
   int64_t gate_ld;
   int gate_hs;
@@ -186,7 +186,8 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         for (int c = 0; c < 2 && ok; ++c) {      // 128 dims
           uint32_t dst, fb;
           if (!(ok = slot(dst, fb))) break;
-          if (one) tma_load_3d(dst, &map_k, fb, 0, kvh * N + kb * kLKeys, 2 * c);
+          if (one && !(g.drop_copy && use == 2))      // tests only: the announced bytes of the second entry never arrive
+            tma_load_3d(dst, &map_k, fb, 0, kvh * N + kb * kLKeys, 2 * c);
         }
       };
       auto values = [&](int kb) {
@@ -272,7 +273,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     int kb = T > 0 ? next_block(0) : 0;
     for (int j = 0; j < T && ok; ++j) {
       const int sb = j & 1;
-      if (!mbar_wait(bar(kLBarSFull + sb), (j >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(kLBarSFull + sb), (j >> 1) & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t s[2][32];
       const uint32_t ts = tmem_base + lanes + kLColS + static_cast<uint32_t>(sb * kLKeys + half * 64);
@@ -300,7 +301,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       x[half * 128 + my] = mx;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(kLBarX + quarter));
-      if (!mbar_wait(bar(kLBarX + quarter), j & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(bar(kLBarX + quarter), j & 1, abort_flag)) { ok = false; break; }
       mx = fmaxf(mx, x[(half ^ 1) * 128 + my]);
       const bool move = mx > m && (m == -INFINITY || (mx - m) * c > kLStale);
       const float f = move && m != -INFINITY ? exp2f_fast((m - mx) * c) : 1.f;      // (a row that has seen no key has O = 0 and l = 0)
@@ -319,7 +320,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
       if (__any_sync(0xffffffffu, f != 1.f)) {
         // P V of the block before has left O at rest, that of this block is not issued before P is there
-        if (!mbar_wait(bar(kLBarRest), (j & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(kLBarRest), (j & 1) ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int i = 0; i < 8; ++i) {
@@ -341,15 +342,15 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (j + 1 < T) kb = next_block(kb + 1);
     }
     // ---- att = bf16(O / l) into the staging tile (which the Q rows must not be on their way to any more)
-    if (T == 0) ok = mbar_wait(bar(kLBarQ), 0, abort_flag);
+    if (T == 0) ok = mbar_wait_warp(bar(kLBarQ), 0, abort_flag);
     if (T > 0 && ok) {
       float* x = xch + (T & 1) * 256;
       x[half * 128 + my] = l;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(kLBarX + quarter));
-      ok = mbar_wait(bar(kLBarX + quarter), T & 1, abort_flag);
+      ok = mbar_wait_warp(bar(kLBarX + quarter), T & 1, abort_flag);
       l += x[(half ^ 1) * 128 + my];
-      if (ok) ok = mbar_wait(bar(kLBarO), 0, abort_flag);
+      if (ok) ok = mbar_wait_warp(bar(kLBarO), 0, abort_flag);
     }
     if (ok) {
       tc_fence_after();
@@ -431,6 +432,7 @@ int tree_attn_long_launch(const void* qt, int64_t NQ, const int64_t* q_rows, con
   a.HKV = static_cast<int>(HKV);
   a.scale_log2e = scale * 1.4426950408889634f;
   a.wait_ms = gemm_wait_limit_ms();
+  a.drop_copy = gemm_drop_copy();
   a.q_rows = q_rows;
   a.gate_ld = gate_ld;
   a.gate_hs = static_cast<int>(gate_hs);

@@ -301,7 +301,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       xch[(2 * slot + half) * 128 + my] = v;
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(kBarX));
-      if (!mbar_wait(bar(kBarX), xphase & 1, abort_flag)) { ok = false; return v; }
+      if (!mbar_wait_warp(bar(kBarX), xphase & 1, abort_flag)) { ok = false; return v; }
       ++xphase;
       return xch[(2 * slot + (half ^ 1)) * 128 + my];
     };
@@ -317,7 +317,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
       // (pass 2 of the one-pass form reads scores that pass 1 has already waited for)
       if (!(one_pass && pass2)) {
-        if (!mbar_wait(bar(kBarSFull + sb), use_s[sb] & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(kBarSFull + sb), use_s[sb] & 1, abort_flag)) { ok = false; break; }
         ++use_s[sb];
       }
       if (stamp && (it == 0 || it == nvis)) trace[it == 0 ? 2 : 3] = global_timer_ns();   // first S of pass 1 / pass 2
@@ -357,7 +357,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             pk[i * 16 + (c >> 1)] = pack2(p0, p1);
           }
         // P V of the previous block must have read P before this block's P is written
-        if (!mbar_wait(bar(kBarPFree), (blk & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(kBarPFree), (blk & 1) ^ 1, abort_flag)) { ok = false; break; }
         // row `my` of the K-major swizzled tile: each 64-key k-block is 128 bytes = 8 chunks of 16, chunk c stored at
         // c ^ (row & 7); this thread's columns start at chunk (half * kCols % 64) / 8 of k-block half * kCols / 64
         uint8_t* prow = Ps + ((half * kCols) / 64) * (128 * 128) + my * 128;
@@ -377,7 +377,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     //      region 0, which no MMA reads any more once O is complete); rows are 16 bytes longer than 512 so that the 32 rows of
     //      a warp spread over the banks
     prefetch_gates(tid);
-    if (ok) ok = mbar_wait(bar(kBarO), 0, abort_flag);
+    if (ok) ok = mbar_wait_warp(bar(kBarO), 0, abort_flag);
     if (stamp) trace[5] = global_timer_ns();                  // O complete
     if (ok) {
       tc_fence_after();

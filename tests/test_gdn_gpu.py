@@ -137,7 +137,8 @@ def test_prep_rows_and_scatter(name):
         assert torch.equal(got.cpu(), O.scatter_slots(rows.cpu(), src))
 
 
-def test_state_pass_bounded_wait_runs_out_and_reports_through_the_status_word():
+@pytest.mark.parametrize("B,HV", [(2, 4), (5, 32)])          # 32 and 640 CTAs: the full form, and the dense one (two to an SM)
+def test_state_pass_bounded_wait_runs_out_and_reports_through_the_status_word(B, HV):
     """The state pass waits for the bulk copies of each step's operands on an mbarrier, with the library's wait limit. With the
     limit at 50 ms and the host-side failure switch on, the copies of the second step are announced but never issued: the wait
     runs out, every CTA leaves its walk, the status word says so, and the next call on the same context is correct."""
@@ -145,7 +146,7 @@ def test_state_pass_bounded_wait_runs_out_and_reports_through_the_status_word():
     import time
     from ojb200 import ext as K, _lib
     lib = _lib.lib()
-    B, T, HK, HV = 2, 150, 2, 4
+    T, HK = 150, 2
     g_ = torch.Generator().manual_seed(12)
     q = torch.nn.functional.normalize(torch.randn(B * T, HK, 128, generator=g_), dim=-1).to(bf16).cuda()
     k = torch.nn.functional.normalize(torch.randn(B * T, HK, 128, generator=g_), dim=-1).to(bf16).cuda()

@@ -287,6 +287,42 @@ def test_few_row_kernel(M, N, K):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("e4m3", [False, True])
+def test_few_row_kernel_bounded_wait(e4m3):
+    """The copies of the few-row kernel's second stage are announced but never issued (host-side switch), the limit is 50 ms: the waits
+    run out, every warp leaves as a whole, the status word says so, and the next call is correct."""
+    import ctypes
+    import time
+    from ojb200 import lt_ext as LT, _lib
+    lib = _lib.lib()
+    x, w = _mk(12, 1000, 2560, 5)
+    if e4m3:
+        xq, wq = LT.quantize_rows_e4m3(x), LT.quantize_weight_e4m3(w)
+        run = lambda: LT.gemm_e4m3(*xq, *wq, 0)
+    else:
+        run = lambda: LT.lt_matmul(x, w, 11)
+    good = run()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    try:
+        assert lib.ojb_gemm_set_wait_limit_ms(ctypes.c_int32(50)) == 0
+        assert lib.ojb_gemm_test_drop_copy(ctypes.c_int32(1)) == 0
+        t0 = time.perf_counter()
+        run()
+        torch.cuda.synchronize()
+        dt = time.perf_counter() - t0
+    finally:
+        lib.ojb_gemm_test_drop_copy(ctypes.c_int32(0))
+        lib.ojb_gemm_set_wait_limit_ms(ctypes.c_int32(0))
+    assert dt < 1.5, dt
+    with pytest.raises(RuntimeError, match="wait ran out"):
+        _lib.check_status()
+    again = run()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(again, good)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 24, 128), (7, 264, 384), (32, 2048, 1280), (12, 1000, 640)])
 def test_few_row_kernel_e4m3(M, N, K):
     """Its 8-bit form against the same products in 64 bits (e4m3 products are exact in fp32)."""

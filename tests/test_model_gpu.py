@@ -149,6 +149,42 @@ def test_one_pass_attention(N_case, HQ, HKV, spread):
         assert (got[keep] - want[keep]).abs().max().item() < 6e-2
 
 
+def test_one_pass_attention_bounded_wait():
+    """The second half of the first keys is announced but never copied (host-side switch), the limit is 50 ms: the issuer's wait runs
+    out, the softmax warps see the flag and leave as whole warps, the status word says so, and the next call is correct."""
+    import ctypes
+    import time
+    from ojb200 import ext as K, _lib
+    lib = _lib.lib()
+    HQ, HKV, N = 12, 2, 1000
+    g = torch.Generator(device="cuda").manual_seed(33)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(bf16)
+    qt, kt, vt_t, q_src = rnd(HQ, N, 256), rnd(HKV, N, 256), rnd(HKV, 256, N), rnd(N, HQ * 512)
+    krange = torch.zeros(N, 8, dtype=torch.int32, device="cuda")
+    krange[:, 0] = torch.arange(1, N + 1)                                # keys [0, row]
+    run = lambda: K.tree_attn_rows(qt, kt, vt_t, q_src, krange, 1 / 16)
+    good = run()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    try:
+        assert lib.ojb_gemm_set_wait_limit_ms(ctypes.c_int32(50)) == 0
+        assert lib.ojb_gemm_test_drop_copy(ctypes.c_int32(1)) == 0
+        t0 = time.perf_counter()
+        run()
+        torch.cuda.synchronize()
+        dt = time.perf_counter() - t0
+    finally:
+        lib.ojb_gemm_test_drop_copy(ctypes.c_int32(0))
+        lib.ojb_gemm_set_wait_limit_ms(ctypes.c_int32(0))
+    assert dt < 1.5, dt
+    with pytest.raises(RuntimeError, match="wait ran out"):
+        _lib.check_status()
+    again = run()
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(again, good)
+
+
 @pytest.mark.parametrize("case", ["doc", "baseline", "nostem"])
 @pytest.mark.parametrize("last", ["full_attention", "linear_attention"])
 @pytest.mark.parametrize("head_dim,fp8", [(256, False), (256, True), (64, False)])
