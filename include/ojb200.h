@@ -92,6 +92,10 @@ int ojb_quantize_rows_e4m3(const void* x, void* q, float* scale, int64_t rows, i
 int64_t ojb_gemm_unit_order(int32_t n_xblk, int32_t tail_rows, int32_t n_xchunk, int32_t BN, int64_t N, int32_t splits,
                             int32_t kb_total, int32_t band_xblk, int32_t* out, int64_t cap);
 
+/* Host-side check (no GPU work): 256-row x blocks per band of that kernel for n_xblk of them, K elements of elt bytes to a row; 0: no
+ * bands. OJB_GEMM_BAND_BLOCKS and OJB_GEMM_BAND_MB in the environment change it for measurements (read once). */
+int ojb_gemm_band_blocks(int32_t n_xblk, int64_t K, int32_t elt);
+
 /* Host-side plan (no GPU work): which kernel variant and how many K ranges the library's cost model picks for a shape.
  * kind = 0 bf16 output, 1 SwiGLU-fused, 2 fp32 split-K partials, 3 those of an 8-bit product with K counted in pairs of
  * elements (the kinds that may use more than one range, up to max_splits). *microseconds (optional) receives the modelled time. Takes the place of the algorithm search of

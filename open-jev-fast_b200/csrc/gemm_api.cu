@@ -174,6 +174,10 @@ extern "C" int ojb_gemm_set_probe(int32_t mma_repeat, int32_t knob) {
 }
 #endif
 
+extern "C" int ojb_gemm_band_blocks(int32_t n_xblk, int64_t K, int32_t elt) {
+  return n_xblk > 0 && K > 0 && (elt == 1 || elt == 2) ? band_blocks(n_xblk, 256 * K * elt) : 0;
+}
+
 extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_splits, int32_t* variant, int32_t* splits,
                              float* microseconds) {
   OJB_REQUIRE(M > 0 && N > 0 && K > 0 && kind >= 0 && kind <= 3 && max_splits >= 1 && max_splits <= 16 && variant && splits);

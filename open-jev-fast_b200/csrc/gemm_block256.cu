@@ -653,19 +653,7 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   if (FP8 && g.BN % 64 != 0) g.BN = (g.BN + 63) / 64 * 64;      // whole 128-byte store tiles (the scaled epilogue needs them)
   g.n_wtile = static_cast<int>(ceil_div(N, g.BN));
   g.n_wtile256 = static_cast<int>(ceil_div(N, 256));
-  {
-    // x beyond what the L2 keeps beside the streaming weight (64 MB) and at least 24 x blocks (with fewer, the CTAs that
-    // run at the same time already cover several weight tiles per x block, and x is re-read only a few times): bands of about
-    // 16 x blocks, equal in size, so that the units under way at any time share both their x blocks and their w tiles about
-    // twelve times (bands of a fixed 40 MB were 4 blocks at K = 17 408). 16 672 rows, blocks per band 8 / 11 / 16 / 22 / 33:
-    // gate/up 4345 / 4329 / 4275 / 4412 / 4554 us, [12352, 5120] 1538 / 1520 / 1496 / 1556 / 1593, [5120, 17408] 2288 / 2283 / 2319 /
-    // 2308 / 2434. OJB_GEMM_BAND_BLOCKS changes the band size (0 = no bands) for measurements.
-    const int64_t xblk_bytes = static_cast<int64_t>(kBlockM) * K * (FP8 ? 1 : 2);
-    static const int band_blocks = [] { const char* e = getenv("OJB_GEMM_BAND_BLOCKS"); return e ? atoi(e) : 16; }();
-    g.band_xblk = 0;
-    if (band_blocks > 0 && g.n_xblk >= 24 && static_cast<int64_t>(g.n_xblk) * xblk_bytes > (64ll << 20))
-      g.band_xblk = static_cast<int>(ceil_div(g.n_xblk, ceil_div(g.n_xblk, band_blocks)));
-  }
+  g.band_xblk = band_blocks(g.n_xblk, static_cast<int64_t>(kBlockM) * K * (FP8 ? 1 : 2));
   const int b_rows = g.n_xblk > 0 ? (g.BN > g.tail_box ? g.BN : g.tail_box) : g.tail_box;
   g.stage_bytes = kABytes + static_cast<uint32_t>(b_rows) * (kBK * 2);
   {

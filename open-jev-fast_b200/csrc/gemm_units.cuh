@@ -118,6 +118,28 @@ __host__ __device__ __forceinline__ Unit decode_unit(const GemmArgs& g, int unit
   return u;
 }
 
+// x blocks per band (0: no bands) for n_xblk blocks of xblk_bytes. x beyond what the L2 keeps beside the streaming weight (64 MB) and
+// at least 24 x blocks (with fewer, the CTAs that run at the same time already cover several weight tiles per x block, and x is
+// re-read only a few times): bands of about 16 x blocks, equal in size, so that the units under way at any time share both their x
+// blocks and their w tiles about twelve times (bands of a fixed 40 MB were 4 blocks at K = 17 408). 16 672 rows, blocks per band
+// 8 / 11 / 16 / 22 / 33: gate/up 4345 / 4329 / 4275 / 4412 / 4554 us, [12352, 5120] 1538 / 1520 / 1496 / 1556 / 1593, [5120, 17408]
+// 2288 / 2283 / 2319 / 2308 / 2434. For measurements OJB_GEMM_BAND_BLOCKS sets the blocks of a band, OJB_GEMM_BAND_MB its size in MB
+// (at least two blocks); 0 switches bands off. With both set the blocks count.
+inline int band_blocks(int n_xblk, int64_t xblk_bytes) {
+  static const char* const blocks_env = getenv("OJB_GEMM_BAND_BLOCKS");
+  static const char* const mb_env = getenv("OJB_GEMM_BAND_MB");
+  int64_t per = 16;
+  if (blocks_env != nullptr) {
+    per = atoi(blocks_env);
+  } else if (mb_env != nullptr) {
+    const int64_t mb = atoi(mb_env);
+    per = mb <= 0 ? 0 : (mb << 20) / xblk_bytes;
+    if (mb > 0 && per < 2) per = 2;
+  }
+  if (per <= 0 || n_xblk < 24 || n_xblk * xblk_bytes <= (64ll << 20)) return 0;
+  return static_cast<int>(ceil_div(n_xblk, ceil_div(n_xblk, per)));
+}
+
 // ---- Cost model (host). Times are SM clocks; the constants come from unit timelines measured on B200 (ojb_gemm_set_trace):
 // the main loops are bound by shared-memory bandwidth (128 bytes per clock per SM shared between the TMA fill of a stage
 // and the operand reads of its MMAs), an MMA with M = 128 never takes less than 64 clocks, a k-block of a

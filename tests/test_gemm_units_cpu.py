@@ -2,6 +2,9 @@
 (x block or chunk, K range, w tile) occurs exactly once, the units of one w tile are adjacent, and with bands — x larger than
 the L2 — every unit of a band comes before the units of the next band. No GPU."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -96,3 +99,24 @@ def test_plan_is_the_same_from_every_thread():
 
     with ThreadPoolExecutor(8) as pool:
         assert all(pool.map(ask, range(8)))
+
+
+@pytest.mark.parametrize("env,want", [
+    ({}, [13, 13, 0, 0]),                                               # five bands of 16 blocks at most
+    ({"OJB_GEMM_BAND_MB": "40"}, [13, 4, 0, 0]),                        # 16 blocks of 2.5 MB, or 4 of 8.5 MB
+    ({"OJB_GEMM_BAND_MB": "1"}, [2, 2, 0, 0]),                          # never less than two blocks
+    ({"OJB_GEMM_BAND_MB": "0"}, [0, 0, 0, 0]),
+    ({"OJB_GEMM_BAND_BLOCKS": "8"}, [8, 8, 0, 0]),
+    ({"OJB_GEMM_BAND_BLOCKS": "0"}, [0, 0, 0, 0]),
+    ({"OJB_GEMM_BAND_BLOCKS": "8", "OJB_GEMM_BAND_MB": "40"}, [8, 8, 0, 0]),
+])
+def test_band_size_and_its_switches(env, want):
+    """Blocks per band at 65 x blocks of K = 5120 and 17 408, at 23 blocks, and where x fits the L2: the rule, and both switches (read
+    once per process)."""
+    code = ("import ctypes; from ojb200 import _lib; f = _lib.lib().ojb_gemm_band_blocks; "
+            "print([f(n, ctypes.c_int64(k), 2) for n, k in ((65, 5120), (65, 17408), (23, 17408), (24, 5120))])")
+    clean = {k: v for k, v in os.environ.items() if not k.startswith("OJB_GEMM_BAND")}
+    path = os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__)))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(clean, PYTHONPATH=path, **env), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip().splitlines()[-1] == str(want)
