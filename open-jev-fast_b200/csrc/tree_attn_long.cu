@@ -18,7 +18,7 @@
 // the issuing thread a wait and a commit, 0.2-0.3 us together: with seven 16 KB entries and P in shared memory a block took 2.5 us
 // of which the tensor pipe needs 1.1.
 // Roles: warps 0-7 softmax and epilogue, warp 8 TMA producer, warp 9 MMA issuer; every wait bounded.
-#include "gemm_common.cuh"
+#include "tree_attn_rows.cuh"
 
 namespace ojb {
 namespace {
@@ -51,6 +51,7 @@ struct LongArgs {
   const int64_t* q_rows;
   int64_t gate_ld;
   int gate_hs;
+  const bf16_t *qt, *kt, *vt_t;
 };
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -84,13 +85,6 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// keys [32 * w, 32 * w + 32) that fall in [lo, hi)
-__device__ __forceinline__ uint32_t key_bits(int lo, int hi, int w) {
-  const int a = max(lo - w * 32, 0), b = min(hi - w * 32, 32);
-  if (a >= b) return 0u;
-  return (b == 32 ? 0xffffffffu : ((1u << b) - 1u)) & ~((1u << a) - 1u);
-}
 
 __global__ void __launch_bounds__(kLThreads, 1)
 tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -286,7 +280,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int w = k0 / 32 + i;
-          const uint32_t bits = key_bits(lo0, hi0, w) | key_bits(lo1, hi1, w) | key_bits(lo2, hi2, w);
+          const uint32_t bits = range_bits(lo0, hi0, w) | range_bits(lo1, hi1, w) | range_bits(lo2, hi2, w);
 #pragma unroll
           for (int e = 0; e < 32; ++e)
             if (!((bits >> e) & 1u)) s[i][e] = 0xff800000u;      // -infinity
@@ -356,6 +350,7 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       tc_fence_after();
       const float inv = l > 0.f ? 1.0f / l : 0.f;
       uint8_t* srow = smem + my * kLPitch;
+      float odd = 0.f;                   // not-a-number if a value of O is not finite
 #pragma unroll 1
       for (int i = 0; i < 4; ++i) {
         const int col = half * 4 + i;
@@ -368,9 +363,20 @@ tree_attn_long_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         for (int v = 0; v < 4; ++v) {
           float a[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) a[e] = l > 0.f ? __uint_as_float(o[v * 8 + e]) * inv : 0.f;      // no visible key: zeros
+          for (int e = 0; e < 8; ++e) {
+            a[e] = l > 0.f ? __uint_as_float(o[v * 8 + e]) * inv : 0.f;      // no visible key: zeros
+            odd = fmaf(a[e], 0.f, odd);
+          }
           *reinterpret_cast<uint4*>(srow + col * 64 + v * 16) = pack8(a);
         }
+      }
+      for (uint32_t again = __ballot_sync(0xffffffffu, odd != odd); again != 0u; again &= again - 1u) {
+        const int src = __ffs(again) - 1, row = quarter * 32 + src;
+        auto of = [&](auto x) { return __shfl_sync(0xffffffffu, x, src); };
+        const float4 a = row_over_its_keys(
+            g.qt + (static_cast<int64_t>(hq0 + row / g.R) * g.NQ + r0 + row % g.R) * kLD, g.kt + static_cast<int64_t>(kvh) * N * kLD,
+            g.vt_t + static_cast<int64_t>(kvh) * kLD * N, N, half * 128, of(lo0), of(hi0), of(lo1), of(hi1), of(lo2), of(hi2), c, of(m) * c, of(inv));
+        *reinterpret_cast<uint2*>(smem + row * kLPitch + half * 256 + lane * 8) = make_uint2(pack2(a.x, a.y), pack2(a.z, a.w));
       }
     }
   }
@@ -436,6 +442,9 @@ int tree_attn_long_launch(const void* qt, int64_t NQ, const int64_t* q_rows, con
   a.q_rows = q_rows;
   a.gate_ld = gate_ld;
   a.gate_hs = static_cast<int>(gate_hs);
+  a.qt = static_cast<const bf16_t*>(qt);
+  a.kt = static_cast<const bf16_t*>(kt);
+  a.vt_t = static_cast<const bf16_t*>(vt_t);
   launch_kernel(tree_attn_long_kernel, dim3(static_cast<unsigned>(HKV * (a.G / a.hp)), static_cast<unsigned>(ceil_div(NQ, a.R))),
                 dim3(kLThreads), kLSmem, st, map_q, map_k, map_vt, a);
   return launch_status(cudaGetLastError());

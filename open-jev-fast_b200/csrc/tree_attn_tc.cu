@@ -24,7 +24,7 @@
 // their loads). An odd number of visible blocks repeats the last one as the second half of the last pair, masked out.
 // Roles: warps 0-7 softmax / epilogue, warp 8 TMA producer, warp 9 MMA issuer; mbarriers between them, every wait bounded (the
 // CTA then reports OJB_DEV_WAIT_TIMEOUT through `status`, frees its tensor memory and returns).
-#include "gemm_common.cuh"
+#include "tree_attn_rows.cuh"
 
 namespace ojb {
 namespace {
@@ -69,15 +69,8 @@ struct AttnArgs {
   const int64_t* q_rows;     // null, or the row of krange that query row n goes by
   int64_t gate_ld;           // gate: elements between rows, and between heads of a row
   int gate_hs;
+  const bf16_t *qt, *kt, *vt_t;
 };
-
-// bits of keys [32 * w, 32 * w + 32) that fall in [lo, hi)
-__device__ __forceinline__ uint32_t range_bits(int lo, int hi, int w) {
-  const int a = max(lo - w * 32, 0), b = min(hi - w * 32, 32);
-  if (a >= b) return 0u;
-  const uint32_t upto_b = b == 32 ? 0xffffffffu : ((1u << b) - 1u);
-  return upto_b & ~((1u << a) - 1u);
-}
 
 __global__ void __launch_bounds__(kTcThreads, 1)
 tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -383,6 +376,7 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       tc_fence_after();
       const float inv_l = l > 0.f ? 1.0f / l : 0.f;
       uint8_t* srow = smem + my * kStagePitch;
+      float odd = 0.f;                         // not-a-number if a value of O is not finite
 #pragma unroll
       for (int cc = 0; cc < kD / 64; ++cc) {
         const int c = half * (kD / 64) + cc;
@@ -393,9 +387,22 @@ tree_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         for (int v8 = 0; v8 < 4; ++v8) {
           float a[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) a[e] = l > 0.f ? __uint_as_float(o[v8 * 8 + e]) * inv_l : 0.f;   // a row that sees no key: zeros, whatever tensor memory holds
+          for (int e = 0; e < 8; ++e) {
+            a[e] = l > 0.f ? __uint_as_float(o[v8 * 8 + e]) * inv_l : 0.f;   // a row that sees no key: zeros, whatever tensor memory holds
+            odd = fmaf(a[e], 0.f, odd);
+          }
           *reinterpret_cast<uint4*>(srow + c * 64 + v8 * 16) = pack8(a);
         }
+      }
+      // (query rows past the last one see no key: l = 0; tile rows past the last head are nobody's)
+      for (uint32_t again = __ballot_sync(0xffffffffu, odd != odd && my < G * kQRows); again != 0u; again &= again - 1u) {
+        const int src = __ffs(again) - 1, row = (warp & 3) * 32 + src;
+        auto of = [&](auto x) { return __shfl_sync(0xffffffffu, x, src); };
+        const float4 a = row_over_its_keys(
+            g.qt + (static_cast<int64_t>(hq0 + (row >> 4)) * g.NQ + r0 + (row & 15)) * kD, g.kt + static_cast<int64_t>(kvh) * N * kD,
+            g.vt_t + static_cast<int64_t>(kvh) * kD * N, N, half * 128, of(a0), of(e0), of(a1), of(e1), of(a2), of(e2), g.scale_log2e,
+            of(m) * g.scale_log2e, of(inv_l));
+        *reinterpret_cast<uint2*>(smem + row * kStagePitch + half * 256 + lane * 8) = make_uint2(pack2(a.x, a.y), pack2(a.z, a.w));
       }
     }
   }
@@ -476,7 +483,8 @@ extern "C" int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_r
   if (!raise_smem_limit(tree_attn_tc_kernel, static_cast<int>(kSmemBytes), smem_set)) return OJB_ERR_LAUNCH;
   AttnArgs a{static_cast<const bf16_t*>(gate), krange, static_cast<bf16_t*>(y), status, static_cast<int>(N), static_cast<int>(HQ),
              static_cast<int>(HKV), static_cast<int>(HQ / HKV), scale * 1.4426950408889634f, gemm_wait_limit_ms(),
-             static_cast<int>(NQ), q_rows, gate_ld, static_cast<int>(gate_hs)};
+             static_cast<int>(NQ), q_rows, gate_ld, static_cast<int>(gate_hs), static_cast<const bf16_t*>(qt),
+             static_cast<const bf16_t*>(kt), static_cast<const bf16_t*>(vt_t)};
   launch_kernel(tree_attn_tc_kernel, dim3(static_cast<unsigned>(HKV), static_cast<unsigned>(ceil_div(NQ, kQRows))), dim3(kTcThreads),
                 kSmemBytes, static_cast<cudaStream_t>(stream), map_q, map_k, map_vt, a);
   return launch_status(cudaGetLastError());

@@ -149,6 +149,44 @@ def test_one_pass_attention(N_case, HQ, HKV, spread):
         assert (got[keep] - want[keep]).abs().max().item() < 6e-2
 
 
+@pytest.mark.parametrize("N_case,HQ,HKV", [("baseline", 24, 4), ("ragged", 4, 2), ("wide", 6, 2), ("nostem", 5, 1), ("single", 3, 3)])
+@pytest.mark.parametrize("one_pass", [False, 2])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_a_value_that_is_not_finite_reaches_the_rows_that_see_it_alone(N_case, HQ, HKV, one_pass, value):
+    """V of single keys (a leaf row, the first row of a leaf, a row of the root) not finite in some dims: rows that see the key are not
+    finite in those dims, everything else is what it is with a finite V (rows whose key block holds it are computed over their
+    own keys: fp32 sums in another order, P in bf16 on both sides)."""
+    from ojb200 import ext as K, _lib
+    from ojb200 import layout as PL
+    D = 256
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()[N_case]
+    ids, lay = PL.gtree_build(seqs, groups, pad_id, NB, PB, dev="cuda", dense=False)
+    N = lay.N
+    g = torch.Generator(device="cuda").manual_seed(37)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(bf16)
+    qt, kt, vt_t, q_src = rnd(HQ, N, D), rnd(HKV, N, D), rnd(HKV, D, N), rnd(N, HQ * 2 * D)
+    run = lambda v: K.tree_attn_rows(qt, kt, v, q_src, lay.krange, D ** -0.5, one_pass=one_pass).float().view(N, HQ, D)
+    clean = run(vt_t)
+    kr = lay.krange.long()
+    e0, a1, e1, a2, e2, a0 = (kr[:, i] for i in range(6))
+    last = int(lay.lastidx[-1])
+    for key in (last, max(last - 3, 0), int(e0[last]) // 2):
+        sees = ((a0 <= key) & (key < e0)) | ((a1 <= key) & (key < e1)) | ((a2 <= key) & (key < e2))
+        assert bool(sees[last if key == last else key])
+        bad = vt_t.clone()
+        bad[:, 3:130:7, key] = value
+        dims = torch.zeros(D, dtype=torch.bool, device="cuda")
+        dims[3:130:7] = True
+        y = run(bad)
+        hit = sees[:, None, None] & dims
+        assert not bool(torch.isfinite(y)[hit.expand_as(y)].any())
+        rest = ~hit.expand_as(y)
+        assert bool(torch.isfinite(y)[rest].all())
+        assert (y - clean)[rest].norm() <= 4e-3 * clean[rest].norm()
+        assert torch.allclose(y[rest], clean[rest], rtol=2 ** -6, atol=2 ** -7)
+    _lib.check_status()
+
+
 def test_one_pass_attention_bounded_wait():
     """The second half of the first keys is announced but never copied (host-side switch), the limit is 50 ms: the issuer's wait runs
     out, the softmax warps see the flag and leave as whole warps, the status word says so, and the next call is correct."""
