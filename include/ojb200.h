@@ -223,16 +223,10 @@ int ojb_gtree_fill(const int64_t* tokens, const int64_t* seq_off, const int32_t*
  * l2norm = 0 leaves q and k un-normalised (src/kernels.cu:96 linattn_prep and linattn_prep2 with do_l2 = false, whose callers
  * let the attention kernel normalise); every other prep variant of the reference normalises. The same entry point serves
  * the reference's older layouts (per-sequence [B, T], single-level tree, src-mapped slots): they differ only in `hist` and in
- * the slot tables, which the Python layer derives.  */
+ * the slot tables, which the Python layer derives. */
 int ojb_gdn_prep(const void* proj, const int32_t* hist, const int32_t* rep_ptr, const int32_t* rep_pos, int64_t n_slots,
                  const void* convw, const void* A_log, const void* dt_bias, void* q, void* k, void* v, float* g,
                  void* beta, int64_t N, int64_t KD, int64_t VD, int64_t HV, int64_t HK, int32_t l2norm, ojb_stream_t stream);
-/* The same; ieee != 0 (packed rows only): sigmoids with expf and an IEEE division instead of the special-function unit's exp2 and
- * reciprocal, a few units of 2^-24 apart before the rounding to bf16. */
-int ojb_gdn_prep_v(const void* proj, const int32_t* hist, const int32_t* rep_ptr, const int32_t* rep_pos, int64_t n_slots,
-                   const void* convw, const void* A_log, const void* dt_bias, void* q, void* k, void* v, float* g,
-                   void* beta, int64_t N, int64_t KD, int64_t VD, int64_t HV, int64_t HK, int32_t l2norm, int32_t ieee,
-                   ojb_stream_t stream);
 
 /* Bytes of scratch that ojb_gdn_chunked needs for n_chunks chunk-table entries and HV value heads. */
 int64_t ojb_gdn_scratch_bytes(int64_t n_chunks, int64_t HV);
@@ -316,9 +310,6 @@ int ojb_gdn_set_trace(uint64_t* records);
  * rstd = 1/sqrt(mean(x^2) + eps) over the 128 dims. x bf16 [*, HV, 128]; proj bf16 [N, P]; w bf16 [128]. */
 int ojb_gated_rmsnorm(const void* x, const int32_t* inv, const void* proj, const void* w, void* out, int64_t N,
                       int64_t HV, int64_t HD, int64_t zoff, int64_t P, float eps, ojb_stream_t stream);
-/* The same; ieee != 0: sigmoids as in ojb_gdn_prep_v (16-byte aligned operands, zoff and P multiples of 8). */
-int ojb_gated_rmsnorm_v(const void* x, const int32_t* inv, const void* proj, const void* w, void* out, int64_t N,
-                        int64_t HV, int64_t HD, int64_t zoff, int64_t P, float eps, int32_t ieee, ojb_stream_t stream);
 
 /* ------------------------------------------------------------------------------------------------------------------
  * Tree attention — replaces src/kernels.cu:4287-4458 fattn_tree (and, above 384 rows, the reference's

@@ -211,7 +211,7 @@ def attn_operands(q_src, kv_src, qw1, kw1, cosb, sinb, HQ, HKV, eps, q_rows=None
 
 
 # ------------------------------------------------------------------------------------------------ Gated DeltaNet
-def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV, HK, HD, l2norm=True, ieee=False):
+def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV, HK, HD, l2norm=True):
     _chk(proj, hist, rep_ptr, rep_pos, convw, A_log, dt_bias)
     if HD != 128 or HK * HD != KD or HV * HD != VD or convw.shape[1] != 4:
         raise RuntimeError("linattn_prep: head dim must be 128 and the conv width 4")
@@ -228,9 +228,9 @@ def _prep(proj, hist, rep_ptr, rep_pos, n_out, convw, A_log, dt_bias, KD, VD, HV
     v = torch.empty(n_out, VD, dtype=bf16, device=dev)
     g = torch.empty(n_out, HV, dtype=torch.float32, device=dev)
     beta = torch.empty(n_out, HV, dtype=bf16, device=dev)
-    call("ojb_gdn_prep_v", ptr(proj), ptr(hist), ptr(rep_ptr), ptr(rep_pos), i64(0 if rep_pos is None else rep_pos.numel()),
+    call("ojb_gdn_prep", ptr(proj), ptr(hist), ptr(rep_ptr), ptr(rep_pos), i64(0 if rep_pos is None else rep_pos.numel()),
          ptr(convw), ptr(A_log), ptr(dt_bias), ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), i64(N), i64(KD), i64(VD),
-         i64(HV), i64(HK), i32(1 if l2norm else 0), i32(1 if ieee else 0), stream_ptr())
+         i64(HV), i64(HK), i32(1 if l2norm else 0), stream_ptr())
     return q, k, v, g, beta
 
 
@@ -238,11 +238,10 @@ def _expand(x, HK, HV, HD):
     return x.view(-1, HK, 1, HD).expand(-1, HK, HV // HK, HD).reshape(-1, HV * HD).contiguous()
 
 
-def linattn_prep_rows(proj, hist, convw, A_log, dt_bias, KD, VD, HV, HK, HD, ieee=False):
+def linattn_prep_rows(proj, hist, convw, A_log, dt_bias, KD, VD, HV, HK, HD):
     """One output row per packed row (no replication): [q [N,KD], k [N,KD], v [N,VD], g f32 [N,HV], beta [N,HV]].
-    Not in the reference; the tree-native Gated DeltaNet pass consumes this layout. ieee: sigmoids with expf and an IEEE
-    division (ojb_gdn_prep_v)."""
-    return list(_prep(proj, hist, None, None, proj.shape[0], convw, A_log, dt_bias, KD, VD, HV, HK, HD, ieee=ieee))
+    Not in the reference; the tree-native Gated DeltaNet pass consumes this layout."""
+    return list(_prep(proj, hist, None, None, proj.shape[0], convw, A_log, dt_bias, KD, VD, HV, HK, HD))
 
 
 def linattn_prep_dedup2(proj, hist, rep_ptr, rep_pos, L2, convw, A_log, dt_bias, KD, VD, HV, HK, HD, rep_qk):
@@ -554,18 +553,18 @@ def gated_rmsnorm_map(x, proj, w, HV, HD, zoff, eps, Lp, Ls):
     return _gated_norm(x, _hist_cache[key], proj, w, HV, HD, zoff, eps)
 
 
-def _gated_norm(x, inv, proj, w, HV, HD, zoff, eps, ieee=False):
+def _gated_norm(x, inv, proj, w, HV, HD, zoff, eps):
     _chk(x, inv, proj, w)
     N, P = proj.shape
     out = torch.empty(N, HV * HD, dtype=bf16, device=proj.device)
-    call("ojb_gated_rmsnorm_v", ptr(x), ptr(inv), ptr(proj), ptr(w), ptr(out), i64(N), i64(HV), i64(HD), i64(zoff), i64(P),
-         f32(eps), i32(1 if ieee else 0), stream_ptr())
+    call("ojb_gated_rmsnorm", ptr(x), ptr(inv), ptr(proj), ptr(w), ptr(out), i64(N), i64(HV), i64(HD), i64(zoff), i64(P),
+         f32(eps), stream_ptr())
     return out
 
 
-def gated_rmsnorm(x, proj, w, HV, HD, zoff, eps, ieee=False):
-    """src/ext.py:9 — x [N, HV, HD] in packed-row order. ieee as in linattn_prep_rows."""
-    return _gated_norm(x, None, proj, w, HV, HD, zoff, eps, ieee)
+def gated_rmsnorm(x, proj, w, HV, HD, zoff, eps):
+    """src/ext.py:9 — x [N, HV, HD] in packed-row order."""
+    return _gated_norm(x, None, proj, w, HV, HD, zoff, eps)
 
 
 def gated_rmsnorm_inv(x, inv, proj, w, HV, HD, zoff, eps):

@@ -298,7 +298,7 @@ class FastQwen35(torch.nn.Module):
                 K.gdn_chunked_proj(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD ** -0.5, lay.chunks,
                                    lay.steps, lay.walk_ptr, lay.n_walks, None, None, o)
                 return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
-            q, k, v, g, beta = K.linattn_prep_rows(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD, self.fp8)
+            q, k, v, g, beta = K.linattn_prep_rows(proj, lay.hist, d.convw, d.A_log, d.dt_bias, d.KD, d.VD, d.HV, d.HK, d.HD)
             if hasattr(lay, "lsteps") and TREE_LEVELS:
                 st = self._bufs.get(("gdn_states", lay.S, d.HV))
                 if st is None:
@@ -309,7 +309,7 @@ class FastQwen35(torch.nn.Module):
             else:
                 K.gdn_chunked(q.view(N, d.HK, d.HD), k.view(N, d.HK, d.HD), v.view(N, d.HV, d.HD), g, beta, d.HD ** -0.5,
                               lay.chunks, lay.steps, lay.walk_ptr, lay.n_walks, None, None, o)
-            return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps, self.fp8)
+            return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
         # the reference's route: every candidate path replicated, one sequence per candidate (src/fastmodel.py:420-454)
         S, L2 = lay.S, lay.L2
         q, k, v, g, beta = K.linattn_prep_dedup2(proj, lay.hist, lay.rep_ptr, lay.rep_pos, L2, d.convw, d.A_log, d.dt_bias,

@@ -284,11 +284,12 @@ def test_prep_of_packed_rows_equals_the_scatter_form(N, l2):
 @pytest.mark.parametrize("gather", [False, True])
 def test_gated_rmsnorm_wide_accesses_equal_the_narrow_ones(N, HV, gather):
     """16-byte form (aligned columns) against the 8-byte form (the same gate four columns further right): sums in the same order, the
-    same bits; with the IEEE sigmoid an ulp of bf16 on few values."""
+    same bits, gates of any magnitude (the two forms compute the sigmoid in different ways)."""
     from ojb200 import ext as K
     gen = torch.Generator().manual_seed(N + HV)
     x = torch.randn(N + 5, HV, 128, generator=gen).to(bf16).cuda()
     proj = torch.randn(N, HV * 128 + 24, generator=gen).to(bf16).cuda()
+    proj[:, 8:8 + HV * 128:5] *= 100
     w = (1 + 0.02 * torch.randn(128, generator=gen)).to(bf16).cuda()
     inv = torch.randint(0, N + 5, (N,), generator=gen).to(torch.int32).cuda() if gather else None
     moved = torch.zeros(N, HV * 128 + 24, dtype=bf16, device="cuda")
@@ -296,10 +297,6 @@ def test_gated_rmsnorm_wide_accesses_equal_the_narrow_ones(N, HV, gather):
     src = x if gather else x[:N].contiguous()
     a = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6)
     assert torch.equal(a, K._gated_norm(src, inv, moved, w, HV, 128, 12, 1e-6))
-    b = K._gated_norm(src, inv, proj, w, HV, 128, 8, 1e-6, ieee=True)
-    a, b = a.float(), b.float()
-    assert bool(((a - b).abs() <= b.abs() * 2 ** -7 + 1e-30).all())
-    assert (a == b).float().mean().item() > 0.99
 
 
 @pytest.mark.parametrize("name,HV,copies", [("baseline", 48, 1), ("example", 40, 1), ("single", 48, 1), ("wide", 16, 4), ("ragged", 32, 3)])
@@ -334,16 +331,20 @@ def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
     assert float(outs[0][0].float().abs().max()) > 0
 
 
-@pytest.mark.parametrize("ieee", [False, True])
-def test_silu_and_sigmoid_of_every_bf16_value(ieee):
-    """The element-wise functions of the preparation on all 65 536 bf16 inputs (a convolution whose last tap is 1), against
-    64 bits: the bf16 result is the correctly rounded one wherever the fp32 value before rounding, a few units of 2^-24 off, does
-    not cross a rounding boundary — all but a handful. Infinities and not-a-numbers as x / (1 + e^-x) gives them."""
+def _every_bf16_value():
+    return torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(torch.int16).view(bf16)
+
+
+@pytest.mark.parametrize("copies", [1, 16])        # 128 and 2048 rows: four and eight rows to a thread
+def test_silu_of_every_bf16_value(copies):
+    """SiLU in the preparation on all 65 536 bf16 inputs (a convolution whose last tap is 1). Against 64 bits: the fp32 value before
+    rounding carries the errors of expf (2^-23), the sum and the quotient (2^-24 each), so at most one value in 2^-22 / 2^-8 = 2^14
+    lies close enough to a rounding boundary to go the other way: a handful. Infinities and not-a-numbers as x / (1 + e^-x) gives them.
+    Against the scatter form, which has the division as it stands: the same bits."""
     from ojb200 import ext as K
-    HK, HV, N = 1, 4, 128                       # 128 rows x 512 value channels: every bf16 value once
+    HK, HV, N = 1, 4, 128 * copies               # 128 rows x 512 value channels: every bf16 value once
     KD, VD = 128, 512
-    bits = torch.arange(65536, dtype=torch.int32).to(torch.uint16).view(torch.int16)
-    x = bits.view(bf16).view(N, VD)
+    x = _every_bf16_value().view(128, VD).repeat(copies, 1)
     proj = torch.zeros(N, 2 * KD + 2 * VD + 2 * HV, dtype=bf16)
     proj[:, 2 * KD:2 * KD + VD] = x
     convw = torch.zeros(2 * KD + VD, 4, dtype=bf16)
@@ -351,14 +352,41 @@ def test_silu_and_sigmoid_of_every_bf16_value(ieee):
     hist = torch.full((N + 1, 4), -1, dtype=torch.int32)
     hist[:N, 3] = torch.arange(N)
     one = torch.zeros(HV, dtype=bf16)
-    _, _, v, _, _ = K._prep(proj.cuda(), hist.cuda(), None, None, N, convw.cuda(), one.cuda(), one.cuda(), KD, VD, HV, HK, 128, False, ieee)
+    args = (convw.cuda(), one.cuda(), one.cuda(), KD, VD, HV, HK, 128, False)
+    v = K._prep(proj.cuda(), hist.cuda(), None, None, N, *args)[2]
+    ptr_ = torch.cat([torch.arange(N + 1), torch.tensor([N])]).to(torch.int32).cuda()
+    scattered = K._prep(proj.cuda(), hist.cuda(), ptr_, torch.arange(N, dtype=torch.int32).cuda(), N, *args)[2]
+    same = (v == scattered) | (torch.isnan(v) & torch.isnan(scattered))
+    assert bool(same.all())
     got, x64 = v.cpu().flatten(), x.double().flatten()
     want = (x64 / (1.0 + torch.exp(-x64)))
     nan = torch.isnan(want)
     assert torch.equal(torch.isnan(got), nan)
     normal = ~nan & (want.abs() > 2.0 ** -120)
     wrong = got[normal] != want[normal].to(bf16)
-    assert wrong.float().mean().item() < 2e-3
+    assert wrong.sum().item() <= 8 * copies
     a, b = got[normal].double(), want[normal]
     assert bool((((a - b).abs() <= b.abs() * 2.0 ** -8) | (a == b)).all())
     assert bool((got[~nan & ~normal].double().abs() <= 2.0 ** -119).all())
+
+
+@pytest.mark.parametrize("copies", [1, 16])        # 128 and 2048 rows: one and two rows to a thread
+def test_gate_of_every_bf16_value(copies):
+    """The gated norm with every bf16 value as the gate: the same bits as the 8-byte form, whose sigmoid has the division as it
+    stands, and, where they are finite, within half a bf16 ulp (2^-8) and the errors of the norm and of the gate (fp32 roundings, 2^-20
+    together) of 64 bits."""
+    from ojb200 import ext as K
+    HV, N = 4, 128 * copies
+    z = _every_bf16_value().view(128, 512).repeat(copies, 1)
+    x = torch.randn(N, HV, 128, generator=torch.Generator().manual_seed(1)).to(bf16)
+    w = torch.ones(128, dtype=bf16)
+    outs = []
+    for off in (8, 12):
+        proj = torch.zeros(N, 512 + 24, dtype=bf16)
+        proj[:, off:off + 512] = z
+        outs.append(K._gated_norm(x.cuda(), None, proj.cuda(), w.cuda(), HV, 128, off, 1e-6).cpu())
+    assert bool(((outs[0] == outs[1]) | (torch.isnan(outs[0]) & torch.isnan(outs[1]))).all())
+    x64, z64 = x.double(), z.double().view(N, HV, 128)
+    want = (x64 / torch.sqrt((x64 * x64).mean(-1, keepdim=True) + 1e-6) * z64 / (1.0 + torch.exp(-z64))).view(N, 512)
+    fin = torch.isfinite(want) & (want.abs() > 2.0 ** -110) & (z.double().abs() < 2.0 ** 120)
+    assert bool(((outs[0].double() - want).abs()[fin] <= want.abs()[fin] * (2.0 ** -8 + 2.0 ** -20)).all())
