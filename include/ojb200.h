@@ -251,12 +251,14 @@ int ojb_gdn_chunked(const void* q, const void* k, const void* v, const float* g,
                     float scale, int32_t* status, ojb_stream_t stream);
 
 /* The same with room for parked states in global memory (ojb_gdn_park_bytes bytes, 16-byte aligned, or null): with it, a state pass of
- * more CTAs (4 * HV * n_walks) than the GPU has SMs runs two to an SM instead of in waves of one. Same results. */
+ * more CTAs (4 * HV * n_walks) than the GPU has SMs runs two to an SM instead of in waves of one. parks = 0 promises that no step of
+ * the walks saves or loads a slot; such a pass needs no room. Same results. ojb_gdn_park_bytes is 0 where the state pass would not use
+ * the room: up to one CTA per SM of the current device, and where it would be more than 256 MiB. */
 int64_t ojb_gdn_park_bytes(int64_t n_walks, int64_t HV);
 int ojb_gdn_chunked_park(const void* q, const void* k, const void* v, const float* g, const void* beta, const int32_t* chunks,
                          int64_t n_chunks, const int32_t* steps, const int32_t* walk_ptr, int64_t n_walks,
                          const float* init_state, float* final_state, void* scratch, void* out, int64_t HK, int64_t HV,
-                         float scale, float* park, int32_t* status, ojb_stream_t stream);
+                         float scale, float* park, int32_t parks, int32_t* status, ojb_stream_t stream);
 
 /* ojb_gdn_chunked with ojb_gdn_prep fused into its first launch (src/kernels.cu:1173 linattn_prep_dedup2 + :4225 gdn_fused6 in
  * two launches instead of three): the state-independent pass reads the in-projection output itself — proj bf16

@@ -14,7 +14,6 @@ from . import _lib
 from ._lib import call, f32, i32, i64, ptr, stream_ptr
 
 bf16 = torch.bfloat16
-SM_COUNT = 148
 
 
 def load(verbose=False):
@@ -421,9 +420,17 @@ def _seq_tables(B, T, device):
     return t
 
 
-def gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walk_ptr, n_walks, init_state=None, final_state=None, out=None):
+def gdn_park_bytes(n_walks, HV):
+    """Bytes that parked states take in a state pass of n_walks walks; 0 where it runs without (ojb_gdn_park_bytes)."""
+    fn = _lib.lib().ojb_gdn_park_bytes
+    fn.restype = _lib.ctypes.c_int64
+    return fn(i64(n_walks), i64(HV))
+
+
+def gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walk_ptr, n_walks, init_state=None, final_state=None, out=None, parks=True):
     """Table-driven chunked gated delta rule (see include/ojb200.h ojb_gdn_chunked). q, k [rows, HK, 128],
-    v [rows, HV, 128], g f32 / beta bf16 [rows, HV]. Returns out bf16 [rows, HV, 128]."""
+    v [rows, HV, 128], g f32 / beta bf16 [rows, HV]. parks=False: no step saves or loads a slot (independent sequences).
+    Returns out bf16 [rows, HV, 128]."""
     _chk(q, k, v, g, beta, chunks, steps, walk_ptr, init_state, final_state)
     rows, HV, HD = v.shape[-3], v.shape[-2], v.shape[-1]
     HK = k.shape[-2]
@@ -436,12 +443,11 @@ def gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walk_ptr, n_walks, init_
     if out is None:
         out = torch.empty(v.shape, dtype=bf16, device=v.device)
     park = None
-    if 4 * HV * n_walks > SM_COUNT:      # more CTAs than SMs in the state pass: room for the form that puts two on an SM
-        pbytes = _lib.lib().ojb_gdn_park_bytes
-        pbytes.restype = _lib.ctypes.c_int64
-        park = torch.empty(pbytes(i64(n_walks), i64(HV)), dtype=torch.uint8, device=v.device)
+    if parks:      # room for the form of the state pass that puts two CTAs on an SM
+        n = gdn_park_bytes(n_walks, HV)
+        park = torch.empty(n, dtype=torch.uint8, device=v.device) if n else None
     call("ojb_gdn_chunked_park", ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(chunks), i64(nch), ptr(steps), ptr(walk_ptr),
-         i64(n_walks), ptr(init_state), ptr(final_state), ptr(scratch), ptr(out), i64(HK), i64(HV), f32(scale), ptr(park),
+         i64(n_walks), ptr(init_state), ptr(final_state), ptr(scratch), ptr(out), i64(HK), i64(HV), f32(scale), ptr(park), i32(1 if parks else 0),
          ptr(_lib.status_word(v.device)), stream_ptr())
     return out
 
@@ -494,7 +500,7 @@ def gdn_fused6(q, k, v, g, beta, scale):
     rows of the last partial chunk beyond T do not exist, pad slots inside T produce zeros only if their inputs are."""
     B, T = v.shape[0], v.shape[1]
     chunks, steps, walks = _seq_tables(B, T, v.device)
-    return gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walks, B)
+    return gdn_chunked(q, k, v, g, beta, scale, chunks, steps, walks, B, parks=False)
 
 
 gdn_fused = gdn_fused2 = gdn_fused3 = gdn_fused4 = gdn_fused8 = gdn_fused9 = gdn_fused6   # src/ext.py:30-33,41-42

@@ -308,7 +308,7 @@ class FastQwen35(torch.nn.Module):
                                   lay, o, st)
             else:
                 K.gdn_chunked(q.view(N, d.HK, d.HD), k.view(N, d.HK, d.HD), v.view(N, d.HV, d.HD), g, beta, d.HD ** -0.5,
-                              lay.chunks, lay.steps, lay.walk_ptr, lay.n_walks, None, None, o)
+                              lay.chunks, lay.steps, lay.walk_ptr, lay.n_walks, None, None, o, getattr(lay, "parks", True))
             return K.gated_rmsnorm(o, proj, d.normw, d.HV, d.HD, 2 * d.KD + d.VD, d.norm_eps)
         # the reference's route: every candidate path replicated, one sequence per candidate (src/fastmodel.py:420-454)
         S, L2 = lay.S, lay.L2

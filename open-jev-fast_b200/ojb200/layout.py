@@ -147,7 +147,8 @@ def pack_requests(requests, pad_id=0, NB=32, PB=16, dev="cuda", pin=False):
 def batch_layout(attention_mask, dev):
     """Layout of a right-padded batch [B, T] of independent sequences (the non-tree forward of src/fastmodel.py:205-241)
     in the vocabulary of the tree kernels: every sequence is its own path, rows are b*T + t, padded up to a multiple of 32
-    rows. Returns a namespace with pos, rowmask, hist, krange, chunks, steps, walk_ptr, n_walks, lastidx, N."""
+    rows. Returns a namespace with pos, rowmask, hist, krange, chunks, steps, walk_ptr, n_walks, lastidx, N and parks = False (no
+    walk parks a state)."""
     m = attention_mask.detach().cpu().numpy().astype(bool)
     B, T = m.shape
     N = -(-(B * T) // 32) * 32
@@ -178,7 +179,7 @@ def batch_layout(attention_mask, dev):
     t32 = lambda a: torch.as_tensor(np.asarray(a, np.int32)).to(dev)
     last = np.array([b * T + max(int(lens[b]) - 1, 0) for b in range(B)], np.int64)
     return SimpleNamespace(N=N, S=B, L2=T, pos=torch.as_tensor(pos).to(dev), rowmask=t32(rowmask), hist=t32(hist),
-                           krange=t32(krange), chunks=t32(chunks), steps=t32(steps), walk_ptr=t32(walks), n_walks=B,
+                           krange=t32(krange), chunks=t32(chunks), steps=t32(steps), walk_ptr=t32(walks), n_walks=B, parks=False,
                            lastidx=torch.as_tensor(last).to(dev))
 
 

@@ -58,6 +58,15 @@ def test_more_query_rows_than_rows_need_their_row_indices():
                                      f32(1e-6), none) == -1
 
 
+def test_parking_room_is_bounded():
+    """ojb_gdn_park_bytes: nothing up to one CTA per SM (4 per head and walk), 128 KiB per head and walk above, nothing where that
+    would pass 256 MiB."""
+    from ojb200 import ext
+    assert ext.gdn_park_bytes(1, 32) == 0 and ext.gdn_park_bytes(1, 37) == 0 and ext.gdn_park_bytes(0, 32) == 0
+    assert ext.gdn_park_bytes(1, 38) == 38 << 17 and ext.gdn_park_bytes(4, 32) == 16 << 20
+    assert ext.gdn_park_bytes(64, 32) == 256 << 20 and ext.gdn_park_bytes(65, 32) == 0 and ext.gdn_park_bytes(20000, 32) == 0
+
+
 def test_gemm_plan_is_host_arithmetic():
     """ojb_gemm_plan needs no GPU: it returns a valid variant, a split count within bounds, and a finite time."""
     from ojb200 import lt_ext

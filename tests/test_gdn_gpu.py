@@ -308,7 +308,7 @@ def test_state_pass_two_to_an_sm_gives_the_same_bits(name, HV, copies):
     HK = 8
     seqs, groups, pad_id, NB, PB = trees.layout_cases()[name]
     ids, lay, _ = PL.pack_requests([(seqs, groups)] * copies, pad_id, NB, PB, dev="cuda")
-    assert 4 * HV * copies > K.SM_COUNT
+    assert K.gdn_park_bytes(copies, HV) > 0
     q, k, v, g, beta = (t.cuda() for t in _inputs(lay.N, HK, HV, 5))
     steps = lay.steps.clone()
     for i in range(copies):
@@ -390,3 +390,30 @@ def test_gate_of_every_bf16_value(copies):
     want = (x64 / torch.sqrt((x64 * x64).mean(-1, keepdim=True) + 1e-6) * z64 / (1.0 + torch.exp(-z64))).view(N, 512)
     fin = torch.isfinite(want) & (want.abs() > 2.0 ** -110) & (z.double().abs() < 2.0 ** 120)
     assert bool(((outs[0].double() - want).abs()[fin] <= want.abs()[fin] * (2.0 ** -8 + 2.0 ** -20)).all())
+
+
+def test_independent_sequences_need_no_parking_room():
+    """A batch of sequences parks nothing: its state pass runs two to an SM without the parking buffer (2 GiB for 512 sequences at 32
+    heads), with the same bits as with it and as the full form, and takes no memory beyond the scratch items and the result."""
+    from ojb200 import ext as K, _lib
+    B, T, HK, HV = 512, 16, 4, 32
+    q, k, v, g, beta = (t.cuda() for t in _inputs(B * T, HK, HV, 7))
+    chunks, steps, walks = K._seq_tables(B, T, torch.device("cuda"))
+    args = (q, k, v, g, beta, 128 ** -0.5)
+    four = lambda t: t.view(B, T, *t.shape[1:])
+    K.gdn_fused6(*(four(t) for t in args[:5]), args[5])
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    got = K.gdn_fused6(*(four(t) for t in args[:5]), args[5])
+    torch.cuda.synchronize()
+    scratch = chunks.shape[0] * HV * 81936
+    assert torch.cuda.max_memory_allocated() - base <= scratch + got.numel() * 2 + (1 << 20)
+    assert torch.equal(got.view(B * T, HV, 128), K.gdn_chunked(*args, chunks, steps, walks, B))          # full form: too much to park
+    few = 16
+    n = few * T
+    some = [t[:n].contiguous() for t in args[:5]]
+    tables = chunks[:few].contiguous(), steps[:few].contiguous(), walks[:few + 1].contiguous(), few
+    assert K.gdn_park_bytes(few, HV) > 0
+    assert torch.equal(K.gdn_chunked(*some, args[5], *tables), K.gdn_chunked(*some, args[5], *tables, parks=False))
+    _lib.check_status()
