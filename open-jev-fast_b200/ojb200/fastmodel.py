@@ -354,12 +354,13 @@ class FastQwen35(torch.nn.Module):
 
     @staticmethod
     def _plain_index(i):
-        """Whether the library's kernels take this index; torch takes the others."""
-        return i.dtype == torch.int64 and i.is_cuda and i.is_contiguous()
+        """Whether the library's kernels take this index: a list of rows; torch takes the others (none at all, tables of rows, other
+        types and strides)."""
+        return i.dtype == torch.int64 and i.is_cuda and i.is_contiguous() and i.dim() == 1 and i.numel() > 0
 
     def _asked_rows_only(self, lay, N):
         i = lay.lastidx
-        return N >= self.ASKED_MIN_ROWS and i.numel() * 4 <= N and self._plain_index(i)
+        return N >= self.ASKED_MIN_ROWS and self._plain_index(i) and i.numel() * 4 <= N
 
     def _mix_asked(self, i, h, hn, rows, lay, cos, sin, linear):
         """Token mixer of the last layer (i) for the asked rows: (their residual stream, their mixer output)."""

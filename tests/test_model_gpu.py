@@ -281,6 +281,30 @@ def test_last_rows_by_index_from_the_end_and_outside(last, asked, fp8, monkeypat
             assert bool(torch.isnan(got[1]).all()) and torch.equal(got[keep], ref[keep])
 
 
+@pytest.mark.parametrize("asked_min", [1, 1 << 30])
+def test_last_rows_in_every_form_of_an_index(asked_min, monkeypatch):
+    """lay.lastidx in the forms torch's indexing takes (a table of rows, no rows, 32 bits, a stride) gives the rows of the plain list in
+    that shape, whether or not the plain list would take the asked-rows path."""
+    from ojb200 import fastmodel as FM
+    from ojb200 import modelgen as MG, _lib, ext
+    cfg = MG.make_config(**dict(MG.SMALL, head_dim=256, num_hidden_layers=2, layer_types=["linear_attention", "full_attention"]))
+    fast = FM.FastQwen35(MG.build_core(cfg, device="cpu", seed=3, std=0.05, draw_on="cpu").to("cuda"))
+    W, b = MG.make_head(cfg.hidden_size, A=2, seed=1, device="cuda")
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()["baseline"]
+    ids, lay = fast.gtree_build([[t % cfg.vocab_size for t in s] for s in seqs], groups, pad_id, NB, PB, dev="cuda")
+    rows = lay.lastidx[:4].contiguous()
+    monkeypatch.setattr(FM.FastQwen35, "ASKED_MIN_ROWS", 1 << 30)
+    every = fast.forward_gtree(ids, lay, return_all=True)
+    monkeypatch.setattr(FM.FastQwen35, "ASKED_MIN_ROWS", asked_min)
+    for index in (rows.view(2, 2), rows[:0], rows.int(), torch.stack([rows, rows], 1)[:, 0]):
+        lay.lastidx = index
+        assert torch.equal(fast.forward_gtree(ids, lay), every[index.long()])
+        if index.dim() == 1:
+            want = fast.score_gtree(ids, lay, W, b)
+            assert want.shape == (index.numel(), 2) and torch.equal(want, ext.score_head(every, index.long().contiguous(), W, b))
+    _lib.check_status()
+
+
 def _small_model(seed=0):
     from ojb200 import modelgen as MG
     cfg = MG.make_config(**MG.SMALL)
