@@ -148,7 +148,8 @@ int ojb_resnorm_f32(float* h, const void* x_init, const void* delta, const float
                     const int32_t* rowmask, void* hn_out, int64_t rows, int64_t H, float eps, ojb_stream_t stream);
 
 /* The same with the normed row handed on as e4m3 operands of the 8-bit GEMM, q [rows, H] bytes and scale fp32 [rows], instead of
- * bf16: what ojb_quantize_rows_e4m3 makes of that bf16 row, bit for bit. */
+ * bf16: bit for bit what ojb_quantize_rows_e4m3 makes of the bf16 rows of ojb_resnorm_f32 above 296 rows. (Up to 296 rows that one adds
+ * the squares of a row in another order, 1024 threads to a row: its rows can differ by an ulp of bf16.) */
 int ojb_resnorm_f32_e4m3(float* h, const void* x_init, const float* parts, int splits, const float* w1, const int32_t* rowmask,
                          void* q, float* scale, int64_t rows, int64_t H, float eps, ojb_stream_t stream);
 

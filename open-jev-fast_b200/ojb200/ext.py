@@ -73,7 +73,7 @@ def resnorm_f32(h, x_init, delta, parts, w1, rowmask, eps):
 
 def resnorm_f32_e4m3(h, x_init, parts, w1, rowmask, eps):
     """resnorm_f32 with the normed rows as e4m3 operands: (bytes [N, H] uint8, scale fp32 [N]), bit for bit those that
-    quantize_rows_e4m3 makes of its bf16 result."""
+    quantize_rows_e4m3 makes of its bf16 result above 296 rows (up to there resnorm_f32 sums a row in another order)."""
     _chk(h, x_init, parts, w1, rowmask)
     N, H = h.shape
     if h.dtype != torch.float32 or (parts is not None and (parts.dtype != torch.float32 or tuple(parts.shape[1:]) != (N, H))):
