@@ -417,3 +417,27 @@ def test_independent_sequences_need_no_parking_room():
     assert K.gdn_park_bytes(few, HV) > 0
     assert torch.equal(K.gdn_chunked(*some, args[5], *tables), K.gdn_chunked(*some, args[5], *tables, parks=False))
     _lib.check_status()
+
+
+def test_dense_state_pass_past_its_staged_steps():
+    """Walks of more steps than a CTA keeps in shared memory (128), two CTAs to an SM: the same bits as the full form."""
+    from ojb200 import ext as K, _lib
+    B, T, HK, HV = 2, 131 * 64 + 17, 4, 32
+    q, k, v, g, beta = (t.cuda() for t in _inputs(B * T, HK, HV, 8))
+    chunks, steps, walks = K._seq_tables(B, T, torch.device("cuda"))
+    outs = []
+    for parks in (False, True):
+        fin = torch.zeros(B, HV, 128, 128, device="cuda")
+        st = steps.clone()
+        for b in range(B):
+            st[int(walks[b + 1]) - 1, 3] = b + 1
+        outs.append((K.gdn_chunked(q, k, v, g, beta, 128 ** -0.5, chunks, st, walks, B, None, fin, None, parks), fin))
+    scratch = torch.empty(chunks.shape[0] * HV * 81936, dtype=torch.uint8, device="cuda")
+    out, fin = torch.empty_like(outs[0][0]), torch.zeros_like(outs[0][1])
+    K.call("ojb_gdn_chunked", *(K.ptr(t) for t in (q, k, v, g, beta, chunks)), K.i64(chunks.shape[0]), K.ptr(st), K.ptr(walks), K.i64(B),
+           K.ptr(None), K.ptr(fin), K.ptr(scratch), K.ptr(out), K.i64(HK), K.i64(HV), K.f32(128 ** -0.5),
+           K.ptr(_lib.status_word(v.device)), K.stream_ptr())
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for o, f in outs:
+        assert torch.equal(o, out) and torch.equal(f, fin)

@@ -149,6 +149,40 @@ def test_one_pass_attention(N_case, HQ, HKV, spread):
         assert (got[keep] - want[keep]).abs().max().item() < 6e-2
 
 
+def test_one_pass_attention_over_thousands_of_keys():
+    """More key blocks than one 32-bit word of the list of visible blocks holds (4096 keys): ranges in words apart with empty words between
+    them, on word boundaries, single keys at both ends of a word, a row that sees everything, one that sees nothing; a key count
+    that fills no block. Asked rows against 64 bits with P rounded to bf16 (relative 2^-9, averaged over the keys)."""
+    from ojb200 import ext as K, _lib
+    HQ, HKV, N, D = 4, 2, 3 * 4096 + 4096 // 2 + 8, 256
+    g = torch.Generator(device="cuda").manual_seed(41)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(bf16)
+    W = 4096
+    ranges = [(0, N, 0, 0, 0, 0), (0, 0, 0, 0, 0, 0), (0, 1, 2 * W, 2 * W + 1, N - 1, N), (W - 1, W + 1, 3 * W - 1, 3 * W, 3 * W, 3 * W + 200),
+              (3 * W, N, 0, 0, 0, 0), (W, 2 * W, 0, 0, 0, 0), (0, 100, 3 * W + 70, 3 * W + 333, 2 * W + 128, 2 * W + 256), (N - 8, N, 0, 5, 0, 0)]
+    q_rows = torch.tensor([5, 9000, N - 1, 77, 4096, 4095, 12000, 300], device="cuda")
+    krange = torch.zeros(N, 8, dtype=torch.int32, device="cuda")
+    for r, (a0, e0, a1, e1, a2, e2) in zip(q_rows.tolist(), ranges):
+        krange[r] = torch.tensor([e0, a1, e1, a2, e2, a0, 0, 0], dtype=torch.int32)
+    kt, vt_t = rnd(HKV, N, D), rnd(HKV, D, N)
+    for pick in ([0, 1, 2, 3, 4, 5, 6, 7], [2], [3, 7], [6, 1]):        # one tile that sees every block, and tiles that see few
+        rows = q_rows[pick]
+        NQ = len(pick)
+        qt, q_src = rnd(HQ, NQ, D), rnd(NQ, HQ * 2 * D)
+        y = K.tree_attn_rows(qt, kt, vt_t, q_src, krange, D ** -0.5, rows).float().view(NQ, HQ, D)
+        two = K.tree_attn_rows(qt, kt, vt_t, q_src, krange, D ** -0.5, rows, one_pass=False).float().view(NQ, HQ, D)
+        gate = torch.sigmoid(q_src.double().view(NQ, HQ, 2, D)[:, :, 1])
+        for i, p in enumerate(pick):
+            a0, e0, a1, e1, a2, e2 = ranges[p]
+            keys = torch.cat([torch.arange(a, e) for a, e in ((a0, e0), (a1, e1), (a2, e2))]).cuda()
+            for h in range(HQ):
+                k, v = kt[h // 2][keys].double(), vt_t[h // 2][:, keys].double()
+                want = v @ torch.softmax(k @ qt[h, i].double() * D ** -0.5, 0) * gate[i, h] if len(keys) else torch.zeros(D, device="cuda")
+                for got in (y[i, h], two[i, h]):
+                    assert (got - want).norm() <= 6e-3 * want.norm(), (p, h)
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("N_case,HQ,HKV", [("baseline", 24, 4), ("ragged", 4, 2), ("wide", 6, 2), ("nostem", 5, 1), ("single", 3, 3)])
 @pytest.mark.parametrize("one_pass", [False, 2])
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
@@ -302,6 +336,24 @@ def test_last_rows_in_every_form_of_an_index(asked_min, monkeypatch):
         if index.dim() == 1:
             want = fast.score_gtree(ids, lay, W, b)
             assert want.shape == (index.numel(), 2) and torch.equal(want, ext.score_head(every, index.long().contiguous(), W, b))
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+def test_preparation_fused_into_the_intra_pass_gives_the_same_scores(fp8, monkeypatch):
+    """OJ_FUSE_PREP in a whole forward, with bf16 and with 8-bit projections: the same bits as the separate preparation."""
+    from ojb200 import fastmodel as FM
+    from ojb200 import modelgen as MG, _lib
+    cfg = MG.make_config(**dict(MG.SMALL, head_dim=256, num_hidden_layers=3,
+                                layer_types=["linear_attention", "full_attention", "linear_attention"]))
+    fast = FM.FastQwen35(MG.build_core(cfg, device="cpu", seed=3, std=0.05, draw_on="cpu").to("cuda"), fp8=fp8)
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()["baseline"]
+    ids, lay = fast.gtree_build([[t % cfg.vocab_size for t in s] for s in seqs], groups, pad_id, NB, PB, dev="cuda")
+    outs = []
+    for fuse in (False, True):
+        monkeypatch.setattr(FM, "FUSE_PREP", fuse)
+        outs.append(fast.forward_gtree(ids, lay))
+    assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0]).all())
     _lib.check_status()
 
 
