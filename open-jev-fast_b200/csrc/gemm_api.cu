@@ -6,7 +6,7 @@
 //             flop), w-tile width chosen per shape, the last M mod 256 <= 128 rows (or all rows when M <= 2048, on request) run with
 //             swapped operands at their true cost.
 //   skinny    (gemm_skinny.cu)    up to 128 rows of x against w tiles of any width, every CTA's shared memory full of weight in
-//             flight; the choice for all shapes it serves.
+//             flight; bf16: the choice up to about 36 to 60 rows (skinny_clocks), e4m3: wherever it serves.
 //   pair256   (gemm_pair256.cu)   the same units on CTA pairs with tcgen05.mma.cta_group::2; measured on par with block256
 //             (both are bound by shared-memory bandwidth), kept as variants 5 / 6.
 // With variant 0 the kernel is the one with the smallest modelled time (plan_kernel): the models replay the round-robin
@@ -43,10 +43,12 @@ double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, in
 }
 
 // The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (its share of a wait, a commit and the MMAs) in less
-// than 220 clocks. Measured against the best of the other kernels (us): [12352, 5120] at 12 / 32 / 64 / 128 rows 24.2 / 24.5 / 27.7 /
-// 27.9 against 36 / 27.2 / 27.3 / 28.7; [2048, 5120] at 32 / 128 rows 15.4 / 18.4 against 21.3 / 21.8; [5120, 4096] at 12 / 128 rows 11.2 /
-// 14.4 against 11.4 / 14.5; [5120, 17408] 32.0 / 38.2 against 32.9 / 39.2.
-constexpr int kSkinnyRows = 128;
+// than 220 clocks. Measured against the best of the other kernels, each with its best K ranges (us; * = what the models pick), at
+// 12 / 32 / 64 / 128 rows: [12352, 5120] 24.6* / 24.8* / 29.6 / 29.7 against 30.4 / 27.4 / 27.8* / 29.0*, [14336, 5120] 28.0* / 27.6* / 30.0 / 31.5
+// against 31.4 / 29.8 / 30.3* / 31.2*, [2048, 5120] 15.4* / 15.4* / 16.5* / 18.6* against 21.3 / 21.3 / 21.2 / 21.8, [5120, 4096]
+// 11.5* / 11.5* / 12.5 / 14.8 against 11.4 / 11.8 / 12.9* / 14.7*, [5120, 6144] 14.9* / 14.5* / 16.0 / 17.9 against 15.0 / 15.0 / 16.2* / 18.4*,
+// [5120, 17408] 32.9* / 33.3 / 35.3 / 39.2 against 33.1 / 33.9* / 36.1* / 39.5*. With many rows the model is too high (30.6 us for
+// [2048, 5120] at 128 rows), and the swapped-operand units take over above about 36 rows where it would still lead by 0 to 5 %.
 double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
   const int bn = skinny_bn(N, splits);
   const double waves = static_cast<double>(ceil_div(ceil_div(N, bn) * splits, sms));
@@ -88,7 +90,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
     const int tail_box = static_cast<int>(ceil_div(ceil_div(M, n_xchunk), 16) * 16);
     consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, model_epi));
   }
-  if (M <= kSkinnyRows && epi != kEpiSwiglu && skinny_serves(M, K) && !eight_bit) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
+  if (epi != kEpiSwiglu && skinny_serves(M, K) && !eight_bit) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz
   if (best.clocks < hbm) best.clocks = hbm;
   return best;

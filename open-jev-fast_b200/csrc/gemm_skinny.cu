@@ -19,7 +19,6 @@ namespace {
 
 constexpr int kSkinnyThreads = 192;
 constexpr int kSkinnyMaxStages = 40;
-constexpr int kSkinnyMaxRows = 128;
 constexpr size_t kSkinnySmem = 227 * 1024;
 
 struct SkinnyArgs {
@@ -236,7 +235,7 @@ int launch_skinny(int bn, const void* x, const void* w, void* out, int64_t M, in
 // bn = 0: the narrowest multiple of 16 (at most 128) with which the tiles times the K ranges fill the SMs at most once
 int gemm_skinny_launch(int epi, int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
                        int64_t ldo, int32_t* status, cudaStream_t stream, const float* sx, const float* sw) {
-  if (M > kSkinnyMaxRows || K % (sx != nullptr ? 128 : kBK) != 0 || (epi != kEpiBf16 && epi != kEpiPartialF32)) return OJB_ERR_LIMIT;
+  if (M > kSkinnyRows || K % (sx != nullptr ? 128 : kBK) != 0 || (epi != kEpiBf16 && epi != kEpiPartialF32)) return OJB_ERR_LIMIT;
   if (bn == 0) bn = skinny_bn(N, splits);
   if (bn < 16 || bn > 128 || bn % 16) return OJB_ERR_ARG;
   if (sx != nullptr)

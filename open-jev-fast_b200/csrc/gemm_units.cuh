@@ -263,7 +263,8 @@ class ModelCache {
 };
 
 // The few-row kernel (gemm_skinny.cu): what it takes, and the rows of its w tile.
-inline bool skinny_serves(int64_t M, int64_t K) { return M <= 128 && K % 64 == 0; }
+constexpr int kSkinnyRows = 128;
+inline bool skinny_serves(int64_t M, int64_t K) { return M <= kSkinnyRows && K % 64 == 0; }
 inline int skinny_bn(int64_t N, int splits) {
   const int64_t per = 148 / splits > 0 ? 148 / splits : 1;
   const int64_t bn = ceil_div(ceil_div(N, per), 16) * 16;

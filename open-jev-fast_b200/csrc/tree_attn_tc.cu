@@ -38,9 +38,9 @@ constexpr uint32_t kQBytes = kMaxG * kQRows * kD * 2;    // 4 k-blocks of [16 G 
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 0, kColS = 256;               // O: 256 columns; S: two buffers of 128 columns
 constexpr int kStagePitch = kD * 2 + 16;                 // bytes per row of the output staging tile
-// Keys from which tree_attn_long.cu is the faster one. Two-pass / one-pass, all rows as queries (us): 128 rows 11.3 / 12.9, 320 rows
-// 17.1 / 16.2, 544 rows 22.6 / 17.9, 1120 rows 53 / 34, 2592 rows 192 / 115, 16 512 rows 5283 / 2804; seven rows as queries: 128 keys
-// 9.8 / 9.5, 320 keys 15.7 / 12.7, 2592 keys 59 / 42.
+// Keys from which tree_attn_long.cu is the faster one. Two-pass / one-pass, all rows as queries (us): 128 rows 10.9 / 13.1, 320 rows
+// 16.2 / 16.6, 544 rows 21.2 / 17.9, 1120 rows 50 / 33.5, 2592 rows 181 / 112, 16 512 rows 5058 / 2512; seven rows as queries: 128 keys
+// 9.9 / 9.7, 320 keys 15.1 / 12.7, 2592 keys 56 / 40.
 constexpr int64_t kOnePassKeys = 256;
 constexpr int kMaxBlocks = 2048;                         // 64-key blocks a CTA can list (131 072 keys)
 constexpr int kSub = 64;               // keys per visibility block

@@ -456,7 +456,8 @@ def gdn_chunked_proj(proj, hist, convw, A_log, dt_bias, KD, VD, HV, HK, scale, c
                      final_state=None, out=None):
     """gdn_chunked with the preparation fused into its first launch (ojb_gdn_chunked_proj): reads the in-projection output
     `proj` [N, 2KD+2VD+2HV] and the history table directly — linattn_prep_rows + gdn_chunked in two launches instead of three,
-    same bits. Chunks must be runs of consecutive packed rows of one tree node (the layout builder's tables).
+    same bits; the state pass is always the full form, one CTA to an SM. Chunks must be runs of consecutive packed rows of one tree
+    node (the layout builder's tables).
     Returns out bf16 [N, HV, 128] (rows outside every chunk are left as they are)."""
     _chk(proj, hist, convw, A_log, dt_bias, chunks, steps, walk_ptr, init_state, final_state)
     N = proj.shape[0]
