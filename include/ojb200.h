@@ -344,8 +344,8 @@ int ojb_tree_attn_tc(const void* qt, const void* kt, const void* vt_t, const voi
  * qt bf16 [HQ, NQ, 256], kt [HKV, N, 256], vt_t [HKV, 256, N], krange [N, 8], y [NQ, HQ*256]. N % 8 == 0; any NQ with q_rows, at most
  * N without. An index -n counts from the end (here and in ojb_attn_operands); one outside [-N, N) is moved to the nearest row, so that
  * nothing outside is read: ojb_gather_rows, which takes the same indices, reports it.
- * one_pass = 1: 256 keys and more (scale > 0) go to a kernel that takes 128 operand rows and goes over the keys once, with a running
- * maximum; 2: any number does; 0: always the two-pass kernel. */
+ * one_pass = 1: from 352 keys on, and from 192 on where NQ is at most a quarter of N (scale > 0), a kernel that takes 128 operand rows and
+ * goes over the keys once, with a running maximum; 2: at any number of keys; 0: always the two-pass kernel. */
 int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N,
                        const void* gate, int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ,
                        int64_t HKV, float scale, int32_t one_pass, int32_t* status, ojb_stream_t stream);

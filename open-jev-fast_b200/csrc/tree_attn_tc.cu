@@ -38,10 +38,12 @@ constexpr uint32_t kQBytes = kMaxG * kQRows * kD * 2;    // 4 k-blocks of [16 G 
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 0, kColS = 256;               // O: 256 columns; S: two buffers of 128 columns
 constexpr int kStagePitch = kD * 2 + 16;                 // bytes per row of the output staging tile
-// Keys from which tree_attn_long.cu is the faster one. Two-pass / one-pass, all rows as queries (us): 128 rows 10.9 / 13.1, 320 rows
-// 16.2 / 16.6, 544 rows 21.2 / 17.9, 1120 rows 50 / 33.5, 2592 rows 181 / 112, 16 512 rows 5058 / 2512; seven rows as queries: 128 keys
-// 9.9 / 9.7, 320 keys 15.1 / 12.7, 2592 keys 56 / 40.
-constexpr int64_t kOnePassKeys = 256;
+// Keys from which tree_attn_long.cu is the faster one (us, two-pass / one-pass). All rows as queries: a long shared root at 128 rows 10.9 /
+// 13.0, 256 13.3 / 14.7, 320 16.1 / 16.4, 352 16.8 / 16.1, 416 18.5 / 16.1, 544 21.2 / 17.9, 1120 50 / 33.5, 2592 181 / 112, 16 512 5058 /
+// 2512; short root and long tails, where the two-pass kernel keeps its scores between the passes, 288 13.5 / 14.8, 384 13.7 / 16.5, 544
+// 14.1 / 16.8, 672 27.3 / 17.1 (more CTAs than SMs). A quarter of the rows or less: 128 keys 9.6 / 9.6, 192 11.7 / 11.1, 256 11.9 /
+// 11.1, 320 15.1 / 12.6, 544 19.7 / 15.7, 2592 56 / 40.
+constexpr int64_t kOnePassKeys = 352, kOnePassKeysFewRows = 192;
 constexpr int kMaxBlocks = 2048;                         // 64-key blocks a CTA can list (131 072 keys)
 constexpr int kSub = 64;               // keys per visibility block
 constexpr int kKB = 128;               // keys per product (two blocks)
@@ -471,7 +473,7 @@ extern "C" int ojb_tree_attn_rows(const void* qt, int64_t NQ, const int64_t* q_r
   OJB_REQUIRE(gate_ld >= 0 && gate_hs >= 0 && gate_ld % 8 == 0 && gate_hs % 8 == 0 && gate_hs < (1 << 30));
   OJB_REQUIRE(aligned16(qt) && aligned16(kt) && aligned16(vt_t) && aligned16(gate) && aligned16(y));
   if ((N + kSub - 1) / kSub > kMaxBlocks || NQ > static_cast<int64_t>(kMaxBlocks) * kSub) return OJB_ERR_LIMIT;
-  if (scale > 0.f && (one_pass == 2 || (one_pass == 1 && N >= kOnePassKeys)))
+  if (scale > 0.f && (one_pass == 2 || (one_pass == 1 && N >= (4 * NQ <= N ? kOnePassKeysFewRows : kOnePassKeys))))
     return tree_attn_long_launch(qt, NQ, q_rows, kt, vt_t, N, gate, gate_ld, gate_hs, krange, y, HQ, HKV, scale, status,
                                  static_cast<cudaStream_t>(stream));
   CUtensorMap map_q, map_k, map_vt;

@@ -149,6 +149,25 @@ def test_one_pass_attention(N_case, HQ, HKV, spread):
         assert (got[keep] - want[keep]).abs().max().item() < 6e-2
 
 
+@pytest.mark.parametrize("N,NQ,one", [(344, 344, False), (352, 352, True), (184, 8, False), (192, 48, True), (192, 49, False), (344, 86, True)])
+def test_which_attention_kernel_serves_a_call(N, NQ, one):
+    """The line between the two kernels: from 352 keys on, from 192 where at most a quarter of the rows ask. The result has the bits of
+    the kernel named."""
+    from ojb200 import ext as K, _lib
+    HQ, HKV = 12, 2
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(bf16)
+    rows = None if NQ == N else torch.randperm(N, generator=g, device="cuda")[:NQ]
+    qt, kt, vt_t, q_src = rnd(HQ, NQ, 256), rnd(HKV, N, 256), rnd(HKV, 256, N), rnd(NQ, HQ * 512)
+    krange = torch.zeros(N, 8, dtype=torch.int32, device="cuda")
+    krange[:, 0] = torch.arange(1, N + 1)
+    run = lambda one_pass: K.tree_attn_rows(qt, kt, vt_t, q_src, krange, 1 / 16, rows, one_pass=one_pass)
+    two, single = run(False), run(2)
+    assert not torch.equal(two, single)
+    assert torch.equal(run(True), single if one else two)
+    _lib.check_status()
+
+
 def test_one_pass_attention_over_thousands_of_keys():
     """More key blocks than one 32-bit word of the list of visible blocks holds (4096 keys): ranges in words apart with empty words between
     them, on word boundaries, single keys at both ends of a word, a row that sees everything, one that sees nothing; a key count
