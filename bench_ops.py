@@ -1,6 +1,6 @@
 """Micro-benchmark of the non-GEMM kernels at the model's dimensions on one tree (for tuning and for ncu captures).
 
-    python bench_ops.py [--tree baseline|example] [--reps 20] [--only gdn|attn|norm]
+    python bench_ops.py [--tree baseline|example] [--reps 20] [--only gdn|attn|norm|gemm]
 
 Prints one JSON line per op: microseconds per call (CUDA events over `reps` back-to-back calls after a warm-up).
 """
@@ -87,9 +87,21 @@ def main():
             out(f"tree_attn ranges gq={gq}", _time(lambda: K.fattn_tree_ranges(qt, kt, vt, gate, lay.krange, D ** -0.5, gq), args.reps))
         if N <= 2048:
             out("tree_attn bits gq=6", _time(lambda: K.fattn_tree(qt, kt, vt, gate, None, lay.vbits, D ** -0.5, 6), args.reps))
-        vt_t = K.fullattn_prep2(proj, w1, w1, cosb, sinb, 1, N, HQ, HKV, D, 1e-6, with_vt_t=True)[4]
         out("fullattn_prep + transposed V", _time(lambda: K.fullattn_prep2(proj, w1, w1, cosb, sinb, 1, N, HQ, HKV, D, 1e-6, with_vt_t=True), args.reps))
-        out("tree_attn tcgen05", _time(lambda: K.fattn_tree_tc(qt, kt, vt_t, gate, lay.krange, D ** -0.5), args.reps))
+        q_src, kv_src = proj[:, :HQ * 2 * D], proj[:, HQ * 2 * D:]
+        ops = lambda: K.attn_operands(q_src, kv_src, w1, w1, cosb, sinb, HQ, HKV, 1e-6)
+        out("attn_operands", _time(ops, args.reps))
+        qt, kt, vt_t = ops()
+        for name, one_pass in (("two passes", False), ("one pass", 2)):
+            out(f"tree_attn tcgen05, {name}", _time(lambda: K.tree_attn_rows(qt, kt, vt_t, q_src, lay.krange, D ** -0.5, one_pass=one_pass), args.reps))
+    if want("gemm"):                       # the few-row kernel, weights larger than the L2 together
+        from ojb200 import lt_ext as LT
+        for rows in (12, 32):
+            x = rnd(rows, H).to(bf16)
+            for n, copies in ((12352, 4), (2048, 14)):
+                ws = [(rnd(n, H) * 0.02).to(bf16) for _ in range(copies)]
+                us = _time(lambda: [LT.lt_matmul(x, w, 11) for w in ws], max(1, args.reps // copies)) / copies
+                out(f"few-row GEMM {rows} x {n} x {H}", us)
     if want("norm"):
         x, d = rnd(N, H).to(bf16), rnd(N, H).to(bf16)
         w1 = torch.ones(H, device="cuda")
