@@ -372,7 +372,8 @@ int ojb_tree_attn_set_trace(uint64_t* records);
 
 /* Scoring head — replaces src/server.py:37 `mdl.head(forward_gtree(...).float())` together with the gather
  * src/fastmodel.py:482 `hn[lay.lastidx]`: out[s, a] = bias[a] + sum_h float(hn[rows[s], h]) * W[a, h], all fp32.
- * hn bf16 [N, H] (final-norm output), rows int64 [S] (last row of each candidate; null: row s), W fp32 [A, H], bias fp32 [A] or null. */
+ * hn bf16 [N, H] (final-norm output), rows int64 [S] (last row of each candidate, inside hn; a negative
+ * one gives not-a-numbers; null: row s), W fp32 [A, H], bias fp32 [A] or null. */
 int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S, int64_t A,
                    int64_t H, ojb_stream_t stream);
 /* The same with the row count of hn: indices as in ojb_gather_rows, the scores of one outside are not-a-number. */

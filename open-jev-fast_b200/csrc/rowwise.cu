@@ -766,7 +766,7 @@ score_head_kernel(const bf16_t* __restrict__ hn, int64_t n_src, const int64_t* _
   pdl_begin();
   __shared__ float red[32];
   const int s = blockIdx.x / A, a = blockIdx.x - s * A;
-  const int64_t n = rows ? row_of_index(rows[s], n_src) : s;
+  const int64_t n = rows == nullptr ? s : (n_src > 0 ? row_of_index(rows[s], n_src) : rows[s]);
   if (n < 0) {      // the whole block
     if (threadIdx.x == 0) {
       out[blockIdx.x] = __int_as_float(0x7fffffff);
@@ -790,20 +790,26 @@ score_head_kernel(const bf16_t* __restrict__ hn, int64_t n_src, const int64_t* _
 }  // namespace
 }  // namespace ojb
 
-extern "C" int ojb_score_head_rows(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out,
-                                   int64_t S, int64_t A, int64_t H, int32_t* status, ojb_stream_t stream) {
+static int launch_score_head(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
+                             int64_t A, int64_t H, int32_t* status, ojb_stream_t stream) {
   if (S == 0 || A == 0) return OJB_OK;
   OJB_REQUIRE(hn && W && out && S > 0 && A > 0 && H > 0 && H % 8 == 0);
-  OJB_REQUIRE(S * A < (int64_t{1} << 31) && n_src > 0 && (rows || S <= n_src));
+  OJB_REQUIRE(S * A < (int64_t{1} << 31));
   launch_kernel(ojb::score_head_kernel, dim3(static_cast<unsigned>(S * A)), dim3(ojb::kHeadThreads), 0, static_cast<cudaStream_t>(stream),
       static_cast<const ojb::bf16_t*>(hn), n_src, rows, W, bias, out, static_cast<int>(A), static_cast<int>(H), status);
   return ojb::launch_status(cudaGetLastError());
 }
 
-// without the row count of hn nothing is known to lie outside (and an index cannot count from the end)
+extern "C" int ojb_score_head_rows(const void* hn, int64_t n_src, const int64_t* rows, const float* W, const float* bias, float* out,
+                                   int64_t S, int64_t A, int64_t H, int32_t* status, ojb_stream_t stream) {
+  OJB_REQUIRE(S == 0 || A == 0 || (n_src > 0 && (rows || S <= n_src)));
+  return launch_score_head(hn, n_src, rows, W, bias, out, S, A, H, status, stream);
+}
+
+// without the row count of hn (n_src = 0) only a negative index is known to lie outside: none counts from the end
 extern "C" int ojb_score_head(const void* hn, const int64_t* rows, const float* W, const float* bias, float* out, int64_t S,
                               int64_t A, int64_t H, ojb_stream_t stream) {
-  return ojb_score_head_rows(hn, INT64_MAX, rows, W, bias, out, S, A, H, nullptr, stream);
+  return launch_score_head(hn, 0, rows, W, bias, out, S, A, H, nullptr, stream);
 }
 
 extern "C" int ojb_quantize_rows_e4m3(const void* x, void* q, float* scale, int64_t rows, int64_t K, ojb_stream_t stream) {

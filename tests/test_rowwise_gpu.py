@@ -176,6 +176,9 @@ def test_row_indices_count_from_the_end_and_an_index_outside_is_reported():
     same = K.score_head(a, ok % n, W, bias)
     assert torch.equal(K.score_head(a, ok, W, bias), same)
     _lib.check_status()
+    out = torch.zeros(5, 3, device="cuda")          # the entry point that does not know the row count: a negative index is outside
+    K.call("ojb_score_head", K.ptr(a), K.ptr(ok), K.ptr(W), K.ptr(bias), K.ptr(out), K.i64(5), K.i64(3), K.i64(24), K.stream_ptr())
+    assert torch.equal(torch.isnan(out).all(1), ok < 0) and torch.equal(out[ok >= 0], same[ok >= 0])
     for bad in (n, -n - 1, 1 << 40, -(1 << 62)):
         idx = ok.clone()
         idx[2] = bad
