@@ -124,6 +124,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// mbar_wait of a whole warp: one result for all lanes. Every role that goes on as a warp (tcgen05.ld / st, mma.sync, votes, shuffles, elected issue)
+// waits with it: were the limit to run out just as the barrier completes, lanes that decide for themselves could part, and those
+// that stay would wait in the next warp-wide instruction for those that left.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // Host-settable limit of those waits and the failure switch of the tests (gemm_api.cu: ojb_gemm_set_wait_limit_ms,
 // ojb_gemm_test_drop_copy); read by every launcher whose kernel waits on an mbarrier.
 int gemm_wait_limit_ms();

@@ -81,12 +81,6 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
   return p != 0;
 }
-// mbar_wait of a whole warp: one result for all lanes. Every role that goes on as a warp (tcgen05.ld / st, votes, shuffles, elected issue)
-// waits with it: were the limit to run out just as the barrier completes, lanes that decide for themselves could part, and those
-// that stay would wait in the next warp-wide instruction for those that left.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
-}
 // Arrive on an mbarrier once every tcgen05.mma issued so far by this thread has finished.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");

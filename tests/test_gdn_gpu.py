@@ -441,3 +441,52 @@ def test_dense_state_pass_past_its_staged_steps():
     _lib.check_status()
     for o, f in outs:
         assert torch.equal(o, out) and torch.equal(f, fin)
+
+
+# steps of 1 to 4 blocks of 16 rows; 31 to 33 and 64 to 66 steps cross the batches in which the step tables are read
+@pytest.mark.parametrize("root,stems,leaf", [(1, 1, [1]), (17, 2, [15, 16, 17]), (64, 1, [32, 33, 48, 49]), (65, 3, [63, 64, 65]),
+                                             (70, 1, [3] * 28), (70, 1, [3] * 29), (70, 1, [3] * 30), (31 * 64, 1, [40]),
+                                             (63 * 64 + 1, 2, [2, 130, 5])])
+@pytest.mark.parametrize("dense", [False, True])
+def test_state_pass_keeps_and_drops_states_as_the_tree_asks(root, stems, leaf, dense):
+    """A leaf's last state is computed only where it is exported, and a state the registers still hold is not loaded again: root ->
+    stems -> leaves against one recurrence per path, with the state of every other leaf exported and an output that starts 4 bytes
+    behind a 16-byte boundary. The error bounds are those of the other comparisons with the recurrence."""
+    from ojb200 import ext as K, _lib
+    HK, HV = 2, (40 if dense else 4)
+    chunks, steps, paths = [], [], []
+    n = 0
+
+    def node(rows, first, save, export=0):
+        nonlocal n
+        begin = n
+        for j in range(0, rows, 64):
+            last = j + 64 >= rows
+            chunks.append([n, min(64, rows - j), 0, 0])
+            steps.append([len(chunks) - 1, first if j == 0 else 0, save if last else 0, export if last else 0])
+            n += chunks[-1][1]
+        return list(range(begin, n))
+    top = node(root, 1, 1)
+    exports = 0
+    for s in range(stems):
+        stem = top + node(7 + 16 * s, 0 if s == 0 else 2, 2)
+        for j, rows in enumerate(leaf):
+            out = j % 2 == 0
+            exports += out
+            paths.append((stem + node(rows, 0 if j == 0 else 3, 0, exports if out else 0), exports - 1 if out else -1))
+    q, k, v, g, beta = _inputs(n, HK, HV, 21)
+    tab = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    fin = torch.zeros(exports, HV, 128, 128, device="cuda")
+    buf = torch.zeros(n * HV * 128 + 2, dtype=bf16, device="cuda")
+    o = buf[2:].view(n, HV, 128)
+    K.gdn_chunked(*(t.cuda() for t in (q, k, v, g, beta)), 128 ** -0.5, tab(chunks), tab(steps), tab([0, len(steps)]), 1, None, fin, o)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    heads = slice(0, 4)                     # (the oracle's time goes with the heads)
+    for rows, export in paths if len(paths) <= 6 else paths[::7]:
+        rows = torch.tensor(rows)
+        ref, state = OG.recurrent(*(t[rows][:, :(2 if i < 2 else 4)] if dense is False else
+                                    t[rows][:, :1 if i < 2 else 4] for i, t in enumerate((q, k, v, g, beta))), 128 ** -0.5)
+        assert _rel(o.cpu()[rows][:, heads], ref) < 4e-3
+        if export >= 0:
+            assert _rel(fin[export, heads], state) < 1e-2
