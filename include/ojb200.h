@@ -71,12 +71,18 @@ int ojb_gemm_bf16_swiglu_v(const void* x, const void* w_blk, void* out, int64_t 
 int ojb_gemm_bf16_splitk(const void* x, const void* w, float* parts, int64_t M, int64_t N, int64_t K, int splits,
                          int variant, int32_t* status, ojb_stream_t stream);
 
+/* h fp32 [M, N] += x · w^T (N % 32 == 0): one K range whose result goes straight to the fp32 residual stream, through bulk reductions of
+ * the block kernel, instead of a plane of ojb_gemm_bf16_splitk that ojb_resnorm_f32 adds afterwards (the same sum, h + product, in fp32;
+ * a product below 2^-126 counts as zero). variant 0 or 3: 256-row blocks, 4: every row in swapped-operand units. */
+int ojb_gemm_bf16_add(const void* x, const void* w, float* h, int64_t M, int64_t N, int64_t K, int variant, int32_t* status,
+                      ojb_stream_t stream);
+
 /* 8-bit variant of the three GEMM forms (the FP8 path the reference measured, README.md:131 / bench/logs/peak_fp8_bench.log,
  * and did not ship): operands are e4m3 bytes with one fp32 scale per row, out = (xq · wq^T) * sx[m] * sw[n], fp32
  * accumulation in tensor memory (tcgen05.mma.kind::f8f6f4, 256-row block kernel). kind 0: out = bf16 [M, N]; kind 1:
  * SwiGLU as in ojb_gemm_bf16_swiglu (wq = the re-laid gate/up weight, sw in the same row order, N % 256 == 0), out = bf16
- * [M, N/2]; kind 2: fp32 partials [splits, M, N] over K ranges of whole 128-column k-blocks. K % 16 == 0; splits = 1
- * unless kind 2. Off by default in the Python layer (OJ_FP8=1): scores move by more than the bf16 tolerance. */
+ * [M, N/2]; kind 2: fp32 partials [splits, M, N] over K ranges of whole 128-column k-blocks; kind 3: added to the fp32 [M, N] at out as
+ * in ojb_gemm_bf16_add (N % 64 == 0). K % 16 == 0; splits = 1 unless kind 2. Off by default in the Python layer (OJ_FP8=1): scores move by more than the bf16 tolerance. */
 int ojb_gemm_e4m3(const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M, int64_t N, int64_t K,
                   int32_t kind, int32_t splits, int32_t* status, ojb_stream_t stream);
 

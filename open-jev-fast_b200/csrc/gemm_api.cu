@@ -142,6 +142,13 @@ extern "C" int ojb_gemm_bf16_splitk(const void* x, const void* w, float* parts, 
   return dispatch(kEpiPartialF32, variant, x, w, parts, M, N, K, splits, N, status, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int ojb_gemm_bf16_add(const void* x, const void* w, float* h, int64_t M, int64_t N, int64_t K, int variant, int32_t* status,
+                                 ojb_stream_t stream) {
+  OJB_REQUIRE(x && w && h && M > 0 && N > 0 && K > 0 && K % 8 == 0 && N % 32 == 0 && (variant == 0 || variant == 3 || variant == 4));
+  OJB_REQUIRE(aligned16(x) && aligned16(w) && aligned16(h));
+  return gemm_block256_add_launch(variant == 4 ? -1 : 0, x, w, h, M, N, K, status, static_cast<cudaStream_t>(stream));
+}
+
 namespace ojb {
 namespace { int g_wait_ms = kDefaultWaitMs, g_drop_copy = 0; }
 int gemm_wait_limit_ms() { return g_wait_ms; }
@@ -213,11 +220,14 @@ extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int3
 extern "C" int ojb_gemm_e4m3(const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M, int64_t N,
                              int64_t K, int32_t kind, int32_t splits, int32_t* status, ojb_stream_t stream) {
   if (M == 0 || N == 0) return OJB_OK;
-  OJB_REQUIRE(xq && sx && wq && sw && out && M > 0 && N > 0 && K > 0 && K % 16 == 0 && kind >= 0 && kind <= 2);
+  OJB_REQUIRE(xq && sx && wq && sw && out && M > 0 && N > 0 && K > 0 && K % 16 == 0 && kind >= 0 && kind <= 3);
   OJB_REQUIRE(aligned16(xq) && aligned16(wq) && aligned16(out));
   OJB_REQUIRE(kind == 2 ? (splits >= 1 && splits <= 16) : splits == 1);
   OJB_REQUIRE(kind != 1 || N % 256 == 0);
+  OJB_REQUIRE(kind != 3 || N % 64 == 0);
   const int epi = kind == 0 ? kEpiBf16 : (kind == 1 ? kEpiSwiglu : kEpiPartialF32);
+  if (kind == 3)
+    return gemm_block256_launch_e4m3(epi, xq, sx, wq, sw, out, M, N, K, 1, N, status, static_cast<cudaStream_t>(stream), true);
   if (M <= kSkinnyRows && K % 128 == 0 && epi != kEpiSwiglu)
     return gemm_skinny_launch(epi, 0, xq, wq, out, M, N, K, splits, N, status, static_cast<cudaStream_t>(stream), sx, sw);
   return gemm_block256_launch_e4m3(epi, xq, sx, wq, sw, out, M, N, K, splits, kind == 1 ? N / 2 : N, status,

@@ -260,7 +260,8 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             fence_proxy_async();
             __syncwarp();
             if (lane == 0 && row0 < g.M) {
-              tma_store_3d(&map_out, tile_s, col, row0, EPI == kEpiPartialF32 ? u.split : 0);
+              if (EPI == kEpiPartialF32 && g.accum) tma_add_3d(&map_out, tile_s, col, row0, 0);
+              else tma_store_3d(&map_out, tile_s, col, row0, EPI == kEpiPartialF32 ? u.split : 0);
               bulk_commit();
             }
           };
@@ -535,7 +536,8 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
               __syncwarp();
               const int col0 = u.wt * 256 + acc_id * kBM + quarter * 32;
               if (lane == 0 && col0 < g.N) {
-                tma_store_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, EPI == kEpiPartialF32 ? u.split : 0);
+                if (EPI == kEpiPartialF32 && g.accum) tma_add_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, 0);
+                else tma_store_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, EPI == kEpiPartialF32 ? u.split : 0);
                 bulk_commit();
               }
               return;
@@ -607,7 +609,7 @@ constexpr size_t kSmemBudget = 227 * 1024;
 
 template <int EPI, bool FP8 = false>
 int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits, int bn_req, int64_t ldo,
-                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr) {
+                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr, bool accum = false) {
   static int smem_set[kMaxDevices] = {};
   auto kern = gemm_block256_kernel<EPI, FP8>;
   if (!raise_smem_limit(kern, static_cast<int>(kSmemBudget), smem_set)) return OJB_ERR_LAUNCH;
@@ -651,6 +653,7 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   if (static_cast<int64_t>(splits - 1) * g.kb_per_split >= g.kb_total) return OJB_ERR_ARG;   // an empty split
   g.BN = EPI == kEpiSwiglu ? 256 : (bn_req > 0 ? bn_req : choose_bn(N, g.n_xblk, g.tail_box, g.n_xchunk, g.tail_rows > 0, splits, g.kb_total, sms, EPI));
   if (FP8 && g.BN % 64 != 0) g.BN = (g.BN + 63) / 64 * 64;      // whole 128-byte store tiles (the scaled epilogue needs them)
+  if (accum) g.BN = (g.BN + 31) / 32 * 32;                       // (a reduction leaves as whole tiles too)
   g.n_wtile = static_cast<int>(ceil_div(N, g.BN));
   g.n_wtile256 = static_cast<int>(ceil_div(N, 256));
   g.band_xblk = band_blocks(g.n_xblk, static_cast<int64_t>(kBlockM) * K * (FP8 ? 1 : 2));
@@ -665,6 +668,8 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   const int out_elt = EPI == kEpiPartialF32 ? 4 : 2;
   g.tma_out = g.n_xblk > 0 && (ldo * out_elt) % 16 == 0 && g.BN % (128 / out_elt) == 0 ? 1 : 0;
   g.tail_tma = (g.tail_rows > 0 && (ldo * out_elt) % 16 == 0 && (EPI != kEpiPartialF32 || (M * N * 4) % 16 == 0)) ? 1 : 0;
+  g.accum = accum ? 1 : 0;
+  if (accum && ((g.n_xblk > 0 && !g.tma_out) || (g.tail_rows > 0 && !g.tail_tma))) return OJB_ERR_LIMIT;
   const size_t fixed = 1024 + (2 * kMaxStages + 2) * 8 + 16 + (g.tma_out ? kStagingBytes : (g.tail_tma ? kEpiWarps * 2048 : 0));
   g.stages = static_cast<int>((kSmemBudget - fixed) / g.stage_bytes);
   if (g.stages > kMaxStages) g.stages = kMaxStages;
@@ -730,11 +735,16 @@ int gemm_block256_launch(int epi, int bn_req, const void* x, const void* w, void
   return launch_gemm<kEpiPartialF32>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
 }
 
+int gemm_block256_add_launch(int bn_req, const void* x, const void* w, float* out, int64_t M, int64_t N, int64_t K, int32_t* status,
+                             cudaStream_t stream) {
+  return launch_gemm<kEpiPartialF32>(x, w, out, M, N, K, 1, bn_req, N, status, stream, nullptr, nullptr, true);
+}
+
 int gemm_block256_launch_e4m3(int epi, const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M,
-                              int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream) {
+                              int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream, bool accum) {
   if (epi == kEpiBf16) return launch_gemm<kEpiBf16, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
   if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
-  return launch_gemm<kEpiPartialF32, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
+  return launch_gemm<kEpiPartialF32, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw, accum);
 }
 
 }  // namespace ojb

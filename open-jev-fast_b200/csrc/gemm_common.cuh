@@ -29,6 +29,12 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
                "r"(y), "r"(z)
                : "memory");
 }
+// The same as an addition to the fp32 values that are there, made by the L2: the tile is not read back by the SM.
+__device__ __forceinline__ void tma_add_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
+  asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(src),
+               "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all bulk stores of this thread have finished reading their shared-memory source
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
@@ -264,11 +270,14 @@ int gemm_tile128_launch(int epi, int bn, const void* x, const void* w, void* out
                         int64_t ldo, int32_t* status, cudaStream_t stream);
 int gemm_block256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,
                          int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
+// out fp32 [M, N] += the product (one K range; N % 32 == 0)
+int gemm_block256_add_launch(int bn_req, const void* x, const void* w, float* out, int64_t M, int64_t N, int64_t K, int32_t* status,
+                             cudaStream_t stream);
 void gemm_block256_set_trace(unsigned long long* buf, int cap);
 // process-wide settings kept in gemm_api.cu: limit of the device-side waits (ms) and the failure-injection switch of the tests
 // e4m3 operands with one fp32 scale per row of x (sx) and per row of w (sw): out = (xq . wq^T) * sx[m] * sw[n]
 int gemm_block256_launch_e4m3(int epi, const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M,
-                              int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
+                              int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream, bool accum = false);
 int tree_attn_long_launch(const void* qt, int64_t NQ, const int64_t* q_rows, const void* kt, const void* vt_t, int64_t N, const void* gate,
                           int64_t gate_ld, int64_t gate_hs, const int32_t* krange, void* y, int64_t HQ, int64_t HKV, float scale,
                           int32_t* status, cudaStream_t st);

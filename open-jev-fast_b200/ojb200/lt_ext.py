@@ -101,6 +101,21 @@ def gemm_splitk(x, w, S, idx=0):
     return parts
 
 
+def gemm_add(x, w, h, idx=0):
+    """h += x @ w^T in place (ojb_gemm_bf16_add): h fp32 [M, N], N a multiple of 32; idx 0 or 3 the block kernel, 7 all rows swapped."""
+    _check(x, w)
+    M, K = x.shape
+    N = w.shape[0]
+    _check_sum(h, M, N, x.device)
+    call("ojb_gemm_bf16_add", ptr(x), ptr(w), ptr(h), i64(M), i64(N), i64(K), i32(VARIANT_BN[idx]), ptr(_lib.status_word(x.device)),
+         stream_ptr())
+
+
+def _check_sum(h, M, N, device):
+    if not (h.is_contiguous() and h.dtype == torch.float32 and h.device == device and tuple(h.shape) == (M, N)):
+        raise RuntimeError("gemm_add: h must be a contiguous fp32 [M, N] on the operands' device")
+
+
 # ---------------------------------------------------------------------------------------------- lt2_* (src/lt.cpp:64-190)
 def quantize_weight_e4m3(w):
     """Offline weight preparation of the 8-bit path: w [N, K] bf16 -> (e4m3 bytes [N, K] as uint8, fp32 scale per row), scale =
@@ -122,9 +137,9 @@ def quantize_rows_e4m3(x):
     return q, s
 
 
-def gemm_e4m3(xq, sx, wq, sw, kind=0, splits=1):
+def gemm_e4m3(xq, sx, wq, sw, kind=0, splits=1, h=None):
     """out = (xq @ wq^T) * sx[:, None] * sw[None, :] on e4m3 operands (ojb_gemm_e4m3). kind 0: bf16 [M, N]; 1: SwiGLU on the
-    re-laid gate/up weight -> bf16 [M, N/2]; 2: fp32 partials [splits, M, N]."""
+    re-laid gate/up weight -> bf16 [M, N/2]; 2: fp32 partials [splits, M, N]; 3: added to h fp32 [M, N] (N a multiple of 64)."""
     for t, dt in ((xq, torch.uint8), (wq, torch.uint8), (sx, torch.float32), (sw, torch.float32)):
         if not (t.is_cuda and t.is_contiguous() and t.dtype == dt):
             raise RuntimeError("gemm_e4m3: contiguous CUDA uint8 operands and fp32 scales expected")
@@ -136,6 +151,9 @@ def gemm_e4m3(xq, sx, wq, sw, kind=0, splits=1):
         out = torch.empty(M, N, dtype=bf16, device=xq.device)
     elif kind == 1:
         out = torch.empty(M, N // 2, dtype=bf16, device=xq.device)
+    elif kind == 3:
+        _check_sum(h, M, N, xq.device)
+        out = h
     else:
         out = torch.empty(splits, M, N, dtype=torch.float32, device=xq.device)
     call("ojb_gemm_e4m3", ptr(xq), ptr(sx), ptr(wq), ptr(sw), ptr(out), i64(M), i64(N), i64(K), i32(kind), i32(splits),

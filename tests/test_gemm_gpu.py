@@ -338,3 +338,43 @@ def test_few_row_kernel_e4m3(M, N, K):
         if (S - 1) * -(-(K // 128) // S) < K // 128:
             assert bool(((LT.gemm_e4m3(xq, sx, wq, sw, 2, S).double().sum(0) - ref).abs() <= bound).all())
     _lib.check_status()
+
+
+# block units alone, with swapped tails of 16 and 128 rows, swapped units alone, a w tile that reaches past the last output
+@pytest.mark.parametrize("M,N,K,idx", [(256, 320, 192, 3), (272, 5120, 640, 0), (640, 96, 1000, 3), (1, 64, 64, 3), (300, 544, 512, 7), (2600, 5120, 320, 3)])
+@pytest.mark.parametrize("e4m3", [False, True])
+def test_product_added_to_the_stream_equals_a_plane_added_afterwards(M, N, K, idx, e4m3):
+    """h + x w^T in place, by the reductions of the block kernel, has the bits of the fp32 plane of one K range added with torch."""
+    from ojb200 import lt_ext as LT, _lib
+    x, w = _mk(M, N, K, 9)
+    h = torch.randn(M, N, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda") * 4
+    guard = torch.full((M + 2, N), 7.0, device="cuda")
+    got = guard[1:M + 1]
+    got.copy_(h)
+    if e4m3:
+        if N % 64 or K % 16:
+            (xq, sx), (wq, sw) = LT.quantize_rows_e4m3(x), LT.quantize_weight_e4m3(w)
+            with pytest.raises(RuntimeError):
+                LT.gemm_e4m3(xq, sx, wq, sw, 3, h=got)
+            return
+        (xq, sx), (wq, sw) = LT.quantize_rows_e4m3(x), LT.quantize_weight_e4m3(w)
+        want = h + LT.gemm_e4m3(xq, sx, wq, sw, 2, 1)[0]
+        LT.gemm_e4m3(xq, sx, wq, sw, 3, h=got)
+    else:
+        want = h + LT.gemm_splitk(x, w, 1, idx)[0]
+        LT.gemm_add(x, w, got, idx)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(got, want)
+    assert bool((guard[0] == 7).all()) and bool((guard[-1] == 7).all())
+
+
+def test_product_added_to_the_stream_refuses_what_it_does_not_take():
+    from ojb200 import lt_ext as LT
+    x, w = _mk(64, 40, 64, 1)
+    with pytest.raises(RuntimeError):
+        LT.gemm_add(x, w, torch.zeros(64, 40, device="cuda"))                      # outputs not in whole tiles
+    x, w = _mk(64, 64, 64, 1)
+    for h in (torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(63, 64, device="cuda"), torch.zeros(64, 128, device="cuda")[:, ::2]):
+        with pytest.raises(RuntimeError):
+            LT.gemm_add(x, w, h)
