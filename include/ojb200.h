@@ -217,6 +217,15 @@ int ojb_gtree_dims(const int64_t* tokens, const int64_t* seq_off, const int32_t*
 int ojb_gtree_fill(const int64_t* tokens, const int64_t* seq_off, const int32_t* groups, int64_t S, int64_t pad_id,
                    int64_t NB, int64_t PB, int64_t* buf64, int32_t* buf32, int32_t* ext32, int32_t flags);
 
+/* Host tables of S sequences (lens[s] <= T rows each) behind a shared prefix of Lp rows whose first `pad` are left padding: the single-level
+ * tree of src/fastmodel.py:247-264 (own_walks = 0: one walk, the prefix state handed to every sequence) or, with Lp = 0 and own_walks = 1,
+ * the right-padded batch of src/fastmodel.py:205-241 (one walk per sequence). Rows: prefix, sequence 0, sequence 1, ..., padding up to
+ * N32 = a multiple of 32. pos [N32], lastidx [S] int64; rowmask [N32], hist [N32 + 1, 4], krange [N32, 8], chunks and steps [cap, 4],
+ * walk_ptr [2 or S + 1] int32, all written in full. OJB_ERR_LIMIT if the sequences have more than cap chunks. */
+int ojb_seq_tables(const int64_t* lens, int64_t S, int64_t Lp, int64_t pad, int64_t T, int32_t own_walks, int64_t cap, int64_t* pos,
+                   int64_t* lastidx, int32_t* rowmask, int32_t* hist, int32_t* krange, int32_t* chunks, int32_t* steps,
+                   int32_t* walk_ptr);
+
 /* ------------------------------------------------------------------------------------------------------------------
  * Gated DeltaNet (linear attention).
  * ------------------------------------------------------------------------------------------------------------------ */

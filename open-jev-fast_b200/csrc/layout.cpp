@@ -329,3 +329,86 @@ extern "C" int ojb_gtree_fill(const int64_t* tokens, const int64_t* seq_off, con
   }
   return OJB_OK;
 }
+
+// Tables of S sequences of at most T rows behind a shared prefix of Lp rows, `pad` of them left padding (in the row order prefix,
+// sequence 0, sequence 1, ..., rows up to a multiple of 32): every entry is written. The loops in Python that this replaces took 1.4 ms
+// for a batch of six sequences of 260 rows and 0.5 ms for five suffixes behind 1900 rows; here 20 us.
+extern "C" int ojb_seq_tables(const int64_t* lens, int64_t S, int64_t Lp, int64_t pad, int64_t T, int32_t own_walks, int64_t cap, int64_t* pos,
+                              int64_t* lastidx, int32_t* rowmask, int32_t* hist, int32_t* krange, int32_t* chunks, int32_t* steps,
+                              int32_t* walk_ptr) {
+  if (!lens || !pos || !lastidx || !rowmask || !hist || !krange || !chunks || !steps || !walk_ptr) return OJB_ERR_ARG;
+  if (S < 0 || Lp < 0 || T < 0 || pad < 0 || pad > Lp || cap < 1 || (own_walks && Lp != 0)) return OJB_ERR_ARG;
+  int64_t need = (Lp - pad + 63) / 64;
+  for (int64_t s = 0; s < S; ++s) {
+    if (lens[s] < 0 || lens[s] > T) return OJB_ERR_ARG;
+    need += (lens[s] + 63) / 64;
+  }
+  if (need > cap) return OJB_ERR_LIMIT;
+  const int64_t N = Lp + S * T, N32 = (N + 31) / 32 * 32;
+  if (N32 > INT32_MAX / 8) return OJB_ERR_LIMIT;
+  auto alone = [&](int64_t n) {                    // padding: a row that sees itself and belongs to no path
+    rowmask[n] = 0;
+    for (int i = 0; i < 4; ++i) hist[n * 4 + i] = -1;
+    int32_t* kr = krange + n * 8;
+    for (int i = 0; i < 8; ++i) kr[i] = 0;
+    kr[3] = static_cast<int32_t>(n);
+    kr[4] = static_cast<int32_t>(n + 1);
+  };
+  for (int64_t n = 0; n < Lp; ++n) {
+    alone(n);
+    pos[n] = n - pad;
+    if (n < pad) continue;
+    rowmask[n] = 1;
+    krange[n * 8 + 3] = static_cast<int32_t>(pad);
+    for (int64_t i = 0; i < 4; ++i) hist[n * 4 + i] = n - 3 + i >= pad ? static_cast<int32_t>(n - 3 + i) : -1;
+  }
+  for (int64_t s = 0; s < S; ++s) {
+    const int64_t first = Lp + s * T;
+    for (int64_t t = 0; t < T; ++t) {
+      const int64_t n = first + t;
+      alone(n);
+      const bool real = t < lens[s];
+      pos[n] = own_walks ? (real ? t : 0) : t + (Lp - pad);
+      if (!real) continue;
+      rowmask[n] = 1;
+      int32_t* kr = krange + n * 8;
+      if (!own_walks) {
+        kr[1] = static_cast<int32_t>(pad);
+        kr[2] = static_cast<int32_t>(Lp);
+      }
+      kr[3] = static_cast<int32_t>(first);
+      for (int64_t i = 0; i < 4; ++i) {            // the last rows of the path: this sequence's, then the prefix's
+        const int64_t back = 3 - i;
+        if (t >= back) hist[n * 4 + i] = static_cast<int32_t>(n - back);
+        else if (Lp - (back - t) >= pad) hist[n * 4 + i] = static_cast<int32_t>(Lp - (back - t));
+      }
+    }
+    lastidx[s] = first + (lens[s] > 0 ? lens[s] - 1 : 0);
+  }
+  for (int64_t n = N; n < N32; ++n) {
+    alone(n);
+    pos[n] = 0;
+  }
+  for (int i = 0; i < 4; ++i) hist[N32 * 4 + i] = -1;
+  int64_t k = 0;
+  auto chunk = [&](int64_t row, int64_t rows, int load) {
+    int32_t *c = chunks + k * 4, *st = steps + k * 4;
+    c[0] = static_cast<int32_t>(row); c[1] = static_cast<int32_t>(rows); c[2] = c[3] = 0;
+    st[0] = static_cast<int32_t>(k); st[1] = load; st[2] = st[3] = 0;
+    ++k;
+  };
+  int64_t w = 0;
+  walk_ptr[w++] = 0;
+  for (int64_t j = pad; j < Lp; j += 64) chunk(j, Lp - j < 64 ? Lp - j : 64, j == pad ? 1 : 0);
+  if (k > 0) steps[(k - 1) * 4 + 2] = 1;           // the prefix state is parked in slot A
+  for (int64_t s = 0; s < S; ++s) {
+    for (int64_t j = 0; j < lens[s]; j += 64)
+      chunk(Lp + s * T + j, lens[s] - j < 64 ? lens[s] - j : 64, j > 0 ? 0 : (Lp > pad ? 2 : 1));
+    if (own_walks) walk_ptr[w++] = static_cast<int32_t>(k);
+  }
+  if (!own_walks) walk_ptr[w++] = static_cast<int32_t>(k);
+  for (int64_t i = k; i < cap; ++i)
+    for (int e = 0; e < 4; ++e) chunks[i * 4 + e] = steps[i * 4 + e] = 0;
+  if (k == 0) steps[1] = 1;
+  return OJB_OK;
+}

@@ -144,43 +144,62 @@ def pack_requests(requests, pad_id=0, NB=32, PB=16, dev="cuda", pin=False):
     return host["ids"].to(dev), lay, host
 
 
+class SeqTables:
+    """Tables of sequences behind a shared prefix (ojb_seq_tables) as views into two buffers, one of int64 and one of int32 fields."""
+
+    def __init__(self, S, N32, cap, walks, device="cpu", pin=False):
+        mk = lambda n, dt: torch.empty(n, dtype=dt, device=device, pin_memory=pin)
+        sizes = [N32, (N32 + 1) * 4, N32 * 8, cap * 4, cap * 4, walks + 1]
+        o = np.cumsum([0] + sizes)
+        self.b64, self.b32 = mk(N32 + S, torch.int64), mk(int(o[-1]), torch.int32)
+        self._shape = (S, N32, cap, walks)
+        self.pos32, self.lastidx = self.b64[:N32], self.b64[N32:]
+        v = [self.b32[int(o[i]):int(o[i + 1])] for i in range(6)]
+        self.rowmask32, self.hist, self.krange, self.chunks, self.steps, self.walk_ptr = (
+            v[0], v[1].view(N32 + 1, 4), v[2].view(N32, 8), v[3].view(cap, 4), v[4].view(cap, 4), v[5])
+
+    @classmethod
+    def build(cls, lens, Lp, pad, T, own_walks, cap=None, pin=False):
+        """On the host. cap: entries of the chunk and step tables (default: as many as there are chunks)."""
+        lens = np.ascontiguousarray(lens, np.int64)
+        S = len(lens)
+        need = max(1, -(-(Lp - pad) // 64) + int((-(-lens // 64)).sum()))
+        if cap is not None and need > max(cap, 1):
+            raise RuntimeError("tree_layout: more chunks than the table capacity")
+        cap = need if cap is None else max(cap, 1)
+        t = cls(S, -(-(Lp + S * T) // 32) * 32, cap, S if own_walks else 1, pin=pin)
+        p = lambda x, ty: ctypes.cast(x.data_ptr(), ty)
+        rc = _lib.lib().ojb_seq_tables(lens.ctypes.data_as(_I64P), *(ctypes.c_int64(x) for x in (S, Lp, pad, T)), ctypes.c_int32(own_walks),
+                                       ctypes.c_int64(cap), p(t.pos32, _I64P), p(t.lastidx, _I64P), *(p(x, _I32P) for x in (
+                                           t.rowmask32, t.hist, t.krange, t.chunks, t.steps, t.walk_ptr)))
+        if rc != 0:
+            raise RuntimeError("layout: the tables of the sequences cannot be built")
+        return t
+
+    def to(self, device):
+        """A copy on `device`, which does not wait where the host buffers are pinned."""
+        if torch.device(device).type == "cpu":
+            return self
+        d = SeqTables(*self._shape, device=device)
+        d.upload(self)
+        return d
+
+    def upload(self, host):
+        """Another request's tables of the same sizes over these."""
+        self.b64.copy_(host.b64, non_blocking=True)
+        self.b32.copy_(host.b32, non_blocking=True)
+
+
 def batch_layout(attention_mask, dev):
     """Layout of a right-padded batch [B, T] of independent sequences (the non-tree forward of src/fastmodel.py:205-241)
     in the vocabulary of the tree kernels: every sequence is its own path, rows are b*T + t, padded up to a multiple of 32
     rows. Returns a namespace with pos, rowmask, hist, krange, chunks, steps, walk_ptr, n_walks, lastidx, N and parks = False (no
     walk parks a state)."""
-    m = attention_mask.detach().cpu().numpy().astype(bool)
-    B, T = m.shape
-    N = -(-(B * T) // 32) * 32
-    lens = m.sum(1)
-    pos = np.zeros(N, np.int64)
-    rowmask = np.zeros(N, np.int32)
-    hist = np.full((N + 1, 4), -1, np.int32)
-    krange = np.zeros((N, 8), np.int32)
-    chunks, steps, walks = [], [], [0]
-    for b in range(B):
-        L = int(lens[b])
-        for t in range(T):
-            n = b * T + t
-            krange[n, 3], krange[n, 4] = (b * T, n + 1) if t < L else (n, n + 1)
-            if t < L:
-                pos[n], rowmask[n] = t, 1
-                for i in range(4):
-                    if t - 3 + i >= 0:
-                        hist[n, i] = n - 3 + i
-        for j in range(0, L, 64):
-            steps.append([len(chunks), 1 if j == 0 else 0, 0, 0])
-            chunks.append([b * T + j, min(64, L - j), 0, 0])
-        walks.append(len(steps))
-    for n in range(B * T, N):
-        krange[n, 3], krange[n, 4] = n, n + 1
-    if not chunks:
-        chunks, steps = [[0, 0, 0, 0]], [[0, 1, 0, 0]]
-    t32 = lambda a: torch.as_tensor(np.asarray(a, np.int32)).to(dev)
-    last = np.array([b * T + max(int(lens[b]) - 1, 0) for b in range(B)], np.int64)
-    return SimpleNamespace(N=N, S=B, L2=T, pos=torch.as_tensor(pos).to(dev), rowmask=t32(rowmask), hist=t32(hist),
-                           krange=t32(krange), chunks=t32(chunks), steps=t32(steps), walk_ptr=t32(walks), n_walks=B, parks=False,
-                           lastidx=torch.as_tensor(last).to(dev))
+    B, T = attention_mask.shape
+    lens = attention_mask.detach().cpu().numpy().astype(bool).sum(1)
+    t = SeqTables.build(lens, 0, 0, T, True, pin=torch.device(dev).type == "cuda").to(dev)
+    return SimpleNamespace(N=t.pos32.shape[0], S=B, L2=T, pos=t.pos32, rowmask=t.rowmask32, hist=t.hist, krange=t.krange, chunks=t.chunks,
+                           steps=t.steps, walk_ptr=t.walk_ptr, n_walks=B, parks=False, lastidx=t.lastidx)
 
 
 def tree_layout(pre_ids, suf_ids, suf_mask, pad=0, dense=True, cap=None):
@@ -194,58 +213,12 @@ def tree_layout(pre_ids, suf_ids, suf_mask, pad=0, dense=True, cap=None):
     S, Ls = (int(x) for x in suf_ids.shape)
     m = suf_mask.detach().cpu().numpy().astype(bool)
     N = Lp + S * Ls
-    N32 = -(-N // 32) * 32
-    pos = np.zeros(N32, np.int64)
-    rowmask = np.zeros(N32, np.int32)
-    hist = np.full((N32 + 1, 4), -1, np.int32)
-    krange = np.zeros((N32, 8), np.int32)
-    for n in range(N32):
-        krange[n, 3], krange[n, 4] = n, n + 1                      # default: a row sees only itself
-    # positions follow the reference for every row, padding included: prefix t - pad, suffix t + (Lp - pad)
-    pos[:Lp] = np.arange(Lp) - pad
-    for s in range(S):
-        pos[Lp + s * Ls: Lp + (s + 1) * Ls] = np.arange(Ls) + (Lp - pad)
-    if Lp > pad:
-        pr = np.arange(pad, Lp)
-        rowmask[pad:Lp] = 1
-        krange[pad:Lp, 3], krange[pad:Lp, 4] = pad, pr + 1
-        hp = pr[:, None] - 3 + np.arange(4)[None, :]
-        hist[pad:Lp] = np.where(hp >= pad, hp, -1)
-    lens = m.sum(1)
-    for s in range(S):
-        for t in range(int(lens[s])):
-            n = Lp + s * Ls + t
-            rowmask[n] = 1
-            krange[n, 1], krange[n, 2] = pad, Lp
-            krange[n, 3], krange[n, 4] = Lp + s * Ls, n + 1
-            tail = list(range(max(pad, Lp - 3), Lp)) + list(range(Lp + s * Ls, n + 1))     # the last rows of this path
-            for i in range(4):
-                if len(tail) - 4 + i >= 0:
-                    hist[n, i] = tail[len(tail) - 4 + i]
-    chunks, steps, walks = [], [], [0]
-    for j in range(pad, Lp, 64):
-        steps.append([len(chunks), 1 if j == pad else 0, 0, 0])
-        chunks.append([j, min(64, Lp - j), 0, 0])
-    if steps:
-        steps[-1][2] = 1                                            # park the prefix state in slot A
-    for s in range(S):
-        for j in range(0, int(lens[s]), 64):
-            steps.append([len(chunks), (2 if Lp > pad else 1) if j == 0 else 0, 0, 0])
-            chunks.append([Lp + s * Ls + j, min(64, int(lens[s]) - j), 0, 0])
-    walks.append(len(steps))
-    if not chunks:
-        chunks, steps = [[0, 0, 0, 0]], [[0, 1, 0, 0]]
-    if cap is not None:
-        if len(chunks) > cap:
-            raise RuntimeError("tree_layout: more chunks than the table capacity")
-        chunks += [[0, 0, 0, 0]] * (cap - len(chunks))
-        steps += [[0, 0, 0, 0]] * (cap - len(steps))
-    t32 = lambda a: torch.as_tensor(np.asarray(a, np.int32)).to(dev)
-    lastidx = np.array([Lp + s * Ls + max(int(lens[s]) - 1, 0) for s in range(S)], np.int64)
+    t = SeqTables.build(m.sum(1), Lp, pad, Ls, False, cap, pin=dev.type == "cuda").to(dev)
+    lay = SimpleNamespace(Lp=Lp, S=S, Ls=Ls, N=N, N32=t.pos32.shape[0], pos=t.pos32[:N], pos32=t.pos32, rowmask=t.rowmask32[:N],
+                          rowmask32=t.rowmask32, lastidx=t.lastidx, hist=t.hist, krange=t.krange, chunks=t.chunks, steps=t.steps,
+                          walk_ptr=t.walk_ptr, n_walks=1, tables=t)
     if not dense:
-        return SimpleNamespace(Lp=Lp, S=S, Ls=Ls, N=N, N32=N32, pos=torch.as_tensor(pos[:N]).to(dev), pos32=torch.as_tensor(pos).to(dev),
-                               rowmask=t32(rowmask[:N]), rowmask32=t32(rowmask), lastidx=torch.as_tensor(lastidx).to(dev),
-                               hist=t32(hist), krange=t32(krange), chunks=t32(chunks), steps=t32(steps), walk_ptr=t32(walks), n_walks=1)
+        return lay
     # dense mask with the reference's semantics for every row (rows that are padding still see valid earlier keys of their
     # own segment and of the prefix); the kernels read krange, where padding rows see only themselves
     seg = np.concatenate([np.zeros(Lp, np.int64), np.repeat(np.arange(1, S + 1), Ls)])
@@ -256,7 +229,6 @@ def tree_layout(pre_ids, suf_ids, suf_mask, pad=0, dense=True, cap=None):
     same_suffix = (seg[None, :] == seg[:, None]) & (seg[:, None] != 0) & earlier
     vis = ((from_prefix | same_suffix) & valid[None, :]) | np.eye(N, dtype=bool)
     repidx = np.array([[p if p < Lp else Lp + s * Ls + (p - Lp) for p in range(Lp + Ls)] for s in range(S)], np.int64)
-    return SimpleNamespace(Lp=Lp, S=S, Ls=Ls, N=N, N32=N32, pos=torch.as_tensor(pos[:N]).to(dev), pos32=torch.as_tensor(pos).to(dev),
-                           amask=torch.as_tensor(vis).to(dev)[None, None], rowmask=t32(rowmask[:N]), rowmask32=t32(rowmask),
-                           lastidx=torch.as_tensor(lastidx).to(dev), repidx=torch.as_tensor(repidx).to(dev), hist=t32(hist),
-                           krange=t32(krange), chunks=t32(chunks), steps=t32(steps), walk_ptr=t32(walks), n_walks=1)
+    lay.amask = torch.as_tensor(vis).to(dev)[None, None]
+    lay.repidx = torch.as_tensor(repidx).to(dev)
+    return lay

@@ -66,6 +66,17 @@ def token_records(records, tok, candidate_prompts):
     return out
 
 
+def _common_prefix(seqs, most):
+    """How many tokens, at most `most`, all candidates begin with."""
+    n = 0
+    if all(type(q) is list for q in seqs):      # 64 at a time while they agree
+        while n < most and all(q[n:min(n + 64, most)] == seqs[0][n:min(n + 64, most)] for q in seqs):
+            n = min(n + 64, most)
+    while n < most and all(q[n] == seqs[0][n] for q in seqs):
+        n += 1
+    return n
+
+
 class Entry:
     """Static buffers + CUDA graph of `score_gtree` for one key (N, S, L2). The tree structure lives in the index tables,
     so every request with the same key replays the same graph after three host-to-device copies. Capture runs in
@@ -133,7 +144,6 @@ class EntryState:
     """Single-level prefix tree with prefix-state hand-off (long shared context, one question): src/server.py:50-70. Static
     prefix / suffix / mask buffers and one CUDA graph per key (Lp bucket, S, Ls bucket); `run` rebuilds the layout on the
     host (tables padded to the key's capacity) and copies it over the static tables."""
-    FIELDS = ("pos32", "rowmask32", "hist", "krange", "chunks", "steps", "walk_ptr", "lastidx")
 
     def __init__(self, scorer, Lpb, S, Lsb):
         fast, dev = scorer.fast, scorer.device
@@ -167,9 +177,8 @@ class EntryState:
         self.pre.copy_(pre, non_blocking=True)
         self.suf.copy_(suf, non_blocking=True)
         self.msk.copy_(msk, non_blocking=True)
-        L = self._fast.tree_layout(pre, suf, msk, pad=pad, dense=False, cap=self.cap)          # host tensors
-        for name in self.FIELDS:
-            getattr(self.lay, name).copy_(getattr(L, name), non_blocking=True)
+        self.lay.tables.upload(_layout.SeqTables.build(msk.numpy().astype(bool).sum(1), pre.shape[0], pad, suf.shape[1], False, self.cap,
+                                                       pin=True))
         if self.g is not None:
             self.g.replay()
         else:
@@ -281,10 +290,7 @@ class Scorer:
         fp32 [S, A] (GPU, not synchronised). The general tree route (score_tokens) serves the same requests; this one keeps
         the reference's key (Lp bucket, S, Ls bucket) and its `tree_layout` / `forward_tree` entry points."""
         t0 = time.perf_counter()
-        mn = min(len(q) for q in seqs)
-        Lp = 0
-        while Lp < mn - 1 and all(q[Lp] == seqs[0][Lp] for q in seqs):
-            Lp += 1
+        Lp = _common_prefix(seqs, min(len(q) for q in seqs) - 1)
         S = len(seqs)
         Ls = max(len(q) - Lp for q in seqs)
         ceil_ = lambda x, b: -(-x // b) * b

@@ -188,3 +188,66 @@ def test_packed_requests_tables():
         assert rows[:, 1].sum() == real.sum()                     # the walk of a request covers each of its real rows once
         assert np.array_equal(host["lastidx"].numpy()[sum(lay.counts[:i]):sum(lay.counts[:i + 1])], r["lastidx"] + base)
         base += n
+
+
+@pytest.mark.parametrize("Lp,pad,lens,T", [(0, 0, [5, 0, 64, 65], 70), (0, 0, [1], 1), (0, 0, [0, 0], 3), (7, 0, [3, 1], 4), (64, 61, [2, 6], 6),
+                                           (130, 2, [0, 65, 1], 65), (33, 33, [4, 2], 4), (3, 1, [1, 2, 3, 4], 4)])
+@pytest.mark.parametrize("own_walks", [True, False])
+def test_sequence_tables(Lp, pad, lens, T, own_walks):
+    """Batch of sequences / single-level tree: every row's path, written out, gives history, key ranges and positions; the chunks cover
+    each path once in order, the prefix parks its state and every sequence starts from it."""
+    from ojb200.layout import SeqTables
+    if own_walks and Lp:
+        pytest.skip("sequences of a batch share no prefix")
+    S, N = len(lens), Lp + len(lens) * T
+    extra = 3
+    t = SeqTables.build(lens, Lp, pad, T, own_walks, cap=sum(-(-n // 64) for n in lens) + -(-(Lp - pad) // 64) + extra)
+    N32 = -(-N // 32) * 32
+    assert t.pos32.shape[0] == N32 and t.hist.shape[0] == N32 + 1
+    prefix = list(range(pad, Lp))
+    paths = {n: prefix[:i + 1] for i, n in enumerate(prefix)}
+    for s, L in enumerate(lens):
+        for i in range(L):
+            paths[Lp + s * T + i] = prefix + list(range(Lp + s * T, Lp + s * T + i + 1))
+    for n in range(N32):
+        path = paths.get(n, [])
+        assert t.hist[n].tolist() == ([-1] * 4 + path)[-4:]
+        assert int(t.rowmask32[n]) == (n in paths)
+        e0, a1, e1, a2, e2, a0 = t.krange[n].tolist()[:6]
+        assert list(range(a0, e0)) + list(range(a1, e1)) + list(range(a2, e2)) == (path or [n])
+        seq = n >= Lp and n < N
+        want = n - pad if n < Lp else ((n - Lp) % T + Lp - pad if seq and (not own_walks or n in paths) else 0)
+        assert int(t.pos32[n]) == want
+    assert t.hist[N32].tolist() == [-1] * 4
+    assert t.lastidx.tolist() == [Lp + s * T + max(L - 1, 0) for s, L in enumerate(lens)]
+    got, w = [], t.walk_ptr.tolist()
+    assert len(w) == (S + 1 if own_walks else 2) and w[0] == 0
+    for i in range(w[-1]):
+        c, load, save, aux = t.steps[i].tolist()
+        first, rows = t.chunks[c].tolist()[:2]
+        assert c == i and 1 <= rows <= 64 and aux == 0
+        starts = first == pad and Lp > pad or first >= Lp and (first - Lp) % T == 0
+        assert load == ((2 if Lp > pad and first >= Lp else 1) if starts else 0) and save == (1 if first + rows == Lp else 0)
+        got += range(first, first + rows)
+    assert got == sorted(paths)
+    assert t.chunks[w[-1]:, 1].sum() == 0
+
+
+def test_sequence_tables_refuse_what_does_not_fit():
+    from ojb200.layout import SeqTables
+    for lens, T in (([5], 4), ([-1], 4)):
+        with pytest.raises(RuntimeError):
+            SeqTables.build(lens, 0, 0, T, True, cap=4)
+    with pytest.raises(RuntimeError):
+        SeqTables.build([64, 64, 65], 0, 0, 65, True, cap=3)
+
+
+def test_common_prefix_of_candidates():
+    from ojb200.server import _common_prefix
+    base = list(range(200))
+    for n in (0, 1, 63, 64, 65, 128, 150):
+        seqs = [base[:n] + [1000 + i] + base[:70] for i in range(3)]
+        for most in (0, 1, n, n + 1, 150):
+            want = min(n, most)
+            assert _common_prefix(seqs, most) == want and _common_prefix([tuple(q) for q in seqs], most) == want
+    assert _common_prefix([base, base, base], 199) == 199
