@@ -40,12 +40,14 @@ int ojb_abi_version(void);
  * GEMM — replaces src/lt.cpp:43 lt_matmul / src/fastmodel.py:168 _mm (cuBLASLt) and src/fastmodel.py:158 _skmm
  * (torch.bmm split-K partials). out[M,N] = x[M,K] · w[N,K]^T, bf16 operands, fp32 accumulation in tensor memory.
  * Requirements: K % 8 == 0, x / w / out 16-byte aligned. variant: 0 = the library chooses (cost model, see ojb_gemm_plan);
- * 1 / 2 = 128-row tile kernel with 128x256 / 128x128 tiles; 3 = 256-row block kernel, automatic w-tile width; 4 = that
+ * 1 / 2 = 128-row tile kernel with 128x256 / 128x128 tiles; 3 = 256-row block kernel, w-tile width and form of the rows
+ * behind the full blocks (as 7 or 8) by the cost model; 4 = that
  * kernel with all rows of x in swapped-operand units (M <= 2048); a multiple of 16 in [16, 256] = that kernel with this
  * w-tile width; 5 = CTA-pair kernel (tcgen05.mma.cta_group::2) with automatic width; 6 = CTA-pair kernel with all rows of
  * x in swapped-operand units (any M: one pass over w per 512 rows of x, up to 512 accumulator columns per unit);
  * 512 + a multiple of 16 in [16, 256] = the pair kernel with that width; 7 = the block kernel with all but the last full
  * 256-row block of x in block units and the remaining 257..511 rows in two swapped-operand chunks that fit them exactly;
+ * 8 = the block kernel with full blocks, a swapped tail of at most 128 rows (a longer remainder is one more block) and automatic width;
  * 1024 = few-row kernel (M <= 128, K % 64 == 0, not SwiGLU; elsewhere as 0) with automatic w-tile width, 1024 + a multiple of 16
  * in [16, 128] = that kernel with this width (OJB_ERR_LIMIT where it does not serve).
  * ------------------------------------------------------------------------------------------------------------------ */
@@ -61,7 +63,7 @@ int ojb_gemm_bf16(const void* x, const void* w, void* out, int64_t M, int64_t N,
  * rows swapped (variant 6) it reads the layout above. */
 int ojb_gemm_bf16_swiglu(const void* x, const void* w_blk, void* out, int64_t M, int64_t N, int64_t K,
                          int32_t* status, ojb_stream_t stream);
-/* The same with the kernel variant forced (0, 1, 3, 4, 5, 6, 7 or 1024 as for ojb_gemm_bf16); for tuning. */
+/* The same with the kernel variant forced (0, 1, 3, 4, 5, 6, 7, 8 or 1024 as for ojb_gemm_bf16); for tuning. */
 int ojb_gemm_bf16_swiglu_v(const void* x, const void* w_blk, void* out, int64_t M, int64_t N, int64_t K, int variant,
                            int32_t* status, ojb_stream_t stream);
 

@@ -18,15 +18,16 @@ using namespace ojb;
 namespace {
 
 // variant: 0 = automatic; 1 = tile128 with 128x256 tiles; 2 = tile128 with 128x128 tiles; a multiple of 16 in [16, 256] =
-// block256 with that w-tile width; 3 = block256 with automatic width; 4 = block256 with every row of x in swapped-operand
-// units (M <= 2048).
+// block256 with that w-tile width; 3 = block256, width and form of the rows behind the full blocks by the model; 4 = block256 with every
+// row of x in swapped-operand units (M <= 2048).
 // 5 = pair256 (CTA pairs, cta_group::2) with automatic width; 6 = pair256 with every row of x in swapped-operand units
 // (any M); 512 + a multiple of 16 in [16, 256] = pair256 with that w-tile width; 7 = block256 with the last 257..511 rows of x in
-// two swapped-operand chunks and the rows before them in block units; 1024 = skinny (M <= 128, K % 64 == 0, not for SwiGLU; else as 0) with automatic
+// two swapped-operand chunks and the rows before them in block units; 8 = block256 with full blocks and a swapped tail of at most 128
+// rows, automatic width; 1024 = skinny (M <= 128, K % 64 == 0, not for SwiGLU; else as 0) with automatic
 // width;
 // 1024 + a multiple of 16 in [16, 128] = skinny with that w-tile width.
 bool variant_ok(int v) {
-  return (v >= 0 && v <= 7) || (v >= 16 && v <= 256 && v % 16 == 0) || (v >= 528 && v <= 768 && v % 16 == 0) ||
+  return (v >= 0 && v <= 8) || (v >= 16 && v <= 256 && v % 16 == 0) || (v >= 528 && v <= 768 && v % 16 == 0) ||
          (v >= 1024 && v <= 1152 && v % 16 == 0);
 }
 
@@ -76,19 +77,13 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
   };
   if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, f32));
   if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, f32));
-  {  // block256: full blocks + swapped tail
-    int n_xblk = static_cast<int>(M / 256), r = static_cast<int>(M % 256);
-    if (r > 128) { n_xblk += 1; r = 0; }
-    if (n_xblk > 0) {
-      const int tail_box = (r + 15) / 16 * 16;
-      const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, model_epi);
-      consider(3, block_kernel_clocks(N, bn, n_xblk, tail_box, 1, r > 0, splits, kb_total, sms, model_epi));
-    }
+  if (plain_form(M).n_xblk > 0) {      // block256
+    if (eight_bit) consider(3, form_clocks(plain_form(M), N, splits, kb_total, sms, model_epi));
+    else consider(3, choose_form(M, N, splits, kb_total, sms, model_epi).clocks);
   }
   if (M <= 2048) {  // block256 with every row in swapped-operand units
-    const int n_xchunk = static_cast<int>(ceil_div(M, 256));
-    const int tail_box = static_cast<int>(ceil_div(ceil_div(M, n_xchunk), 16) * 16);
-    consider(4, block_kernel_clocks(N, 256, 0, tail_box, n_xchunk, true, splits, kb_total, sms, model_epi));
+    const BlockForm f = chunked_form(M, 0);
+    consider(4, block_kernel_clocks(N, 256, 0, f.tail_box, f.n_xchunk, true, splits, kb_total, sms, model_epi));
   }
   if (epi != kEpiSwiglu && skinny_serves(M, K) && !eight_bit) consider(1024, skinny_clocks(M, N, kb_total, splits, sms));
   const double hbm = (static_cast<double>(N) * K * 2.0) / 3500.0 + 7000.0;     // bytes per clock at 6.3 TB/s and 1.8 GHz
@@ -111,7 +106,7 @@ int dispatch(int epi, int variant, const void* x, const void* w, void* out, int6
     return gemm_pair256_launch(epi, variant == 5 ? 0 : (variant == 6 ? -1 : variant - 512), x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 1 || variant == 2)
     return gemm_tile128_launch(epi, variant == 1 ? 256 : 128, x, w, out, M, N, K, splits, ldo, status, st);
-  return gemm_block256_launch(epi, variant == 3 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : variant)), x, w, out, M, N, K, splits, ldo, status, st);
+  return gemm_block256_launch(epi, variant == 3 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : (variant == 8 ? -3 : variant))), x, w, out, M, N, K, splits, ldo, status, st);
 }
 
 }  // namespace
@@ -126,7 +121,7 @@ extern "C" int ojb_gemm_bf16(const void* x, const void* w, void* out, int64_t M,
 extern "C" int ojb_gemm_bf16_swiglu_v(const void* x, const void* w_blk, void* out, int64_t M, int64_t N, int64_t K, int variant,
                                       int32_t* status, ojb_stream_t stream) {
   OJB_REQUIRE(x && w_blk && out && M > 0 && N > 0 && K > 0 && K % 8 == 0 && N % 256 == 0);
-  OJB_REQUIRE(aligned16(x) && aligned16(w_blk) && aligned16(out) && (variant == 0 || variant == 1 || variant == 3 || variant == 4 || variant == 5 || variant == 6 || variant == 7 || variant == 1024));
+  OJB_REQUIRE(aligned16(x) && aligned16(w_blk) && aligned16(out) && (variant == 0 || variant == 1 || variant == 3 || variant == 4 || variant == 5 || variant == 6 || variant == 7 || variant == 8 || variant == 1024));
   return dispatch(kEpiSwiglu, variant, x, w_blk, out, M, N, K, 1, N / 2, status, static_cast<cudaStream_t>(stream));
 }
 

@@ -620,37 +620,29 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   g.M = static_cast<int>(M);
   g.N = static_cast<int>(N);
   g.K = static_cast<int>(K);
-  // bn_req == -1: every row of x goes through swapped-operand units (M <= 2048: chunks of <= 256 rows); bn_req == -2: all
-  // but the last full 256-row block go through block units and the remaining 257..511 rows through two swapped-operand
-  // chunks that fit them exactly (544 rows = one block + 2 x 144: no MMA runs at the 64-clock floor of a short tail);
-  // otherwise full 256-row blocks plus a swapped tail of <= 128 rows (a longer remainder is cheaper as one more zero-padded
-  // block)
-  const bool hybrid = bn_req == -2 && M > kBlockM;
-  const bool all_swapped = (bn_req < 0 && !hybrid) || M <= kBM;
-  if (bn_req < 0) bn_req = 0;
-  if (all_swapped) {
-    if (M > 2048) return OJB_ERR_LIMIT;
-    g.n_xblk = 0;
-    g.tail_rows = static_cast<int>(M);
-    g.n_xchunk = static_cast<int>(ceil_div(M, 256));
-    g.tail_box = static_cast<int>(ceil_div(ceil_div(M, g.n_xchunk), 16) * 16);
-  } else if (hybrid) {
-    g.n_xblk = static_cast<int>(M / kBlockM) - 1;
-    g.tail_rows = static_cast<int>(M - static_cast<int64_t>(g.n_xblk) * kBlockM);      // 256 .. 511 rows
-    g.n_xchunk = static_cast<int>(ceil_div(g.tail_rows, 256));
-    g.tail_box = static_cast<int>(ceil_div(ceil_div(g.tail_rows, g.n_xchunk), 16) * 16);
-  } else {
-    g.n_xblk = static_cast<int>(M / kBlockM);
-    int r = static_cast<int>(M % kBlockM);
-    if (r > kBM) { g.n_xblk += 1; r = 0; }
-    g.tail_rows = r;
-    g.tail_box = (r + 15) / 16 * 16;
-    g.n_xchunk = 1;
-  }
   g.splits = splits;
   g.kb_total = static_cast<int>(ceil_div(K, FP8 ? 128 : kBK));
   g.kb_per_split = static_cast<int>(ceil_div(g.kb_total, splits));
   if (static_cast<int64_t>(splits - 1) * g.kb_per_split >= g.kb_total) return OJB_ERR_ARG;   // an empty split
+  // bn_req > 0: full blocks with w tiles of that width and a swapped tail; 0: blocks, the form of the rest and the width by the model;
+  // -1: every row of x in swapped-operand units (M <= 2048: chunks of <= 256 rows), as always up to 128 rows; -2: the last 257..511 rows
+  // in two swapped chunks; -3: full blocks and a swapped tail, the width by the model
+  BlockForm form;
+  if (bn_req == -1 || M <= kBM) {
+    if (M > 2048) return OJB_ERR_LIMIT;
+    form = chunked_form(M, 0);
+  } else if (bn_req == -2 && M > kBlockM) {
+    form = hybrid_form(M);
+  } else if (bn_req == 0 && !FP8) {
+    form = choose_form(M, N, splits, g.kb_total, sms, EPI).form;
+  } else {
+    form = plain_form(M);
+  }
+  if (bn_req < 0) bn_req = 0;
+  g.n_xblk = form.n_xblk;
+  g.tail_rows = form.tail_rows;
+  g.tail_box = form.tail_box;
+  g.n_xchunk = form.n_xchunk;
   g.BN = EPI == kEpiSwiglu ? 256 : (bn_req > 0 ? bn_req : choose_bn(N, g.n_xblk, g.tail_box, g.n_xchunk, g.tail_rows > 0, splits, g.kb_total, sms, EPI));
   if (FP8 && g.BN % 64 != 0) g.BN = (g.BN + 63) / 64 * 64;      // whole 128-byte store tiles (the scaled epilogue needs them)
   if (accum) g.BN = (g.BN + 31) / 32 * 32;                       // (a reduction leaves as whole tiles too)
@@ -704,7 +696,7 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   const int64_t units = static_cast<int64_t>(g.n_xblk) * g.n_wtile * splits +
                         (g.tail_rows > 0 ? static_cast<int64_t>(g.n_wtile256) * splits * g.n_xchunk : 0);
   int grid = static_cast<int>(units < sms ? units : sms);
-  if (units > grid && g.tail_rows > 0) {
+  if (units > grid && g.tail_rows > 0 && g.n_xblk > 0) {      // (swapped units alone are all alike: every SM takes part)
     const int group = (g.n_xblk + g.n_xchunk) * splits;   // units per w tile when BN = 256
     auto gcd = [](int a, int b) { while (b) { const int t = a % b; a = b; b = t; } return a; };
     while (grid > 1 && gcd(grid, group) != 1) --grid;

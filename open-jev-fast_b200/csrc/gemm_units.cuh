@@ -289,5 +289,56 @@ inline int choose_bn(int64_t N, int n_xblk, int tail_box, int n_xchunk, bool has
   });
 }
 
+// How the 256-row block kernel takes the rows behind its full blocks, for M > 128 rows.
+struct BlockForm {
+  int n_xblk;       // 256-row blocks of x in block units
+  int tail_rows;    // rows of x in swapped-operand units, in n_xchunk chunks of tail_box (a multiple of 16, at most 256)
+  int tail_box, n_xchunk;
+};
+// Full blocks and a swapped tail of at most 128 rows (a longer remainder as one more, zero-padded block).
+inline BlockForm plain_form(int64_t M) {
+  BlockForm f{static_cast<int>(M / kBlockM), static_cast<int>(M % kBlockM), 0, 1};
+  if (f.tail_rows > kBM) { f.n_xblk += 1; f.tail_rows = 0; }
+  f.tail_box = (f.tail_rows + 15) / 16 * 16;
+  return f;
+}
+// `blocks` full blocks and everything else in swapped chunks.
+inline BlockForm chunked_form(int64_t M, int64_t blocks) {
+  BlockForm f{static_cast<int>(blocks), static_cast<int>(M - blocks * kBlockM), 0, 0};
+  f.n_xchunk = static_cast<int>(ceil_div(f.tail_rows, 256));
+  f.tail_box = static_cast<int>(ceil_div(ceil_div(f.tail_rows, f.n_xchunk), 16) * 16);
+  return f;
+}
+// All but the last full block in block units, the remaining 257 .. 511 rows in two swapped chunks that fit them (M > 256): no MMA
+// runs at the 64-clock floor of a short tail, and none on the zero rows of a padded block.
+inline BlockForm hybrid_form(int64_t M) { return chunked_form(M, M / kBlockM - 1); }
+
+inline double form_clocks(const BlockForm& f, int64_t N, int splits, int kb_total, int sms, int epi) {
+  const bool tail = f.tail_rows > 0;
+  const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, f.n_xblk, f.tail_box, f.n_xchunk, tail, splits, kb_total, sms, epi);
+  return block_kernel_clocks(N, bn, f.n_xblk, f.tail_box, f.n_xchunk, tail, splits, kb_total, sms, epi);
+}
+// The cheaper of the two by the model, and its clocks. (Not for e4m3 operands: a block and a swapped unit round SiLU differently, and
+// that path keeps its bits.) Measured under the power cap, without / with the choice: [12352, 5120] at 1066 / 1184 rows 126 / 140 us
+// and 109 / 122, gate/up at 1984 rows 561 and 532, [5120, 17408] in one K range at 1312 rows 210 and 193.
+struct FormChoice {
+  BlockForm form;
+  double clocks;
+};
+inline FormChoice choose_form(int64_t M, int64_t N, int splits, int kb_total, int sms, int epi) {
+  static ModelCache<6, FormChoice> cache;
+  const int64_t key[6] = {M, N, splits, kb_total, sms, epi};
+  return cache.get(key, [&] {
+    const BlockForm plain = plain_form(M);
+    FormChoice best{plain, form_clocks(plain, N, splits, kb_total, sms, epi)};
+    if (M > kBlockM && M % kBlockM != 0) {
+      const BlockForm hybrid = hybrid_form(M);
+      const double clocks = form_clocks(hybrid, N, splits, kb_total, sms, epi);
+      if (clocks < best.clocks) best = FormChoice{hybrid, clocks};
+    }
+    return best;
+  });
+}
+
 }  // namespace
 }  // namespace ojb

@@ -166,7 +166,7 @@ class FastQwen35(torch.nn.Module):
         if q8 is not None:
             yq, sy = LT.quantize_rows_e4m3(y)
             S8 = S if S > 0 else LT.plan_splitk(M, w.shape[0], Kd // 2, eight_bit=True)      # a 128-byte k-block holds twice the elements
-            if S8 == 1 and self._adds(M, w.shape[0]):
+            if S8 == 1 and self._adds(M, w.shape[0], w.shape[1]):
                 LT.gemm_e4m3(yq, sy, q8[0], q8[1], 3, h=h)
                 return [h, self._norm(h, None, None, w1, mask, last)]
             return [h, self._norm(h, None, LT.gemm_e4m3(yq, sy, q8[0], q8[1], 2, S8), w1, mask, last)]
@@ -174,21 +174,21 @@ class FastQwen35(torch.nn.Module):
             idx, S = self._force.get("res", self._plan.get(("res", M, w.shape[0], Kd), (0, 0)))
             if S == 0:
                 S = LT.plan_splitk(M, w.shape[0], Kd)
-        if S == 1 and idx in self.ADD_KERNELS and self._adds(M, w.shape[0]):
+        if S == 1 and idx in self.ADD_KERNELS and self._adds(M, *w.shape):
             LT.gemm_add(y, w, h, idx)
             return [h, self._norm(h, None, None, w1, mask, last)]
         return [h, self._norm(h, None, LT.gemm_splitk(y, w, S, idx), w1, mask, last)]
 
     # One K range of many rows: the product goes straight to the residual stream instead of a plane that the norm kernel adds (the same
     # sum). The norm is then bound by half the bytes (30 -> 18 us at 2560 rows, 56 -> 36 at 4192, 193 -> 115 at 16 672); the product
-    # itself pays where its epilogues run under no other unit, because the stream comes from HBM for the addition: 117 -> 122 us on average at
-    # 1560 rows, more than the norm saves; from nine blocks of rows on (180 units and more for 148 SMs) a few us of 200.
-    ADD_MIN_ROWS = 2304
-    ADD_KERNELS = (0, 3)
+    # itself pays where the stream has left the L2 and its epilogues run under no other unit, because the addition then waits for HBM. That
+    # is the down projection (K = 17 408) below about nine blocks of rows: both projections together 117 -> 122 us on average at 1560 rows. A short
+    # K moves little through the L2: from 1024 rows on it gains (K = 4096 at 1066 / 1568 rows, with the norm: 60 / 79 us -> 54 / 71).
+    @staticmethod
+    def _adds(M, N, K):
+        return M >= (1024 if K <= 8192 else 2304) and N % 64 == 0
 
-    @classmethod
-    def _adds(cls, M, N):
-        return M >= cls.ADD_MIN_ROWS and N % 64 == 0
+    ADD_KERNELS = (0, 3)
 
     def _mlp_in(self, hn, d):
         if d.fused_mlp and self.fp8:
@@ -252,7 +252,7 @@ class FastQwen35(torch.nn.Module):
                     out.setdefault(tuple(w.shape), []).append(d)
             return out
 
-        kernels = [1, 3] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
+        kernels = [1, 12] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
         few = [11] if M <= 128 else []
         for (N, Kd), layers in groups("w_in").items():
             x = rnd(M, Kd)

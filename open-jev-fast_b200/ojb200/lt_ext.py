@@ -2,11 +2,12 @@
 
 The reference enumerates cuBLASLt algorithms per shape (lt_setup) and runs one by index (lt_matmul); split-K plans go
 through lt2_*. Here an "algorithm" is one of the library's GEMM variants: index 0 lets the library choose, 1 / 2 force the
-128-row tile kernel with 256 / 128-wide tiles, 3 the 256-row block kernel with automatic w-tile width, 4..6 that kernel
+128-row tile kernel with 256 / 128-wide tiles, 3 the 256-row block kernel with w-tile width and the form of the remaining rows by the cost model, 4..6 that kernel
 with w-tile width 256, 192, 128, 7 that kernel with all of x in swapped-operand units (M <= 2048), 8 / 9 the CTA-pair
 kernel (tcgen05.mma.cta_group::2) with automatic width / all of x in swapped-operand units, 10 the block kernel with
 block units for all but the last full block of x and two swapped-operand chunks for the remaining 257..511 rows, 11 the
-few-row kernel (at most 128 rows, K a multiple of 64, not SwiGLU; as 0 elsewhere).
+few-row kernel (at most 128 rows, K a multiple of 64, not SwiGLU; as 0 elsewhere), 12 the block kernel with full blocks and a swapped tail
+of at most 128 rows.
 Two entry points have no counterpart in the reference: gemm_swiglu (SwiGLU fused into the epilogue) and gemm_splitk
 (fp32 partial sums from the un-split [N, K] weight).
 """
@@ -19,7 +20,7 @@ from . import _lib
 from ._lib import call, i32, i64, ptr, stream_ptr
 
 bf16 = torch.bfloat16
-VARIANT_BN = [0, 1, 2, 3, 256, 192, 128, 4, 5, 6, 7, 1024]
+VARIANT_BN = [0, 1, 2, 3, 256, 192, 128, 4, 5, 6, 7, 1024, 8]
 N_VARIANTS = len(VARIANT_BN)
 SM_COUNT = 148
 _plans = []          # lt2 plans: dicts

@@ -378,3 +378,25 @@ def test_product_added_to_the_stream_refuses_what_it_does_not_take():
     for h in (torch.zeros(64, 64, device="cuda", dtype=torch.bfloat16), torch.zeros(63, 64, device="cuda"), torch.zeros(64, 128, device="cuda")[:, ::2]):
         with pytest.raises(RuntimeError):
             LT.gemm_add(x, w, h)
+
+
+# rows where the forms part: a remainder of 1, 128, 129 and 255 rows behind one and behind several blocks; swapped units alone with more units than
+# SMs (2 and 6 chunks of 38 w tiles)
+@pytest.mark.parametrize("M,N", [(257, 320), (384, 320), (385, 320), (511, 320), (513, 4160), (640, 4160), (1153, 4160), (1407, 4160),
+                                 (500, 9728), (1500, 9728)])
+@pytest.mark.parametrize("idx", [0, 3, 7, 10, 12])
+def test_forms_of_the_block_kernel(M, N, idx):
+    """Every form takes every row once: bf16 and fp32 results against fp64, sums of K products within K * 2^-24 of sum |x w| (the bf16
+    result half an ulp, 2^-8, beside it)."""
+    from ojb200 import _lib, lt_ext as LT
+    K = 192
+    x, w = _mk(M, N, K, M + N)
+    ref = x.double() @ w.double().t()
+    bound = (x.double().abs() @ w.double().abs().t()) * K * 2.0 ** -24
+    out = LT.lt_matmul(x, w, idx)
+    assert bool(((out.double() - ref).abs() <= bound + ref.abs() * 2.0 ** -8).all())
+    for S in (1, 3):
+        parts = LT.gemm_splitk(x, w, S, idx)
+        assert bool(((parts.double().sum(0) - ref).abs() <= bound).all())
+    torch.cuda.synchronize()
+    _lib.check_status()
