@@ -9,10 +9,17 @@
 // MMAs and commit (0.2 us) sets the pace, 21 us for K = 5120 whatever the weight's size, against 12.9 us with four.
 //
 // One CTA per (w tile, K range), 192 threads: warp 0 asks for the tiles (plain cp.async.bulk.tensor, 128-byte swizzle, mbarrier), one
-// lane of warp 1 issues tcgen05.mma, warps 2-5 read the accumulator back and store. The MMA has M = 128 whatever the number of
-// rows: its A operand starts at the stage's x rows and runs on into whatever shared memory follows them (the w tile, the next
-// stage); a row of the product depends on its own row of A alone, and the rows past M are never read back.
+// lane of warp 1 issues tcgen05.mma, warps 2-5 read the accumulator back and store. The MMA has M = 128 whatever its A operand: that runs on
+// behind its own rows into whatever shared memory follows (the other operand, the next k-block, the next stage); a row of the product
+// depends on its own row of A alone, and the rows past the operand are never read back. So a k-step costs 128 products for every row
+// of the N side, and the narrower of the two operands is the N side: the rows of x (rounded up to 16) under most tiles, the w tile where
+// that has fewer rows (2048 outputs: 16). With x always the M side a weight cost 128 products, most of them of other weights taken for
+// rows of x, and the products of random operands are what the board's power goes to. 28 rows, in runs at the 1 kW cap, x as the
+// M side / as the N side: [12352, 5120] 26.7 / 25.0 us, [5120, 17408] in six K ranges 41.6 / 39.1, in e4m3 17.4 / 15.4 and 28.9 / 24.7; [2048,
+// 5120] 15.3 / 16.3. Same bits.
 #include "gemm_units.cuh"
+
+#include <type_traits>
 
 namespace ojb {
 namespace {
@@ -23,7 +30,7 @@ constexpr size_t kSkinnySmem = 227 * 1024;
 
 struct SkinnyArgs {
   int M, N;
-  int BN, x_rows;                  // rows of w and of x in a stage
+  int BN, x_rows;                  // rows of w and of x (a multiple of 16 as the N side, else of 8) in a stage
   int splits, kb_per_split, kb_total;
   int nk;                          // k-blocks per stage
   int stages;
@@ -36,7 +43,8 @@ struct SkinnyArgs {
   const float* sw;
 };
 
-template <int EPI, bool FP8>
+// WSIDE: w is the M side, the rows of x the N side.
+template <int EPI, bool FP8, bool WSIDE>
 __global__ void __launch_bounds__(kSkinnyThreads, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, SkinnyArgs g) {
   pdl_launch_dependents();
@@ -97,14 +105,16 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       const bool one = elect_one();
       int stage = 0;
       uint32_t phase = 0;
-      const uint32_t idesc = FP8 ? umma_idesc_e4m3(g.BN) : umma_idesc(g.BN);
+      const int n_side = WSIDE ? g.x_rows : g.BN;
+      const uint32_t idesc = FP8 ? umma_idesc_e4m3(n_side) : umma_idesc(n_side);
       bool ok = true;
       for (int kb = 0; kb < nkb; kb += g.nk) {
         if (!mbar_wait_warp(full0 + 8 * stage, phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t src = tiles0 + stage * g.stage_bytes;
         for (int j = 0; j < g.nk && kb + j < nkb; ++j) {
-          const uint64_t adesc = smem_desc_sw128(src + j * x_bytes), bdesc = smem_desc_sw128(src + g.nk * x_bytes + j * w_bytes);
+          const uint64_t xdesc = smem_desc_sw128(src + j * x_bytes), wdesc = smem_desc_sw128(src + g.nk * x_bytes + j * w_bytes);
+          const uint64_t adesc = WSIDE ? wdesc : xdesc, bdesc = WSIDE ? xdesc : wdesc;
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             const uint32_t accum = (kb + j > 0 || k > 0) ? 1u : 0u;
@@ -120,53 +130,80 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       if (ok && one) umma_commit(accfull);
     }
   } else {
-    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const int quarter = warp & 3, row = quarter * 32 + lane;      // this thread's row of the M side
     if (mbar_wait_warp(accfull, 0, abort_flag)) {
       tc_fence_after();
-      if (quarter * 32 < g.M) {
-        const bool row_ok = row < g.M;
-        const int ncols = min(g.N - n0, g.BN);
-        float rs = 1.f;
-        if constexpr (FP8) rs = row_ok ? __ldg(g.sx + row) : 1.f;
-        const int64_t off = static_cast<int64_t>(split) * g.split_stride + static_cast<int64_t>(row) * g.ldo + n0;
-        const bool vec_ok = (g.ldo & 7) == 0 && (g.split_stride & 3) == 0;      // n0 and the 16-column steps keep the alignment
+      const int ncols = min(g.N - n0, g.BN);
+      if constexpr (WSIDE) {
+        if (quarter * 32 < ncols) {
+          const bool col_ok = row < ncols;
+          float ws = 1.f;
+          if constexpr (FP8) ws = __ldg(g.sw + min(n0 + row, g.N - 1));
+          const int64_t off = static_cast<int64_t>(split) * g.split_stride + n0 + row;
 #pragma unroll 1
-        for (int c = 0; c < ncols; c += 16) {
-          uint32_t r[16];
-          tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
-          tmem_ld_wait();
-          if (row_ok) {
-            float v[16];
+          for (int m0 = 0; m0 < g.M; m0 += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + m0, r);
+            tmem_ld_wait();
+            const int left = g.M - m0;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              v[e] = __uint_as_float(r[e]);
-              if constexpr (FP8) v[e] *= rs * __ldg(g.sw + min(n0 + c + e, g.N - 1));
-            }
-            if constexpr (EPI == kEpiPartialF32) {
-              float* o = reinterpret_cast<float*>(g.out) + off + c;
-              if (vec_ok && c + 16 <= ncols) {
-#pragma unroll
-                for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(o + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-              } else {
-#pragma unroll
-                for (int e = 0; e < 16; ++e)
-                  if (c + e < ncols) o[e] = v[e];
-              }
-            } else {
-              bf16_t* o = reinterpret_cast<bf16_t*>(g.out) + off + c;
-              if (vec_ok && c + 16 <= ncols) {
-#pragma unroll
-                for (int e = 0; e < 16; e += 8)
-                  *reinterpret_cast<uint4*>(o + e) = make_uint4(pack2(v[e], v[e + 1]), pack2(v[e + 2], v[e + 3]), pack2(v[e + 4], v[e + 5]),
-                                                                pack2(v[e + 6], v[e + 7]));
-              } else {
-#pragma unroll
-                for (int e = 0; e < 16; ++e)
-                  if (c + e < ncols) o[e] = f2bf(v[e]);
+            for (int e = 0; e < 16; ++e) {      // neighbouring lanes hold neighbouring columns: whole 128- or 64-byte pieces of a row
+              if (col_ok && e < left) {
+                float v = __uint_as_float(r[e]);
+                if constexpr (FP8) v *= __ldg(g.sx + m0 + e) * ws;
+                const int64_t at = off + static_cast<int64_t>(m0 + e) * g.ldo;
+                if constexpr (EPI == kEpiPartialF32) reinterpret_cast<float*>(g.out)[at] = v;
+                else reinterpret_cast<bf16_t*>(g.out)[at] = f2bf(v);
               }
             }
+            __syncwarp();
           }
-          __syncwarp();
+        }
+      } else {
+        if (quarter * 32 < g.M) {
+          const bool row_ok = row < g.M;
+          float rs = 1.f;
+          if constexpr (FP8) rs = row_ok ? __ldg(g.sx + row) : 1.f;
+          const int64_t off = static_cast<int64_t>(split) * g.split_stride + static_cast<int64_t>(row) * g.ldo + n0;
+          const bool vec_ok = (g.ldo & 7) == 0 && (g.split_stride & 3) == 0;      // n0 and the 16-column steps keep the alignment
+#pragma unroll 1
+          for (int c = 0; c < ncols; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + c, r);
+            tmem_ld_wait();
+            if (row_ok) {
+              float v[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) {
+                v[e] = __uint_as_float(r[e]);
+                if constexpr (FP8) v[e] *= rs * __ldg(g.sw + min(n0 + c + e, g.N - 1));
+              }
+              if constexpr (EPI == kEpiPartialF32) {
+                float* o = reinterpret_cast<float*>(g.out) + off + c;
+                if (vec_ok && c + 16 <= ncols) {
+#pragma unroll
+                  for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4*>(o + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 16; ++e)
+                    if (c + e < ncols) o[e] = v[e];
+                }
+              } else {
+                bf16_t* o = reinterpret_cast<bf16_t*>(g.out) + off + c;
+                if (vec_ok && c + 16 <= ncols) {
+#pragma unroll
+                  for (int e = 0; e < 16; e += 8)
+                    *reinterpret_cast<uint4*>(o + e) = make_uint4(pack2(v[e], v[e + 1]), pack2(v[e + 2], v[e + 3]), pack2(v[e + 4], v[e + 5]),
+                                                                  pack2(v[e + 6], v[e + 7]));
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 16; ++e)
+                    if (c + e < ncols) o[e] = f2bf(v[e]);
+                }
+              }
+            }
+            __syncwarp();
+          }
         }
       }
       tc_fence_before();
@@ -185,17 +222,17 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
-template <int EPI, bool FP8>
+template <int EPI, bool FP8, bool WSIDE>
 int launch_skinny(int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits, int64_t ldo,
                   int32_t* status, cudaStream_t stream, const float* sx, const float* sw) {
   static int smem_set[kMaxDevices] = {};
-  auto kern = gemm_skinny_kernel<EPI, FP8>;
+  auto kern = gemm_skinny_kernel<EPI, FP8, WSIDE>;
   if (!raise_smem_limit(kern, static_cast<int>(kSkinnySmem - 2048), smem_set)) return OJB_ERR_LAUNCH;      // 2 KB: the static part
   SkinnyArgs g{};
   g.M = static_cast<int>(M);
   g.N = static_cast<int>(N);
   g.BN = bn;
-  g.x_rows = static_cast<int>(ceil_div(M, 8) * 8);
+  g.x_rows = static_cast<int>(WSIDE ? ceil_div(M, 16) * 16 : ceil_div(M, 8) * 8);
   g.splits = splits;
   g.kb_total = static_cast<int>(ceil_div(K, FP8 ? 128 : kBK));
   g.kb_per_split = static_cast<int>(ceil_div(g.kb_total, splits));
@@ -207,12 +244,12 @@ int launch_skinny(int bn, const void* x, const void* w, void* out, int64_t M, in
   while (g.nk > 1 && (g.nk * kb_bytes * 6 > budget || g.nk > g.kb_per_split)) --g.nk;
   g.stage_bytes = g.nk * kb_bytes;
   // the A operand of the last k-block may run on behind the last stage
-  const uint32_t reach = (g.nk - 1) * static_cast<uint32_t>(g.x_rows) * 128 + kBM * 128u;
+  const uint32_t reach = WSIDE ? g.stage_bytes + (kBM - bn) * 128u : (g.nk - 1) * static_cast<uint32_t>(g.x_rows) * 128 + kBM * 128u;
   const uint32_t over = reach > g.stage_bytes ? reach - g.stage_bytes : 0u;
   g.stages = static_cast<int>((budget - over) / g.stage_bytes);
   if (g.stages > kSkinnyMaxStages) g.stages = kSkinnyMaxStages;
   g.tmem_cols = 32;
-  while (static_cast<int>(g.tmem_cols) < bn) g.tmem_cols *= 2;
+  while (static_cast<int>(g.tmem_cols) < (WSIDE ? g.x_rows : bn)) g.tmem_cols *= 2;
   g.out = out;
   g.ldo = ldo;
   g.split_stride = EPI == kEpiPartialF32 ? M * N : 0;
@@ -238,11 +275,16 @@ int gemm_skinny_launch(int epi, int bn, const void* x, const void* w, void* out,
   if (M > kSkinnyRows || K % (sx != nullptr ? 128 : kBK) != 0 || (epi != kEpiBf16 && epi != kEpiPartialF32)) return OJB_ERR_LIMIT;
   if (bn == 0) bn = skinny_bn(N, splits);
   if (bn < 16 || bn > 128 || bn % 16) return OJB_ERR_ARG;
-  if (sx != nullptr)
-    return epi == kEpiBf16 ? launch_skinny<kEpiBf16, true>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw)
-                           : launch_skinny<kEpiPartialF32, true>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw);
-  return epi == kEpiBf16 ? launch_skinny<kEpiBf16, false>(bn, x, w, out, M, N, K, splits, ldo, status, stream, nullptr, nullptr)
-                         : launch_skinny<kEpiPartialF32, false>(bn, x, w, out, M, N, K, splits, ldo, status, stream, nullptr, nullptr);
+  const bool wside = ceil_div(M, 16) * 16 < bn;
+  auto pick = [&](auto fp8, auto side) {
+    constexpr bool kFp8 = decltype(fp8)::value, kSide = decltype(side)::value;
+    return epi == kEpiBf16 ? launch_skinny<kEpiBf16, kFp8, kSide>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw)
+                           : launch_skinny<kEpiPartialF32, kFp8, kSide>(bn, x, w, out, M, N, K, splits, ldo, status, stream, sx, sw);
+  };
+  using std::false_type;
+  using std::true_type;
+  if (sx != nullptr) return wside ? pick(true_type{}, true_type{}) : pick(true_type{}, false_type{});
+  return wside ? pick(false_type{}, true_type{}) : pick(false_type{}, false_type{});
 }
 
 }  // namespace ojb

@@ -400,3 +400,20 @@ def test_forms_of_the_block_kernel(M, N, idx):
         assert bool(((parts.double().sum(0) - ref).abs() <= bound).all())
     torch.cuda.synchronize()
     _lib.check_status()
+
+
+# x as the N side (w tile wider than the rows) and as the M side (2048 outputs: tiles of 16), edges of 16 rows and of the last w tile
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 100, 128])
+@pytest.mark.parametrize("N", [2048, 2056, 12352])
+def test_few_row_kernel_e4m3_has_the_bits_of_the_block_kernel(M, N):
+    """The same rows among 256, which the 256-row block kernel takes, give the same bits: sums run over K in the same order."""
+    from ojb200 import lt_ext as LT, _lib
+    K = 640
+    x, w = _mk(256, N, K, M)
+    (xq, sx), (wq, sw) = LT.quantize_rows_e4m3(x), LT.quantize_weight_e4m3(w)
+    few = LT.gemm_e4m3(xq[:M].contiguous(), sx[:M].contiguous(), wq, sw, 0)
+    assert torch.equal(few, LT.gemm_e4m3(xq, sx, wq, sw, 0)[:M])
+    few = LT.gemm_e4m3(xq[:M].contiguous(), sx[:M].contiguous(), wq, sw, 2, 2)
+    assert torch.equal(few, LT.gemm_e4m3(xq, sx, wq, sw, 2, 2)[:, :M])
+    torch.cuda.synchronize()
+    _lib.check_status()
