@@ -320,9 +320,10 @@ int ojb_gdn_chunked_static(const void* q, const void* k, const void* v, const fl
 
 /* Measurement hook of the state pass (no counterpart in the reference): `records` = null switches it off; otherwise a device
  * buffer of 4 + 12 uint64 words per walk step. The CTA of head 0 / column slice 0 / walk 0 stores %globaltimer at kernel entry,
- * when its tables are staged and its first operands requested, and at its exit (words 0-2), then at six points of every step
- * (step begin, operands ready, phase 1 done, v' visible, phase 2 done, step end), words 0-5 of the step's record from its
- * state-chain warp and 6-11 from its output warp. Synchronises the device (it writes a device variable). */
+ * when its barriers are set up, and at its exit (words 0-2), then six stamps of every step: words 0-5 of the step's record from a warp that
+ * carries the state (step begin, operands there, first product and v' done, fragments handed on, state update done, step end), words 6-11
+ * from a warp that forms the outputs (step begin, fragments taken over, operands there, and three times around the end of its products
+ * and stores). Synchronises the device (it writes a device variable). */
 int ojb_gdn_set_trace(uint64_t* records);
 
 /* src/kernels.cu:1333-1374 gated_rmsnorm_inv2 (inv != null) and :143 gated_rmsnorm (inv == null).

@@ -336,7 +336,7 @@ extern "C" int ojb_gtree_fill(const int64_t* tokens, const int64_t* seq_off, con
 extern "C" int ojb_seq_tables(const int64_t* lens, int64_t S, int64_t Lp, int64_t pad, int64_t T, int32_t own_walks, int64_t cap, int64_t* pos,
                               int64_t* lastidx, int32_t* rowmask, int32_t* hist, int32_t* krange, int32_t* chunks, int32_t* steps,
                               int32_t* walk_ptr) {
-  if (!lens || !pos || !lastidx || !rowmask || !hist || !krange || !chunks || !steps || !walk_ptr) return OJB_ERR_ARG;
+  if (!hist || !chunks || !steps || !walk_ptr || (S > 0 && (!lens || !lastidx))) return OJB_ERR_ARG;
   if (S < 0 || Lp < 0 || T < 0 || pad < 0 || pad > Lp || cap < 1 || (own_walks && Lp != 0)) return OJB_ERR_ARG;
   int64_t need = (Lp - pad + 63) / 64;
   for (int64_t s = 0; s < S; ++s) {
@@ -346,6 +346,7 @@ extern "C" int ojb_seq_tables(const int64_t* lens, int64_t S, int64_t Lp, int64_
   if (need > cap) return OJB_ERR_LIMIT;
   const int64_t N = Lp + S * T, N32 = (N + 31) / 32 * 32;
   if (N32 > INT32_MAX / 8) return OJB_ERR_LIMIT;
+  if (N32 > 0 && (!pos || !rowmask || !krange)) return OJB_ERR_ARG;      // (tables of no rows have no address)
   auto alone = [&](int64_t n) {                    // padding: a row that sees itself and belongs to no path
     rowmask[n] = 0;
     for (int i = 0; i < 4; ++i) hist[n * 4 + i] = -1;

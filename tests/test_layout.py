@@ -190,7 +190,7 @@ def test_packed_requests_tables():
         base += n
 
 
-@pytest.mark.parametrize("Lp,pad,lens,T", [(0, 0, [5, 0, 64, 65], 70), (0, 0, [1], 1), (0, 0, [0, 0], 3), (7, 0, [3, 1], 4), (64, 61, [2, 6], 6),
+@pytest.mark.parametrize("Lp,pad,lens,T", [(0, 0, [], 5), (0, 0, [0, 0], 0), (0, 0, [5, 0, 64, 65], 70), (0, 0, [1], 1), (0, 0, [0, 0], 3), (7, 0, [3, 1], 4), (64, 61, [2, 6], 6),
                                            (130, 2, [0, 65, 1], 65), (33, 33, [4, 2], 4), (3, 1, [1, 2, 3, 4], 4)])
 @pytest.mark.parametrize("own_walks", [True, False])
 def test_sequence_tables(Lp, pad, lens, T, own_walks):
