@@ -125,6 +125,26 @@ def test_quantize_rows_e4m3(M, K):
     assert (_deq(q, s) - x.float()).abs().max().item() <= amax.max().item() * 2 ** -4 + 1e-6
 
 
+@pytest.mark.parametrize("K", [8, 1032, 4096, 4104, 6144, 6152, 17408, 18432, 18440])
+def test_quantize_rows_e4m3_forms(K):
+    """Every form of the row quantisation at both ends of its row lengths: the bits of fp32 arithmetic (no tolerance: a maximum, one
+    product, one division, and one product and rounding per value)."""
+    from ojb200 import lt_ext
+    x = (torch.randn(9, K, generator=torch.Generator().manual_seed(K)) * 3).to(bf16)
+    x[1] = 0
+    x[2, :-1] = 0
+    x[3, -1], x[4, 0], x[5, -1], x[6, 0] = 3e38, 2.0 ** -130, float("nan"), -float("inf")
+    x[7] = 2.0 ** -133
+    q, s = (t.cpu() for t in lt_ext.quantize_rows_e4m3(x.cuda()))
+    amax = torch.where(x.isnan(), 0.0, x.float().abs()).amax(dim=1)
+    sc = torch.where(amax > 0, amax * torch.tensor(1.0 / 448.0), torch.ones(9))
+    assert torch.equal(s, sc)
+    v = x.float() * (1.0 / sc)[:, None]
+    want = v.clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+    odd = v.isnan()
+    assert torch.equal(q[~odd], want[~odd]) and bool(((q[odd] & 0x7f) == 0x7f).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 512, 256), (256, 256, 128), (544, 1024, 640), (539, 12352, 5120), (288, 1280, 5120), (300, 520, 1008)])
 def test_gemm_e4m3_plain(M, N, K):
     """8-bit GEMM against fp32 matmul of the same dequantised operands: only the accumulation order differs."""
