@@ -66,7 +66,8 @@ struct Plan {
 // time HBM needs for the weight.
 // eight_bit: the ranges of K of an 8-bit product. They regroup its sums, and on e4m3 operands a regrouped sum moves the result of
 // a deep model by percents, so that choice stays on the model it was first made with.
-Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eight_bit = false) {
+// plain_forms: as if the block kernel had its plain form alone, for choices that a result depends on.
+Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool plain_forms, bool eight_bit = false) {
   const int sms = 148;
   const int kb_total = static_cast<int>(ceil_div(K, 64));
   Plan best{3, 1e30};
@@ -78,7 +79,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
   if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, f32));
   if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, f32));
   if (plain_form(M).n_xblk > 0) {      // block256
-    if (eight_bit) consider(3, form_clocks(plain_form(M), N, splits, kb_total, sms, model_epi));
+    if (plain_forms) consider(3, form_clocks(plain_form(M), N, splits, kb_total, sms, model_epi));
     else consider(3, choose_form(M, N, splits, kb_total, sms, model_epi).clocks);
   }
   if (M <= 2048) {  // block256 with every row in swapped-operand units
@@ -94,7 +95,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool eig
 Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   static ModelCache<5, Plan> cache;
   const int64_t key[5] = {epi, M, N, K, splits};
-  return cache.get(key, [&] { return model_kernel(epi, M, N, K, splits); });
+  return cache.get(key, [&] { return model_kernel(epi, M, N, K, splits, false); });
 }
 
 int dispatch(int epi, int variant, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
@@ -199,10 +200,15 @@ extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int3
     for (int s = 1; s <= (parts ? max_splits : 1); ++s) {
       const int per = static_cast<int>(ceil_div(kb_total, s));
       if (static_cast<int64_t>(s - 1) * per >= kb_total) continue;
-      Plan p = model_kernel(eight_bit ? kEpiPartialF32 : kind, M, N, K, s, eight_bit);
+      // (K ranges regroup the sums, so they are chosen over the plain forms: another form of the block kernel changes no result)
+      Plan p = model_kernel(eight_bit ? kEpiPartialF32 : kind, M, N, K, s, parts, eight_bit);
       // the kernel that sums the partial planes reads S * M * N floats (mostly from L2)
       if (parts) p.clocks += (s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
       if (p.clocks < best.clocks * 0.97) { best = p; best_s = s; }
+    }
+    if (kind == 2) {
+      best = model_kernel(kind, M, N, K, best_s, false);
+      best.clocks += (best_s - 1) * static_cast<double>(M) * N * 4.0 / 5000.0;
     }
     return Ranges{best, best_s};
   });

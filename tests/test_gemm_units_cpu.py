@@ -101,6 +101,16 @@ def test_plan_is_the_same_from_every_thread():
         assert all(pool.map(ask, range(8)))
 
 
+# K ranges by the plain form of the block kernel, at row counts where ranges chosen over all its forms would differ
+@pytest.mark.parametrize("M,K,want", [(1824, 4096, 2), (1888, 4096, 2), (2720, 4096, 2), (928, 6144, 1), (1824, 6144, 2), (1216, 17408, 1),
+                                      (1248, 17408, 1)])
+def test_k_ranges_do_not_move_with_the_forms(M, K, want):
+    """Ranges of K regroup the sums of a product; the form of the block kernel does not. So what the model knows of the forms must not
+    move the ranges, and with them the results."""
+    from ojb200 import lt_ext
+    assert lt_ext.plan_splitk(M, 5120, K) == want
+
+
 @pytest.mark.parametrize("env,want", [
     ({}, [13, 13, 0, 0]),                                               # five bands of 16 blocks at most
     ({"OJB_GEMM_BAND_MB": "40"}, [13, 4, 0, 0]),                        # 16 blocks of 2.5 MB, or 4 of 8.5 MB
