@@ -60,6 +60,7 @@ double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
 struct Plan {
   int variant;
   double clocks;
+  int pair_rows = -1;      // see gemm_block256_launch
 };
 
 // Cheapest kernel for this shape and number of K ranges according to the cost models (gemm_units.cuh), never below the
@@ -74,7 +75,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool pla
   const bool f32 = epi == kEpiPartialF32 && !eight_bit;
   const int model_epi = eight_bit ? kEpi8BitRanges : epi;
   auto consider = [&](int variant, double clocks) {
-    if (clocks < best.clocks) best = Plan{variant, clocks};
+    if (clocks < best.clocks) best = Plan{variant, clocks, -1};
   };
   if (epi != kEpiSwiglu || M > 64) consider(1, tile128_clocks(M, N, kb_total, splits, 256, sms, f32));
   if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, f32));
@@ -95,19 +96,30 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool pla
 Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   static ModelCache<5, Plan> cache;
   const int64_t key[5] = {epi, M, N, K, splits};
-  return cache.get(key, [&] { return model_kernel(epi, M, N, K, splits, false); });
+  return cache.get(key, [&] {
+    Plan p = model_kernel(epi, M, N, K, splits, false);
+    // SwiGLU: which rows take their SiLU in pairs follows from the kernel that the plain forms would get
+    if (epi == kEpiSwiglu && p.variant == 3 && model_kernel(epi, M, N, K, splits, true).variant != 3) p.pair_rows = 0;
+    return p;
+  });
 }
 
 int dispatch(int epi, int variant, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
              int64_t ldo, int32_t* status, cudaStream_t st) {
   if (variant == 1024 && (epi == kEpiSwiglu || !skinny_serves(M, K))) variant = 0;
-  if (variant == 0) variant = plan_kernel(epi, M, N, K, splits).variant;
+  int pair_rows = -1;
+  if (variant == 0) {
+    const Plan p = plan_kernel(epi, M, N, K, splits);
+    variant = p.variant;
+    pair_rows = p.pair_rows;
+  }
   if (variant >= 1024) return gemm_skinny_launch(epi, variant - 1024, x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 5 || variant == 6 || variant >= 512)
     return gemm_pair256_launch(epi, variant == 5 ? 0 : (variant == 6 ? -1 : variant - 512), x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 1 || variant == 2)
     return gemm_tile128_launch(epi, variant == 1 ? 256 : 128, x, w, out, M, N, K, splits, ldo, status, st);
-  return gemm_block256_launch(epi, variant == 3 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : (variant == 8 ? -3 : variant))), x, w, out, M, N, K, splits, ldo, status, st);
+  return gemm_block256_launch(epi, variant == 3 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : (variant == 8 ? -3 : variant))), x, w, out, M, N, K, splits, ldo, status, st,
+                              pair_rows);
 }
 
 }  // namespace

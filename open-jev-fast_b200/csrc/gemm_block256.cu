@@ -25,6 +25,8 @@
 // OJB_DEV_WAIT_TIMEOUT in the status word, lets copies in flight land, frees its TMEM and returns.
 #include "gemm_units.cuh"
 
+#include <type_traits>
+
 namespace ojb {
 namespace {
 
@@ -270,37 +272,46 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             __syncwarp();
           };
           if constexpr (EPI == kEpiSwiglu) {
+            auto tiles = [&](auto paired) {      // (chosen once per unit: asked per pair, the choice cost 4 % of the kernel)
 #pragma unroll 1
-            for (int t = 0; t < 2; ++t) {          // two tiles of 64 output columns
-              uint32_t gr[32], ur[32];
+              for (int t = 0; t < 2; ++t) {          // two tiles of 64 output columns
+                uint32_t gr[32], ur[32];
 #pragma unroll 1
-              for (int c = 0; c < 2; ++c) {
-                tmem_ld32(taddr + t * 64 + c * 32, gr);
-                tmem_ld32(taddr + 128 + t * 64 + c * 32, ur);
-                tmem_ld_wait();
-                if (c == 0) reuse();
+                for (int c = 0; c < 2; ++c) {
+                  tmem_ld32(taddr + t * 64 + c * 32, gr);
+                  tmem_ld32(taddr + 128 + t * 64 + c * 32, ur);
+                  tmem_ld_wait();
+                  if (c == 0) reuse();
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  float o[8];
+                  for (int j = 0; j < 4; ++j) {
+                    float o[8];
 #pragma unroll
-                  for (int e = 0; e < 8; e += 2) {
-                    float g0 = __uint_as_float(gr[8 * j + e]), g1 = __uint_as_float(gr[8 * j + e + 1]);
-                    float u0 = __uint_as_float(ur[8 * j + e]), u1 = __uint_as_float(ur[8 * j + e + 1]);
-                    if constexpr (FP8) {
-                      const int wr = u.wt * 256 + t * 64 + c * 32 + 8 * j + e;      // gate row of w; its up row is 128 further
-                      g0 *= rs * sw_at(wr); g1 *= rs * sw_at(wr + 1);
-                      u0 *= rs * sw_at(wr + 128); u1 *= rs * sw_at(wr + 129);
+                    for (int e = 0; e < 8; e += 2) {
+                      float g0 = __uint_as_float(gr[8 * j + e]), g1 = __uint_as_float(gr[8 * j + e + 1]);
+                      float u0 = __uint_as_float(ur[8 * j + e]), u1 = __uint_as_float(ur[8 * j + e + 1]);
+                      if constexpr (FP8) {
+                        const int wr = u.wt * 256 + t * 64 + c * 32 + 8 * j + e;      // gate row of w; its up row is 128 further
+                        g0 *= rs * sw_at(wr); g1 *= rs * sw_at(wr + 1);
+                        u0 *= rs * sw_at(wr + 128); u1 *= rs * sw_at(wr + 129);
+                      }
+                      float s0, s1;
+                      if constexpr (decltype(paired)::value) {
+                        silu2_f(g0, g1, s0, s1);
+                      } else {
+                        s0 = silu_f(g0);
+                        s1 = silu_f(g1);
+                      }
+                      o[e] = s0 * u0;
+                      o[e + 1] = s1 * u1;
                     }
-                    float s0, s1;
-                    silu2_f(g0, g1, s0, s1);
-                    o[e] = s0 * u0;
-                    o[e + 1] = s1 * u1;
+                    put(c * 4 + j, pack8(o));
                   }
-                  put(c * 4 + j, pack8(o));
                 }
+                if (u.wt * 128 + t * 64 < g.N / 2) flush(u.wt * 128 + t * 64);
               }
-              if (u.wt * 128 + t * 64 < g.N / 2) flush(u.wt * 128 + t * 64);
-            }
+            };
+            if (FP8 || u.xb * kBlockM < g.pair_rows) tiles(std::true_type{});
+            else tiles(std::false_type{});
           } else if constexpr (EPI == kEpiBf16) {
             const int nt = g.BN / 64;              // BN is a multiple of 64 on this path
 #pragma unroll 1
@@ -471,13 +482,17 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                   if (lane == 0) bulk_wait_read1();
                   __syncwarp();
                 }
+                auto tile = [&](auto paired) {
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                  const float xs = sx_at(m0 + c * 16 + e);
-                  const float gv = __uint_as_float(gr[e]) * (FP8 ? xs * swg : 1.f);
-                  const float uv = __uint_as_float(ur[e]) * (FP8 ? xs * swu : 1.f);
-                  t[e * 32 + lane] = f2bf(silu_f(gv) * uv);
-                }
+                  for (int e = 0; e < 16; ++e) {
+                    const float xs = sx_at(m0 + c * 16 + e);
+                    const float gv = __uint_as_float(gr[e]) * (FP8 ? xs * swg : 1.f);
+                    const float uv = __uint_as_float(ur[e]) * (FP8 ? xs * swu : 1.f);
+                    t[e * 32 + lane] = f2bf((decltype(paired)::value ? silu2_lanes_f(gv) : silu_f(gv)) * uv);
+                  }
+                };
+                if (!FP8 && m0 + c * 16 < g.pair_rows) tile(std::true_type{});      // (a multiple of 256: all 16 rows are on one side)
+                else tile(std::false_type{});
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0 && u.wt * 128 + quarter * 32 < g.N / 2) {
@@ -609,7 +624,7 @@ constexpr size_t kSmemBudget = 227 * 1024;
 
 template <int EPI, bool FP8 = false>
 int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits, int bn_req, int64_t ldo,
-                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr, bool accum = false) {
+                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr, bool accum = false, int pair_rows = -1) {
   static int smem_set[kMaxDevices] = {};
   auto kern = gemm_block256_kernel<EPI, FP8>;
   if (!raise_smem_limit(kern, static_cast<int>(kSmemBudget), smem_set)) return OJB_ERR_LAUNCH;
@@ -638,6 +653,9 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   } else {
     form = plain_form(M);
   }
+  // The two forms of SiLU differ in the last bits, so which one a row takes follows from the plain form, whatever form the model chooses.
+  if (pair_rows < 0) pair_rows = (bn_req == 0 && M > kBM ? plain_form(M) : form).n_xblk * kBlockM;
+  g.pair_rows = pair_rows;
   if (bn_req < 0) bn_req = 0;
   g.n_xblk = form.n_xblk;
   g.tail_rows = form.tail_rows;
@@ -721,9 +739,9 @@ void gemm_block256_set_probe(int repeat, int knob) {
 #endif
 
 int gemm_block256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,
-                         int splits, int64_t ldo, int32_t* status, cudaStream_t stream) {
+                         int splits, int64_t ldo, int32_t* status, cudaStream_t stream, int pair_rows) {
   if (epi == kEpiBf16) return launch_gemm<kEpiBf16>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
-  if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
+  if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream, nullptr, nullptr, false, pair_rows);
   return launch_gemm<kEpiPartialF32>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
 }
 

@@ -161,6 +161,14 @@ __device__ __forceinline__ void silu2_f(float x0, float x1, float& s0, float& s1
   s1 = x1 * (r * d0);
 }
 
+// silu2_f where the two values are on neighbouring lanes (of a whole warp): the same bits for each.
+__device__ __forceinline__ float silu2_lanes_f(float x) {
+  const float d = 1.0f + exp2f_fast(fminf(-x * 1.4426950408889634f, 60.0f)), other = __shfl_xor_sync(0xffffffffu, d, 1);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d * other));
+  return x * (r * other);
+}
+
 enum Epilogue { kEpiBf16 = 0, kEpiSwiglu = 1, kEpiPartialF32 = 2 };
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -268,8 +276,9 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Launchers of the two kernels (defined in gemm_tile128.cu and gemm_block256.cu). epi is an Epilogue value.
 int gemm_tile128_launch(int epi, int bn, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits,
                         int64_t ldo, int32_t* status, cudaStream_t stream);
+// pair_rows: rows of x that take their SiLU as in block units, -1 = those of the plain form (bn_req 0) or of the form asked for
 int gemm_block256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,
-                         int splits, int64_t ldo, int32_t* status, cudaStream_t stream);
+                         int splits, int64_t ldo, int32_t* status, cudaStream_t stream, int pair_rows = -1);
 // out fp32 [M, N] += the product (one K range; N % 32 == 0)
 int gemm_block256_add_launch(int bn_req, const void* x, const void* w, float* out, int64_t M, int64_t N, int64_t K, int32_t* status,
                              cudaStream_t stream);

@@ -43,6 +43,7 @@ struct GemmArgs {
   int tail_sub;                // bytes of a tail sub-stage (128 rows of w + the x rows), 0 = one k-block per stage
   int tma_out;                 // the block epilogue stores through shared-memory tiles and bulk tensor stores
   int accum;                   // block kernel, fp32 output: the product is added to what out holds (bulk reductions in place of bulk stores)
+  int pair_rows;               // block kernel, SwiGLU: rows of x below it take their SiLU in pairs (silu2_f), the others by silu_f
   int dbg;                     // probe builds only (see below); 0 otherwise
   int mma_repeat;              // probe builds only; 1 otherwise
   // CTA-pair kernel, swapped-operand units: the tail_box accumulator columns (= rows of x) of a unit are produced by
@@ -318,9 +319,10 @@ inline double form_clocks(const BlockForm& f, int64_t N, int splits, int kb_tota
   const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, f.n_xblk, f.tail_box, f.n_xchunk, tail, splits, kb_total, sms, epi);
   return block_kernel_clocks(N, bn, f.n_xblk, f.tail_box, f.n_xchunk, tail, splits, kb_total, sms, epi);
 }
-// The cheaper of the two by the model, and its clocks. (Not for e4m3 operands: a block and a swapped unit round SiLU differently, and
-// that path keeps its bits.) Measured under the power cap, without / with the choice: [12352, 5120] at 1066 / 1184 rows 126 / 140 us
-// and 109 / 122, gate/up at 1984 rows 561 and 532, [5120, 17408] in one K range at 1312 rows 210 and 193.
+// The cheaper of the two by the model, and its clocks; no result depends on it (GemmArgs::pair_rows). Not for e4m3 operands, whose results
+// would move: a block and a swapped unit multiply the two scales in another order. Measured under the power cap, without / with
+// the choice: [12352, 5120] at 1066 / 1184 rows 126 / 140 us and 109 / 122, gate/up at 544 / 1984 / 2208 rows 196 / 563 / 624 and 187 / 553 /
+// 615, [5120, 17408] in one K range at 1312 rows 210 and 193.
 struct FormChoice {
   BlockForm form;
   double clocks;

@@ -422,6 +422,31 @@ def test_forms_of_the_block_kernel(M, N, idx):
     _lib.check_status()
 
 
+# rows of x and the 256-row blocks that the plain form has for them, 0 where all rows in swapped-operand units are weighed as cheaper than that form
+@pytest.mark.parametrize("M,blocks", [(288, 0), (416, 0), (704, 0), (1056, 4), (1248, 0), (1568, 0), (1984, 0), (2049, 8), (2208, 9), (2400, 9),
+                                      (2623, 10), (2624, 10)])
+def test_swiglu_result_does_not_depend_on_the_form(M, blocks):
+    """Block and swapped-operand units round SiLU differently. Whatever form the model chooses, a row keeps the bits that it has in the plain
+    form, its rows in full blocks and a swapped tail of at most 128 rows, or in swapped units throughout where those are preferred to it."""
+    from ojb200 import _lib, lt_ext as LT
+    K, I = 5120, 17408
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, generator=g, device="cuda").to(bf16)
+    w = (torch.randn(2 * I, K, generator=g, device="cuda") * 0.02).to(bf16)
+    head = min(M, blocks * 256)
+    want = torch.empty(M, I, device="cuda", dtype=bf16)
+    if head:
+        full = x.new_zeros(blocks * 256, K)
+        full[:head] = x[:head]
+        want[:head] = LT.gemm_swiglu(full, w, 12)[:head]
+    for m in range(head, M, 1024):
+        want[m:m + 1024] = LT.gemm_swiglu(x[m:m + 1024].contiguous(), w, 7)
+    assert torch.equal(LT.gemm_swiglu(x, w, 0), want)
+    if blocks:
+        assert torch.equal(LT.gemm_swiglu(x, w, 3), want)
+    _lib.check_status()
+
+
 # x as the N side (w tile wider than the rows) and as the M side (2048 outputs: tiles of 16), edges of 16 rows and of the last w tile
 @pytest.mark.parametrize("M", [1, 16, 17, 33, 100, 128])
 @pytest.mark.parametrize("N", [2048, 2056, 12352])
