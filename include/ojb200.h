@@ -40,14 +40,14 @@ int ojb_abi_version(void);
  * GEMM — replaces src/lt.cpp:43 lt_matmul / src/fastmodel.py:168 _mm (cuBLASLt) and src/fastmodel.py:158 _skmm
  * (torch.bmm split-K partials). out[M,N] = x[M,K] · w[N,K]^T, bf16 operands, fp32 accumulation in tensor memory.
  * Requirements: K % 8 == 0, x / w / out 16-byte aligned. variant: 0 = the library chooses (cost model, see ojb_gemm_plan);
- * 1 / 2 = 128-row tile kernel with 128x256 / 128x128 tiles; 3 = 256-row block kernel, w-tile width and form of the rows
- * behind the full blocks (as 7 or 8) by the cost model; 4 = that
+ * 1 / 2 = 128-row tile kernel with 128x256 / 128x128 tiles; 3 = 256-row block kernel with full blocks, a swapped tail of at most 128 rows (a
+ * longer remainder is one more block) and automatic w-tile width; 4 = that
  * kernel with all rows of x in swapped-operand units (M <= 2048); a multiple of 16 in [16, 256] = that kernel with this
  * w-tile width; 5 = CTA-pair kernel (tcgen05.mma.cta_group::2) with automatic width; 6 = CTA-pair kernel with all rows of
  * x in swapped-operand units (any M: one pass over w per 512 rows of x, up to 512 accumulator columns per unit);
  * 512 + a multiple of 16 in [16, 256] = the pair kernel with that width; 7 = the block kernel with all but the last full
  * 256-row block of x in block units and the remaining 257..511 rows in two swapped-operand chunks that fit them exactly;
- * 8 = the block kernel with full blocks, a swapped tail of at most 128 rows (a longer remainder is one more block) and automatic width;
+ * 8 = the block kernel as 3 or 7, whichever the cost model prefers (variant 0 takes it so);
  * 1024 = few-row kernel (M <= 128, K % 64 == 0, not SwiGLU; elsewhere as 0) with automatic w-tile width, 1024 + a multiple of 16
  * in [16, 128] = that kernel with this width (OJB_ERR_LIMIT where it does not serve).
  * ------------------------------------------------------------------------------------------------------------------ */
@@ -75,7 +75,7 @@ int ojb_gemm_bf16_splitk(const void* x, const void* w, float* parts, int64_t M, 
 
 /* h fp32 [M, N] += x · w^T (N % 32 == 0): one K range whose result goes straight to the fp32 residual stream, through bulk reductions of
  * the block kernel, instead of a plane of ojb_gemm_bf16_splitk that ojb_resnorm_f32 adds afterwards (the same sum, h + product, in fp32;
- * a product below 2^-126 counts as zero). variant 0 or 3: 256-row blocks, 4: every row in swapped-operand units. */
+ * a product below 2^-126 counts as zero). variant 0: as 8, 3: full blocks and a swapped tail, 4: every row in swapped-operand units. */
 int ojb_gemm_bf16_add(const void* x, const void* w, float* h, int64_t M, int64_t N, int64_t K, int variant, int32_t* status,
                       ojb_stream_t stream);
 
@@ -106,7 +106,7 @@ int ojb_gemm_band_blocks(int32_t n_xblk, int64_t K, int32_t elt);
 
 /* Host-side plan (no GPU work): which kernel variant and how many K ranges the library's cost model picks for a shape.
  * kind = 0 bf16 output, 1 SwiGLU-fused, 2 fp32 split-K partials, 3 those of an 8-bit product with K counted in pairs of
- * elements (the kinds that may use more than one range, up to max_splits). *microseconds (optional) receives the modelled time. Takes the place of the algorithm search of
+ * elements (the kinds that may use more than one range, up to max_splits). Variant 3 stands for the block kernel in either form. *microseconds (optional) receives the modelled time. Takes the place of the algorithm search of
  * src/lt.cpp:93 (lt2_search), which times cuBLASLt candidates on the device. */
 int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int32_t max_splits, int32_t* variant, int32_t* splits,
                   float* microseconds);

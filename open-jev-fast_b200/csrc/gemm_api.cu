@@ -18,13 +18,12 @@ using namespace ojb;
 namespace {
 
 // variant: 0 = automatic; 1 = tile128 with 128x256 tiles; 2 = tile128 with 128x128 tiles; a multiple of 16 in [16, 256] =
-// block256 with that w-tile width; 3 = block256, width and form of the rows behind the full blocks by the model; 4 = block256 with every
-// row of x in swapped-operand units (M <= 2048).
+// block256 with that w-tile width; 3 = block256 with full blocks and a swapped tail of at most 128 rows, automatic width; 4 = block256 with
+// every row of x in swapped-operand units (M <= 2048).
 // 5 = pair256 (CTA pairs, cta_group::2) with automatic width; 6 = pair256 with every row of x in swapped-operand units
 // (any M); 512 + a multiple of 16 in [16, 256] = pair256 with that w-tile width; 7 = block256 with the last 257..511 rows of x in
-// two swapped-operand chunks and the rows before them in block units; 8 = block256 with full blocks and a swapped tail of at most 128
-// rows, automatic width; 1024 = skinny (M <= 128, K % 64 == 0, not for SwiGLU; else as 0) with automatic
-// width;
+// two swapped-operand chunks and the rows before them in block units; 8 = block256 as 3 or 7, by the model; 1024 = skinny (M <= 128,
+// K % 64 == 0, not for SwiGLU; else as 0) with automatic width;
 // 1024 + a multiple of 16 in [16, 128] = skinny with that w-tile width.
 bool variant_ok(int v) {
   return (v >= 0 && v <= 8) || (v >= 16 && v <= 256 && v % 16 == 0) || (v >= 528 && v <= 768 && v % 16 == 0) ||
@@ -81,7 +80,7 @@ Plan model_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits, bool pla
   if (epi != kEpiSwiglu) consider(2, tile128_clocks(M, N, kb_total, splits, 128, sms, f32));
   if (plain_form(M).n_xblk > 0) {      // block256
     if (plain_forms) consider(3, form_clocks(plain_form(M), N, splits, kb_total, sms, model_epi));
-    else consider(3, choose_form(M, N, splits, kb_total, sms, model_epi).clocks);
+    else consider(8, choose_form(M, N, splits, kb_total, sms, model_epi).clocks);
   }
   if (M <= 2048) {  // block256 with every row in swapped-operand units
     const BlockForm f = chunked_form(M, 0);
@@ -99,7 +98,7 @@ Plan plan_kernel(int epi, int64_t M, int64_t N, int64_t K, int splits) {
   return cache.get(key, [&] {
     Plan p = model_kernel(epi, M, N, K, splits, false);
     // SwiGLU: which rows take their SiLU in pairs follows from the kernel that the plain forms would get
-    if (epi == kEpiSwiglu && p.variant == 3 && model_kernel(epi, M, N, K, splits, true).variant != 3) p.pair_rows = 0;
+    if (epi == kEpiSwiglu && p.variant == 8 && model_kernel(epi, M, N, K, splits, true).variant != 3) p.pair_rows = 0;
     return p;
   });
 }
@@ -118,7 +117,7 @@ int dispatch(int epi, int variant, const void* x, const void* w, void* out, int6
     return gemm_pair256_launch(epi, variant == 5 ? 0 : (variant == 6 ? -1 : variant - 512), x, w, out, M, N, K, splits, ldo, status, st);
   if (variant == 1 || variant == 2)
     return gemm_tile128_launch(epi, variant == 1 ? 256 : 128, x, w, out, M, N, K, splits, ldo, status, st);
-  return gemm_block256_launch(epi, variant == 3 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : (variant == 8 ? -3 : variant))), x, w, out, M, N, K, splits, ldo, status, st,
+  return gemm_block256_launch(epi, variant == 8 ? 0 : (variant == 4 ? -1 : (variant == 7 ? -2 : (variant == 3 ? -3 : variant))), x, w, out, M, N, K, splits, ldo, status, st,
                               pair_rows);
 }
 
@@ -154,7 +153,7 @@ extern "C" int ojb_gemm_bf16_add(const void* x, const void* w, float* h, int64_t
                                  ojb_stream_t stream) {
   OJB_REQUIRE(x && w && h && M > 0 && N > 0 && K > 0 && K % 8 == 0 && N % 32 == 0 && (variant == 0 || variant == 3 || variant == 4));
   OJB_REQUIRE(aligned16(x) && aligned16(w) && aligned16(h));
-  return gemm_block256_add_launch(variant == 4 ? -1 : 0, x, w, h, M, N, K, status, static_cast<cudaStream_t>(stream));
+  return gemm_block256_add_launch(variant == 4 ? -1 : (variant == 3 ? -3 : 0), x, w, h, M, N, K, status, static_cast<cudaStream_t>(stream));
 }
 
 namespace ojb {
@@ -224,7 +223,7 @@ extern "C" int ojb_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t kind, int3
     }
     return Ranges{best, best_s};
   });
-  *variant = r.plan.variant;
+  *variant = r.plan.variant == 8 ? 3 : r.plan.variant;      // (the block kernel, whatever its form)
   *splits = r.splits;
   if (microseconds) *microseconds = static_cast<float>(r.plan.clocks / 1800.0);
   return OJB_OK;

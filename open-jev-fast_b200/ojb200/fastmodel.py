@@ -252,7 +252,7 @@ class FastQwen35(torch.nn.Module):
                     out.setdefault(tuple(w.shape), []).append(d)
             return out
 
-        kernels = [1, 12] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
+        kernels = [1, 3] + ([7] if M <= 2048 else []) + ([10] if M > 256 and M % 256 else []) + self.TUNE_EXTRA
         few = [11] if M <= 128 else []
         for (N, Kd), layers in groups("w_in").items():
             x = rnd(M, Kd)

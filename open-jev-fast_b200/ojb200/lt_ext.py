@@ -2,12 +2,12 @@
 
 The reference enumerates cuBLASLt algorithms per shape (lt_setup) and runs one by index (lt_matmul); split-K plans go
 through lt2_*. Here an "algorithm" is one of the library's GEMM variants: index 0 lets the library choose, 1 / 2 force the
-128-row tile kernel with 256 / 128-wide tiles, 3 the 256-row block kernel with w-tile width and the form of the remaining rows by the cost model, 4..6 that kernel
+128-row tile kernel with 256 / 128-wide tiles, 3 the 256-row block kernel with automatic w-tile width, 4..6 that kernel
 with w-tile width 256, 192, 128, 7 that kernel with all of x in swapped-operand units (M <= 2048), 8 / 9 the CTA-pair
 kernel (tcgen05.mma.cta_group::2) with automatic width / all of x in swapped-operand units, 10 the block kernel with
 block units for all but the last full block of x and two swapped-operand chunks for the remaining 257..511 rows, 11 the
-few-row kernel (at most 128 rows, K a multiple of 64, not SwiGLU; as 0 elsewhere), 12 the block kernel with full blocks and a swapped tail
-of at most 128 rows.
+few-row kernel (at most 128 rows, K a multiple of 64, not SwiGLU; as 0 elsewhere), 12 the block kernel as 3 or 10, whichever the cost
+model prefers. The indices keep their meaning: plans are kept as indices (OJ_TUNE_CACHE).
 Two entry points have no counterpart in the reference: gemm_swiglu (SwiGLU fused into the epilogue) and gemm_splitk
 (fp32 partial sums from the un-split [N, K] weight).
 """
@@ -103,7 +103,8 @@ def gemm_splitk(x, w, S, idx=0):
 
 
 def gemm_add(x, w, h, idx=0):
-    """h += x @ w^T in place (ojb_gemm_bf16_add): h fp32 [M, N], N a multiple of 32; idx 0 or 3 the block kernel, 7 all rows swapped."""
+    """h += x @ w^T in place (ojb_gemm_bf16_add): h fp32 [M, N], N a multiple of 32; idx 0 or 3 the block kernel in its own choice of form or
+    with full blocks and a swapped tail, 7 all rows swapped."""
     _check(x, w)
     M, K = x.shape
     N = w.shape[0]

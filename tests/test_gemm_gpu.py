@@ -438,12 +438,33 @@ def test_swiglu_result_does_not_depend_on_the_form(M, blocks):
     if head:
         full = x.new_zeros(blocks * 256, K)
         full[:head] = x[:head]
-        want[:head] = LT.gemm_swiglu(full, w, 12)[:head]
+        want[:head] = LT.gemm_swiglu(full, w, 3)[:head]
     for m in range(head, M, 1024):
         want[m:m + 1024] = LT.gemm_swiglu(x[m:m + 1024].contiguous(), w, 7)
     assert torch.equal(LT.gemm_swiglu(x, w, 0), want)
     if blocks:
-        assert torch.equal(LT.gemm_swiglu(x, w, 3), want)
+        assert torch.equal(LT.gemm_swiglu(x, w, 3), want) and torch.equal(LT.gemm_swiglu(x, w, 12), want)
+    _lib.check_status()
+
+
+@pytest.mark.parametrize("idx,blocks,swapped", [(3, 4, 1), (10, 3, 2), (12, 3, 2)])
+def test_algorithm_indices_name_the_same_kernels(idx, blocks, swapped):
+    """Kept plans hold bare indices, so each goes on naming the kernel that was timed under it: the block and swapped-operand units per 256
+    outputs of a 1056-row product, from the kernel's own record of its units."""
+    import ctypes
+    from ojb200 import _lib, lt_ext as LT
+    x, w = _mk(1056, 34816, 5120, 5)
+    rec = torch.zeros(1 + 4 * 4096, dtype=torch.int64, device="cuda")
+    _lib.call("ojb_gemm_set_trace", _lib.ptr(rec), ctypes.c_int32(4096))
+    try:
+        LT.gemm_swiglu(x, w, idx)
+        torch.cuda.synchronize()
+    finally:
+        _lib.call("ojb_gemm_set_trace", None, ctypes.c_int32(0))
+    n = int(rec[0])
+    units = rec[1:1 + 4 * n].view(n, 4)[:, 0]
+    tails = int(((units >> 31) & 1).sum())
+    assert (n - tails, tails) == (blocks * 136, swapped * 136)
     _lib.check_status()
 
 
