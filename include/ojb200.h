@@ -46,7 +46,8 @@ int ojb_abi_version(void);
  * w-tile width; 5 = CTA-pair kernel (tcgen05.mma.cta_group::2) with automatic width; 6 = CTA-pair kernel with all rows of
  * x in swapped-operand units (any M: one pass over w per 512 rows of x, up to 512 accumulator columns per unit);
  * 512 + a multiple of 16 in [16, 256] = the pair kernel with that width; 7 = the block kernel with all but the last full
- * 256-row block of x in block units and the remaining 257..511 rows in two swapped-operand chunks that fit them exactly;
+ * 256-row block of x in block units and the remaining 257..511 rows in two swapped-operand chunks that fit them exactly (up
+ * to 256 rows: as 4);
  * 8 = the block kernel as 3 or 7, whichever the cost model prefers (variant 0 takes it so);
  * 1024 = few-row kernel (M <= 128, K % 64 == 0, not SwiGLU; elsewhere as 0) with automatic w-tile width, 1024 + a multiple of 16
  * in [16, 128] = that kernel with this width (OJB_ERR_LIMIT where it does not serve).

@@ -641,12 +641,12 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   if (static_cast<int64_t>(splits - 1) * g.kb_per_split >= g.kb_total) return OJB_ERR_ARG;   // an empty split
   // bn_req > 0: full blocks with w tiles of that width and a swapped tail; 0: blocks, the form of the rest and the width by the model;
   // -1: every row of x in swapped-operand units (M <= 2048: chunks of <= 256 rows), as always up to 128 rows; -2: the last 257..511 rows
-  // in two swapped chunks; -3: full blocks and a swapped tail, the width by the model
+  // in two swapped chunks (up to 256 rows: as -1); -3: full blocks and a swapped tail, the width by the model
   BlockForm form;
-  if (bn_req == -1 || M <= kBM) {
+  if (bn_req == -1 || M <= kBM || (bn_req == -2 && M <= kBlockM)) {
     if (M > 2048) return OJB_ERR_LIMIT;
     form = chunked_form(M, 0);
-  } else if (bn_req == -2 && M > kBlockM) {
+  } else if (bn_req == -2) {
     form = hybrid_form(M);
   } else if (bn_req == 0 && !FP8) {
     form = choose_form(M, N, splits, g.kb_total, sms, EPI).form;

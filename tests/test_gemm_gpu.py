@@ -447,6 +447,16 @@ def test_swiglu_result_does_not_depend_on_the_form(M, blocks):
     _lib.check_status()
 
 
+@pytest.mark.parametrize("M", [129, 200, 256])
+def test_two_chunk_form_of_one_block_swaps_all_rows(M):
+    """Up to 256 rows the form of index 10 has no block before its chunks: every row is in swapped units, with their bits."""
+    from ojb200 import lt_ext as LT, _lib
+    x, w = _mk(M, 34816, 1280, M)
+    w *= 8
+    assert torch.equal(LT.gemm_swiglu(x, w, 10), LT.gemm_swiglu(x, w, 7))
+    _lib.check_status()
+
+
 @pytest.mark.parametrize("idx,blocks,swapped", [(3, 4, 1), (10, 3, 2), (12, 3, 2)])
 def test_algorithm_indices_name_the_same_kernels(idx, blocks, swapped):
     """Kept plans hold bare indices, so each goes on naming the kernel that was timed under it: the block and swapped-operand units per 256
