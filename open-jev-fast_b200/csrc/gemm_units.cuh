@@ -169,6 +169,19 @@ inline UnitCost unit_cost(int bn, int tail_box, int epi) {
   return c;
 }
 
+// Never more than block_kernel_clocks of the same arguments: the mean load of the workers. A width search passes over what cannot win by
+// this instead of dealing its units out.
+inline double block_kernel_floor(int64_t N, int bn, int n_xblk, int tail_box, int n_xchunk, bool has_tail, int splits, int kb_total,
+                                 int workers, int epi) {
+  const UnitCost c = unit_cost(bn, tail_box, epi);
+  const int64_t blocks = n_xblk * ceil_div(N, bn), tails = has_tail ? n_xchunk * ceil_div(N, 256) : 0;      // per K range
+  const int64_t units = (blocks + tails) * splits;
+  if (units <= 0) return 0.0;
+  const double all = static_cast<double>(blocks) * (kb_total * c.block_kb + splits * c.block_epi) +
+                     static_cast<double>(tails) * (kb_total * c.tail_kb + splits * c.tail_epi);
+  return static_cast<double>(static_cast<int64_t>(all / static_cast<double>(units < workers ? units : workers))) + 5000.0;
+}
+
 // Longest per-worker sum when the units of the block kernels (order of decode_unit) are dealt round-robin to `workers`
 // CTAs (or CTA pairs). n_xblk == 0: swapped-operand units only.
 inline double block_kernel_clocks(int64_t N, int bn, int n_xblk, int tail_box, int n_xchunk, bool has_tail, int splits,
@@ -283,6 +296,7 @@ inline int choose_bn(int64_t N, int n_xblk, int tail_box, int n_xchunk, bool has
     int best = 256;
     double best_cost = 1e30;
     for (int bn = 256; bn >= 64; bn -= 16) {
+      if (block_kernel_floor(N, bn, n_xblk, tail_box, n_xchunk, has_tail, splits, kb_total, workers, epi) >= best_cost * 0.98) continue;
       const double cost = block_kernel_clocks(N, bn, n_xblk, tail_box, n_xchunk, has_tail, splits, kb_total, workers, epi);
       if (cost < best_cost * 0.98) { best_cost = cost; best = bn; }
     }
@@ -314,6 +328,14 @@ inline BlockForm chunked_form(int64_t M, int64_t blocks) {
 // runs at the 64-clock floor of a short tail, and none on the zero rows of a padded block.
 inline BlockForm hybrid_form(int64_t M) { return chunked_form(M, M / kBlockM - 1); }
 
+inline double form_floor(const BlockForm& f, int64_t N, int splits, int kb_total, int sms, int epi) {
+  double least = 1e30;
+  for (int bn = 256; bn >= (epi == kEpiSwiglu ? 256 : 64); bn -= 16) {
+    const double floor = block_kernel_floor(N, bn, f.n_xblk, f.tail_box, f.n_xchunk, f.tail_rows > 0, splits, kb_total, sms, epi);
+    least = floor < least ? floor : least;
+  }
+  return least;
+}
 inline double form_clocks(const BlockForm& f, int64_t N, int splits, int kb_total, int sms, int epi) {
   const bool tail = f.tail_rows > 0;
   const int bn = epi == kEpiSwiglu ? 256 : choose_bn(N, f.n_xblk, f.tail_box, f.n_xchunk, tail, splits, kb_total, sms, epi);
@@ -335,8 +357,10 @@ inline FormChoice choose_form(int64_t M, int64_t N, int splits, int kb_total, in
     FormChoice best{plain, form_clocks(plain, N, splits, kb_total, sms, epi)};
     if (M > kBlockM && M % kBlockM != 0) {
       const BlockForm hybrid = hybrid_form(M);
-      const double clocks = form_clocks(hybrid, N, splits, kb_total, sms, epi);
-      if (clocks < best.clocks) best = FormChoice{hybrid, clocks};
+      if (form_floor(hybrid, N, splits, kb_total, sms, epi) < best.clocks) {
+        const double clocks = form_clocks(hybrid, N, splits, kb_total, sms, epi);
+        if (clocks < best.clocks) best = FormChoice{hybrid, clocks};
+      }
     }
     return best;
   });

@@ -111,6 +111,21 @@ def test_k_ranges_do_not_move_with_the_forms(M, K, want):
     assert lt_ext.plan_splitk(M, 5120, K) == want
 
 
+# (M, N, K, kind): K ranges and modelled clocks when every tile width is dealt out unit by unit
+PLANS = [(144, 12352, 5120, 0, 1, 75180), (400, 5120, 17408, 2, 3, 119845), (544, 34816, 5120, 1, 1, 282892), (1066, 12352, 5120,
+         0, 1, 188176), (1184, 12352, 5120, 0, 1, 203144), (1984, 34816, 5120, 1, 1, 892832), (2208, 5120, 6144, 2, 1, 207824), (2500,
+         5120, 17408, 2, 2, 565524), (3001, 14336, 5120, 0, 1, 545820), (4160, 5120, 4096, 2, 1, 257204), (9037, 12352, 5120, 0, 1,
+         1411132), (16672, 5120, 17408, 2, 1, 3580080), (600, 264, 640, 2, 5, 12611), (777, 1000, 136, 0, 1, 10384)]
+
+
+def test_width_search_passes_over_no_winner():
+    """The search of tile widths and forms leaves out what a lower bound rules out; the answers are those of the search over all of them."""
+    from ojb200 import lt_ext
+    for M, N, K, kind, splits, clocks in PLANS:
+        _, s, us = lt_ext.gemm_plan(M, N, K, kind)
+        assert (s, round(us * 1800)) == (splits, clocks), (M, N, K, kind)
+
+
 @pytest.mark.parametrize("env,want", [
     ({}, [13, 13, 0, 0]),                                               # five bands of 16 blocks at most
     ({"OJB_GEMM_BAND_MB": "40"}, [13, 4, 0, 0]),                        # 16 blocks of 2.5 MB, or 4 of 8.5 MB
