@@ -256,7 +256,8 @@ int64_t ojb_gdn_scratch_bytes(int64_t n_chunks, int64_t HV);
  *   chunks int32 [n_chunks, 4] = (first row, rows <= 64 (0 = unused entry), -, -)
  *   steps  int32 [*, 4]        = (chunk, load, save, aux) in execution order; load: 0 carry on, 1 zero state, 2 / 3 restore
  *                                parked slot A / B, 4 initial state number (aux >> 16) - 1; save: bit 0 park in slot A,
- *                                bit 1 in slot B; (aux & 0xffff) - 1 = index in final_state written after the step
+ *                                bit 1 in slot B; (aux & 0xffff) - 1 = index in final_state written after the step. The
+ *                                step of an unused entry leaves the state as it loads it
  *   walk_ptr int32 [n_walks+1] = step ranges that are independent of each other (one CTA column each)
  * q, k bf16 [rows, HK, 128]; v bf16 [rows, HV, 128]; g fp32 (natural-log decay) and beta bf16 [rows, HV];
  * init_state / final_state fp32 [*, HV, 128(dk), 128(dv)] or null; out bf16 [rows, HV, 128], rows not covered by a chunk

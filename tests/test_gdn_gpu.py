@@ -490,3 +490,38 @@ def test_state_pass_keeps_and_drops_states_as_the_tree_asks(root, stems, leaf, d
         assert _rel(o.cpu()[rows][:, heads], ref) < 4e-3
         if export >= 0:
             assert _rel(fin[export, heads], state) < 1e-2
+
+
+@pytest.mark.parametrize("HV", [4, 40])      # full form and, above one CTA per SM, dense form
+def test_steps_of_unused_entries_leave_the_state_alone(HV):
+    """Steps that name a chunk of no rows, among others and first in a walk: they load, park and export the state and change nothing, and
+    the state pass reads nothing that the first pass has not written (the scratch starts as not-a-numbers). The error bounds are those
+    of the other comparisons with the recurrence."""
+    from ojb200 import ext as K, _lib
+    HK, n = 2, 85
+    chunks = [[0, 40, 0, 0], [40, 0, 0, 0], [40, 30, 0, 0], [0, 0, 0, 0], [70, 5, 0, 0], [75, 10, 0, 0]]
+    steps = [[0, 1, 0, 0], [1, 0, 1, 1], [2, 0, 0, 0], [3, 2, 2, 2], [4, 0, 0, 3], [1, 3, 0, 4], [3, 1, 0, 0], [5, 0, 0, 5]]
+    walks = [0, 6, 8]
+    host = _inputs(n, HK, HV, 31)
+    q, k, v, g, beta = (t.cuda() for t in host)
+    tab = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    chunks, steps, walks = tab(chunks), tab(steps), tab(walks)
+    fin, out = torch.zeros(5, HV, 128, 128, device="cuda"), torch.zeros(n, HV, 128, dtype=bf16, device="cuda")
+    scratch = torch.full((6 * HV * 81936,), 255, dtype=torch.uint8, device="cuda")
+    park = torch.full((max(16, K.gdn_park_bytes(2, HV)),), 255, dtype=torch.uint8, device="cuda")
+    K.call("ojb_gdn_chunked_park", *(K.ptr(t) for t in (q, k, v, g, beta, chunks)), K.i64(6), K.ptr(steps), K.ptr(walks), K.i64(2), K.ptr(None),
+           K.ptr(fin), K.ptr(scratch), K.ptr(out), K.i64(HK), K.i64(HV), K.f32(128 ** -0.5), K.ptr(park if HV == 40 else None), K.i32(1),
+           K.ptr(_lib.status_word(v.device)), K.stream_ptr())
+    torch.cuda.synchronize()
+    _lib.check_status()
+    root = list(range(40))
+    heads = [0, 1, HV - 2, HV - 1]
+    for rows, shown, exports in ((root, root, (0, 1, 3)), (root + list(range(40, 70)), range(40, 70), ()),
+                                 (root + list(range(70, 75)), range(70, 75), (2,)), (list(range(75, 85)), range(75, 85), (4,))):
+        for h in heads:
+            one = [t[rows][:, [h * HK // HV if i < 2 else h]] for i, t in enumerate(host)]
+            ref, state = OG.recurrent(*one, 128 ** -0.5)
+            assert _rel(out[list(shown), h], ref[-len(shown):, 0]) < 4e-3
+            for e in exports:
+                assert _rel(fin[e, h], state[0]) < 1e-2
+    assert torch.equal(fin[0], fin[1])
