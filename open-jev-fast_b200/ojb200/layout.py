@@ -164,9 +164,9 @@ class SeqTables:
         lens = np.ascontiguousarray(lens, np.int64)
         S = len(lens)
         need = max(1, -(-(Lp - pad) // 64) + int((-(-lens // 64)).sum()))
-        if cap is not None and need > max(cap, 1):
+        if cap is not None and need > cap:
             raise RuntimeError("tree_layout: more chunks than the table capacity")
-        cap = need if cap is None else max(cap, 1)
+        cap = need if cap is None else cap
         t = cls(S, -(-(Lp + S * T) // 32) * 32, cap, S if own_walks else 1, pin=pin)
         p = lambda x, ty: ctypes.cast(x.data_ptr(), ty)
         rc = _lib.lib().ojb_seq_tables(lens.ctypes.data_as(_I64P), *(ctypes.c_int64(x) for x in (S, Lp, pad, T)), ctypes.c_int32(own_walks),

@@ -238,8 +238,9 @@ def test_sequence_tables_refuse_what_does_not_fit():
     for lens, T in (([5], 4), ([-1], 4)):
         with pytest.raises(RuntimeError):
             SeqTables.build(lens, 0, 0, T, True, cap=4)
-    with pytest.raises(RuntimeError):
-        SeqTables.build([64, 64, 65], 0, 0, 65, True, cap=3)
+    for lens, cap in (([64, 64, 65], 3), ([3], 0), ([0], 0)):      # (tables of no chunk hold one unused entry)
+        with pytest.raises(RuntimeError):
+            SeqTables.build(lens, 0, 0, 65, True, cap=cap)
 
 
 def test_common_prefix_of_candidates():
