@@ -482,11 +482,12 @@ def test_state_pass_keeps_and_drops_states_as_the_tree_asks(root, stems, leaf, d
     K.gdn_chunked(*(t.cuda() for t in (q, k, v, g, beta)), 128 ** -0.5, tab(chunks), tab(steps), tab([0, len(steps)]), 1, None, fin, o)
     torch.cuda.synchronize()
     _lib.check_status()
-    heads = slice(0, 4)                     # (the oracle's time goes with the heads)
-    for rows, export in paths if len(paths) <= 6 else paths[::7]:
+    heads = [0, 1, HV - 2, HV - 1]          # (the oracle's time goes with the heads)
+    inputs = [t[:, [h * HK // HV for h in heads] if i < 2 else heads] for i, t in enumerate((q, k, v, g, beta))]
+    # many leaves: every 7th, and the last three, which follow the end of a batch of 32 steps
+    for rows, export in paths if len(paths) <= 9 else paths[::7] + paths[-3:]:
         rows = torch.tensor(rows)
-        ref, state = OG.recurrent(*(t[rows][:, :(2 if i < 2 else 4)] if dense is False else
-                                    t[rows][:, :1 if i < 2 else 4] for i, t in enumerate((q, k, v, g, beta))), 128 ** -0.5)
+        ref, state = OG.recurrent(*(t[rows] for t in inputs), 128 ** -0.5)
         assert _rel(o.cpu()[rows][:, heads], ref) < 4e-3
         if export >= 0:
             assert _rel(fin[export, heads], state) < 1e-2

@@ -389,6 +389,33 @@ def test_product_added_to_the_stream_equals_a_plane_added_afterwards(M, N, K, id
     assert bool((guard[0] == 7).all()) and bool((guard[-1] == 7).all())
 
 
+# bands (24 and more blocks of x over 64 MB) with a remainder behind them, one w tile and several
+@pytest.mark.parametrize("M,N,K", [(24 * 256 + 40, 320, 5504), (30 * 256, 1280, 4608)])
+@pytest.mark.parametrize("e4m3", [False, True])
+def test_product_added_to_the_stream_in_bands(M, N, K, e4m3):
+    """Rows taken in bands, as long prefixes are, add every element of the product once: the bits of the plane added afterwards."""
+    import ctypes
+    from ojb200 import lt_ext as LT, _lib
+    K = K * 2 if e4m3 else K
+    assert 0 < _lib.lib().ojb_gemm_band_blocks(M // 256, ctypes.c_int64(K), 1 if e4m3 else 2) < M // 256
+    x, w = _mk(M, N, K, 11)
+    h = torch.randn(M, N, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda") * 4
+    guard = torch.full((M + 2, N), 7.0, device="cuda")
+    got = guard[1:M + 1]
+    got.copy_(h)
+    if e4m3:
+        (xq, sx), (wq, sw) = LT.quantize_rows_e4m3(x), LT.quantize_weight_e4m3(w)
+        want = h + LT.gemm_e4m3(xq, sx, wq, sw, 2, 1)[0]
+        LT.gemm_e4m3(xq, sx, wq, sw, 3, h=got)
+    else:
+        want = h + LT.gemm_splitk(x, w, 1, 0)[0]
+        LT.gemm_add(x, w, got, 0)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(got, want)
+    assert bool((guard[0] == 7).all()) and bool((guard[-1] == 7).all())
+
+
 def test_product_added_to_the_stream_refuses_what_it_does_not_take():
     from ojb200 import lt_ext as LT
     x, w = _mk(64, 40, 64, 1)
@@ -481,9 +508,9 @@ def test_algorithm_indices_name_the_same_kernels(idx, blocks, swapped):
 # x as the N side (w tile wider than the rows) and as the M side (2048 outputs: tiles of 16), edges of 16 rows and of the last w tile
 @pytest.mark.parametrize("M", [1, 16, 17, 33, 100, 128])
 @pytest.mark.parametrize("N", [2048, 2056, 12352])
-def test_few_row_kernel_e4m3_has_the_bits_of_the_block_kernel(M, N):
-    """The same rows among 256, which the 256-row block kernel takes, give the same bits: sums run over K in the same order. (fp32 partials:
-    the two scales are multiplied in another order there, two roundings of 2^-24 each.)"""
+def test_few_row_kernel_e4m3_agrees_with_the_block_kernel(M, N):
+    """The same rows among 256, which the 256-row block kernel takes: sums run over K in the same order, so bf16 results have the same bits
+    here, and fp32 partials differ by the order in which the two scales are multiplied, two roundings of 2^-24 in either kernel."""
     from ojb200 import lt_ext as LT, _lib
     K = 640
     x, w = _mk(256, N, K, M)

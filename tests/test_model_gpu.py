@@ -476,6 +476,31 @@ def test_e4m3_projections_stay_close_to_the_bf16_forward():
     assert c > 0.8, c
 
 
+@pytest.mark.parametrize("fp8", [False, True])
+def test_forward_that_adds_its_projections_to_the_stream(fp8, monkeypatch):
+    """Output and down projections of one K range, added to the residual stream by the product itself or as a plane by the norm kernel: the
+    same sums, so the same hidden states bit for bit. (Few rows keep the plane in both: there the e4m3 plane comes from another kernel.)"""
+    from ojb200 import fastmodel as FM, modelgen as MG, _lib
+    cfg, core = _small_model()
+    seqs, groups, pad_id, NB, PB = trees.layout_cases()["baseline"]
+    fast = FM.FastQwen35(core.to("cuda"), fp8=fp8)
+    ids, lay = fast.gtree_build([[t % cfg.vocab_size for t in s] for s in seqs], groups, pad_id % cfg.vocab_size, NB, PB)
+    added = []
+    add, e4m3 = FM.LT.gemm_add, FM.LT.gemm_e4m3
+    monkeypatch.setattr(FM.LT, "plan_splitk", lambda *a, **k: 1)
+    monkeypatch.setattr(FM.LT, "gemm_add", lambda *a, **k: (added.append("bf16"), add(*a, **k))[1])
+    monkeypatch.setattr(FM.LT, "gemm_e4m3", lambda *a, **k: (added.append("e4m3") if a[4] == 3 else None, e4m3(*a, **k))[1])
+    monkeypatch.setattr(FM.FastQwen35, "_adds", staticmethod(lambda M, N, K: False))
+    want = fast.forward_gtree(ids, lay)
+    assert not added
+    monkeypatch.setattr(FM.FastQwen35, "_adds", staticmethod(lambda M, N, K: M > 128 and N % 64 == 0))
+    got = fast.forward_gtree(ids, lay)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert added == ["e4m3" if fp8 else "bf16"] * (2 * len(fast.L) - 2)      # (the last layer runs on the asked rows)
+    assert torch.equal(got, want)
+
+
 def test_full_width_tree_forward_equals_its_candidates_scored_alone():
     """Size-independent property at the model's full width (hidden 5120, MLP 17408, 32 / 16 GDN heads, 24 / 4 attention
     heads; 4 layers = 3 Gated DeltaNet + 1 attention) on the 539-row benchmark tree: packing candidates into a prefix tree
