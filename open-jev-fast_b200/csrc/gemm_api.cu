@@ -48,7 +48,9 @@ double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, in
 // against 31.4 / 29.8 / 30.3* / 31.2*, [2048, 5120] 15.4* / 15.4* / 16.5* / 18.6* against 21.3 / 21.3 / 21.2 / 21.8, [5120, 4096]
 // 11.5* / 11.5* / 12.5 / 14.8 against 11.4 / 11.8 / 12.9* / 14.7*, [5120, 6144] 14.9* / 14.5* / 16.0 / 17.9 against 15.0 / 15.0 / 16.2* / 18.4*,
 // [5120, 17408] 32.9* / 33.3 / 35.3 / 39.2 against 33.1 / 33.9* / 36.1* / 39.5*. With many rows the model is too high (30.6 us for
-// [2048, 5120] at 128 rows), and the swapped-operand units take over above about 36 rows where it would still lead by 0 to 5 %.
+// [2048, 5120] at 128 rows), and the swapped-operand units take over above about 36 rows where it would still lead by 0 to 5 %. (Rows are
+// counted in eights; a launch with x as the N side loads them in sixteens, at most eight more. The K ranges of few rows are chosen by this
+// figure, so it stays as fitted.)
 double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
   const int bn = skinny_bn(N, splits);
   const double waves = static_cast<double>(ceil_div(ceil_div(N, bn) * splits, sms));

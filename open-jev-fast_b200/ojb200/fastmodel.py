@@ -174,8 +174,8 @@ class FastQwen35(torch.nn.Module):
             idx, S = self._force.get("res", self._plan.get(("res", M, w.shape[0], Kd), (0, 0)))
             if S == 0:
                 S = LT.plan_splitk(M, w.shape[0], Kd)
-        if S == 1 and idx in self.ADD_KERNELS and self._adds(M, *w.shape):
-            LT.gemm_add(y, w, h, idx)
+        if S == 1 and idx == 0 and self._adds(M, *w.shape):
+            LT.gemm_add(y, w, h)
             return [h, self._norm(h, None, None, w1, mask, last)]
         return [h, self._norm(h, None, LT.gemm_splitk(y, w, S, idx), w1, mask, last)]
 
@@ -183,12 +183,13 @@ class FastQwen35(torch.nn.Module):
     # sum). The norm is then bound by half the bytes (30 -> 18 us at 2560 rows, 56 -> 36 at 4192, 193 -> 115 at 16 672); the product
     # itself pays where the stream has left the L2 and its epilogues run under no other unit, because the addition then waits for HBM. That
     # is the down projection (K = 17 408) below about nine blocks of rows: both projections together 117 -> 122 us on average at 1560 rows. A short
-    # K moves little through the L2: from 1024 rows on it gains (K = 4096 at 1066 / 1568 rows, with the norm: 60 / 79 us -> 54 / 71).
+    # K moves little through the L2: from 1024 rows on it ties or gains (bf16 with the norm, weights from HBM, K = 4096 / 6144 at 1056 rows 57 / 77 us ->
+    # 54 / 74, at 1568 rows 73 / 98 -> 74 / 99, at 2560 rows 123 / 167 -> 117 / 162, K = 17 408 at 2560 / 8224 rows 411 / 1240 -> 401 / 1219). The same
+    # thresholds serve e4m3 operands, which gain throughout (K = 4096 / 6144 at 1056 rows 48 / 60 -> 41 / 51, at 2560 rows 99 / 123 -> 85 / 112,
+    # K = 17 408 at 2560 / 4192 rows 253 / 440 -> 236 / 427). Choices made by tune(), timed with a plane, keep the plane.
     @staticmethod
     def _adds(M, N, K):
         return M >= (1024 if K <= 8192 else 2304) and N % 64 == 0
-
-    ADD_KERNELS = (0, 3)
 
     def _mlp_in(self, hn, d):
         if d.fused_mlp and self.fp8:

@@ -171,7 +171,7 @@ class EntryState:
         else:
             self.out = body()
         self.launches = _lib.launch_count() - n0
-        self._body, self._fast = body, fast
+        self._body = body
 
     def run(self, pre, suf, msk, pad):
         self.pre.copy_(pre, non_blocking=True)
