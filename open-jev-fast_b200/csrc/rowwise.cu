@@ -148,8 +148,9 @@ resnorm_f32_kernel(float* __restrict__ h, const bf16_t* __restrict__ x_init, con
   float v[kVecs][8];
   float ss = 0.f;
   // Few rows: the norm's weights and the row mask are asked for with the row, not behind the sum over it (another trip to the L2 on a
-  // chain of a few microseconds). 28 / 288 rows, three planes: 3.25 / 5.37 -> 3.04 / 5.17 us.
-  constexpr bool kEarly = THREADS == 1024;
+  // chain of a few microseconds). 32 / 288 rows, three planes: 3.34 / 5.60 -> 3.09 / 5.37 us. Not with five planes or more: those registers
+  // would leave one row of 640 threads to an SM in place of two (6 planes at 192 rows 6.5 us, with early weights 7.5).
+  constexpr bool kEarly = THREADS == 1024 && SPLITS < 5;
   float4 wa[kEarly ? kVecs : 1], wb[kEarly ? kVecs : 1];
   const bool keep_early = kEarly && (rowmask ? rowmask[row] != 0 : true);
   if constexpr (kEarly) {
