@@ -52,7 +52,10 @@ constexpr int g_mma_repeat = 1, g_max_stages = 0, g_dbg = 0;
 // FP8: the operands are e4m3 bytes (a k-block of 128 bytes is then 128 elements of K and an MMA covers 32 of them); the
 // epilogue multiplies the accumulator by the scale of its row of x and of its row of w. Everything counted in bytes (stages,
 // swizzle, descriptors) is the same for both operand types.
-template <int EPI, bool FP8>
+// ALT, with fp32 results: the product is added to what out holds (bulk reductions in place of bulk stores); with SwiGLU: a row's SiLU follows from
+// g.pair_rows, not from its kind of unit. Kernels of their own, because asked at run time the first cost fp32 results 2 to 4 % where epilogues are
+// much of the work ([5120, 4096] in six K ranges), the second SwiGLU 0.5 %.
+template <int EPI, bool FP8, bool ALT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     const __grid_constant__ CUtensorMap map_w256, const __grid_constant__ CUtensorMap map_xt,
@@ -262,7 +265,7 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             fence_proxy_async();
             __syncwarp();
             if (lane == 0 && row0 < g.M) {
-              if (EPI == kEpiPartialF32 && g.accum) tma_add_3d(&map_out, tile_s, col, row0, 0);
+              if constexpr (EPI == kEpiPartialF32 && ALT) tma_add_3d(&map_out, tile_s, col, row0, 0);
               else tma_store_3d(&map_out, tile_s, col, row0, EPI == kEpiPartialF32 ? u.split : 0);
               bulk_commit();
             }
@@ -310,7 +313,7 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                 if (u.wt * 128 + t * 64 < g.N / 2) flush(u.wt * 128 + t * 64);
               }
             };
-            if (FP8 || u.xb * kBlockM < g.pair_rows) tiles(std::true_type{});
+            if (!ALT || u.xb * kBlockM < g.pair_rows) tiles(std::true_type{});
             else tiles(std::false_type{});
           } else if constexpr (EPI == kEpiBf16) {
             const int nt = g.BN / 64;              // BN is a multiple of 64 on this path
@@ -491,7 +494,7 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                     t[e * 32 + lane] = f2bf((decltype(paired)::value ? silu2_lanes_f(gv) : silu_f(gv)) * uv);
                   }
                 };
-                if (!FP8 && m0 + c * 16 < g.pair_rows) tile(std::true_type{});      // (a multiple of 256: all 16 rows are on one side)
+                if (ALT && m0 + c * 16 < g.pair_rows) tile(std::true_type{});      // (a multiple of 256: all 16 rows are on one side)
                 else tile(std::false_type{});
                 fence_proxy_async();
                 __syncwarp();
@@ -551,7 +554,7 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
               __syncwarp();
               const int col0 = u.wt * 256 + acc_id * kBM + quarter * 32;
               if (lane == 0 && col0 < g.N) {
-                if (EPI == kEpiPartialF32 && g.accum) tma_add_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, 0);
+                if constexpr (EPI == kEpiPartialF32 && ALT) tma_add_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, 0);
                 else tma_store_3d(&map_tail, smem_u32(t), col0, m0 + c * 16, EPI == kEpiPartialF32 ? u.split : 0);
                 bulk_commit();
               }
@@ -622,11 +625,12 @@ gemm_block256_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
 
 constexpr size_t kSmemBudget = 227 * 1024;
 
-template <int EPI, bool FP8 = false>
+template <int EPI, bool FP8 = false, bool ALT = false>
 int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K, int splits, int bn_req, int64_t ldo,
-                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr, bool accum = false, int pair_rows = -1) {
+                int32_t* status, cudaStream_t stream, const float* sx = nullptr, const float* sw = nullptr, int pair_rows = -1) {
   static int smem_set[kMaxDevices] = {};
-  auto kern = gemm_block256_kernel<EPI, FP8>;
+  constexpr bool kAdd = EPI == kEpiPartialF32 && ALT;
+  auto kern = gemm_block256_kernel<EPI, FP8, ALT>;
   if (!raise_smem_limit(kern, static_cast<int>(kSmemBudget), smem_set)) return OJB_ERR_LAUNCH;
   const int sms = sm_count();
   if (sms <= 0) return OJB_ERR_LAUNCH;
@@ -653,8 +657,12 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   } else {
     form = plain_form(M);
   }
-  // The two forms of SiLU differ in the last bits, so which one a row takes follows from the plain form, whatever form the model chooses.
-  if (pair_rows < 0) pair_rows = (bn_req == 0 && M > kBM ? plain_form(M) : form).n_xblk * kBlockM;
+  if constexpr (EPI == kEpiSwiglu && !FP8 && !ALT) {
+    // the two forms of SiLU differ in the last bits, so which one a row takes follows from the plain form, whatever form the model chooses
+    if (pair_rows < 0) pair_rows = (bn_req == 0 && M > kBM ? plain_form(M) : form).n_xblk * kBlockM;
+    if (pair_rows != form.n_xblk * kBlockM)
+      return launch_gemm<EPI, FP8, true>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream, sx, sw, pair_rows);
+  }
   g.pair_rows = pair_rows;
   if (bn_req < 0) bn_req = 0;
   g.n_xblk = form.n_xblk;
@@ -663,7 +671,7 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   g.n_xchunk = form.n_xchunk;
   g.BN = EPI == kEpiSwiglu ? 256 : (bn_req > 0 ? bn_req : choose_bn(N, g.n_xblk, g.tail_box, g.n_xchunk, g.tail_rows > 0, splits, g.kb_total, sms, EPI));
   if (FP8 && g.BN % 64 != 0) g.BN = (g.BN + 63) / 64 * 64;      // whole 128-byte store tiles (the scaled epilogue needs them)
-  if (accum) g.BN = (g.BN + 31) / 32 * 32;                       // (a reduction leaves as whole tiles too)
+  if (kAdd) g.BN = (g.BN + 31) / 32 * 32;                       // (a reduction leaves as whole tiles too)
   g.n_wtile = static_cast<int>(ceil_div(N, g.BN));
   g.n_wtile256 = static_cast<int>(ceil_div(N, 256));
   g.band_xblk = band_blocks(g.n_xblk, static_cast<int64_t>(kBlockM) * K * (FP8 ? 1 : 2));
@@ -678,8 +686,7 @@ int launch_gemm(const void* x, const void* w, void* out, int64_t M, int64_t N, i
   const int out_elt = EPI == kEpiPartialF32 ? 4 : 2;
   g.tma_out = g.n_xblk > 0 && (ldo * out_elt) % 16 == 0 && g.BN % (128 / out_elt) == 0 ? 1 : 0;
   g.tail_tma = (g.tail_rows > 0 && (ldo * out_elt) % 16 == 0 && (EPI != kEpiPartialF32 || (M * N * 4) % 16 == 0)) ? 1 : 0;
-  g.accum = accum ? 1 : 0;
-  if (accum && ((g.n_xblk > 0 && !g.tma_out) || (g.tail_rows > 0 && !g.tail_tma))) return OJB_ERR_LIMIT;
+  if (kAdd && ((g.n_xblk > 0 && !g.tma_out) || (g.tail_rows > 0 && !g.tail_tma))) return OJB_ERR_LIMIT;
   const size_t fixed = 1024 + (2 * kMaxStages + 2) * 8 + 16 + (g.tma_out ? kStagingBytes : (g.tail_tma ? kEpiWarps * 2048 : 0));
   g.stages = static_cast<int>((kSmemBudget - fixed) / g.stage_bytes);
   if (g.stages > kMaxStages) g.stages = kMaxStages;
@@ -741,20 +748,21 @@ void gemm_block256_set_probe(int repeat, int knob) {
 int gemm_block256_launch(int epi, int bn_req, const void* x, const void* w, void* out, int64_t M, int64_t N, int64_t K,
                          int splits, int64_t ldo, int32_t* status, cudaStream_t stream, int pair_rows) {
   if (epi == kEpiBf16) return launch_gemm<kEpiBf16>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
-  if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream, nullptr, nullptr, false, pair_rows);
+  if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream, nullptr, nullptr, pair_rows);
   return launch_gemm<kEpiPartialF32>(x, w, out, M, N, K, splits, bn_req, ldo, status, stream);
 }
 
 int gemm_block256_add_launch(int bn_req, const void* x, const void* w, float* out, int64_t M, int64_t N, int64_t K, int32_t* status,
                              cudaStream_t stream) {
-  return launch_gemm<kEpiPartialF32>(x, w, out, M, N, K, 1, bn_req, N, status, stream, nullptr, nullptr, true);
+  return launch_gemm<kEpiPartialF32, false, true>(x, w, out, M, N, K, 1, bn_req, N, status, stream);
 }
 
 int gemm_block256_launch_e4m3(int epi, const void* xq, const float* sx, const void* wq, const float* sw, void* out, int64_t M,
                               int64_t N, int64_t K, int splits, int64_t ldo, int32_t* status, cudaStream_t stream, bool accum) {
   if (epi == kEpiBf16) return launch_gemm<kEpiBf16, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
   if (epi == kEpiSwiglu) return launch_gemm<kEpiSwiglu, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
-  return launch_gemm<kEpiPartialF32, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw, accum);
+  if (accum) return launch_gemm<kEpiPartialF32, true, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
+  return launch_gemm<kEpiPartialF32, true>(xq, wq, out, M, N, K, splits, 0, ldo, status, stream, sx, sw);
 }
 
 }  // namespace ojb

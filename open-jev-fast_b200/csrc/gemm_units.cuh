@@ -42,7 +42,6 @@ struct GemmArgs {
   int trace_cap;
   int tail_sub;                // bytes of a tail sub-stage (128 rows of w + the x rows), 0 = one k-block per stage
   int tma_out;                 // the block epilogue stores through shared-memory tiles and bulk tensor stores
-  int accum;                   // block kernel, fp32 output: the product is added to what out holds (bulk reductions in place of bulk stores)
   int pair_rows;               // block kernel, SwiGLU: rows of x below it take their SiLU in pairs (silu2_f), the others by silu_f
   int dbg;                     // probe builds only (see below); 0 otherwise
   int mma_repeat;              // probe builds only; 1 otherwise
