@@ -526,3 +526,34 @@ def test_steps_of_unused_entries_leave_the_state_alone(HV):
             for e in exports:
                 assert _rel(fin[e, h], state[0]) < 1e-2
     assert torch.equal(fin[0], fin[1])
+
+
+@pytest.mark.parametrize("HV", [4, 40])      # full form and, above one CTA per SM, dense form
+def test_walks_of_one_step_among_others(HV):
+    """Tables of no more chunks than walks go to the kernel that knows walks of one step: one step from zero and from an initial state, with its
+    state exported or not, beside a walk of two steps and one of none. The same walks with unused chunk entries behind, which the other
+    kernel takes, give the same bits."""
+    from ojb200 import ext as K, _lib
+    HK, n = 2, 64 + 17 + 33 + 1 + 48
+    chunks = [[0, 64, 0, 0], [64, 17, 0, 0], [81, 33, 0, 0], [114, 1, 0, 0], [115, 48, 0, 0]]
+    steps = [[0, 1, 0, 0], [1, 4, 0, (1 << 16) | 1], [2, 1, 0, 0], [3, 0, 0, 2], [4, 4, 0, (2 << 16) | 3]]
+    walks = [0, 1, 2, 2, 4, 5]
+    tab = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    q, k, v, g, beta = (t.cuda() for t in _inputs(n, HK, HV, 41))
+    init = torch.randn(2, HV, 128, 128, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda") * 0.1
+    results = []
+    for more in (0, 3):
+        fin = torch.zeros(3, HV, 128, 128, device="cuda")
+        out = K.gdn_chunked(q, k, v, g, beta, 128 ** -0.5, tab(chunks + [[0, 0, 0, 0]] * more), tab(steps), tab(walks), 5, init, fin, None, False)
+        results.append((out, fin))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    (out, fin), (other, other_fin) = results
+    assert torch.equal(out, other) and torch.equal(fin, other_fin)
+    for rows, first, export in ((range(0, 64), None, None), (range(64, 81), 0, 0), (range(81, 115), None, 1), (range(115, 163), 1, 2)):
+        for h in (0, HV - 1):
+            one = [t[list(rows)][:, [h * HK // HV if i < 2 else h]].cpu() for i, t in enumerate((q, k, v, g, beta))]
+            ref, state = OG.recurrent(*one, 128 ** -0.5, None if first is None else init[first, [h]].cpu())
+            assert _rel(out[list(rows), h], ref[:, 0]) < 4e-3
+            if export is not None:
+                assert _rel(fin[export, h], state[0]) < 1e-2
