@@ -14,9 +14,10 @@
 // depends on its own row of A alone, and the rows past the operand are never read back. So a k-step costs 128 products for every row
 // of the N side, and the narrower of the two operands is the N side: the rows of x (rounded up to 16) under most tiles, the w tile where
 // that has fewer rows (2048 outputs: 16). With x always the M side a weight cost 128 products, most of them of other weights taken for
-// rows of x, and the products of random operands are what the board's power goes to. 28 rows, in runs at the 1 kW cap, x as the
-// M side / as the N side: [12352, 5120] 26.7 / 25.0 us, [5120, 17408] in six K ranges 41.6 / 39.1, in e4m3 17.4 / 15.4 and 28.9 / 24.7; [2048,
-// 5120] 15.3 / 16.3. Same bits.
+// rows of x, and the products of random operands are what the board's power goes to. x as the M side / the choice, in runs at the 1 kW cap
+// (us): 28 rows [12352, 5120] 26.8 / 24.2, [5120, 4096] in two K ranges 11.8 / 11.2, [5120, 17408] in three 35.6 / 32.0; 64 rows 30.5 / 28.9, 12.5 /
+// 11.5 and 39.7 / 35.7. In short runs 0 to 25 % faster too, e4m3 up to 33 %. Same bits. With w as the M side the accumulator leaves 16 rows of x at a time,
+// loads ahead of the stores: with each load waited for and addresses formed per value it cost 0.3 us for every 16 rows and lost up to 9 %.
 #include "gemm_units.cuh"
 
 #include <type_traits>
@@ -140,23 +141,36 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           float ws = 1.f;
           if constexpr (FP8) ws = __ldg(g.sw + min(n0 + row, g.N - 1));
           const int64_t off = static_cast<int64_t>(split) * g.split_stride + n0 + row;
-#pragma unroll 1
-          for (int m0 = 0; m0 < g.M; m0 += 16) {
-            uint32_t r[16];
-            tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + m0, r);
-            tmem_ld_wait();
-            const int left = g.M - m0;
+          using Out = std::conditional_t<EPI == kEpiPartialF32, float, bf16_t>;
+          Out* const out = reinterpret_cast<Out*>(g.out) + off;
+          const uint32_t acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+          // neighbouring lanes hold neighbouring columns: whole 128- or 64-byte pieces of a row; TMEM loads run 16 rows ahead of the stores
+          auto emit = [&](int m0, const uint32_t (&r)[16]) {
+            Out* p = out + static_cast<int64_t>(m0) * g.ldo;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {      // neighbouring lanes hold neighbouring columns: whole 128- or 64-byte pieces of a row
-              if (col_ok && e < left) {
+            for (int e = 0; e < 16; ++e, p += g.ldo) {
+              if (col_ok && m0 + e < g.M) {
                 float v = __uint_as_float(r[e]);
                 if constexpr (FP8) v *= __ldg(g.sx + m0 + e) * ws;
-                const int64_t at = off + static_cast<int64_t>(m0 + e) * g.ldo;
-                if constexpr (EPI == kEpiPartialF32) reinterpret_cast<float*>(g.out)[at] = v;
-                else reinterpret_cast<bf16_t*>(g.out)[at] = f2bf(v);
+                if constexpr (EPI == kEpiPartialF32) *p = v;
+                else *p = f2bf(v);
               }
             }
             __syncwarp();
+          };
+          uint32_t ra[16], rb[16];
+          tmem_ld16(acc, ra);
+          tmem_ld_wait();
+#pragma unroll 1
+          for (int m0 = 0; m0 < g.M; m0 += 32) {
+            if (m0 + 16 < g.M) tmem_ld16(acc + m0 + 16, rb);
+            emit(m0, ra);
+            tmem_ld_wait();
+            if (m0 + 16 < g.M) {
+              if (m0 + 32 < g.M) tmem_ld16(acc + m0 + 32, ra);
+              emit(m0 + 16, rb);
+              tmem_ld_wait();
+            }
           }
         }
       } else {
