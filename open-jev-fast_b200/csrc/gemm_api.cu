@@ -44,13 +44,13 @@ double tile128_clocks(int64_t M, int64_t N, int kb_total, int splits, int bn, in
 
 // The few-row kernel: a CTA takes in about 30 bytes per clock, and no k-block (its share of a wait, a commit and the MMAs) in less
 // than 220 clocks. Measured against the best of the other kernels, each with its best K ranges (us; * = what the models pick), at
-// 12 / 32 / 64 / 128 rows: [12352, 5120] 24.6* / 24.8* / 29.6 / 29.7 against 30.4 / 27.4 / 27.8* / 29.0*, [14336, 5120] 28.0* / 27.6* / 30.0 / 31.5
-// against 31.4 / 29.8 / 30.3* / 31.2*, [2048, 5120] 15.4* / 15.4* / 16.5* / 18.6* against 21.3 / 21.3 / 21.2 / 21.8, [5120, 4096]
-// 11.5* / 11.5* / 12.5 / 14.8 against 11.4 / 11.8 / 12.9* / 14.7*, [5120, 6144] 14.9* / 14.5* / 16.0 / 17.9 against 15.0 / 15.0 / 16.2* / 18.4*,
-// [5120, 17408] 32.9* / 33.3 / 35.3 / 39.2 against 33.1 / 33.9* / 36.1* / 39.5*. With many rows the model is too high (30.6 us for
-// [2048, 5120] at 128 rows), and the swapped-operand units take over above about 36 rows where it would still lead by 0 to 5 %. (Rows are
-// counted in eights; a launch with x as the N side loads them in sixteens, at most eight more. The K ranges of few rows are chosen by this
-// figure, so it stays as fitted.)
+// 12 / 32 / 64 / 128 rows: [12352, 5120] 23.7* / 23.9* / 27.1 / 28.2 against 30.1 / 26.7 / 27.2* / 28.2*, [14336, 5120] 26.1* / 26.5* / 28.9 / 30.8
+// against 30.7 / 28.9 / 29.7* / 30.4*, [2048, 5120] 15.3* / 15.2* / 16.3* / 18.3* against 21.2 / 21.2 / 21.4 / 21.9, [5120, 4096]
+// 10.7* / 11.0* / 11.5 / 15.3 against 11.7 / 12.0 / 13.4* / 15.8*, [5120, 6144] 14.0* / 14.2* / 15.1 / 19.0 against 15.2 / 15.4 / 16.8* / 19.2*,
+// [5120, 17408] 31.1* / 31.8 / 33.1 / 38.0 against 32.1 / 33.2* / 35.1* / 38.3*. With many rows the model is too high (30.6 us for
+// [2048, 5120] at 128 rows), and the swapped-operand units take over above about 36 rows where this kernel still leads, by 4 to 20 % up to 96 rows
+// where there are K ranges: those are chosen by the same figures, and another fit would move results. tune() times both. (Rows are
+// counted in eights; a launch with x as the N side loads them in sixteens, at most eight more.)
 double skinny_clocks(int64_t M, int64_t N, int kb_total, int splits, int sms) {
   const int bn = skinny_bn(N, splits);
   const double waves = static_cast<double>(ceil_div(ceil_div(N, bn) * splits, sms));
