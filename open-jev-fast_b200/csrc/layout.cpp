@@ -337,8 +337,8 @@ extern "C" int ojb_seq_tables(const int64_t* lens, int64_t S, int64_t Lp, int64_
                               int64_t* lastidx, int32_t* rowmask, int32_t* hist, int32_t* krange, int32_t* chunks, int32_t* steps,
                               int32_t* walk_ptr) {
   if (!hist || !chunks || !steps || !walk_ptr || (S > 0 && (!lens || !lastidx))) return OJB_ERR_ARG;
-  if (S < 0 || Lp < 0 || T < 0 || pad < 0 || pad > Lp || cap < 1 || (own_walks && Lp != 0)) return OJB_ERR_ARG;
-  int64_t need = (Lp - pad + 63) / 64;
+  if (S < 0 || Lp < 0 || T < 0 || pad < 0 || cap < 1 || (own_walks && Lp != 0)) return OJB_ERR_ARG;
+  int64_t need = Lp > pad ? (Lp - pad + 63) / 64 : 0;      // (pad > Lp: a prefix without a real row, positions shifted all the same)
   for (int64_t s = 0; s < S; ++s) {
     if (lens[s] < 0 || lens[s] > T) return OJB_ERR_ARG;
     need += (lens[s] + 63) / 64;

@@ -163,7 +163,7 @@ class SeqTables:
         """On the host. cap: entries of the chunk and step tables (default: as many as there are chunks)."""
         lens = np.ascontiguousarray(lens, np.int64)
         S = len(lens)
-        need = max(1, -(-(Lp - pad) // 64) + int((-(-lens // 64)).sum()))
+        need = max(1, -(-max(Lp - pad, 0) // 64) + int((-(-lens // 64)).sum()))
         if cap is not None and need > cap:
             raise RuntimeError("tree_layout: more chunks than the table capacity")
         cap = need if cap is None else cap

@@ -243,6 +243,17 @@ def test_sequence_tables_refuse_what_does_not_fit():
             SeqTables.build(lens, 0, 0, 65, True, cap=cap)
 
 
+def test_tree_layout_with_more_padding_than_prefix():
+    """Left padding beyond the prefix, as a caller with a fixed prefix length may state it: no prefix row is real, and positions start at Lp - pad."""
+    import torch
+    from ojb200 import layout as PL
+    lay = PL.tree_layout(torch.zeros(4, dtype=torch.long), torch.ones(2, 3, dtype=torch.long), torch.ones(2, 3, dtype=torch.long), pad=6, dense=False)
+    assert lay.pos.tolist() == [-6, -5, -4, -3, -2, -1, 0, -2, -1, 0]
+    assert lay.rowmask.tolist() == [0] * 4 + [1] * 6 and lay.walk_ptr.tolist() == [0, 2]
+    assert lay.steps.tolist() == [[0, 1, 0, 0], [1, 1, 0, 0]] and lay.chunks[:, :2].tolist() == [[4, 3], [7, 3]]
+    assert lay.hist[4].tolist() == [-1, -1, -1, 4] and lay.hist[9].tolist() == [-1, 7, 8, 9] and lay.lastidx.tolist() == [6, 9]
+
+
 def test_common_prefix_of_candidates():
     from ojb200.server import _common_prefix
     base = list(range(200))
